@@ -832,12 +832,27 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
 
     uint32_t* deg = ar.get<uint32_t>(n);
     unsigned long long* off = ar.get<unsigned long long>((size_t)n + 1);
-    uint32_t* parent = ar.get<uint32_t>(n);
-    uint32_t* seed = ar.get<uint32_t>(n);
-    uint32_t* cstart = ar.get<uint32_t>(n);
-    uint32_t* best = ar.get<uint32_t>(n);
-    uint32_t* cluster_no = ar.get<uint32_t>((size_t)n + 1);
-    uint32_t* pos_flag = ar.get<uint32_t>(n);
+    // union-find state: over cells for all minpts of a group at once (grids
+    // whose cells are cliques), or over points, one variant at a time
+    unsigned long long* cbest = nullptr;
+    uint32_t* cells_buf = nullptr;
+    uint32_t* cells_ws = nullptr;
+    size_t cells_slots = 0, cells_ws_slots = 0;
+    const uint32_t nw = start_words(n);
+    uint2* crng = nullptr;  // neighbour cells of every cell and row
+    size_t crng_cap = 0;
+    UfState whole;
+    memset(&whole, 0, sizeof whole);
+    auto new_state = [&]() {
+        UfState u;
+        u.parent = ar.get<uint32_t>(n);
+        u.seed = ar.get<uint32_t>(n);
+        u.cstart = ar.get<uint32_t>(n);
+        u.best = ar.get<uint32_t>(n);
+        u.cluster_no = ar.get<uint32_t>((size_t)n + 1);
+        u.pos_flag = ar.get<uint32_t>(n);
+        return u;
+    };
     uint32_t asym_cap = kAsymCap;  // grows when a count pass finds more one-way pairs
     AsymPair* asym = ar.get<AsymPair>(asym_cap);
     uint32_t* asym_n = ar.get<uint32_t>(4);
@@ -856,7 +871,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* tiles = ar.get<uint32_t>((size_t)n + 1);
     uint32_t* cscan = ar.get<uint32_t>((size_t)n + 1);
     uint32_t* clist = ar.get<uint32_t>((size_t)n + 1);
-    uint32_t* crep = ar.get<uint32_t>(n);
     unsigned long long* tboff = ar.get<unsigned long long>((size_t)n + 1);
     uint32_t* tunits = ar.get<uint32_t>(n);
     uint32_t* tuoff = ar.get<uint32_t>((size_t)n + 1);
@@ -913,14 +927,18 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         }
         return nullptr;
     };
-    auto save_comp = [&](const ClusterArgs& ca, uint64_t mp) {
-        // (nothing reads the components of the last epsilon group)
-        if (!o.reuse || mp == ~0ull || group_index + 1 >= groups.size()) return;
+    // where the components of this group's minpts mp are kept (nullptr: not;
+    // nothing reads those of the last epsilon group)
+    auto comp_dest = [&](uint64_t mp) -> uint32_t* {
+        if (!o.reuse || mp == ~0ull || group_index + 1 >= groups.size()) return nullptr;
         auto it = saved_comp.find(mp);
         if (it == saved_comp.end())
             it = saved_comp.emplace(mp, SavedComp{group_index, ar.get<uint32_t>(n)}).first;
         it->second.group = group_index;
-        launch_save_components(ca, it->second.comp, s);
+        return it->second.comp;
+    };
+    auto save_comp = [&](const ClusterArgs& ca, uint64_t mp) {
+        if (uint32_t* comp = comp_dest(mp)) launch_save_components(ca, comp, s);
     };
     // builds the rows of chunk c into nbr (expand from the bitmap, or the
     // fill pass when there is no bitmap)
@@ -966,12 +984,16 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         // the labels of the variant before it
         std::vector<std::pair<uint32_t, uint64_t>> slots;    // (variant, minpts)
         std::vector<std::pair<uint32_t, uint32_t>> copies;   // (variant, source variant)
+        std::vector<uint32_t> ncopies;                       // variants per slot
         for (auto& mv : gr.vars) {
             const uint64_t mp = mv.first > 0x7fffffffu ? ~0ull : (uint64_t)mv.first;
-            if (!slots.empty() && slots.back().second == mp)
+            if (!slots.empty() && slots.back().second == mp) {
                 copies.push_back({mv.second, slots.back().first});
-            else
+                ncopies.back()++;
+            } else {
                 slots.push_back({mv.second, mp});
+                ncopies.push_back(1);
+            }
         }
         EpsParams ep;
         memset(&ep, 0, sizeof ep);
@@ -1362,16 +1384,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 // one union-find state per minpts of the group (the rows of
                 // every chunk serve all of them), then the largest chunk
                 // that the remaining memory allows
-                while (states.size() < slots.size()) {
-                    UfState u;
-                    u.parent = ar.get<uint32_t>(n);
-                    u.seed = ar.get<uint32_t>(n);
-                    u.cstart = ar.get<uint32_t>(n);
-                    u.best = ar.get<uint32_t>(n);
-                    u.cluster_no = ar.get<uint32_t>((size_t)n + 1);
-                    u.pos_flag = ar.get<uint32_t>(n);
-                    states.push_back(u);
-                }
+                while (!clique && states.size() < slots.size()) states.push_back(new_state());
                 if (nbr) ar.put(nbr);
                 nbr = nullptr;
                 nbr_cap_bytes = 0;
@@ -1420,40 +1433,21 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ca.unit_words = unit_words;
             ca.gpos = gpos;
             ca.gorig = gorig;
-            if (chunked) {
-                const UfState& u = states[si];
-                ca.parent = u.parent;
-                ca.seed = u.seed;
-                ca.cstart = u.cstart;
-                ca.best = u.best;
-                ca.cluster_no = u.cluster_no;
-                ca.pos_flag = u.pos_flag;
-            } else {
-                ca.parent = parent;
-                ca.seed = seed;
-                ca.cstart = cstart;
-                ca.best = best;
-                ca.cluster_no = cluster_no;
-                ca.pos_flag = pos_flag;
-            }
+            if (!chunked && !whole.parent) whole = new_state();
+            const UfState& u = chunked ? states[si] : whole;
+            ca.parent = u.parent;
+            ca.seed = u.seed;
+            ca.cstart = u.cstart;
+            ca.best = u.best;
+            ca.cluster_no = u.cluster_no;
+            ca.pos_flag = u.pos_flag;
             ca.asym = asym;
             ca.asym_count = asym_n;
             ca.asym_cap = asym_cap;
             ca.labels_out = labels + (size_t)slots[si].first * n;
             ca.st = d_st;
-            ca.g = g;
+            ca.copies = ncopies[si];
             ca.ep = d_ep;
-            ca.gkey = gkey;
-            ca.cell_start = cell_start;
-            ca.crow = crow;
-            ca.ccx = ccx;
-            ca.clist = clist;
-            ca.ncl = cscan + n;
-            ca.cscan = cscan;
-            ca.crep = crep;
-            ca.glocal = glocal;
-            ca.gxy = gxy;
-            ca.gbox = gbox;
             return ca;
         };
         auto chunk_rows = [&](ClusterArgs& ca, const RowChunk& c) {
@@ -1461,7 +1455,82 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ca.row_lo = c.r_lo;
             ca.row_hi = c.r_hi;
         };
-        if (!chunked) {
+        if (clique) {
+            // (the labelling does not read the table: a chunked table's rows
+            // are written, chunk by chunk, and that is all)
+            if (chunked)
+                for (const RowChunk& c : chunk_list) build_chunk(ta_args, c, group_asym);
+            const size_t want = std::min<size_t>(slots.size(), kSlots);
+            const size_t n8 = ((size_t)n + 7) & ~(size_t)7;  // (keeps the bit words aligned)
+            if (want > cells_slots) {
+                if (cells_buf) ar.put(cells_buf);
+                cells_buf = ar.get<uint32_t>(want * (3 * n8 + 2 * (size_t)nw));
+                cells_slots = want;
+            }
+            if (!cbest) cbest = ar.get<unsigned long long>(n);
+            const int nrows = 2 * ep.rho + 1;
+            if ((size_t)n * nrows > crng_cap) {
+                if (crng) ar.put(crng);
+                crng_cap = (size_t)n * nrows;
+                crng = ar.get<uint2>(crng_cap);
+            }
+            if (!ccx) ccx = ar.get<uint32_t>(n);
+            if (group_asym && want > cells_ws_slots) {
+                if (cells_ws) ar.put(cells_ws);
+                cells_ws = ar.get<uint32_t>(want * (resolve_scratch_bytes() / 4));
+                cells_ws_slots = want;
+            }
+            for (size_t s0 = 0; s0 < slots.size(); s0 += kSlots) {
+                CellArgs ca;
+                memset(&ca, 0, sizeof ca);
+                ca.n = n;
+                ca.deg = deg;
+                ca.gpos = gpos;
+                ca.gorig = gorig;
+                ca.gkey = gkey;
+                ca.glocal = glocal;
+                ca.gxy = gxy;
+                ca.gbox = gbox;
+                ca.g = g;
+                ca.ep = d_ep;
+                ca.cell_start = cell_start;
+                ca.crow = crow;
+                ca.ccx = ccx;
+                ca.crng = crng;
+                ca.clist = clist;
+                ca.ncl = cscan + n;
+                ca.cscan = cscan;
+                ca.cbest = cbest;
+                ca.m = (int)std::min<size_t>(slots.size() - s0, kSlots);
+                ca.chain = o.reuse ? 1 : 0;
+                ca.parent = cells_buf;
+                ca.seed = cells_buf + cells_slots * n8;
+                ca.cst = cells_buf + 2 * cells_slots * n8;
+                ca.bits = cells_buf + 3 * cells_slots * n8;
+                ca.brank = ca.bits + cells_slots * nw;
+                ca.nw = nw;
+                ca.asym = asym;
+                ca.asym_count = asym_n;
+                ca.asym_cap = asym_cap;
+                ca.st = d_st;
+                for (int v = 0; v < ca.m; v++) {
+                    const uint64_t mp = slots[s0 + v].second;
+                    ca.mp[v] = mp == ~0ull ? 0xffffffffu : (uint32_t)mp;
+                    ca.copies[v] = ncopies[s0 + v];
+                    ca.labels[v] = labels + (size_t)slots[s0 + v].first * n;
+                    ca.comp_prev[v] = comp_source(mp);
+                }
+                for (int v = 0; v < ca.m; v++) ca.comp_out[v] = comp_dest(slots[s0 + v].second);
+                if (s0 > 0 && ca.chain) {
+                    // go on from the last slot before
+                    CK(cudaMemcpyAsync(ca.parent, ca.parent + (size_t)(kSlots - 1) * n,
+                                       (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
+                    ca.continued = 1;
+                }
+                launch_cells(ca, nrows, group_asym != 0, cells_ws, s);
+                CK(cudaGetLastError());
+            }
+        } else if (!chunked) {
             // the whole table is resident: one variant after the other on one
             // state; with reuse, a variant starts from the components of the
             // one before it (a larger minpts of the same epsilon: its cores
@@ -1470,14 +1539,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 ClusterArgs ca = cluster_args(si);
                 const bool chain = o.reuse && si > 0 && !none;
                 if (chain) ca.minpts_prev = slots[si - 1].second;
-                if (!none) ca.comp_prev = comp_source(slots[si].second);
                 launch_uf_init(ca, !chain, s);
-                if (!none) {
-                    if (clique)
-                        launch_cell_union(ca, nb_warps, s);
-                    else
-                        launch_uf_union(ca, nb_warps, s);
-                }
+                if (!none) launch_uf_union(ca, nb_warps, s);
                 launch_uf_finish(ca, scratch, scratch + resolve_scratch_bytes(), s);
                 if (!none) save_comp(ca, slots[si].second);
                 launch_border_and_write(ca, nb_warps, s);
@@ -1485,23 +1548,18 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             }
         } else {
             // row chunks: every variant keeps its own state while the chunks
-            // pass.  Cells that are cliques are united without the table;
-            // otherwise every chunk is built once for the unions and once
-            // more for the border pull.
+            // pass, each built once for the unions and once more for the
+            // border pull
             std::vector<ClusterArgs> cas;
             for (size_t si = 0; si < slots.size(); si++) {
                 cas.push_back(cluster_args(si));
-                cas.back().comp_prev = comp_source(slots[si].second);
                 launch_uf_init(cas.back(), true, s);
-                if (clique) launch_cell_union(cas.back(), nb_warps, s);
             }
-            if (!clique) {
-                for (const RowChunk& c : chunk_list) {
-                    build_chunk(ta_args, c, group_asym);
-                    for (ClusterArgs& ca : cas) {
-                        chunk_rows(ca, c);
-                        launch_uf_union(ca, nb_warps, s);
-                    }
+            for (const RowChunk& c : chunk_list) {
+                build_chunk(ta_args, c, group_asym);
+                for (ClusterArgs& ca : cas) {
+                    chunk_rows(ca, c);
+                    launch_uf_union(ca, nb_warps, s);
                 }
             }
             for (size_t si = 0; si < cas.size(); si++) {
@@ -1527,7 +1585,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         group_spans.push_back(GroupSpan{tcl0, tcl1, table_marks, table_marks_before});
         group_index++;
     }
-    launch_count_clusters(labels, n, V, ar.get<uint32_t>(V), d_st, s);
     if (capturing) {
         // the labels and the status block come back through pinned buffers
         // of the graph, after the last IF body
@@ -2276,7 +2333,6 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* tiles = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* cscan = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* clist = cv.take<uint32_t>((size_t)n + 1);
-    uint32_t* crep = cv.take<uint32_t>(n);
     EpsParams* d_ep = cv.take<EpsParams>(1);
     uint32_t* deg = cv.take<uint32_t>(n);
     unsigned long long* off = cv.take<unsigned long long>((size_t)n + 1);
@@ -2286,7 +2342,11 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* parent = cv.take<uint32_t>(n);
     uint32_t* seed = cv.take<uint32_t>(n);
     uint32_t* cstart = cv.take<uint32_t>(n);
+    // cells that are cliques are clustered without the table
+    const bool clique = 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
     uint32_t* best = cv.take<uint32_t>(n);
+    cv.take<uint32_t>(n);  // (cbest: both pieces, 8 bytes per cell)
+    unsigned long long* cbest = (unsigned long long*)best;
     uint32_t* cluster_no = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* pos_flag = cv.take<uint32_t>(n);
 
@@ -2356,60 +2416,95 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     CK(cudaMemcpyAsync(&hs, st, sizeof hs, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     check_flags(hs);
-    // the neighbour table takes the rest of the array
+    // the neighbour table has the rest of the array
     const size_t room = (kNoallocBytes - cv.used) / sizeof(uint32_t);
     if (E > room)
         throw VdbError{VDB_ERR_TOO_LARGE, "neighbour table exceeds the fixed scratch array"};
-    uint32_t* nbr = cv.take<uint32_t>(E ? E : 1);
-    ta.nbr = nbr;
-    ta.off_base = 0;
-    CK(cudaMemsetAsync(tile_counter, 0, 4, s));
-    launch_fill(ta, nsm * table_blocks_per_sm(true, ep.mixed != 0), s);
-
-    ClusterArgs ca;
-    memset(&ca, 0, sizeof ca);
-    ca.n = n;
-    ca.deg = deg;
-    ca.unit_words = kUnitWords;
-    ca.minpts = minpts > 0x7fffffffu ? ~0ull : (unsigned long long)minpts;
-    ca.minpts_prev = ~0ull;
-    ca.off = off;
-    ca.row_lo = 0;
-    ca.row_hi = n;
-    ca.nbr = nbr;
-    ca.gpos = gpos;
-    ca.gorig = gorig;
-    ca.parent = parent;
-    ca.seed = seed;
-    ca.cstart = cstart;
-    ca.best = best;
-    ca.cluster_no = cluster_no;
-    ca.pos_flag = pos_flag;
-    ca.asym = asym;
-    ca.asym_count = asym_n;
-    ca.asym_cap = kNoallocAsymCap;
-    ca.labels_out = labels;
-    ca.st = st;
-    ca.g = g;
-    ca.ep = d_ep;
-    ca.gkey = gkey;
-    ca.cell_start = cell_start;
-    ca.clist = clist;
-    ca.ncl = cscan + n;
-    ca.cscan = cscan;
-    ca.crep = crep;
-    ca.glocal = glocal;
-    ca.gxy = gxy;
-    ca.gbox = gbox;
+    uint32_t* nbr = nullptr;
+    uint2* crng = nullptr;
+    uint32_t *ccx = nullptr, *bits = nullptr, *brank = nullptr;
+    if (clique) {
+        // cells that are cliques are labelled without the table: its room
+        // holds the cells' neighbour lists and the start bits
+        bits = cv.take<uint32_t>(start_words(n));
+        brank = cv.take<uint32_t>(start_words(n));
+        ccx = cv.take<uint32_t>(n);
+        crng = cv.take<uint2>((size_t)n * (2 * ep.rho + 1));
+    } else {
+        nbr = cv.take<uint32_t>(E ? E : 1);
+        ta.nbr = nbr;
+        ta.off_base = 0;
+        CK(cudaMemsetAsync(tile_counter, 0, 4, s));
+        launch_fill(ta, nsm * table_blocks_per_sm(true, ep.mixed != 0), s);
+    }
     const int nb_warps = nsm * 8;
-    launch_uf_init(ca, true, s);
-    const bool clique = 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
-    if (clique)
-        launch_cell_union(ca, nb_warps, s);
-    else
+    if (clique) {
+        CellArgs ca;
+        memset(&ca, 0, sizeof ca);
+        ca.n = n;
+        ca.deg = deg;
+        ca.gpos = gpos;
+        ca.gorig = gorig;
+        ca.gkey = gkey;
+        ca.glocal = glocal;
+        ca.gxy = gxy;
+        ca.gbox = gbox;
+        ca.g = g;
+        ca.ep = d_ep;
+        ca.cell_start = cell_start;
+        ca.clist = clist;
+        ca.ncl = cscan + n;
+        ca.cscan = cscan;
+        ca.cbest = cbest;
+        ca.ccx = ccx;
+        ca.crng = crng;
+        ca.m = 1;
+        ca.mp[0] = minpts > 0x7fffffffu ? 0xffffffffu : minpts;
+        ca.copies[0] = 1;
+        ca.labels[0] = labels;
+        ca.parent = parent;
+        ca.seed = seed;
+        ca.cst = cstart;
+        ca.bits = bits;
+        ca.brank = brank;
+        ca.nw = start_words(n);
+        ca.asym = asym;
+        ca.asym_count = asym_n;
+        ca.asym_cap = kNoallocAsymCap;
+        ca.st = st;
+        launch_cells(ca, 2 * ep.rho + 1, true, scratch, s);
+    } else {
+        ClusterArgs ca;
+        memset(&ca, 0, sizeof ca);
+        ca.n = n;
+        ca.deg = deg;
+        ca.unit_words = kUnitWords;
+        ca.minpts = minpts > 0x7fffffffu ? ~0ull : (unsigned long long)minpts;
+        ca.minpts_prev = ~0ull;
+        ca.off = off;
+        ca.row_lo = 0;
+        ca.row_hi = n;
+        ca.nbr = nbr;
+        ca.gpos = gpos;
+        ca.gorig = gorig;
+        ca.parent = parent;
+        ca.seed = seed;
+        ca.cstart = cstart;
+        ca.best = best;
+        ca.cluster_no = cluster_no;
+        ca.pos_flag = pos_flag;
+        ca.asym = asym;
+        ca.asym_count = asym_n;
+        ca.asym_cap = kNoallocAsymCap;
+        ca.labels_out = labels;
+        ca.st = st;
+        ca.copies = 1;
+        ca.ep = d_ep;
+        launch_uf_init(ca, true, s);
         launch_uf_union(ca, nb_warps, s);
-    launch_uf_finish(ca, scratch, scratch + resolve_scratch_bytes(), s);
-    launch_border_and_write(ca, nb_warps, s);
+        launch_uf_finish(ca, scratch, scratch + resolve_scratch_bytes(), s);
+        launch_border_and_write(ca, nb_warps, s);
+    }
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(&hs, st, sizeof hs, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));

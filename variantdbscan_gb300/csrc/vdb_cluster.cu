@@ -126,220 +126,6 @@ __device__ __forceinline__ uint32_t uf_find_ro(const uint32_t* parent, uint32_t 
     return x;
 }
 
-// Cell union, step 1.  With cells of width <= eps/sqrt(2), every two points
-// of a cell are neighbours in both directions, so the cell's cores form a
-// clique: all of them are linked to the cell's first core (the smallest index,
-// so parents still only decrease).  Point-parallel: crep[c] = first core of
-// cell c (one atomic per cell and warp), then every other core links to it.
-// The cell of point k is cscan[k + 1] - 1 (cscan: exclusive scan of the
-// cell-start flags).
-__global__ void cell_rep_min_kernel(ClusterArgs a) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool core = k < a.n && is_core(a.deg[k], a.minpts);
-    const uint32_t c = core ? a.cscan[k + 1] - 1u : kNone;
-    const uint32_t act = __ballot_sync(kFull, core);
-    if (!core) return;
-    const uint32_t same = __match_any_sync(act, c);
-    // lanes are in point order: the lowest lane of a cell holds its first core
-    if ((threadIdx.x & 31) == (uint32_t)(__ffs(same) - 1) && VDB_GUARD(a.st, c < a.n, 15, c))
-        atomicMin(&a.crep[c], k);
-}
-
-// From scratch every other core of the cell takes the first core as parent
-// (rep <= k, so parents still only decrease).  When parent holds the
-// components of a larger minpts (minpts_prev), a core that is new at this
-// minpts is still a root of its own and is linked the same way; the cores
-// that were already cores form one component, which is united with the first
-// core only when that first core is new.
-__global__ void cell_rep_link_kernel(ClusterArgs a) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n || !is_core(a.deg[k], a.minpts)) return;
-    const uint32_t c = a.cscan[k + 1] - 1u;
-    if (!VDB_GUARD(a.st, c < a.n, 16, c)) return;
-    const uint32_t rep = a.crep[c];
-    if (rep == k) return;
-    if (a.minpts_prev == ~0ull || !is_core(a.deg[k], a.minpts_prev))
-        a.parent[k] = rep;
-    else if (!is_core(a.deg[rep], a.minpts_prev))
-        uf_union(a.parent, k, rep, a.st);
-}
-
-// Cell union, step 2 (one warp per cell A with cores): for every cell B within
-// reach with a larger key that also has cores and is not yet in A's
-// component, look for one core-core pair (a, b) accepted in both directions
-// and unite the two cells on the first one.  One edge per connected cell pair
-// replaces the union of every edge.  The lanes first screen up to 32
-// neighbour cells at once (range, cores, roots); then, for each cell still to
-// test, lanes hold A's cores and B's points are broadcast; the test is the
-// table kernels' (FP32 on cell-relative coordinates, exact FP64 predicate
-// inside the error band).
-__global__ void cell_pairs_kernel(ClusterArgs a) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint32_t ncl = *a.ncl;
-    const EpsParams* __restrict__ ep = a.ep;
-    const int R = ep->rho;
-    const bool mixed = ep->mixed != 0;
-    const float lo = ep->lo32, hi = ep->hi32;
-    const double eps = ep->eps, thr = ep->thr, tbox = ep->tbox;
-    const ExactBounds xb = exact_bounds(eps, thr, tbox);
-    const float wf = (float)a.g.w;
-    const uint32_t ncx_pad = a.g.ncx_pad;
-    const float fnan = __int_as_float(0x7fc00000);
-    const float near2 = (float)(eps * eps * (1.0 + 0x1p-8));
-    // neighbours of the half neighbourhood: row dy = 0 to the right, rows
-    // dy = 1..R across their reach
-    int nnb = 0;
-    for (int dy = 0; dy <= R; dy++) nnb += dy == 0 ? ep->reach[R] : 2 * ep->reach[dy + R] + 1;
-    uint32_t skipped = 0;  // lane 0: cell pairs of different components at a larger epsilon
-    for (uint64_t c = warp; c < ncl; c += nwarps) {
-        const uint32_t repA = a.crep[c];
-        if (repA == kNone) continue;
-        const uint32_t compA = a.comp_prev ? a.comp_prev[a.gpos[repA]] : kNone;
-        const uint32_t sA = a.clist[c], eA = a.clist[c + 1];
-        const uint32_t keyA = a.gkey[sA];
-        const int cy = (int)(keyA / ncx_pad), cx = (int)(keyA - (uint32_t)cy * ncx_pad);
-        // A's first 32 points, kept for every neighbour cell
-        const bool va0 = sA + lane < eA && is_core(a.deg[sA + lane], a.minpts);
-        float2 pa0 = make_float2(fnan, fnan);
-        double2 Pa0 = make_double2(0.0, 0.0);
-        if (va0) {
-            pa0 = a.glocal[sA + lane];
-            Pa0 = a.gxy[sA + lane];
-        }
-        for (int base = 0; base < nnb; base += 32) {
-            // lane -> neighbour (dy, dx) number base + lane
-            int my_dy = 0, my_dx = 0;
-            bool valid = false;
-            {
-                int idx = base + (int)lane, acc = 0;
-                for (int dy = 0; dy <= R && !valid; dy++) {
-                    const int reach = ep->reach[dy + R];
-                    const int cnt = dy == 0 ? reach : 2 * reach + 1;
-                    if (idx < acc + cnt) {
-                        my_dy = dy;
-                        my_dx = (dy == 0 ? 1 : -reach) + (idx - acc);
-                        valid = true;
-                    }
-                    acc += cnt;
-                }
-            }
-            const int ry = cy + my_dy, rx = cx + my_dx;
-            uint32_t sB = 0, eB = 0, repB = kNone;
-            bool need = false;
-            if (valid && ry < (int)a.g.ncy && rx >= 0 && rx < (int)a.g.ncx) {
-                cell_row_range(a.g, a.cell_start, a.crow, a.ccx, a.clist, (uint32_t)ry,
-                               (uint32_t)rx, (uint32_t)rx, &sB, &eB);
-                if (sB < eB) {
-                    repB = a.crep[a.cscan[sB]];
-                    need = repB != kNone && uf_find(a.parent, repA) != uf_find(a.parent, repB);
-                    // cores in different components at the larger epsilon are
-                    // not connected at this one (its components refine those)
-                    if (need && a.comp_prev && a.comp_prev[a.gpos[repB]] != compA) need = false;
-                }
-            }
-            if (a.comp_prev) {
-                const bool skip = valid && repB != kNone && !need && sB < eB &&
-                                  a.comp_prev[a.gpos[repB]] != compA;
-                skipped += __popc(__ballot_sync(kFull, skip));
-            }
-            // nearest cells first (their pairs are found soonest, and the unions
-            // they make often connect the farther cells already): squared gap
-            // between the cells in cell widths, then lane
-            const int gx = max(abs(my_dx) - 1, 0), gy = max(my_dy - 1, 0);
-            const uint32_t order = ((uint32_t)(gx * gx + gy * gy) << 5) | lane;
-            for (uint32_t todo = __ballot_sync(kFull, need); todo;) {
-                const uint32_t pick = __reduce_min_sync(kFull, (todo >> lane) & 1u ? order : 0xffffffffu);
-                const int src = (int)(pick & 31u);
-                todo &= ~(1u << src);
-                const uint32_t sBb = __shfl_sync(kFull, sB, src), eBb = __shfl_sync(kFull, eB, src);
-                const int dx = __shfl_sync(kFull, my_dx, src), dy = __shfl_sync(kFull, my_dy, src);
-                // unions made since the screen may have joined the two cells
-                const uint32_t repBb = __shfl_sync(kFull, repB, src);
-                if (uf_find(a.parent, repA) == uf_find(a.parent, repBb)) continue;
-                const float dyw = __fmul_rn((float)dy, wf);
-                const float dxw = __fmul_rn((float)dx, wf);
-                bool found = false;
-                for (uint32_t b = sA; b < eA && !found; b += 32) {
-                    const uint32_t ka = b + lane;
-                    bool va = va0;
-                    float2 pa = pa0;
-                    double2 Pa = Pa0;
-                    if (b != sA) {  // cells of more than 32 points: the next 32
-                        va = ka < eA && is_core(a.deg[ka], a.minpts);
-                        pa = make_float2(fnan, fnan);
-                        if (va) {
-                            pa = a.glocal[ka];
-                            Pa = a.gxy[ka];
-                        }
-                    }
-                    // only points within eps of the other cell's square can pair
-                    // (cell-relative FP32 coordinates, eps^2 widened by 2^-8)
-                    if (mixed && va) {
-                        const float ex = fmaxf(fmaxf(dxw - pa.x, pa.x - (dxw + wf)), 0.0f);
-                        const float ey = fmaxf(fmaxf(dyw - pa.y, pa.y - (dyw + wf)), 0.0f);
-                        va = __fmaf_rn(ex, ex, ey * ey) <= near2;
-                    }
-                    if (!__any_sync(kFull, va)) continue;
-                    // B's points 32 at a time: one coalesced load of their
-                    // core flags and coordinates, then broadcast core by core
-                    for (uint32_t kb0 = sBb; kb0 < eBb && !found; kb0 += 32) {
-                        const uint32_t kbl = kb0 + lane;
-                        bool vb = kbl < eBb && is_core(a.deg[kbl], a.minpts);
-                        float2 lbl = make_float2(fnan, fnan);
-                        if (vb && mixed) {
-                            lbl = a.glocal[kbl];
-                            const float bx = __fmaf_rn((float)dx, wf, lbl.x);
-                            const float by = __fadd_rn(lbl.y, dyw);
-                            const float ex = fmaxf(fmaxf(-bx, bx - wf), 0.0f);
-                            const float ey = fmaxf(fmaxf(-by, by - wf), 0.0f);
-                            vb = __fmaf_rn(ex, ex, ey * ey) <= near2;
-                        }
-                        for (uint32_t cm = __ballot_sync(kFull, vb); cm; cm &= cm - 1u) {
-                            const int t = __ffs(cm) - 1;
-                            const uint32_t kb = kb0 + (uint32_t)t;
-                            const float lbx = __shfl_sync(kFull, lbl.x, t);
-                            const float lby = __shfl_sync(kFull, lbl.y, t);
-                            bool in = false;
-                            if (va) {
-                                uint32_t cls;  // 0 out, 1 in (both directions), 2 band
-                                double2 Qb = make_double2(0.0, 0.0);  // FP64 tests only
-                                if (mixed) {
-                                    const float bx = __fmaf_rn((float)dx, wf, lbx);
-                                    const float by = __fadd_rn(lby, dyw);
-                                    const float ddx = __fsub_rn(pa.x, bx), ddy = __fsub_rn(pa.y, by);
-                                    const float d2 = __fmaf_rn(ddx, ddx, __fmul_rn(ddy, ddy));
-                                    cls = d2 < lo ? 1u : (d2 <= hi ? 2u : 0u);
-                                } else {
-                                    Qb = a.gxy[kb];
-                                    const double ddx = __dsub_rn(Pa.x, Qb.x), ddy = __dsub_rn(Pa.y, Qb.y);
-                                    const double d2 = __dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy));
-                                    cls = d2 <= tbox ? 1u : (d2 <= thr ? 2u : 0u);
-                                }
-                                if (cls == 2u) {
-                                    if (mixed) Qb = a.gxy[kb];
-                                    cls = exact_pair(Pa, Qb, ka, kb, xb, a.gbox) == 3u
-                                              ? 1u : 0u;
-                                }
-                                in = cls == 1u;
-                            }
-                            const uint32_t hit = __ballot_sync(kFull, in);
-                            if (hit) {
-                                const uint32_t u = __shfl_sync(kFull, ka, __ffs(hit) - 1);
-                                if (lane == 0) uf_union(a.parent, u, kb, a.st);
-                                found = true;
-                                break;
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-    if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
-}
-
 __global__ void save_components_kernel(ClusterArgs a, uint32_t* __restrict__ comp) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
@@ -494,6 +280,7 @@ __global__ void asym_push_kernel(ClusterArgs a) {
 __global__ void write_labels_kernel(ClusterArgs a) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
+    if (k == 0) atomicAdd(&a.st->clusters, (unsigned long long)a.cluster_no[a.n] * a.copies);
     uint32_t lab;
     if (is_core(a.deg[k], a.minpts)) {
         const uint32_t t = start_time(a, k);
@@ -505,50 +292,589 @@ __global__ void write_labels_kernel(ClusterArgs a) {
     if (VDB_GUARD(a.st, a.gorig[k] < a.n, 13, a.gorig[k])) a.labels_out[a.gorig[k]] = lab;
 }
 
-// vmax[v] = largest label of variant v (one atomic per variant and warp)
-// Largest label of each variant: block b reduces part b % bpv of variant
-// b / bpv and raises vmax[v] once.
-__global__ void label_max_kernel(const uint32_t* __restrict__ labels, uint32_t n, uint32_t bpv,
-                                 uint32_t* __restrict__ vmax) {
-    __shared__ uint32_t s_max[kThreads / 32];
-    const uint32_t v = blockIdx.x / bpv, part = blockIdx.x % bpv;
-    const uint32_t* __restrict__ lv = labels + (size_t)v * n;
-    uint32_t mx = 0;
-    for (unsigned long long i = (unsigned long long)part * kThreads + threadIdx.x; i < n;
-         i += (unsigned long long)bpv * kThreads)
-        mx = max(mx, lv[i]);
-    mx = __reduce_max_sync(kFull, mx);
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        mx = threadIdx.x < kThreads / 32 ? s_max[threadIdx.x] : 0u;
-        mx = __reduce_max_sync(kFull, mx);
-        if (threadIdx.x == 0 && mx) atomicMax(&vmax[v], mx);
+// ------------------------------------------------------------- cell clusters
+//
+// Grids whose cells are cliques (cell width <= eps/sqrt(2), 2 w^2 below the
+// thresholds): the cores of a cell always share a component, so the
+// union-find runs over the non-empty cells, and a border point is settled by
+// its neighbour cells' cluster starts.  The neighbour table is not read.  All
+// minpts of one epsilon (slots, largest minpts first) share the kernels that
+// do not depend on one another.
+
+// Neighbour cells: crng[i * n + c] = the non-empty cells [x, y) of row
+// i - rho within reach of cell c, ccx[c] = the column of cell c.  One thread
+// per cell and row looks them up once for all slots and kernels (in sparse
+// grids by binary search), so that the kernels below walk lists of cells that
+// exist instead of probing every offset.
+__global__ void cell_ranges_kernel(CellArgs a) {
+    const uint32_t rho = (uint32_t)a.ep->rho;
+    const uint32_t ncl = *a.ncl;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+    if (c >= ncl || r > 2u * rho) return;
+    const uint32_t key = a.gkey[a.clist[c]];
+    const int cy = (int)(key / a.g.ncx_pad), cx = (int)(key - (uint32_t)cy * a.g.ncx_pad);
+    if (r == rho && !a.g.sparse) a.ccx[c] = (uint32_t)cx;
+    const int ry = cy + (int)r - (int)rho, reach = a.ep->reach[r];
+    const uint32_t lo = (uint32_t)max(cx - reach, 0);
+    const uint32_t hi = (uint32_t)min(cx + reach, (int)a.g.ncx - 1);
+    uint2 out = make_uint2(0u, 0u);
+    if (ry >= 0 && ry < (int)a.g.ncy) {
+        if (a.g.sparse) {
+            const uint32_t re = a.crow[ry + 1];
+            out.x = cx_lower_bound(a.ccx, a.crow[ry], re, lo);
+            out.y = out.x;
+            while (out.y < re && a.ccx[out.y] <= hi) out.y++;
+        } else {
+            const uint32_t base = (uint32_t)ry * a.g.ncx_pad;
+            out.x = a.cscan[a.cell_start[base + lo]];
+            out.y = a.cscan[a.cell_start[base + hi + 1]];
+        }
+    }
+    if (!VDB_GUARD(a.st, out.x <= out.y && out.y <= ncl, 16, out.y)) out = make_uint2(0u, 0u);
+    a.crng[(size_t)r * a.n + c] = out;
+}
+
+// cbest[c] = largest degree of the cell (high word) and the first point that
+// has it (complemented, low word): the cell has cores at minpts m iff the
+// high word is >= m, and that point is one of them.
+__device__ __forceinline__ uint32_t best_deg(unsigned long long b) { return (uint32_t)(b >> 32); }
+__device__ __forceinline__ uint32_t best_point(unsigned long long b) { return ~(uint32_t)b; }
+
+struct PairTest {
+    bool mixed;
+    float lo, hi, wf;
+    ExactBounds xb;
+};
+__device__ __forceinline__ PairTest pair_test(const CellArgs& a) {
+    PairTest t;
+    t.mixed = a.ep->mixed != 0;
+    t.lo = a.ep->lo32;
+    t.hi = a.ep->hi32;
+    t.wf = (float)a.g.w;
+    t.xb = exact_bounds(a.ep->eps, a.ep->thr, a.ep->tbox);
+    return t;
+}
+// bit0: v in N(u), bit1: u in N(v), for points ku and kv whose cells lie
+// (dx, dy) cells apart; pu, pv: their FP32 coordinates in their own cells.
+__device__ __forceinline__ uint32_t test_pair(const CellArgs& a, const PairTest& t, uint32_t ku,
+                                              uint32_t kv, float2 pu, float2 pv, int dx, int dy) {
+    if (t.mixed) {
+        const float ddx = __fsub_rn(pu.x, __fmaf_rn((float)dx, t.wf, pv.x));
+        const float ddy = __fsub_rn(pu.y, __fadd_rn(pv.y, __fmul_rn((float)dy, t.wf)));
+        const float d2 = __fmaf_rn(ddx, ddx, __fmul_rn(ddy, ddy));
+        if (d2 < t.lo) return 3u;
+        if (!(d2 <= t.hi)) return 0u;
+    }
+    return exact_pair(a.gxy[ku], a.gxy[kv], ku, kv, t.xb, a.gbox);
+}
+
+// Start state of all slots: every cell its own root in the first slot's
+// forest (the others copy their predecessor's), no seeds, no cluster starts.
+__global__ void cells_init_kernel(CellArgs a) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < a.nw)
+        for (int v = 0; v < a.m; v++) a.bits[(size_t)v * a.nw + k] = 0u;
+    if (k >= a.n) return;
+    a.cbest[k] = 0ull;
+    for (int v = 0; v < a.m; v++) {
+        const size_t o = (size_t)v * a.n + k;
+        a.seed[o] = kNone;
+        if (v == 0 ? !a.continued : !a.chain) a.parent[o] = k;
     }
 }
 
-__global__ void sum_clusters_kernel(const uint32_t* __restrict__ vmax, uint32_t V,
-                                    DeviceStatus* st) {
-    unsigned long long acc = 0;
-    for (uint32_t v = threadIdx.x; v < V; v += blockDim.x) acc += vmax[v];
-    for (int d = 16; d > 0; d >>= 1) acc += __shfl_down_sync(kFull, acc, d);
-    if ((threadIdx.x & 31) == 0 && acc) atomicAdd(&st->clusters, acc);
+__global__ void cell_best_kernel(CellArgs a) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = k < a.n;
+    const uint32_t c = in ? a.cscan[k + 1] - 1u : kNone;
+    const uint32_t d = in ? a.deg[k] : 0u;
+    const uint32_t same = __match_any_sync(kFull, c);
+    const uint32_t mx = __reduce_max_sync(same, d);
+    const uint32_t first = __reduce_min_sync(same, d == mx ? k : kNone);
+    if (in && first == k && VDB_GUARD(a.st, c < a.n, 15, c))
+        atomicMax(&a.cbest[c], ((unsigned long long)mx << 32) | (uint32_t)~k);
+}
+
+// First unions of slot v: a thread per cell and row (its own and the next)
+// tests the points of largest degree of the cell and of its adjacent cells.
+// In dense regions that joins almost every pair of adjacent cells, so that
+// the search below finds most pairs already joined.
+__global__ void cell_near_kernel(CellArgs a, int v) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, dy = blockIdx.y;
+    if (c >= *a.ncl) return;
+    const uint32_t mp = a.mp[v];
+    const unsigned long long bA = a.cbest[c];
+    if (best_deg(bA) < mp) return;
+    const uint32_t rho = (uint32_t)a.ep->rho;
+    const uint2 rg = a.crng[(size_t)(rho + dy) * a.n + c];
+    const int cx = (int)a.ccx[c];
+    const uint32_t ku = best_point(bA);
+    if (ku >= a.n) return;
+    const PairTest t = pair_test(a);
+    const float2 pu = a.glocal[ku];
+    uint32_t* parent = a.parent + (size_t)v * a.n;
+    for (uint32_t o = dy ? rg.x : c + 1; o < rg.y; o++) {
+        const int dx = (int)a.ccx[o] - cx;
+        if (dx > 1) break;
+        if (dx < -1) continue;
+        const unsigned long long bB = a.cbest[o];
+        if (best_deg(bB) < mp || parent[c] == parent[o]) continue;
+        const uint32_t kv = best_point(bB);
+        if (kv < a.n && test_pair(a, t, ku, kv, pu, a.glocal[kv], dx, (int)dy) == 3u)
+            uf_union(parent, c, o, a.st);
+    }
+}
+
+constexpr uint32_t kLanePairs = 4;     // cells of at most so many point pairs: one lane
+constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes over the pairs
+
+// Remaining unions of slot v: every pair of cells within reach whose roots
+// still differ is searched for one core-core pair accepted in both
+// directions.  A lane takes a cell and one row of its half neighbourhood; it
+// screens the roots and tests the pairs of next to empty cells itself; the
+// other pairs are searched by the whole warp, lanes over the point pairs (or,
+// for large cells, over the first cell's points within eps of the second).
+__global__ void cell_pairs_kernel(CellArgs a, int v) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t ncl = *a.ncl;
+    const uint32_t mp = a.mp[v];
+    const PairTest t = pair_test(a);
+    const double eps = a.ep->eps;
+    const float near2 = (float)(eps * eps * (1.0 + 0x1p-8));
+    const float wf = t.wf;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, dy = blockIdx.y;
+    if (c - lane >= ncl) return;  // (whole warps)
+    uint32_t* parent = a.parent + (size_t)v * a.n;
+    const uint32_t* __restrict__ comp = a.comp_prev[v];
+    uint32_t skipped = 0;  // cell pairs of different components at a larger epsilon
+    uint32_t o = 0, oe = 0, sA = 0, eA = 0, compA = kNone;
+    int cx = 0;
+    if (c < ncl) {
+        const unsigned long long bA = a.cbest[c];
+        if (best_deg(bA) >= mp) {
+            const uint2 rg = a.crng[(size_t)((uint32_t)a.ep->rho + dy) * a.n + c];
+            o = dy ? rg.x : c + 1;
+            oe = rg.y;
+            if (o < oe) {
+                cx = (int)a.ccx[c];
+                sA = a.clist[c];
+                eA = a.clist[c + 1];
+                if (comp) compA = comp[a.gpos[best_point(bA)]];
+            }
+        }
+    }
+    // every lane walks its row; each step's pairs that need more than a
+    // lane are then searched one after the other
+    while (__any_sync(kFull, o < oe)) {
+        bool need = false;
+        uint32_t sB = 0, eB = 0;
+        int dx = 0;
+        const uint32_t ob = o;
+        if (o < oe) {
+            const unsigned long long bB = a.cbest[o];
+            need = best_deg(bB) >= mp && uf_find(parent, c) != uf_find(parent, o);
+            // cores in different components at the larger epsilon are not
+            // connected at this one (its components refine those)
+            if (need && comp && comp[a.gpos[best_point(bB)]] != compA) {
+                need = false;
+                skipped++;
+            }
+            if (need) {
+                sB = a.clist[o];
+                eB = a.clist[o + 1];
+                dx = (int)a.ccx[o] - cx;
+                if ((uint64_t)(eA - sA) * (eB - sB) <= kLanePairs) {
+                    for (uint32_t u = sA; u < eA && need; u++)
+                        for (uint32_t w = sB; w < eB && need; w++)
+                            if (a.deg[u] >= mp && a.deg[w] >= mp &&
+                                test_pair(a, t, u, w, a.glocal[u], a.glocal[w], dx, (int)dy) == 3u) {
+                                uf_union(parent, c, o, a.st);
+                                need = false;
+                            }
+                    need = false;
+                }
+            }
+            o++;
+        }
+        for (uint32_t todo = __ballot_sync(kFull, need); todo; todo &= todo - 1u) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t cA = __shfl_sync(kFull, c, src), cB = __shfl_sync(kFull, ob, src);
+            // unions made since the screen may have joined the two cells
+            bool joined = false;
+            if (lane == 0) joined = uf_find(parent, cA) == uf_find(parent, cB);
+            if (__shfl_sync(kFull, (int)joined, 0)) continue;
+            const uint32_t As = __shfl_sync(kFull, sA, src), Ae = __shfl_sync(kFull, eA, src);
+            const uint32_t Bs = __shfl_sync(kFull, sB, src), Be = __shfl_sync(kFull, eB, src);
+            const int ox = __shfl_sync(kFull, dx, src), oy = __shfl_sync(kFull, (int)dy, src);
+            const uint32_t na = Ae - As, nb = Be - Bs;
+            bool found = false;
+            if ((uint64_t)na * nb <= kFlatPairs) {
+                const uint32_t tot = na * nb;
+                for (uint32_t p0 = 0; p0 < tot && !found; p0 += 32) {
+                    const uint32_t p = p0 + lane;
+                    bool in = false;
+                    if (p < tot) {
+                        const uint32_t u = As + p / nb, w = Bs + p % nb;
+                        in = a.deg[u] >= mp && a.deg[w] >= mp &&
+                             test_pair(a, t, u, w, a.glocal[u], a.glocal[w], ox, oy) == 3u;
+                    }
+                    found = __any_sync(kFull, in);
+                }
+            } else {
+                const float dxw = __fmul_rn((float)ox, wf), dyw = __fmul_rn((float)oy, wf);
+                for (uint32_t u0 = As; u0 < Ae && !found; u0 += 32) {
+                    const uint32_t u = u0 + lane;
+                    bool va = u < Ae && a.deg[u] >= mp;
+                    float2 pu = make_float2(0.f, 0.f);
+                    if (va) {
+                        // only points within eps of the other cell's square can
+                        // pair (FP32 coordinates, eps^2 widened by 2^-8)
+                        pu = a.glocal[u];
+                        const float ex = fmaxf(fmaxf(dxw - pu.x, pu.x - (dxw + wf)), 0.0f);
+                        const float ey = fmaxf(fmaxf(dyw - pu.y, pu.y - (dyw + wf)), 0.0f);
+                        va = !t.mixed || __fmaf_rn(ex, ex, ey * ey) <= near2;
+                    }
+                    if (!__any_sync(kFull, va)) continue;
+                    for (uint32_t w0 = Bs; w0 < Be && !found; w0 += 32) {
+                        const uint32_t wl = w0 + lane;
+                        bool vb = wl < Be && a.deg[wl] >= mp;
+                        float2 pw = make_float2(0.f, 0.f);
+                        if (vb) {
+                            pw = a.glocal[wl];
+                            const float bx = __fmaf_rn((float)ox, wf, pw.x);
+                            const float by = __fadd_rn(pw.y, dyw);
+                            const float ex = fmaxf(fmaxf(-bx, bx - wf), 0.0f);
+                            const float ey = fmaxf(fmaxf(-by, by - wf), 0.0f);
+                            vb = !t.mixed || __fmaf_rn(ex, ex, ey * ey) <= near2;
+                        }
+                        for (uint32_t cm = __ballot_sync(kFull, vb); cm && !found; cm &= cm - 1u) {
+                            const int s1 = __ffs(cm) - 1;
+                            const float2 q = make_float2(__shfl_sync(kFull, pw.x, s1),
+                                                         __shfl_sync(kFull, pw.y, s1));
+                            const bool in = va && test_pair(a, t, u, w0 + (uint32_t)s1, pu, q, ox,
+                                                            oy) == 3u;
+                            found = __any_sync(kFull, in);
+                        }
+                    }
+                }
+            }
+            if (found && lane == 0) uf_union(parent, cA, cB, a.st);
+            __syncwarp();
+        }
+    }
+    skipped = __reduce_add_sync(kFull, skipped);
+    if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
+}
+
+// Roots of slot v, which are also the next slot's start (a smaller minpts
+// keeps every core and every connection).
+__global__ void cell_flatten_kernel(CellArgs a, int v) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= *a.ncl) return;
+    uint32_t* parent = a.parent + (size_t)v * a.n;
+    const uint32_t r = uf_find_ro(parent, c);
+    parent[c] = r;
+    if (a.chain && v + 1 < a.m) parent[a.n + c] = r;
+}
+
+// seed[root] = first visit position among the component's cores (y: slot).
+__global__ void cell_seed_kernel(CellArgs a) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int v = blockIdx.y;
+    if (k >= a.n || a.deg[k] < a.mp[v]) return;
+    const uint32_t c = a.cscan[k + 1] - 1u;
+    if (!VDB_GUARD(a.st, c < a.n, 16, c)) return;
+    const uint32_t r = a.parent[(size_t)v * a.n + c];
+    // neighbours in cell order mostly share a root: one atomic per root and warp
+    const uint32_t same = __match_any_sync(__activemask(), r);
+    const uint32_t mn = __reduce_min_sync(same, a.gpos[k]);
+    if ((threadIdx.x & 31) == (uint32_t)(__ffs(same) - 1) && r < a.n)
+        atomicMin(&a.seed[(size_t)v * a.n + r], mn);
+}
+
+// Core-core edges accepted in one direction only, between components (one
+// thread per slot; run only when the table has one-way pairs): the components
+// that an earlier cluster's expansion absorbs take its start as their seed.
+__global__ void cell_resolve_kernel(CellArgs a, uint32_t* ws, uint32_t cap) {
+    if (threadIdx.x != 0) return;
+    const int v = blockIdx.x;
+    const uint32_t mp = a.mp[v];
+    const uint32_t* parent = a.parent + (size_t)v * a.n;
+    uint32_t* seed = a.seed + (size_t)v * a.n;
+    uint32_t* cs = a.cst + (size_t)v * a.n;  // start component of the edges' components
+    ws += (size_t)v * 6 * cap;
+    uint32_t na = *a.asym_count;
+    if (na > a.asym_cap) na = a.asym_cap;
+    uint32_t* efrom = ws;
+    uint32_t* eto = ws + cap;
+    uint32_t* nodes = ws + 2 * cap;
+    uint32_t* stack = ws + 4 * cap;  // 2*cap entries
+    uint32_t ne = 0;
+    for (uint32_t i = 0; i < na; i++) {
+        const AsymPair p = a.asym[i];
+        if (a.deg[p.a] < mp || a.deg[p.b] < mp) continue;
+        const uint32_t ra = parent[a.cscan[p.a + 1] - 1u], rb = parent[a.cscan[p.b + 1] - 1u];
+        if (ra == rb) continue;
+        if (ne >= cap) {
+            atomicOr(&a.st->flags, kStatResolveOverflow);
+            return;
+        }
+        // dir 1: b in N(a) only, a's expansion reaches b
+        efrom[ne] = p.dir == 1u ? ra : rb;
+        eto[ne] = p.dir == 1u ? rb : ra;
+        ne++;
+    }
+    if (ne == 0) return;
+    // distinct endpoint components in seed order
+    uint32_t nn = 0;
+    for (uint32_t i = 0; i < 2 * ne; i++) {
+        const uint32_t r = i < ne ? efrom[i] : eto[i - ne];
+        bool dup = false;
+        for (uint32_t j = 0; j < nn && !dup; j++) dup = nodes[j] == r;
+        if (dup) continue;
+        uint32_t j = nn++;
+        while (j > 0 && seed[nodes[j - 1]] > seed[r]) {
+            nodes[j] = nodes[j - 1];
+            j--;
+        }
+        nodes[j] = r;
+    }
+    for (uint32_t i = 0; i < nn; i++) cs[nodes[i]] = kNone;
+    for (uint32_t i = 0; i < nn; i++) {
+        const uint32_t u = nodes[i];
+        if (cs[u] != kNone) continue;
+        cs[u] = u;
+        uint32_t top = 0;
+        stack[top++] = u;
+        while (top) {
+            const uint32_t x = stack[--top];
+            for (uint32_t e = 0; e < ne; e++) {
+                if (efrom[e] != x) continue;
+                const uint32_t y = eto[e];
+                if (cs[y] != kNone) continue;
+                cs[y] = u;
+                stack[top++] = y;
+            }
+        }
+    }
+    for (uint32_t i = 0; i < nn; i++) seed[nodes[i]] = seed[cs[nodes[i]]];
+}
+
+// cst = visit position at which the cluster of the cell's cores starts (kNone:
+// no cores); the starts' bits (y: slot).
+__global__ void cell_starts_kernel(CellArgs a) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int v = blockIdx.y;
+    if (c >= *a.ncl) return;
+    const size_t o = (size_t)v * a.n;
+    uint32_t s = kNone;
+    if (best_deg(a.cbest[c]) >= a.mp[v]) {
+        const uint32_t r = a.parent[o + c];
+        s = r < a.n ? a.seed[o + r] : kNone;
+        if (!VDB_GUARD(a.st, s < a.n, 12, s)) s = kNone;
+        else if (r == c) atomicOr(&a.bits[(size_t)v * a.nw + (s >> 5)], 1u << (s & 31u));
+    }
+    a.cst[o + c] = s;
+}
+
+// brank[w] = cluster starts before word w of the slot's bits; the slot's
+// number of clusters (one block per slot).
+constexpr int kRankThreads = 1024;
+constexpr int kRankItems = 8;
+__global__ void __launch_bounds__(kRankThreads) cell_rank_kernel(CellArgs a) {
+    __shared__ uint32_t s_tot[32];
+    const int v = blockIdx.x;
+    const uint32_t* __restrict__ bits = a.bits + (size_t)v * a.nw;
+    uint32_t* rank = a.brank + (size_t)v * a.nw;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < a.nw; base += kRankThreads * kRankItems) {
+        const uint32_t w0 = base + threadIdx.x * kRankItems;
+        uint32_t c[kRankItems], sum = 0;
+        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+        if (w0 < a.nw) {  // (nw is a multiple of kRankItems)
+            lo = reinterpret_cast<const uint4*>(bits + w0)[0];
+            hi = reinterpret_cast<const uint4*>(bits + w0)[1];
+        }
+        c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w;
+        c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
+#pragma unroll
+        for (int i = 0; i < kRankItems; i++) {
+            c[i] = __popc(c[i]);
+            sum += c[i];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, d);
+            if (lane >= (uint32_t)d) incl += t;
+        }
+        if (lane == 31) s_tot[wid] = incl;
+        __syncthreads();
+        uint32_t t = s_tot[lane], ti = t;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(kFull, ti, d);
+            if (lane >= (uint32_t)d) ti += o;
+        }
+        const uint32_t before = __shfl_sync(kFull, ti - t, (int)wid);
+        const uint32_t all = __shfl_sync(kFull, ti, 31);
+        uint32_t run = carry + before + incl - sum;
+#pragma unroll
+        for (int i = 0; i < kRankItems; i++) {
+            const uint32_t t2 = c[i];
+            c[i] = run;
+            run += t2;
+        }
+        if (w0 < a.nw) {
+            reinterpret_cast<uint4*>(rank + w0)[0] = make_uint4(c[0], c[1], c[2], c[3]);
+            reinterpret_cast<uint4*>(rank + w0)[1] = make_uint4(c[4], c[5], c[6], c[7]);
+        }
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && carry)
+        atomicAdd(&a.st->clusters, (unsigned long long)carry * a.copies[v]);
+}
+
+// Label of the cluster that starts at visit position s.
+__device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32_t s) {
+    const size_t w = (size_t)v * a.nw + (s >> 5);
+    return a.brank[w] + __popc(a.bits[w] & ((1u << (s & 31u)) - 1u)) + 1u;
+}
+
+// Labels of the cores, and the saved components (comp[visit position] =
+// cluster start of the core there, kNone for other points).
+__global__ void cell_core_labels_kernel(CellArgs a) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.n) return;
+    const uint32_t d = a.deg[k], c = a.cscan[k + 1] - 1u, o = a.gorig[k], p = a.gpos[k];
+    if (!VDB_GUARD(a.st, c < a.n && o < a.n && p < a.n, 13, o)) return;
+    for (int v = 0; v < a.m; v++) {
+        const bool core = d >= a.mp[v];
+        uint32_t s = kNone;
+        if (core) {
+            s = a.cst[(size_t)v * a.n + c];
+            if (VDB_GUARD(a.st, s < a.n, 14, s)) a.labels[v][o] = start_label(a, v, s);
+        }
+        if (a.comp_out[v]) a.comp_out[v][p] = s;
+    }
+}
+
+// Labels of the points that are not core, a thread per point.  Such a point p
+// takes the earliest cluster start among the cores u with p in N(u): the
+// start of its own cell if that has cores (a clique), or of a neighbour cell
+// if one of that cell's cores lists p.  Only neighbour cells whose start is
+// earlier than what p has are searched, earliest start first: a point whose
+// neighbour cells all belong to its own cell's cluster searches nothing, and
+// one surrounded by a single other cluster ends at the first core found.  A
+// start after p's own visit position cannot label it (p was visited first, as
+// noise).  A lane searches up to kLaneCores points itself; larger searches are
+// done by the warp, lanes over the cells' points.
+constexpr uint32_t kLaneCores = 16;
+__global__ void cell_border_kernel(CellArgs a) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t d = k < a.n ? a.deg[k] : kNone;
+    if (!__any_sync(kFull, d < a.mp[0])) return;  // (slots in descending minpts: all cores)
+    const PairTest t = pair_test(a);
+    const int rho = a.ep->rho, nrows = 2 * rho + 1;
+    uint32_t c = 0, p = 0, out = 0;
+    int cx = 0;
+    float2 loc = make_float2(0.f, 0.f);
+    bool ok = d < a.mp[0];
+    if (ok) {
+        c = a.cscan[k + 1] - 1u;
+        p = a.gpos[k];
+        out = a.gorig[k];
+        ok = VDB_GUARD(a.st, c < a.n && out < a.n, 13, out);
+    }
+    if (ok) {
+        cx = (int)a.ccx[c];
+        loc = a.glocal[k];
+    }
+    const uint2* __restrict__ rng = a.crng + c;  // row i: rng[i * n]
+    for (int v = 0; v < a.m; v++) {
+        const uint32_t mp = a.mp[v];
+        const bool border = ok && d < mp;
+        if (!__any_sync(kFull, border)) break;  // (nor at a smaller minpts)
+        const uint32_t* __restrict__ cst = a.cst + (size_t)v * a.n;
+        uint32_t best = border ? cst[c] : 0u;
+        uint32_t floor_s = 0;  // starts below this one have been searched
+        bool busy = border;
+        while (__any_sync(kFull, busy)) {
+            // the earliest start that is left among the neighbour cells, and
+            // the points of its cells
+            uint32_t ms = kNone, npts = 0;
+            if (busy) {
+                const uint32_t lim = min(best, p);
+                for (int i = 0; i < nrows; i++) {
+                    const uint2 rg = rng[(size_t)i * a.n];
+                    for (uint32_t o = rg.x; o < rg.y; o++) {
+                        const uint32_t st = cst[o];
+                        if (st >= lim || st < floor_s || st > ms) continue;
+                        if (st < ms) npts = 0;
+                        ms = st;
+                        npts += a.clist[o + 1] - a.clist[o];
+                    }
+                }
+                if (ms == kNone) busy = false;
+            }
+            bool hit = false;
+            const bool wide = busy && npts > kLaneCores;
+            if (busy && !wide) {
+                for (int i = 0; i < nrows && !hit; i++) {
+                    const uint2 rg = rng[(size_t)i * a.n];
+                    for (uint32_t o = rg.x; o < rg.y && !hit; o++) {
+                        if (cst[o] != ms) continue;
+                        const int dx = (int)a.ccx[o] - cx;
+                        const uint32_t e = a.clist[o + 1];
+                        for (uint32_t u = a.clist[o]; u < e && !hit; u++)
+                            hit = a.deg[u] >= mp &&
+                                  (test_pair(a, t, k, u, loc, a.glocal[u], dx, i - rho) & 2u);
+                    }
+                }
+            }
+            for (uint32_t todo = __ballot_sync(kFull, wide); todo; todo &= todo - 1u) {
+                const int src = __ffs(todo) - 1;
+                const uint32_t kk = __shfl_sync(kFull, k, src), cc = __shfl_sync(kFull, c, src);
+                const uint32_t mss = __shfl_sync(kFull, ms, src);
+                const int cxx = __shfl_sync(kFull, cx, src);
+                const float2 l = make_float2(__shfl_sync(kFull, loc.x, src),
+                                             __shfl_sync(kFull, loc.y, src));
+                bool found = false;
+                // nearest rows first
+                for (int j = 0; j < nrows && !found; j++) {
+                    const int dy = (j + 1) / 2 * ((j & 1) ? 1 : -1);
+                    const uint2 rg = a.crng[(size_t)(dy + rho) * a.n + cc];
+                    for (uint32_t o = rg.x; o < rg.y && !found; o++) {
+                        if (cst[o] != mss) continue;
+                        const int dx = (int)a.ccx[o] - cxx;
+                        const uint32_t b = a.clist[o], e = a.clist[o + 1];
+                        for (uint32_t u0 = b; u0 < e && !found; u0 += 32) {
+                            const uint32_t u = u0 + lane;
+                            const bool in = u < e && a.deg[u] >= mp &&
+                                            (test_pair(a, t, kk, u, l, a.glocal[u], dx, dy) & 2u);
+                            found = __any_sync(kFull, in);
+                        }
+                    }
+                }
+                if (found && (int)lane == src) hit = true;
+            }
+            if (busy) {
+                if (hit) {
+                    best = ms;
+                    busy = false;  // (no earlier start is left)
+                } else {
+                    floor_s = ms + 1u;
+                }
+            }
+        }
+        if (border) a.labels[v][out] = best < p ? start_label(a, v, best) : 0u;
+    }
 }
 
 }  // namespace
-
-void launch_count_clusters(const uint32_t* labels, uint32_t n, uint32_t V, uint32_t* vmax,
-                           DeviceStatus* st, cudaStream_t s) {
-    if (!n || !V) return;
-    cudaMemsetAsync(vmax, 0, (size_t)V * sizeof(uint32_t), s);
-    // about 8 labels per thread, at most 64 blocks per variant
-    const uint32_t bpv = (uint32_t)std::min<unsigned long long>(
-        64, std::max<unsigned long long>(1, ((unsigned long long)n + 8 * kThreads - 1) / (8 * kThreads)));
-    VDB_COUNT_LAUNCH();
-    label_max_kernel<<<bpv * V, kThreads, 0, s>>>(labels, n, bpv, vmax);
-    VDB_COUNT_LAUNCH();
-    sum_clusters_kernel<<<1, kThreads, 0, s>>>(vmax, V, st);
-}
 
 size_t resolve_scratch_bytes() { return (size_t)kResolveCap * 6 * sizeof(uint32_t); }
 
@@ -561,18 +887,6 @@ void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s) {
 
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s) {
     if (a.row_hi > a.row_lo) { VDB_COUNT_LAUNCH(); uf_union_kernel<<<nblocks, kThreads, 0, s>>>(a); }
-}
-
-void launch_cell_union(const ClusterArgs& a, int nblocks, cudaStream_t s) {
-    if (!a.n) return;
-    // crep[c] starts as "no core" for every cell (ncl <= n)
-    cudaMemsetAsync(a.crep, 0xff, (size_t)a.n * sizeof(uint32_t), s);
-    VDB_COUNT_LAUNCH();
-    cell_rep_min_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_rep_link_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_pairs_kernel<<<nblocks, kThreads, 0, s>>>(a);
 }
 
 void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, void* scan_scratch,
@@ -611,6 +925,40 @@ void launch_border_and_write(const ClusterArgs& a, int nblocks, cudaStream_t s) 
     if (!a.n) return;
     launch_border_pull(a, nblocks, s);
     launch_label_write(a, s);
+}
+
+void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
+                  cudaStream_t s) {
+    if (!a.n) return;
+    const dim3 per_slot(nblk(a.n), (unsigned)a.m);
+    VDB_COUNT_LAUNCH();
+    cells_init_kernel<<<nblk(std::max(a.n, a.nw)), kThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_ranges_kernel<<<dim3(nblk(a.n), (unsigned)nrows), kThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_best_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    for (int v = 0; v < a.m; v++) {
+        VDB_COUNT_LAUNCH();
+        cell_near_kernel<<<dim3(nblk(a.n), nrows > 1 ? 2 : 1), kThreads, 0, s>>>(a, v);
+        VDB_COUNT_LAUNCH();
+        cell_pairs_kernel<<<dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, 0, s>>>(a, v);
+        VDB_COUNT_LAUNCH();
+        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v);
+    }
+    VDB_COUNT_LAUNCH();
+    cell_seed_kernel<<<per_slot, kThreads, 0, s>>>(a);
+    if (one_way) {
+        VDB_COUNT_LAUNCH();
+        cell_resolve_kernel<<<a.m, 32, 0, s>>>(a, (uint32_t*)resolve_ws, kResolveCap);
+    }
+    VDB_COUNT_LAUNCH();
+    cell_starts_kernel<<<per_slot, kThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_rank_kernel<<<a.m, kRankThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_core_labels_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_border_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
 }
 
 }  // namespace vdb

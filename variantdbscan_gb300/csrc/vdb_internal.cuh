@@ -485,26 +485,60 @@ struct ClusterArgs {
     uint32_t asym_cap;
     uint32_t* labels_out;       // n labels in input order
     DeviceStatus* st;
-    // cell structure (cell union): cells of width <= eps/sqrt(2) are cliques
-    GridParams g;
+    uint32_t copies;            // variants that get these labels (equal minpts)
     const EpsParams* ep;        // reach pattern of the grid
+};
+// Clustering on grids whose cells are cliques: all minpts of one epsilon
+// (slots, largest minpts first), up to kSlots at a time.
+constexpr int kSlots = 8;
+struct CellArgs {
+    uint32_t n;
+    const uint32_t* deg;
+    const uint32_t* gpos;
+    const uint32_t* gorig;
     const uint32_t* gkey;
-    const uint32_t* cell_start;
-    const uint32_t* crow;       // sparse grids: row directory (see cell_row_range)
-    const uint32_t* ccx;
-    const uint32_t* clist;      // first point of every non-empty cell (ncl+1 entries)
-    const uint32_t* ncl;        // device scalar
-    const uint32_t* cscan;      // cell index of the first point of each cell
-    uint32_t* crep;             // per non-empty cell: its first core point or ~0
     const float2* glocal;       // FP32 coordinates relative to the own cell's origin
     const double2* gxy;         // FP64 coordinates, cell order
     const MpbBox* gbox;         // multiple-point box of each cell-ordered point
-    // nested-epsilon reuse: comp_prev[pos] = component (its seed) of the core
-    // at visit position pos in a variant with a larger or equal epsilon and a
-    // smaller or equal minpts (nullptr: none); cores of different components
-    // there cannot be connected here
-    const uint32_t* comp_prev;
+    GridParams g;
+    const EpsParams* ep;
+    const uint32_t* cell_start;
+    const uint32_t* crow;       // sparse grids: row directory (see cell_row_range)
+    uint32_t* ccx;              // column of every non-empty cell
+    uint2* crng;                // [2*rho+1][n] neighbour cells per row
+    const uint32_t* clist;      // first point of every non-empty cell (ncl+1 entries)
+    const uint32_t* ncl;        // device scalar
+    const uint32_t* cscan;      // cell of point k: cscan[k + 1] - 1
+    unsigned long long* cbest;  // per cell: largest degree and a point that has it (n entries)
+    int m;                      // slots
+    int chain;                  // nonzero: a slot starts from the components of the one before
+    int continued;              // nonzero: parent of slot 0 holds such a start already
+    uint32_t mp[kSlots];        // minpts (0xffffffff: no cores)
+    uint32_t copies[kSlots];    // variants that get the slot's labels
+    // nested-epsilon reuse: comp_prev[v][pos] = component (its cluster start)
+    // of the core at visit position pos in a variant with a larger or equal
+    // epsilon and a smaller or equal minpts (nullptr: none); cores of
+    // different components there cannot be connected here.  comp_out[v]
+    // receives this slot's (nullptr: not kept).
+    const uint32_t* comp_prev[kSlots];
+    uint32_t* comp_out[kSlots];
+    uint32_t* labels[kSlots];   // n labels in input order
+    uint32_t* parent;           // [m][n] union-find over cells
+    uint32_t* seed;             // [m][n] per root: min visit position of its cores
+    uint32_t* cst;              // [m][n] per cell: start of its cores' cluster
+    uint32_t* bits;             // [m][nw] visit positions at which clusters start
+    uint32_t* brank;            // [m][nw] starts before each word
+    uint32_t nw;                // start_words(n)
+    const AsymPair* asym;
+    const uint32_t* asym_count;
+    uint32_t asym_cap;
+    DeviceStatus* st;
 };
+// Words of the start bits of n visit positions (whole 32-byte groups).
+inline uint32_t start_words(uint32_t n) { return ((n + 31u) / 32u + 7u) & ~7u; }
+// nrows: 2*rho+1; one_way: the table has one-way pairs; resolve_ws:
+// m * resolve_scratch_bytes()
+void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws, cudaStream_t s);
 size_t resolve_scratch_bytes();
 // comp[gpos[k]] = seed of the component of core k, kNone for other points
 // (after launch_uf_finish)
@@ -538,7 +572,6 @@ void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphCondition
 // *dst = v by a kernel (a captured host-to-device copy would read the host
 // buffer at replay time).
 void launch_store_eps(EpsParams* dst, const EpsParams& v, cudaStream_t s);
-void launch_cell_union(const ClusterArgs& a, int nblocks, cudaStream_t s);
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s);
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s);
 void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, void* scan_scratch,
@@ -548,9 +581,6 @@ void launch_border_and_write(const ClusterArgs& a, int nblocks, cudaStream_t s);
 // [row_lo, row_hi) of the table held in nbr (from off_base), then the
 // one-way in-edges and the label write (after every row has been pulled)
 void launch_border_pull(const ClusterArgs& a, int nblocks, cudaStream_t s);
-// st->clusters += sum over the V variants of their largest label (labels[v*n + i])
-void launch_count_clusters(const uint32_t* labels, uint32_t n, uint32_t V, uint32_t* vmax,
-                           DeviceStatus* st, cudaStream_t s);
 void launch_label_write(const ClusterArgs& a, cudaStream_t s);
 
 }  // namespace vdb
