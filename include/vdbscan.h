@@ -74,9 +74,9 @@ typedef struct vdb_context vdb_context;
 #define VDB_SCHEDULE_PLAIN 1   /* one neighbour table and one clustering per variant */
 
 #define VDB_TABLE_ALL 0        /* every row of each neighbour table is written */
-#define VDB_TABLE_BORDER 1     /* only the rows the labelling reads: points that are not
-                                  core for some minpts of their epsilon (labels only;
-                                  needs cells that are cliques, else all rows) */
+#define VDB_TABLE_BORDER 1     /* only the rows the labelling reads (labels only): none
+                                  where the grid's cells are cliques (the default cell
+                                  size), else all rows */
 
 typedef struct {
     const double *x;        /* n coordinates; host or device pointer (see location) */

@@ -1,0 +1,69 @@
+"""Counting and cell clustering at the sizes where they can go wrong: tiles of
+0, 1 and 2 query slots, ragged last words, tiles tested lane = candidate and
+lane = query, words settled by their boxes, more minpts of one epsilon than
+one pass of the clustering takes, sparse and dense cells.  Labels and table
+hashes must equal the oracle's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+M64 = (1 << 64) - 1
+
+
+@pytest.fixture(scope="module")
+def vdb():
+    import variantdbscan_gb300 as v
+    from variantdbscan_gb300 import build
+    build.build()
+    return v
+
+
+@pytest.fixture(scope="module")
+def ctx(vdb):
+    c = vdb.Context()
+    yield c
+    c.close()
+
+
+def _check(ctx, vdb, orc, x, y, eps, mp, mbb=70, **kw):
+    want = orc.variants(x, y, eps, mp, mbb)
+    out, st = ctx.run([vdb.BatchItem(x, y, eps, mp, mbb)], table_hash=True, **kw)
+    np.testing.assert_array_equal(out[0], want)
+    assert st["table_hash"] == sum(orc.table_hash(x, y, e, mbb) for e in np.unique(eps)) & M64
+    assert st["clusters"] == int(want.max(axis=1).sum())
+    out, _ = ctx.run([vdb.BatchItem(x, y, eps, mp, mbb)], table="border", **kw)
+    np.testing.assert_array_equal(out[0], want)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [2, 15, 16, 17, 31, 33, 63, 65, 129, 1025, 4099])
+def test_ragged_sizes(ctx, vdb, orc, n, precision):
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0, 2, n), rng.uniform(0, 1, n)
+    # one epsilon with 11 minpts (two passes of the clustering), one repeated
+    eps = np.array([0.4] * 12 + [0.05, 0.05, 1.7])
+    mp = np.array([1, 2, 3, 5, 8, 13, 21, 34, 55, 144, 500, 3, 2, 4, 30], np.uint32)
+    _check(ctx, vdb, orc, x, y, eps, mp, precision=precision)
+
+
+@pytest.mark.parametrize("lattice", [False, True])
+@pytest.mark.parametrize("n", [32768, 40007])
+def test_words_settled_by_their_boxes(ctx, vdb, orc, n, lattice):
+    # hundreds of points per cell: most words lie inside or outside eps of a
+    # whole tile; on the lattice many pairs are exactly eps apart
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0, 3, n), rng.uniform(0, 2, n)
+    x[: n // 8] = rng.normal(1.0, 0.05, n // 8)
+    if lattice:
+        x, y = np.rint(x * 50) / 50, np.rint(y * 50) / 50
+    _check(ctx, vdb, orc, x, y, np.array([0.5, 0.2, 0.2]), np.array([50, 20, 400], np.uint32))
+
+
+def test_sparse_cells_over_a_wide_box(ctx, vdb, orc):
+    # a row directory instead of a dense cell array, cells of one point
+    rng = np.random.default_rng(8)
+    x, y = rng.uniform(0, 3000, 20000), rng.uniform(0, 3000, 20000)
+    x[:6000] = rng.normal(700, 2, 6000)
+    y[:6000] = rng.normal(700, 2, 6000)
+    _check(ctx, vdb, orc, x, y, np.array([0.3, 0.3, 5.0]), np.array([4, 12, 3], np.uint32))

@@ -274,6 +274,13 @@ int bits_for(uint64_t v) {
     return b;
 }
 
+// Subcell bits per axis that the sort key has room for without another 8-bit
+// pass of the sort: they order the points of a cell, nothing depends on them.
+uint32_t sub_bits(uint64_t ncells) {
+    const int kb = bits_for(ncells - 1);
+    return (uint32_t)std::min(3, ((kb + 7) / 8 * 8 - kb) / 2);
+}
+
 // Distance-test parameters of eps on grid g.  Cells (i, j) relative to a query
 // cell are scanned when their nearest points can be within eps:
 // (max(|i|-1,0)^2 + max(|j|-1,0)^2) * w^2 <= eps^2 (1 + 2^-16).  The margin
@@ -431,6 +438,7 @@ constexpr int kCellsPerEps = 2;
 // which track the exact sums within a few percent on the tables above.
 constexpr double kCostSlot = 6.9e-13, kCostTile = 2.8e-9;  // seconds
 constexpr uint32_t kTuneMinPoints = 131072;
+constexpr uint32_t kBoxPoints = 1u << 15;        // word boxes from this many points on
 constexpr uint32_t kSmallUnitPoints = 1u << 18;  // smaller work units below this many points
 
 uint32_t choose_tile_cells(const unsigned long long* sums) {
@@ -874,6 +882,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     unsigned long long* tboff = ar.get<unsigned long long>((size_t)n + 1);
     uint32_t* tunits = ar.get<uint32_t>(n);
     uint32_t* tuoff = ar.get<uint32_t>((size_t)n + 1);
+    float4* wbox = nullptr;  // boxes of runs of points
     uint32_t* bitmap = nullptr;
     uint64_t bitmap_cap = 0;
     uint32_t* unit_tile = nullptr;
@@ -958,8 +967,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         } else {
             launch_fill(t, nb_fill, s);
         }
-        // hash of the rows just built (tables written in full only)
-        if (o.table_hash && t.row_deg_lim == 0) launch_table_hash(t, gorig, nb_warps, s);
+        // hash of the rows just built
+        if (o.table_hash) launch_table_hash(t, gorig, nb_warps, s);
         CK(cudaGetLastError());
         table_marks.push_back({m0, tm.mark()});
         chunks++;
@@ -978,6 +987,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         uint32_t group_asym = 0;
         bool chunked = false;
         bool compact = false;  // 16-bit table entries for this group's table
+        bool no_rows = false;  // labels only: the degrees are all that is needed
         chunk_list.assign(1, RowChunk{0, 0xffffffffu, 0, 0, 0, n, 0, 0});
         table_marks.clear();
         // unique minpts of the group, largest first; a repeated minpts copies
@@ -1038,8 +1048,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // directory of the non-empty cells instead of a dense cell array,
             // so that the grid costs O(points + rows), not O(cells)
             g.sparse = g.ncells > 32ull * n + (1ull << 22) ? 1u : 0u;
+            g.sub = isfinite(g.w) ? sub_bits(g.ncells) : 0u;
             launch_grid_keys(x, y, n, g, gkey, gorig, s);
-            radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1), scratch, s);
+            radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1) + 2 * (int)g.sub, scratch, s);
             launch_grid_gather(x, y, gorig, pos, n, g, gkey, gxy, glocal, gpos, s);
             launch_point_boxes(gpos, n, mpb, ds.mbb_size, gbox, s);
             auto build_cell_start = [&]() {
@@ -1113,6 +1124,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 // cells: such a shape is not taken)
                 if (G != g.G && g2.ncx == g.ncx && g2.ncy == g.ncy && g2.w == g.w) {
                     g2.sparse = g.sparse;
+                    g2.sub = g.sub;
                     launch_grid_rekey(gkey, n, g.ncx_pad, g2.ncx_pad, s);
                     g = g2;
                     build_cell_start();
@@ -1153,7 +1165,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // only (small, read entry by entry) keep 32-bit entries.
             const bool compact_ok = o.entry_bytes != 4 && 2 * ep.rho + 1 <= 32 &&
                                     (o.entry_bytes == 2 || o.table_rows != VDB_TABLE_BORDER);
-            if (g.sparse || compact_ok) {
+            // VDB_TABLE_BORDER writes the rows that the labelling reads: none
+            // on grids whose cells are cliques
+            no_rows = o.table_rows == VDB_TABLE_BORDER && clique;
+            if (g.sparse || (compact_ok && !no_rows)) {
                 const size_t nr = (size_t)n * (size_t)(2 * ep.rho + 1);
                 if (nr > trow_cap) {
                     if (trow_s) ar.put(trow_s);
@@ -1184,7 +1199,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // 32 candidates of its tile), which the table pass expands
             ta_args.unit_words = unit_words;
             launch_tile_words(ta_args, tflags, tunits, nb_warps, s);
-            scan_u32_to_u64(tflags, tboff, n, scratch, s);
+            if (!no_rows) scan_u32_to_u64(tflags, tboff, n, scratch, s);
             scan_u32(tunits, tuoff, n, scratch, s);
             uint64_t bm_words = 0;
             uint32_t nunits = 0;
@@ -1199,18 +1214,22 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 st_flags = (uint32_t)rec->take();
                 GraphCheck chk;
                 memset(&chk, 0, sizeof chk);
-                chk.c[0] = graph_cond(tboff + n, kGcLe64, bm_words);
-                chk.c[1] = graph_cond(tuoff + n, kGcLe32, nunits);
-                chk.c[2] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
-                chk.n = 3;
+                chk.c[0] = graph_cond(tuoff + n, kGcLe32, nunits);
+                chk.n = 1;
+                if (!no_rows) {
+                    chk.c[1] = graph_cond(tboff + n, kGcLe64, bm_words);
+                    chk.c[2] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
+                    chk.n = 3;
+                }
                 capture_checkpoint(*rec, s, chk);
             } else {
-                CK(cudaMemcpyAsync(ctx->h_pinned, tboff + n, 8, cudaMemcpyDeviceToHost, s));
+                if (!no_rows)
+                    CK(cudaMemcpyAsync(ctx->h_pinned, tboff + n, 8, cudaMemcpyDeviceToHost, s));
                 CK(cudaMemcpyAsync((char*)ctx->h_pinned + 8, tuoff + n, 4,
                                    cudaMemcpyDeviceToHost, s));
                 read_status(ctx, s);
                 status_before_count = *ctx->h_status;
-                memcpy(&bm_words, ctx->h_pinned, 8);
+                if (!no_rows) memcpy(&bm_words, ctx->h_pinned, 8);
                 memcpy(&nunits, (char*)ctx->h_pinned + 8, 4);
                 st_flags = ctx->h_status->flags & kStatBitmapTooLarge;
                 if (recording) {
@@ -1222,7 +1241,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // 16-bit entries (positions within work units)
             compact = compact_ok;
             ta_args.compact = compact ? 1 : 0;
-            if (compact) {
+            if (compact && !no_rows) {
                 if (!ptile) ptile = ar.get<uint32_t>(n);
                 ta_args.ptile = ptile;
                 launch_tile_owner(ta_args, ptile, nb_warps, s);
@@ -1233,17 +1252,20 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 if (parts) ar.put(parts);
                 unit_cap = (uint64_t)nunits + 1;
                 unit_tile = ar.get<uint32_t>(unit_cap);
-                parts = ar.get<uint32_t>(unit_cap * kUnitQ);
+                parts = nullptr;
             }
+            if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
             ta_args.tile_uoff = tuoff;
             ta_args.nunits = tuoff + n;
             ta_args.unit_tile = unit_tile;
-            ta_args.parts = parts;
+            ta_args.parts = no_rows ? nullptr : parts;
+            ta_args.pair_sum = no_rows ? &d_st->pairs : nullptr;
             launch_unit_list(ta_args, unit_tile, nb_warps, s);
             CK(cudaMemsetAsync(deg, 0, (size_t)n * 4, s));
             ta_args.bitmap = nullptr;
             ta_args.tile_boff = tboff;
-            if (capturing) {
+            if (no_rows) {
+            } else if (capturing) {
                 // the recorded choice between the bitmap and the fill pass
                 const bool want = rec->take() != 0;
                 if (want && bm_words > bitmap_cap) {
@@ -1269,16 +1291,22 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 }
                 if (bitmap && bm_words <= bitmap_cap) ta_args.bitmap = bitmap;
             }
-            if (recording) rec->put(ta_args.bitmap ? 1 : 0);
+            if (recording && !no_rows) rec->put(ta_args.bitmap ? 1 : 0);
+            if (mixed && n >= kBoxPoints) {
+                if (!wbox) wbox = ar.get<float4>((n + 3u) / 4u);
+                ta_args.wbox = wbox;
+                launch_word_boxes(ta_args, s);
+            }
             size_t tc = 0;
             for (;;) {
                 CK(cudaMemsetAsync(tile_counter, 0, 4, s));
                 launch_count(ta_args, nb_count, s);
                 CK(cudaGetLastError());
                 tc = tm.mark();
-                scan_u32_to_u64(deg, off, n, scratch, s);
+                if (!no_rows) scan_u32_to_u64(deg, off, n, scratch, s);
                 if (capturing) break;
-                CK(cudaMemcpyAsync(ctx->h_pinned, off + n, 8, cudaMemcpyDeviceToHost, s));
+                if (!no_rows)
+                    CK(cudaMemcpyAsync(ctx->h_pinned, off + n, 8, cudaMemcpyDeviceToHost, s));
                 CK(cudaMemcpyAsync((char*)ctx->h_pinned + 8, asym_n, 4, cudaMemcpyDeviceToHost, s));
                 read_status(ctx, s);
                 if (!(ctx->h_status->flags & kStatAsymOverflow)) break;
@@ -1310,14 +1338,15 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 // pairs only if the record had some (their flag pass runs then)
                 GraphCheck chk;
                 memset(&chk, 0, sizeof chk);
-                chk.c[0] = graph_cond(off + n, kGcLe64, E, 0, &d_st->pairs);
-                chk.c[1] = graph_cond(asym_n, kGcLe32, group_asym ? asym_cap : 0u);
-                chk.c[2] = graph_cond(&d_st->flags, kGcMask32, kStatAsymOverflow, 0);
-                chk.n = 3;
+                chk.c[0] = graph_cond(asym_n, kGcLe32, group_asym ? asym_cap : 0u);
+                chk.c[1] = graph_cond(&d_st->flags, kGcMask32, kStatAsymOverflow, 0);
+                chk.n = 2;
+                if (!no_rows) chk.c[chk.n++] = graph_cond(off + n, kGcLe64, E, 0, &d_st->pairs);
                 capture_checkpoint(*rec, s, chk);
             } else {
                 check_flags(*ctx->h_status);
-                memcpy(&E, ctx->h_pinned, 8);
+                if (no_rows) E = ctx->h_status->pairs - status_before_count.pairs;
+                else memcpy(&E, ctx->h_pinned, 8);
                 memcpy(&group_asym, (char*)ctx->h_pinned + 8, 4);
                 if (recording) {
                     rec->put(E);
@@ -1327,32 +1356,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             asym_total += group_asym;
             ms_index_extra += tm.ms(ta, tb);
             ms_count += tm.ms(tb, tc);
-            // rows to write: all, or (VDB_TABLE_BORDER, cells that are
-            // cliques) those of points that are not core for the group's
-            // largest minpts: the border pulls of every minpts read only
-            // those, and off becomes the scan of their degrees
-            uint64_t Erows = E;
-            if (o.table_rows == VDB_TABLE_BORDER && clique && !slots.empty() &&
-                slots.front().second > 0) {
-                const uint64_t mp_max = slots.front().second;
-                const uint32_t lim = mp_max >= 0xffffffffull ? 0xffffffffu : (uint32_t)mp_max;
-                launch_masked_degrees(deg, n, lim, tflags, s);
-                scan_u32_to_u64(tflags, off, n, scratch, s);
-                if (capturing) {
-                    Erows = graph_table_room(rec->take(), compact ? 2 : 4, o.budget);
-                    GraphCheck chk;
-                    memset(&chk, 0, sizeof chk);
-                    chk.c[0] = graph_cond(off + n, kGcLe64, Erows);
-                    chk.n = 1;
-                    capture_checkpoint(*rec, s, chk);
-                } else {
-                    CK(cudaMemcpyAsync(ctx->h_pinned, off + n, 8, cudaMemcpyDeviceToHost, s));
-                    CK(cudaStreamSynchronize(s));
-                    memcpy(&Erows, ctx->h_pinned, 8);
-                    if (recording) rec->put(Erows);
-                }
-                ta_args.row_deg_lim = lim;
-            }
+            // rows to write: all (of 16- or 32-bit entries), or none
+            const uint64_t Erows = no_rows ? 0 : E;
             chunk_list[0].e_hi = Erows;
             // neighbour table: whole when its entries (2 or 4 bytes each)
             // fit the budget (free device memory plus blocks cached by this
@@ -1361,7 +1366,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             const uint64_t esz = compact ? 2 : 4;
             auto words_for = [&](uint64_t entries) { return (size_t)((entries * esz + 3) / 4); };
             chunked = o.budget > 0 && (int64_t)(Erows * esz) > o.budget;
-            if (!chunked && Erows * esz > nbr_cap_bytes) {
+            if (!no_rows && !chunked && Erows * esz > nbr_cap_bytes) {
                 if (nbr) ar.put(nbr);
                 nbr = nullptr;
                 nbr_cap_bytes = 0;
@@ -1399,7 +1404,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             }
             ta_args.nbr = nbr;
             table_alloc_max = std::max(table_alloc_max, nbr_cap_bytes);
-            if (!chunked) {
+            if (no_rows) {
+                chunks++;
+            } else if (!chunked) {
                 build_chunk(ta_args, chunk_list[0], group_asym);
             }
             tables++;
@@ -2318,8 +2325,8 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     MpbBox* mpb = cv.take<MpbBox>(nmpb);
     launch_mpb_boxes(x, y, vorder, n, mbb, mpb, s);
 
-    const GridParams g = make_grid(hb, eps / kCellsPerEps, 1,
-                                   kNoallocMaxCells);
+    GridParams g = make_grid(hb, eps / kCellsPerEps, 1, kNoallocMaxCells);
+    g.sub = sub_bits(g.ncells);
     const EpsParams ep = make_eps(eps, g, hb, true);
     uint32_t* gkey = cv.take<uint32_t>(n);
     uint32_t* gorig = cv.take<uint32_t>(n);
@@ -2351,7 +2358,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* pos_flag = cv.take<uint32_t>(n);
 
     launch_grid_keys(x, y, n, g, gkey, gorig, s);
-    radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1), scratch, s);
+    radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1) + 2 * (int)g.sub, scratch, s);
     launch_grid_gather(x, y, gorig, pos, n, g, gkey, gxy, glocal, gpos, s);
     launch_point_boxes(gpos, n, mpb, mbb, gbox, s);
     CK(cudaMemsetAsync(cell_start, 0xff, (g.ncells + 1) * 4, s));

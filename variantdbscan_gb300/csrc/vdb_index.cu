@@ -82,10 +82,16 @@ __global__ void mpb_kernel(const double* __restrict__ x, const double* __restric
     if (lane == 0) boxes[b] = MpbBox{x0, x1, y0, y1};
 }
 
-__device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, uint32_t nc) {
-    double f = floor(__ddiv_rn(__dsub_rn(v, v0), w));
+// Cell of v and its subcell (of 2^sub per cell), which only orders the points
+// of a cell.
+__device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, uint32_t nc,
+                                            uint32_t sub, uint32_t* sc) {
+    const double q = __ddiv_rn(__dsub_rn(v, v0), w);
+    double f = floor(q);
     if (!(f >= 0.0)) f = 0.0;
     if (f > (double)(nc - 1)) f = (double)(nc - 1);
+    const float r = (float)(q - f) * (float)(1u << sub);
+    *sc = (uint32_t)fminf(fmaxf(r, 0.f), (float)((1u << sub) - 1u));
     return (uint32_t)f;
 }
 
@@ -94,9 +100,13 @@ __global__ void grid_keys_kernel(const double* __restrict__ x, const double* __r
                                  uint32_t* __restrict__ idx) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    uint32_t cx = cell_of(x[i], g.x0, g.w, g.ncx);
-    uint32_t cy = cell_of(y[i], g.y0, g.w, g.ncy);
-    keys[i] = cy * g.ncx_pad + cx;
+    uint32_t sx = 0, sy = 0;
+    uint32_t cx = cell_of(x[i], g.x0, g.w, g.ncx, g.sub, &sx);
+    uint32_t cy = cell_of(y[i], g.y0, g.w, g.ncy, g.sub, &sy);
+    uint32_t key = cy * g.ncx_pad + cx;
+    for (int b = (int)g.sub - 1; b >= 0; b--)
+        key = (key << 2) | (((sy >> b) & 1u) << 1) | ((sx >> b) & 1u);
+    keys[i] = key;
     idx[i] = i;
 }
 
@@ -106,13 +116,17 @@ __global__ void grid_keys_kernel(const double* __restrict__ x, const double* __r
 __global__ void grid_gather_kernel(const double* __restrict__ x, const double* __restrict__ y,
                                    const uint32_t* __restrict__ gorig,
                                    const uint32_t* __restrict__ pos, uint32_t n, GridParams g,
-                                   const uint32_t* __restrict__ gkey, double2* __restrict__ gxy,
+                                   uint32_t* __restrict__ gkey, double2* __restrict__ gxy,
                                    float2* __restrict__ glocal, uint32_t* __restrict__ gpos) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     uint32_t o = gorig[k];
     double xv = x[o], yv = y[o];
     uint32_t key = gkey[k];
+    if (g.sub) {
+        key >>= 2u * g.sub;
+        gkey[k] = key;
+    }
     uint32_t cy = key / g.ncx_pad, cx = key - cy * g.ncx_pad;
     double ox = __dadd_rn(g.x0, __dmul_rn((double)cx, g.w));
     double oy = __dadd_rn(g.y0, __dmul_rn((double)cy, g.w));
@@ -297,7 +311,7 @@ void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g
 }
 
 void launch_grid_gather(const double* x, const double* y, const uint32_t* gorig,
-                        const uint32_t* pos, uint32_t n, GridParams g, const uint32_t* gkey,
+                        const uint32_t* pos, uint32_t n, GridParams g, uint32_t* gkey,
                         double2* gxy, float2* glocal, uint32_t* gpos, cudaStream_t s) {
     if (n) VDB_COUNT_LAUNCH();
     if (n)

@@ -87,7 +87,9 @@ struct GridParams {
     // 1: many more cells than points - a row directory of the non-empty
     //    cells (crow, ccx, clist) replaces it
     uint32_t sparse;
-    uint32_t pad;
+    // points are sorted by cell and, within a cell, along a Morton curve of
+    // 2^sub x 2^sub subcells (neighbours in the order are near each other)
+    uint32_t sub;
 };
 
 // Points [*s, *e) of the cells lo_c..hi_c of grid row ry (cell order).
@@ -294,8 +296,9 @@ void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g
 // gbox[k] = mpb[gpos[k] / mbb]: the multiple-point box of cell-ordered point k
 void launch_point_boxes(const uint32_t* gpos, uint32_t n, const MpbBox* mpb, int mbb,
                         MpbBox* gbox, cudaStream_t s);
+// (takes the subcell bits off gkey)
 void launch_grid_gather(const double* x, const double* y, const uint32_t* gorig,
-                        const uint32_t* pos, uint32_t n, GridParams g, const uint32_t* gkey,
+                        const uint32_t* pos, uint32_t n, GridParams g, uint32_t* gkey,
                         double2* gxy, float2* glocal, uint32_t* gpos, cudaStream_t s);
 // Row directory of a sparse grid: ccx[c] = column of non-empty cell c,
 // crow[r] = first non-empty cell of row >= r (crow[ncy] = number of cells;
@@ -353,6 +356,7 @@ struct TableArgs {
     const uint32_t* gkey;
     const float2* glocal;
     const double2* gxy;
+    float4* wbox;               // boxes of runs of points (launch_word_boxes), (n+3)/4; may be null
     const uint32_t* gpos;
     const MpbBox* gbox;         // multiple-point box of each cell-ordered point
     uint32_t n;
@@ -373,15 +377,13 @@ struct TableArgs {
     const uint32_t* tile_uoff;
     const uint32_t* nunits;         // device scalar
     uint32_t* parts;                // per unit and query slot: neighbours in that chunk
+    unsigned long long* pair_sum;   // count pass: adds the neighbours counted (nullptr: not)
     // one row chunk of the table (zero: the whole table): the fill pass takes
     // tiles from tile_lo on, the expand pass units [unit_lo, unit_hi), and the
     // asymmetric flags touch rows [row_lo, row_hi) only
     uint32_t tile_lo;
     uint32_t unit_lo, unit_hi;
     uint32_t row_lo, row_hi;
-    // nonzero: the table holds only the rows of points with deg < row_deg_lim
-    // (off is the scan of those rows' degrees); the other rows are skipped
-    uint32_t row_deg_lim;
 };
 // Work units hold 4096 candidates of a tile (kUnitWords bitmap words) or, for
 // small datasets, 1024 (kUnitWordsSmall): a warp's longest unit bounds the
@@ -434,6 +436,7 @@ static __device__ __forceinline__ void walk_compact_row(
     }
 }
 void launch_count(const TableArgs& a, int nblocks, cudaStream_t s);
+void launch_word_boxes(const TableArgs& a, cudaStream_t s);
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s);
 void launch_tile_words(const TableArgs& a, uint32_t* words, uint32_t* units, int nblocks,
                        cudaStream_t s);
@@ -441,9 +444,6 @@ void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, int nblocks, cuda
 // adds the hash of rows [row_lo, row_hi) of the table to st->table_hash
 // (gorig: input index of every cell-ordered point)
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s);
-// out[k] = deg[k] < lim ? deg[k] : 0
-void launch_masked_degrees(const uint32_t* deg, uint32_t n, uint32_t lim, uint32_t* out,
-                           cudaStream_t s);
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s);
 // ptile[k] = t for the points [tiles[t], tiles[t+1]) of every tile t
 void launch_tile_owner(const TableArgs& a, uint32_t* ptile, int nblocks, cudaStream_t s);

@@ -149,6 +149,71 @@ __device__ __forceinline__ void warp_rows(const TableArgs& a, const EpsParams* _
     __syncwarp();
 }
 
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// Records a pair accepted in one direction only (once per pair: kp < kq).
+__device__ __forceinline__ void record_one_way(const TableArgs& a, uint32_t kp, uint32_t kq,
+                                               uint32_t r) {
+    if ((r != 1u && r != 2u) || kp >= kq) return;
+    const uint32_t slot = atomicAdd(a.asym_n, 1u);
+    if (slot < a.asym_cap) {
+        AsymPair ap;
+        ap.a = kp;
+        ap.b = kq;
+        ap.dir = r;
+        ap.pad = 0u;
+        a.asym[slot] = ap;
+    } else {
+        atomicOr(&a.st->flags, kStatAsymOverflow);
+    }
+}
+
+// Tiles of at most kLaneCand queries are tested lane = candidate (a step per
+// query) instead of lane = query (a step per candidate pair): a step costs
+// about the same either way, so the lanes that a small tile leaves empty cost
+// more than they test.  FP64 tests always go lane = candidate: they are bound
+// by the FP64 pipe (2 lanes per cycle and SM), and only the last word of a
+// tile has idle lanes.
+constexpr uint32_t kLaneCand = 16;
+// Word boxes.  A run of points that are next to each other in the cell order
+// lies in a small box where the data are dense (points of a cell are ordered
+// by subcell).  box[i] bounds the points [4i, 4i + 36), relative to the cell
+// origin of point 4i, so it covers the 32 candidates of any word that starts
+// at points 4i..4i+3; x0 > x1 when the run spans two grid rows.  Tiles of at
+// least kBoxCand candidates compare each word's box with their queries' first:
+// a box wholly inside or outside eps settles 64 x 32 pairs without a test.
+constexpr uint32_t kBoxCand = 2048;
+constexpr uint32_t kBoxRun = 36;
+__global__ void word_boxes_kernel(TableArgs a) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t k0 = 4u * i;
+    if (k0 >= a.n) return;
+    const uint32_t key0 = a.gkey[k0], cy0 = key0 / a.g.ncx_pad;
+    const uint32_t e = min(k0 + kBoxRun, a.n);
+    const float wf = (float)a.g.w;
+    float4 b = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
+    if (a.gkey[e - 1] / a.g.ncx_pad == cy0) {
+        for (uint32_t k = k0; k < e; k++) {
+            const float2 loc = a.glocal[k];
+            const float x = __fmaf_rn((float)(a.gkey[k] - key0), wf, loc.x);
+            b.x = fminf(b.x, x);
+            b.y = fmaxf(b.y, x);
+            b.z = fminf(b.z, loc.y);
+            b.w = fmaxf(b.w, loc.y);
+        }
+    }
+    a.wbox[i] = b;
+}
+
 // Count pass over work units (tile, chunk of unit_words*32 candidates): adds
 // each query's neighbours in the chunk to deg, records them in parts (for the
 // table pass) and, when a.bitmap is set, stores the chunk's test bitmap
@@ -156,31 +221,24 @@ __device__ __forceinline__ void warp_rows(const TableArgs& a, const EpsParams* _
 template <bool MIXED>
 __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
     __shared__ WarpRows s_rows[kWPB];
-    __shared__ double2 s_xy[kWPB][MIXED ? 1 : kWC];
-    __shared__ uint32_t s_id[kWPB][kWC];
+    __shared__ uint32_t s_id[kWPB][MIXED ? kWC : 1];
+    // lane = query: candidate pairs (x_a, x_b, y_a, y_b); lane = candidate:
+    // queries (x, y, (L - |q|^2)/2)
     __shared__ float4 s_relp[kWPB][MIXED ? kWC / 2 : 1];
     __shared__ float2 s_hcp[kWPB][MIXED ? kWC / 2 : 1];
     // band pairs of a word are re-tested in FP64 32 at a time, whatever query
     // they belong to: queue of (query slot, candidate) entries, the queries'
     // FP64 coordinates and the accepted bits per query slot
-    __shared__ uint16_t s_rq[kWPB][kRQ];
+    __shared__ uint16_t s_rq[kWPB][MIXED ? kRQ : 1];
     __shared__ double2 s_qd[kWPB][kWQ];
-    __shared__ uint32_t s_madd[kWPB][kWQ];
+    __shared__ uint32_t s_madd[kWPB][MIXED ? kWQ : 1];
+    static_assert(kWC / 2 >= kWQ, "queries fit the candidate pairs' array");
 
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     WarpRows& rows = s_rows[wib];
-    uint16_t* rq = s_rq[wib];
     double2* sqd = s_qd[wib];
-    uint32_t* madd = s_madd[wib];
-    madd[lane] = 0u;
-    madd[lane + 32] = 0u;
-    float4* relp = s_relp[wib];
-    float2* hcp = s_hcp[wib];
-    double2* cxy = s_xy[wib];
-    uint32_t* ids = s_id[wib];
     const EpsParams* __restrict__ ep = a.ep;
-    const double eps = ep->eps, thr = ep->thr, tbox = ep->tbox;
-    const ExactBounds xb = exact_bounds(eps, thr, tbox);
+    const ExactBounds xb = exact_bounds(ep->eps, ep->thr, ep->tbox);
     const float L = ep->L32, wq = ep->w32;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
@@ -189,7 +247,11 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     const float fnan = __int_as_float(0x7fc00000);
     const double dnan = __longlong_as_double(0x7ff8000000000000ll);
-    unsigned long long my_retest = 0;
+    unsigned long long my_retest = 0, my_pairs = 0;
+    if (MIXED) {
+        s_madd[wib][lane] = 0u;
+        s_madd[wib][lane + 32] = 0u;
+    }
 
     for (;;) {
         uint32_t u = 0;
@@ -217,219 +279,388 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
         const unsigned long long bm0 = a.bitmap ? a.tile_boff[t] : 0ull;
 
         float qx[2], qy[2];
-        double2 qd[2];
-        uint32_t qk[2], cnt[2];
+        uint32_t cnt[2] = {0u, 0u};
+        const uint32_t qk[2] = {qs + (uint32_t)lane, qs + (uint32_t)lane + 32u};
 #pragma unroll
         for (int q = 0; q < 2; q++) {
-            const uint32_t k = qs + (uint32_t)lane + 32u * q;
-            qk[q] = k;
-            cnt[q] = 0;
-            if (k < qe) {
-                const float2 loc = a.glocal[k];
-                const int dcx = (int)(a.gkey[k] - tile_base);
-                qx[q] = __fmaf_rn((float)dcx, wf, loc.x);
-                qy[q] = loc.y;
-                qd[q] = a.gxy[k];
-            } else {
-                qx[q] = qy[q] = fnan;
-                qd[q] = make_double2(dnan, dnan);
+            double2 qd = make_double2(dnan, dnan);
+            qx[q] = qy[q] = fnan;
+            if (qk[q] < qe) {
+                if (MIXED) {
+                    const float2 loc = a.glocal[qk[q]];
+                    const int dcx = (int)(a.gkey[qk[q]] - tile_base);
+                    qx[q] = __fmaf_rn((float)dcx, wf, loc.x);
+                    qy[q] = loc.y;
+                }
+                qd = a.gxy[qk[q]];
             }
+            sqd[lane + 32 * q] = qd;
         }
         const bool two = Q > 32;  // second query slot used by some lane
-        sqd[lane] = qd[0];
-        sqd[lane + 32] = qd[1];
-        unsigned long long qxx[2], qyy[2], nhq2[2];
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            qxx[q] = f2_pack(qx[q], qx[q]);
-            qyy[q] = f2_pack(qy[q], qy[q]);
-            // -(|q|^2 - L)/2 (halving and negation are exact)
-            const float q2 = __fmaf_rn(qx[q], qx[q], __fmul_rn(qy[q], qy[q]));
-            const float nhq = -0.5f * __fsub_rn(q2, L);
-            nhq2[q] = f2_pack(nhq, nhq);
-        }
         // the float above w (w > 0)
         const float wup = __uint_as_float(__float_as_uint(wq) + 1u);
         const unsigned long long w2p = f2_pack(wup, wup);
 
-        for (uint32_t cb = cbeg; cb < cend; cb += kWC) {
-            const uint32_t len = min((uint32_t)kWC, cend - cb);
-#pragma unroll
-            for (int s = 0; s < kWC / 32; s++) {
-                const uint32_t j = (uint32_t)lane + 32u * s;
-                uint32_t k = 0xffffffffu;
-                int i = 0;
-                if (j < len) {
-                    k = tile_candidate(rows.start, rows.off, nrows, cb + j, &i);
-                    if (!VDB_GUARD(a.st, k < a.n, 3, k)) k = 0xffffffffu;
-                }
-                // pair slot of candidate j: (j>>5)*16 + (j&15), element j>>4 & 1
-                float* pslot = reinterpret_cast<float*>(&relp[(j >> 5) * 16 + (j & 15)]) +
-                               ((j >> 4) & 1);
-                float* hslot = reinterpret_cast<float*>(&hcp[(j >> 5) * 16 + (j & 15)]) +
-                               ((j >> 4) & 1);
-                if (k != 0xffffffffu) {
-                    if (MIXED) {
-                        const float2 loc = a.glocal[k];
-                        const int dcx = (int)(a.gkey[k] - rows.base[i]);
-                        const float rx = __fmaf_rn((float)dcx, wf, loc.x);
-                        const float ry = __fadd_rn(loc.y, rows.dyw[i]);
-                        pslot[0] = rx;
-                        pslot[2] = ry;
-                        hslot[0] = 0.5f * __fmaf_rn(rx, rx, __fmul_rn(ry, ry));
-                    } else {
-                        cxy[j] = a.gxy[k];
-                    }
-                    ids[j] = k;
-                } else {
-                    if (MIXED) {
-                        pslot[0] = fnan;
-                        pslot[2] = fnan;
-                        hslot[0] = fnan;
-                    } else {
-                        cxy[j] = make_double2(dnan, dnan);
-                    }
-                    ids[j] = 0;
-                }
-            }
+        if (!MIXED) {
             __syncwarp();
-            for (uint32_t j0 = 0; j0 < len; j0 += 32) {
-                uint32_t m[2] = {0u, 0u}, amb[2] = {0u, 0u};
-                if (MIXED) {
-                    // Candidates jj and jj+16 are tested together with packed FP32
-                    // pair instructions (each element rounds exactly like the
-                    // scalar __f*_rn operations of the fill pass); sign bits are
-                    // gathered by funnel shifts (bit 31-jj, reversed below).
-                    // nS =|c|^2/2 - (q.c - (|q|^2 - L)/2) = (d2 - L)/2: two
-                    // fma and one subtraction per test; its sign is the
-                    // in-mask.  The sign of nS - w' (w' the float above w, so
-                    // negative <=> nS <= w; a difference of floats is zero only
-                    // for equal operands, so its sign is exact) marks the tests
-                    // that are not out; band = not out and not in.  NaN (empty
-                    // query or candidate slots) has both signs clear.
-                    uint32_t ma[2] = {0u, 0u}, mb[2] = {0u, 0u}, oa[2] = {0u, 0u}, ob[2] = {0u, 0u};
-                    const ulonglong2* pr = reinterpret_cast<const ulonglong2*>(relp) + (j0 >> 5) * 16;
-                    const unsigned long long* ph =
-                        reinterpret_cast<const unsigned long long*>(hcp) + (j0 >> 5) * 16;
-#pragma unroll
-                    for (int jj = 0; jj < 16; jj++) {
-                        const ulonglong2 c = pr[jj];  // (x_a, x_b), (y_a, y_b)
-                        const unsigned long long hc = ph[jj];  // (|c_a|^2/2, |c_b|^2/2)
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            if (q == 1 && !two) break;
-                            const unsigned long long ay = f2_fma(qyy[q], c.y, nhq2[q]);
-                            const unsigned long long qc = f2_fma(qxx[q], c.x, ay);
-                            const unsigned long long s = f2_sub(hc, qc);
-                            const unsigned long long nw = f2_sub(s, w2p);
-                            ma[q] = __funnelshift_l((uint32_t)s, ma[q], 1);
-                            mb[q] = __funnelshift_l((uint32_t)(s >> 32), mb[q], 1);
-                            oa[q] = __funnelshift_l((uint32_t)nw, oa[q], 1);
-                            ob[q] = __funnelshift_l((uint32_t)(nw >> 32), ob[q], 1);
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < 2; q++) {
-                        m[q] = __brev((ma[q] << 16) | (mb[q] & 0xffffu));
-                        amb[q] = __brev((oa[q] << 16) | (ob[q] & 0xffffu)) & ~m[q];
-                    }
-                } else {
-                    uint32_t hm[2] = {0u, 0u};
-#pragma unroll
-                    for (int jj = 0; jj < 32; jj++) {
-                        const double2 c = cxy[j0 + jj];
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            if (q == 1 && !two) break;
-                            const double dx = __dsub_rn(qd[q].x, c.x);
-                            const double dy = __dsub_rn(qd[q].y, c.y);
-                            const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-                            m[q] |= (d2 <= tbox) ? (1u << jj) : 0u;
-                            hm[q] |= (d2 <= thr) ? (1u << jj) : 0u;
-                        }
-                    }
-                    amb[0] = hm[0] & ~m[0];
-                    amb[1] = hm[1] & ~m[1];
+            for (uint32_t cb = cbeg; cb < cend; cb += 32) {
+                uint32_t k = 0;
+                int i;
+                double2 cd = make_double2(dnan, dnan);
+                if (cb + (uint32_t)lane < cend) {
+                    k = tile_candidate(rows.start, rows.off, nrows, cb + (uint32_t)lane, &i);
+                    if (VDB_GUARD(a.st, k < a.n, 3, k)) cd = a.gxy[k];
                 }
-                // pairs in the band: exact FP64 predicate, 32 pairs per step
-                // of the warp (queued in shared memory, whatever their query)
-                if (__any_sync(kFull, (amb[0] | amb[1]) != 0u)) {
-                    const uint32_t c = __popc(amb[0]) + __popc(amb[1]);
-                    uint32_t incl = c;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const uint32_t v = __shfl_up_sync(kFull, incl, d);
-                        if (lane >= d) incl += v;
-                    }
-                    const uint32_t excl = incl - c;
-                    const uint32_t total = __shfl_sync(kFull, incl, 31);
-                    for (uint32_t pb = 0; pb < total; pb += kRQ) {
-                        uint32_t idx = excl;
-#pragma unroll
-                        for (int q = 0; q < 2; q++) {
-                            for (uint32_t bits = amb[q]; bits; bits &= bits - 1u, idx++) {
-                                if (idx >= pb && idx < pb + kRQ)
-                                    rq[idx - pb] = (uint16_t)(((uint32_t)lane << 6) |
-                                                              ((uint32_t)q << 5) |
-                                                              (uint32_t)(__ffs(bits) - 1));
-                            }
-                        }
-                        __syncwarp();
-                        const uint32_t ne = min((uint32_t)kRQ, total - pb);
-                        for (uint32_t e = lane; e < ne; e += 32) {
-                            const uint32_t ent = rq[e];
-                            const uint32_t slot_q = (ent >> 6) + 32u * ((ent >> 5) & 1u);
-                            const uint32_t jj = ent & 31u;
-                            const uint32_t kp = qs + slot_q;
-                            const uint32_t kq = ids[j0 + jj];
-                            const uint32_t r =
-                                exact_pair(sqd[slot_q], a.gxy[kq], kp, kq, xb, a.gbox);
+                uint32_t w[2] = {0u, 0u};
+                auto step = [&](uint32_t q, uint32_t* word) {
+                    // d2 is >= +0 or NaN; compared as ordered integers
+                    // (ExactBounds), NaN by its bits above those of infinity
+                    const double2 qd = sqd[q];
+                    const double dx = __dsub_rn(qd.x, cd.x), dy = __dsub_rn(qd.y, cd.y);
+                    const long long d2b =
+                        __double_as_longlong(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)));
+                    const bool num = (unsigned long long)d2b <= 0x7ff0000000000000ull;
+                    bool in = num && d2b <= xb.tbox;
+                    const bool band = num && !in && d2b <= xb.thr;
+                    if (__any_sync(kFull, band)) {
+                        if (band) {
+                            const uint32_t r = exact_pair(qd, cd, qs + q, k, xb, a.gbox);
                             my_retest++;
-                            if (r & 1u) atomicOr(&madd[slot_q], 1u << jj);
-                            if ((r == 1u || r == 2u) && kp < kq) {
-                                const uint32_t slot = atomicAdd(a.asym_n, 1u);
-                                if (slot < a.asym_cap) {
-                                    AsymPair ap;
-                                    ap.a = kp;
-                                    ap.b = kq;
-                                    ap.dir = r;
-                                    ap.pad = 0u;
-                                    a.asym[slot] = ap;
-                                } else {
-                                    atomicOr(&a.st->flags, kStatAsymOverflow);
-                                }
-                            }
+                            in = (r & 1u) != 0u;
+                            record_one_way(a, qs + q, k, r);
                         }
-                        __syncwarp();
                     }
-                    m[0] |= madd[lane];
-                    m[1] |= madd[lane + 32];
-                    madd[lane] = 0u;
-                    madd[lane + 32] = 0u;
-                    __syncwarp();
-                }
-                const unsigned long long wrow = bm0 + (unsigned long long)((cb + j0) >> 5) * Q;
+                    const uint32_t m = __ballot_sync(kFull, in);
+                    if ((uint32_t)lane == (q & 31u)) *word = m;
+                };
+                for (uint32_t q = 0; q < min(Q, 32u); q++) step(q, &w[0]);
+                for (uint32_t q = 32; q < Q; q++) step(q, &w[1]);
+                const unsigned long long wrow = bm0 + (unsigned long long)(cb >> 5) * Q;
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
                     if (qk[q] < qe) {
-                        cnt[q] += __popc(m[q]);
-                        if (a.bitmap) a.bitmap[wrow + (qk[q] - qs)] = m[q];
+                        cnt[q] += __popc(w[q]);
+                        if (a.bitmap) a.bitmap[wrow + (qk[q] - qs)] = w[q];
                     }
                 }
             }
             __syncwarp();
+        } else if (Q <= kLaneCand) {
+            float4* sq = s_relp[wib];
+            if ((uint32_t)lane < Q) {
+                const float q2 = __fmaf_rn(qx[0], qx[0], __fmul_rn(qy[0], qy[0]));
+                sq[lane] = make_float4(qx[0], qy[0], -0.5f * __fsub_rn(q2, L), 0.f);
+            }
+            __syncwarp();
+            for (uint32_t cb = cbeg; cb < cend; cb += kWC) {
+                // this lane's four candidates (words s = 0..3)
+                unsigned long long X[2], Y[2], H[2];
+                uint32_t id[4];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    float rx[2], ry[2], hc[2];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const uint32_t g = cb + 32u * (2 * h + e) + (uint32_t)lane;
+                        rx[e] = ry[e] = hc[e] = fnan;
+                        id[2 * h + e] = 0;
+                        if (g < cend) {
+                            int i;
+                            const uint32_t k = tile_candidate(rows.start, rows.off, nrows, g, &i);
+                            if (VDB_GUARD(a.st, k < a.n, 3, k)) {
+                                const float2 loc = a.glocal[k];
+                                const int dcx = (int)(a.gkey[k] - rows.base[i]);
+                                rx[e] = __fmaf_rn((float)dcx, wf, loc.x);
+                                ry[e] = __fadd_rn(loc.y, rows.dyw[i]);
+                                hc[e] = 0.5f * __fmaf_rn(rx[e], rx[e], __fmul_rn(ry[e], ry[e]));
+                                id[2 * h + e] = k;
+                            }
+                        }
+                    }
+                    X[h] = f2_pack(rx[0], rx[1]);
+                    Y[h] = f2_pack(ry[0], ry[1]);
+                    H[h] = f2_pack(hc[0], hc[1]);
+                }
+                const uint32_t nwv = (min((uint32_t)kWC, cend - cb) + 31u) >> 5;
+                uint32_t w[4] = {0u, 0u, 0u, 0u};
+                for (uint32_t q = 0; q < Q; q++) {
+                    const float4 Qv = sq[q];
+                    const unsigned long long qxx = f2_pack(Qv.x, Qv.x), qyy = f2_pack(Qv.y, Qv.y),
+                                             nh = f2_pack(Qv.z, Qv.z);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        if (h == 1 && nwv <= 2) break;
+                        // the filter of the lane = query form below, two words at a time
+                        const unsigned long long s =
+                            f2_sub(H[h], f2_fma(qxx, X[h], f2_fma(qyy, Y[h], nh)));
+                        const unsigned long long nwm = f2_sub(s, w2p);
+                        bool in0 = (int)(uint32_t)s < 0, in1 = (int)(uint32_t)(s >> 32) < 0;
+                        const bool b0 = !in0 && (int)(uint32_t)nwm < 0;
+                        const bool b1 = !in1 && (int)(uint32_t)(nwm >> 32) < 0;
+                        if (__any_sync(kFull, b0 || b1)) {
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                if (e ? b1 : b0) {
+                                    const uint32_t k = id[2 * h + e];
+                                    const uint32_t r = exact_pair(sqd[q], a.gxy[k], qs + q, k, xb, a.gbox);
+                                    my_retest++;
+                                    (e ? in1 : in0) = (r & 1u) != 0u;
+                                    record_one_way(a, qs + q, k, r);
+                                }
+                            }
+                        }
+                        const uint32_t m0 = __ballot_sync(kFull, in0), m1 = __ballot_sync(kFull, in1);
+                        if ((uint32_t)lane == q) {
+                            w[2 * h] = m0;
+                            w[2 * h + 1] = m1;
+                        }
+                    }
+                }
+                if ((uint32_t)lane < Q) {
+                    const unsigned long long wrow = bm0 + (unsigned long long)(cb >> 5) * Q + (uint32_t)lane;
+#pragma unroll
+                    for (int s = 0; s < 4; s++) {
+                        cnt[0] += __popc(w[s]);
+                        if (a.bitmap && (uint32_t)s < nwv) a.bitmap[wrow + (unsigned long long)s * Q] = w[s];
+                    }
+                }
+            }
+            __syncwarp();
+        } else {
+            uint16_t* rq = s_rq[wib];
+            uint32_t* madd = s_madd[wib];
+            float4* relp = s_relp[wib];
+            float2* hcp = s_hcp[wib];
+            uint32_t* ids = s_id[wib];
+            unsigned long long qxx[2], qyy[2], nhq2[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                qxx[q] = f2_pack(qx[q], qx[q]);
+                qyy[q] = f2_pack(qy[q], qy[q]);
+                // -(|q|^2 - L)/2 (halving and negation are exact)
+                const float q2 = __fmaf_rn(qx[q], qx[q], __fmul_rn(qy[q], qy[q]));
+                const float nhq = -0.5f * __fsub_rn(q2, L);
+                nhq2[q] = f2_pack(nhq, nhq);
+            }
+            const bool boxes = a.wbox && C >= kBoxCand;
+            float bx0 = 0.f, bx1 = 0.f, by0 = 0.f, by1 = 0.f;  // the queries' box (fmin/fmax skip NaN)
+            float pad = 0.f;  // more than the roundings of a box's edges (16 of them)
+            if (boxes) {
+                bx0 = warp_min(fminf(qx[0], qx[1]));
+                bx1 = warp_max(fmaxf(qx[0], qx[1]));
+                by0 = warp_min(fminf(qy[0], qy[1]));
+                by1 = warp_max(fmaxf(qy[0], qy[1]));
+                pad = 0x1p-20f * wf * (float)((int)G + 2 * ep->reach[rho] + 4);
+            }
+
+            // blocks of 32 words: lane l looks at word wb + l
+            for (uint32_t wb = cbeg >> 5; wb * 32u < cend; wb += 32) {
+                const uint32_t nwb = min(32u, ((cend + 31u) >> 5) - wb);
+                uint32_t todo = nwb >= 32u ? kFull : (1u << nwb) - 1u;  // words to test
+                if (boxes) {
+                    bool in = false, out = false;
+                    const uint32_t g0 = (wb + (uint32_t)lane) * 32u, g1 = min(g0 + 32u, cend);
+                    if ((uint32_t)lane < nwb) {
+                        int i;
+                        const uint32_t k = tile_candidate(rows.start, rows.off, nrows, g0, &i);
+                        if (g1 <= rows.off[i + 1] && VDB_GUARD(a.st, k < a.n, 3, k)) {
+                            const float4 b = a.wbox[k >> 2];
+                            if (b.x <= b.y) {
+                                // Rounding is monotone: the largest |q - c| per
+                                // axis, rounded, is at least every rounded
+                                // |q - c|, and its FP32 d2 at least every
+                                // pair's; the smallest likewise.  So d2max <
+                                // lo32 (d2min > hi32) decides all pairs of the
+                                // two boxes as their own FP32 d2 would.
+                                const float dcx = (float)(int)(a.gkey[k & ~3u] - rows.base[i]);
+                                const float x0 = __fmaf_rn(dcx, wf, b.x) - pad;
+                                const float x1 = __fmaf_rn(dcx, wf, b.y) + pad;
+                                const float y0 = b.z + rows.dyw[i] - pad, y1 = b.w + rows.dyw[i] + pad;
+                                const float mx = fmaxf(__fsub_rn(x1, bx0), __fsub_rn(bx1, x0));
+                                const float my = fmaxf(__fsub_rn(y1, by0), __fsub_rn(by1, y0));
+                                const float nx = fmaxf(fmaxf(__fsub_rn(x0, bx1), __fsub_rn(bx0, x1)), 0.f);
+                                const float ny = fmaxf(fmaxf(__fsub_rn(y0, by1), __fsub_rn(by0, y1)), 0.f);
+                                in = __fmaf_rn(mx, mx, __fmul_rn(my, my)) < ep->lo32;
+                                out = __fmaf_rn(nx, nx, __fmul_rn(ny, ny)) > ep->hi32;
+                            }
+                        }
+                    }
+                    const uint32_t mi = __ballot_sync(kFull, in), mo = __ballot_sync(kFull, out);
+                    todo &= ~(mi | mo);
+                    const uint32_t add = __reduce_add_sync(kFull, in ? g1 - g0 : 0u);
+                    if (qk[0] < qe) cnt[0] += add;
+                    if (qk[1] < qe) cnt[1] += add;
+                    if (a.bitmap) {
+                        for (uint32_t l = mi | mo; l; l &= l - 1u) {
+                            const uint32_t w = (uint32_t)__ffs(l) - 1u, word = wb + w;
+                            const uint32_t left = cend - word * 32u;
+                            const uint32_t m = !((mi >> w) & 1u) ? 0u
+                                               : left >= 32u     ? kFull
+                                                                 : (1u << left) - 1u;
+                            const unsigned long long wrow = bm0 + (unsigned long long)word * Q;
+                            if (qk[0] < qe) a.bitmap[wrow + (qk[0] - qs)] = m;
+                            if (qk[1] < qe) a.bitmap[wrow + (qk[1] - qs)] = m;
+                        }
+                    }
+                }
+                while (todo) {
+                // the next (up to) four words
+                uint32_t word[kWC / 32];
+                uint32_t nst = 0;
+#pragma unroll
+                for (int s = 0; s < kWC / 32; s++) {
+                    word[s] = 0xffffffffu;
+                    if (todo) {
+                        word[s] = wb + (uint32_t)__ffs(todo) - 1u;
+                        todo &= todo - 1u;
+                        nst = (uint32_t)s + 1u;
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < kWC / 32; s++) {
+                    const uint32_t j = (uint32_t)lane + 32u * s;
+                    const uint32_t cg = word[s] * 32u + (uint32_t)lane;
+                    uint32_t k = 0;
+                    float rx = fnan, ry = fnan;
+                    if (word[s] != 0xffffffffu && cg < cend) {
+                        int i;
+                        k = tile_candidate(rows.start, rows.off, nrows, cg, &i);
+                        if (VDB_GUARD(a.st, k < a.n, 3, k)) {
+                            const float2 loc = a.glocal[k];
+                            const int dcx = (int)(a.gkey[k] - rows.base[i]);
+                            rx = __fmaf_rn((float)dcx, wf, loc.x);
+                            ry = __fadd_rn(loc.y, rows.dyw[i]);
+                        } else {
+                            k = 0;
+                        }
+                    }
+                    // pair slot of candidate j: (j>>5)*16 + (j&15), element j>>4 & 1
+                    float* pslot = reinterpret_cast<float*>(&relp[(j >> 5) * 16 + (j & 15)]) +
+                                   ((j >> 4) & 1);
+                    float* hslot = reinterpret_cast<float*>(&hcp[(j >> 5) * 16 + (j & 15)]) +
+                                   ((j >> 4) & 1);
+                    pslot[0] = rx;
+                    pslot[2] = ry;
+                    hslot[0] = 0.5f * __fmaf_rn(rx, rx, __fmul_rn(ry, ry));
+                    ids[j] = k;
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t j0 = 0; j0 < nst * 32u; j0 += 32) {
+                    uint32_t m[2] = {0u, 0u}, amb[2] = {0u, 0u};
+                    {
+                        // Candidates jj and jj+16 are tested together with packed FP32
+                        // pair instructions; sign bits are gathered by funnel shifts
+                        // (bit 31-jj, reversed below).
+                        // nS =|c|^2/2 - (q.c - (|q|^2 - L)/2) = (d2 - L)/2: two
+                        // fma and one subtraction per test; its sign is the
+                        // in-mask.  The sign of nS - w' (w' the float above w, so
+                        // negative <=> nS <= w; a difference of floats is zero only
+                        // for equal operands, so its sign is exact) marks the tests
+                        // that are not out; band = not out and not in.  NaN (empty
+                        // query or candidate slots) has both signs clear.
+                        uint32_t ma[2] = {0u, 0u}, mb[2] = {0u, 0u}, oa[2] = {0u, 0u}, ob[2] = {0u, 0u};
+                        const ulonglong2* pr = reinterpret_cast<const ulonglong2*>(relp) + (j0 >> 5) * 16;
+                        const unsigned long long* ph =
+                            reinterpret_cast<const unsigned long long*>(hcp) + (j0 >> 5) * 16;
+#pragma unroll
+                        for (int jj = 0; jj < 16; jj++) {
+                            const ulonglong2 c = pr[jj];  // (x_a, x_b), (y_a, y_b)
+                            const unsigned long long hc = ph[jj];  // (|c_a|^2/2, |c_b|^2/2)
+#pragma unroll
+                            for (int q = 0; q < 2; q++) {
+                                if (q == 1 && !two) break;
+                                const unsigned long long ay = f2_fma(qyy[q], c.y, nhq2[q]);
+                                const unsigned long long qc = f2_fma(qxx[q], c.x, ay);
+                                const unsigned long long s = f2_sub(hc, qc);
+                                const unsigned long long nw = f2_sub(s, w2p);
+                                ma[q] = __funnelshift_l((uint32_t)s, ma[q], 1);
+                                mb[q] = __funnelshift_l((uint32_t)(s >> 32), mb[q], 1);
+                                oa[q] = __funnelshift_l((uint32_t)nw, oa[q], 1);
+                                ob[q] = __funnelshift_l((uint32_t)(nw >> 32), ob[q], 1);
+                            }
+                        }
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            m[q] = __brev((ma[q] << 16) | (mb[q] & 0xffffu));
+                            amb[q] = __brev((oa[q] << 16) | (ob[q] & 0xffffu)) & ~m[q];
+                        }
+                        // pairs in the band: exact FP64 predicate, 32 pairs per step
+                        // of the warp (queued in shared memory, whatever their query)
+                        if (__any_sync(kFull, (amb[0] | amb[1]) != 0u)) {
+                            const uint32_t c = __popc(amb[0]) + __popc(amb[1]);
+                            uint32_t incl = c;
+#pragma unroll
+                            for (int d = 1; d < 32; d <<= 1) {
+                                const uint32_t v = __shfl_up_sync(kFull, incl, d);
+                                if (lane >= d) incl += v;
+                            }
+                            const uint32_t excl = incl - c;
+                            const uint32_t total = __shfl_sync(kFull, incl, 31);
+                            for (uint32_t pb = 0; pb < total; pb += kRQ) {
+                                uint32_t idx = excl;
+#pragma unroll
+                                for (int q = 0; q < 2; q++) {
+                                    for (uint32_t bits = amb[q]; bits; bits &= bits - 1u, idx++) {
+                                        if (idx >= pb && idx < pb + kRQ)
+                                            rq[idx - pb] = (uint16_t)(((uint32_t)lane << 6) |
+                                                                      ((uint32_t)q << 5) |
+                                                                      (uint32_t)(__ffs(bits) - 1));
+                                    }
+                                }
+                                __syncwarp();
+                                const uint32_t ne = min((uint32_t)kRQ, total - pb);
+                                for (uint32_t e = lane; e < ne; e += 32) {
+                                    const uint32_t ent = rq[e];
+                                    const uint32_t slot_q = (ent >> 6) + 32u * ((ent >> 5) & 1u);
+                                    const uint32_t jj = ent & 31u;
+                                    const uint32_t kp = qs + slot_q;
+                                    const uint32_t kq = ids[j0 + jj];
+                                    const uint32_t r =
+                                        exact_pair(sqd[slot_q], a.gxy[kq], kp, kq, xb, a.gbox);
+                                    my_retest++;
+                                    if (r & 1u) atomicOr(&madd[slot_q], 1u << jj);
+                                    record_one_way(a, kp, kq, r);
+                                }
+                                __syncwarp();
+                            }
+                            m[0] |= madd[lane];
+                            m[1] |= madd[lane + 32];
+                            madd[lane] = 0u;
+                            madd[lane + 32] = 0u;
+                            __syncwarp();
+                        }
+                    }
+                    const uint32_t wj = j0 == 0 ? word[0] : j0 == 32 ? word[1] : j0 == 64 ? word[2] : word[3];
+                    const unsigned long long wrow = bm0 + (unsigned long long)wj * Q;
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        if (qk[q] < qe) {
+                            cnt[q] += __popc(m[q]);
+                            if (a.bitmap) a.bitmap[wrow + (qk[q] - qs)] = m[q];
+                        }
+                    }
+                }
+                __syncwarp();
+                }
+            }
         }
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             if (qk[q] < qe) {
                 if (cnt[q]) atomicAdd(&a.deg[qk[q]], cnt[q]);
                 if (a.parts) a.parts[(unsigned long long)u * kUnitQ + lane + 32u * q] = cnt[q];
+                my_pairs += cnt[q];
             }
         }
     }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) my_retest += __shfl_down_sync(kFull, my_retest, d);
+    for (int d = 16; d > 0; d >>= 1) {
+        my_retest += __shfl_down_sync(kFull, my_retest, d);
+        my_pairs += __shfl_down_sync(kFull, my_pairs, d);
+    }
     if (lane == 0 && my_retest) atomicAdd(&a.st->retested, my_retest);
+    if (lane == 0 && my_pairs && a.pair_sum) atomicAdd(a.pair_sum, my_pairs);
 }
 
 // Table pass over the same work units: neighbour ids from the count pass's
@@ -547,11 +778,6 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
         const unsigned long long bm0 = a.tile_boff[t];
         // row cursors: lane l holds queries l and l+32
         const bool v0 = qs + lane < qe, v1 = qs + lane + 32 < qe;
-        // rows written: all, or (row_deg_lim) those of points with deg < lim
-        const uint32_t lim = a.row_deg_lim;
-        const bool w0row = v0 && (!lim || a.deg[qs + lane] < lim);
-        const bool w1row = v1 && (!lim || a.deg[qs + lane + 32] < lim);
-        if (!__any_sync(kFull, w0row || w1row)) continue;
         unsigned long long cur0 = v0 ? a.off[qs + lane] - a.off_base : 0;
         unsigned long long cur1 = v1 ? a.off[qs + lane + 32] - a.off_base : 0;
         for (uint32_t uu = u0; uu < u; uu++) {
@@ -583,7 +809,7 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
             for (uint32_t qh = 0; qh < Q; qh += 32) {
                 const uint32_t q = qh + (uint32_t)lane;
                 __syncwarp();  // the previous slots have been read
-                const bool wrow = qh == 0 ? w0row : w1row;
+                const bool wrow = qh == 0 ? v0 : v1;
                 uint32_t todo = __ballot_sync(kFull, wrow);  // queries whose rows are written
                 if (wrow) {
                     uint32_t wd[kWXW], pm[kWXW];
@@ -760,10 +986,6 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
         const uint32_t wend = min(words, wbeg + a.unit_words);
         const unsigned long long bm0 = a.tile_boff[t];
         const bool v0 = qs + lane < qe, v1 = qs + lane + 32 < qe;
-        const uint32_t lim = a.row_deg_lim;
-        const bool w0row = v0 && (!lim || a.deg[qs + lane] < lim);
-        const bool w1row = v1 && (!lim || a.deg[qs + lane + 32] < lim);
-        if (!__any_sync(kFull, w0row || w1row)) continue;
         unsigned long long cur0 = v0 ? a.off[qs + lane] - a.off_base : 0;
         unsigned long long cur1 = v1 ? a.off[qs + lane + 32] - a.off_base : 0;
         for (uint32_t uu = u0; uu < u; uu++) {
@@ -781,7 +1003,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
             for (uint32_t qh = 0; qh < Q; qh += 32) {
                 const uint32_t q = qh + (uint32_t)lane;
                 __syncwarp();  // the previous slots have been read
-                const bool wrow = qh == 0 ? w0row : w1row;
+                const bool wrow = qh == 0 ? v0 : v1;
                 uint32_t todo = __ballot_sync(kFull, wrow);
                 if (wrow) {
                     uint32_t wd[kWXW], pm[kWXW];
@@ -963,14 +1185,12 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
         double2 qd[kQPT];
         uint32_t qk[kQPT], cnt[kQPT];
         unsigned long long cur[kQPT], rend[kQPT];
-        bool wr[kQPT];
 #pragma unroll
         for (int q = 0; q < kQPT; q++) {
             const uint32_t k = qs + (uint32_t)tid * kQPT + q;
             qk[q] = k;
             cnt[q] = 0;
             cur[q] = rend[q] = 0;
-            wr[q] = false;
             if (k < qe) {
                 const float2 loc = a.glocal[k];
                 const int dcx = (int)(a.gkey[k] - tile_base);
@@ -980,8 +1200,6 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
                 if (FILL) {
                     cur[q] = a.off[k] - a.off_base;
                     rend[q] = a.off[k + 1] - a.off_base;
-                    // rows of points with deg >= row_deg_lim are not written
-                    wr[q] = !a.row_deg_lim || a.deg[k] < a.row_deg_lim;
                 }
             } else {
                 qx[q] = qy[q] = __int_as_float(0x7fc00000);
@@ -1088,7 +1306,7 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
                 if (FILL) {
 #pragma unroll
                     for (int q = 0; q < kQPT; q++) {
-                        uint32_t act = __ballot_sync(kFull, m[q] != 0u && wr[q]);
+                        uint32_t act = __ballot_sync(kFull, m[q] != 0u);
                         while (act) {
                             const int src = __ffs(act) - 1;
                             act &= act - 1u;
@@ -1194,12 +1412,6 @@ __global__ void tile_owner_kernel(TableArgs a, uint32_t* __restrict__ ptile) {
     }
 }
 
-__global__ void masked_degrees_kernel(const uint32_t* __restrict__ deg, uint32_t n, uint32_t lim,
-                                      uint32_t* __restrict__ out) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) out[k] = deg[k] < lim ? deg[k] : 0u;
-}
-
 // unit_tile[u] = t for the units [tile_uoff[t], tile_uoff[t+1]) of tile t.
 __global__ void unit_list_kernel(TableArgs a, uint32_t* unit_tile) {
     const uint32_t lane = threadIdx.x & 31;
@@ -1270,7 +1482,6 @@ __global__ void asym_flags_kernel(TableArgs a) {
         const uint32_t row = p.dir == 1u ? p.a : p.b;
         const uint32_t target = p.dir == 1u ? p.b : p.a;
         if (a.row_hi && (row < a.row_lo || row >= a.row_hi)) continue;  // row not in this chunk
-        if (a.row_deg_lim && a.deg[row] >= a.row_deg_lim) continue;     // row not written
         unsigned long long lo = a.off[row] - a.off_base, hi = a.off[row + 1] - a.off_base;
         const unsigned long long end = hi;
         if (a.compact) {
@@ -1332,6 +1543,12 @@ void launch_count(const TableArgs& a, int nblocks, cudaStream_t s) {
         count_kernel<false><<<nblocks, kWPB * 32, 0, s>>>(a);
 }
 
+void launch_word_boxes(const TableArgs& a, cudaStream_t s) {
+    const uint32_t nb = (a.n + 3u) / 4u;
+    VDB_COUNT_LAUNCH();
+    word_boxes_kernel<<<(nb + kTT - 1) / kTT, kTT, 0, s>>>(a);
+}
+
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s) {
     VDB_COUNT_LAUNCH();
     if (a.mixed)
@@ -1349,13 +1566,6 @@ void launch_tile_words(const TableArgs& a, uint32_t* words, uint32_t* units, int
 void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, int nblocks, cudaStream_t s) {
     VDB_COUNT_LAUNCH();
     unit_list_kernel<<<nblocks, kTT, 0, s>>>(a, unit_tile);
-}
-
-void launch_masked_degrees(const uint32_t* deg, uint32_t n, uint32_t lim, uint32_t* out,
-                           cudaStream_t s) {
-    if (!n) return;
-    VDB_COUNT_LAUNCH();
-    masked_degrees_kernel<<<(n + kTT - 1) / kTT, kTT, 0, s>>>(deg, n, lim, out);
 }
 
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
