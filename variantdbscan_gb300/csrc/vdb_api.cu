@@ -274,12 +274,37 @@ int bits_for(uint64_t v) {
     return b;
 }
 
-// Subcell bits per axis that the sort key has room for without another 8-bit
-// pass of the sort: they order the points of a cell, nothing depends on them.
+// Subcell bits per axis that the sort key has room for without another pass
+// of the sort: they order the points of a cell, nothing depends on them.
 uint32_t sub_bits(uint64_t ncells) {
     const int kb = bits_for(ncells - 1);
-    return (uint32_t)std::min(3, ((kb + 7) / 8 * 8 - kb) / 2);
+    return (uint32_t)std::min(3, (std::min(32, sort_passes(kb) * kDigitBits) - kb) / 2);
 }
+
+// Zeroed device memory, carved in 256-byte pieces: first measured (base null),
+// then taken.
+struct ZeroCarve {
+    char* base;
+    size_t used;
+    void* take(size_t bytes) {
+        void* p = base ? base + used : nullptr;
+        used += (bytes + 255) & ~(size_t)255;
+        return p;
+    }
+};
+// The zeroed memory of one epsilon: look-back states and counters.
+struct GroupZero {
+    uint32_t* counts;   // asym_n, count and expand tile counters
+    void *sort, *order, *tiles, *words, *off;
+    GroupZero(ZeroCarve& z, uint32_t n, bool with_sort) {
+        counts = (uint32_t*)z.take(4 * sizeof(uint32_t));
+        order = z.take(order_state_bytes(n));
+        tiles = z.take(order_state_bytes(n));
+        words = z.take(words_state_bytes(n));
+        off = z.take(scan_state_bytes(n));
+        sort = with_sort ? z.take(sort_zero_bytes(n, 32)) : nullptr;
+    }
+};
 
 // Distance-test parameters of eps on grid g.  Cells (i, j) relative to a query
 // cell are scanned when their nearest points can be within eps:
@@ -527,7 +552,7 @@ struct RowChunk {
 
 // Union-find state of one variant.
 struct UfState {
-    uint32_t *parent, *seed, *cstart, *best, *cluster_no, *pos_flag;
+    uint32_t *parent, *seed, *cstart, *best, *bits, *brank;
 };
 
 // Splits the table into row chunks of whole tiles holding at most cap
@@ -739,15 +764,23 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     }
     uint32_t* labels = host ? ar.get<uint32_t>((size_t)n * V) : ds.labels;
 
-    // scratch sized for the largest primitive call
-    size_t scr = std::max({radix_sort_scratch_bytes(n), scan_u32_to_u64_scratch_bytes(n + 1),
-                           bbox_scratch_bytes(n),
-                           resolve_scratch_bytes() + scan_u32_scratch_bytes(n)});
+    // scratch of the sorts, the box and the one-way edges' components
+    const size_t scr = std::max({sort_scratch_bytes(n), bbox_scratch_bytes(), resolve_scratch_bytes()});
     char* scratch = ar.get<char>(scr);
+    // memory that the look-back kernels want zeroed: once for the visit order,
+    // then for every epsilon
+    size_t zero_bytes = 0;
+    {
+        ZeroCarve z{nullptr, 0};
+        GroupZero gz(z, n, true);
+        zero_bytes = std::max(z.used, 256 + sort_zero_bytes(n, kVisitBits));
+    }
+    char* zeroed = ar.get<char>(zero_bytes);
 
     CK(cudaMemsetAsync(d_st, 0, sizeof(DeviceStatus), s));
+    CK(cudaMemsetAsync(zeroed, 0, 256 + sort_zero_bytes(n, kVisitBits), s));
     BBox* d_bb = ar.get<BBox>(1);
-    launch_bbox(x, y, n, d_bb, scratch, s);
+    launch_bbox(x, y, n, d_bb, scratch, (uint32_t*)zeroed, s);
     if (!capturing) {
         CK(cudaMemcpyAsync(ctx->h_pinned, d_bb, sizeof(BBox), cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->box_ready, s));
@@ -761,9 +794,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* pos = ar.get<uint32_t>(n);
     const uint32_t nmpb = (uint32_t)(((uint64_t)n + (uint32_t)ds.mbb_size - 1) / (uint32_t)ds.mbb_size);
     MpbBox* mpb = ar.get<MpbBox>(nmpb);
-    launch_visit_keys(x, y, n, d_bb, vkey, vorder, d_st, s);
-    radix_sort_pairs(vkey, vorder, n, bits_for(kVisitBins * kVisitBins - 1), scratch, s);
-    launch_invert(vorder, n, pos, s);
+    launch_visit_keys(x, y, n, d_bb, vkey, (uint32_t*)(zeroed + 256), d_st, s);
+    radix_sort(vkey, n, kVisitBits, 0, zeroed + 256, scratch, nullptr, vorder, pos, d_st, s);
     launch_mpb_boxes(x, y, vorder, n, ds.mbb_size, mpb, s);
     BBox hb_ref;
     memset(&hb_ref, 0, sizeof hb_ref);
@@ -807,7 +839,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     }
     if (hb_ref.nonfinite) throw VdbError{VDB_ERR_INVALID_ARG, "non-finite coordinate"};
     HostBox hb{hb_ref.minx, hb_ref.tmaxx, hb_ref.miny, hb_ref.tmaxy};
-    ar.put(vkey);
+    uint32_t* const skey = vkey;  // unsorted cell keys of each epsilon
 
     // variant groups
     std::vector<Group> groups;
@@ -857,14 +889,21 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         u.seed = ar.get<uint32_t>(n);
         u.cstart = ar.get<uint32_t>(n);
         u.best = ar.get<uint32_t>(n);
-        u.cluster_no = ar.get<uint32_t>((size_t)n + 1);
-        u.pos_flag = ar.get<uint32_t>(n);
+        u.bits = ar.get<uint32_t>(nw);
+        u.brank = ar.get<uint32_t>(nw);
         return u;
     };
     uint32_t asym_cap = kAsymCap;  // grows when a count pass finds more one-way pairs
     AsymPair* asym = ar.get<AsymPair>(asym_cap);
-    uint32_t* asym_n = ar.get<uint32_t>(4);
-    uint32_t* tile_counter = asym_n + 1;
+    ZeroCarve zc{zeroed, 0};
+    const GroupZero gz(zc, n, true);
+    uint32_t* asym_n = gz.counts;
+    uint32_t* count_counter = asym_n + 1;  // next unit of the count pass
+    uint32_t* table_counter = asym_n + 2;  // next unit (tile) of the table pass
+    unsigned long long* d_totals = ar.get<unsigned long long>(4);
+    unsigned long long* d_nwords = d_totals;            // bitmap words
+    uint32_t* d_nunits = (uint32_t*)(d_totals + 1);     // work units
+    uint32_t* d_ntiles = (uint32_t*)(d_totals + 2);
     EpsParams* d_ep = ar.get<EpsParams>(1);
     unsigned long long* tune_sums = ar.get<unsigned long long>(2 * kTuneShapes);
     uint32_t tile_cells_hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // tables per log2(G)
@@ -874,13 +913,13 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     float2* glocal = ar.get<float2>(n);
     uint32_t* gpos = ar.get<uint32_t>(n);
     MpbBox* gbox = ar.get<MpbBox>(n);
-    uint32_t* tflags = ar.get<uint32_t>(n);
-    uint32_t* tscan = ar.get<uint32_t>((size_t)n + 1);
     uint32_t* tiles = ar.get<uint32_t>((size_t)n + 1);
+    uint32_t* ptile = ar.get<uint32_t>(n);  // tile of every cell-ordered point
     uint32_t* cscan = ar.get<uint32_t>((size_t)n + 1);
     uint32_t* clist = ar.get<uint32_t>((size_t)n + 1);
+    uint32_t* ckey = ar.get<uint32_t>(n);  // keys and columns of the non-empty cells
+    uint32_t* ccx = ar.get<uint32_t>(n);
     unsigned long long* tboff = ar.get<unsigned long long>((size_t)n + 1);
-    uint32_t* tunits = ar.get<uint32_t>(n);
     uint32_t* tuoff = ar.get<uint32_t>((size_t)n + 1);
     float4* wbox = nullptr;  // boxes of runs of points
     uint32_t* bitmap = nullptr;
@@ -891,12 +930,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* nbr = nullptr;
     size_t nbr_cap_bytes = 0;
     size_t table_alloc_max = 0;  // largest neighbour-table (or chunk) allocation
-    uint32_t* ptile = nullptr;  // compact tables: tile of every cell-ordered point
     uint32_t* cell_start = nullptr;
     uint64_t cell_cap = 0;
     uint32_t* crow = nullptr;   // sparse grids: row directory
     uint64_t crow_cap = 0;
-    uint32_t* ccx = nullptr;
     uint32_t *trow_s = nullptr, *trow_e = nullptr;  // tile row ranges (sparse grids, compact tables)
     size_t trow_cap = 0;
 
@@ -949,6 +986,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     auto save_comp = [&](const ClusterArgs& ca, uint64_t mp) {
         if (uint32_t* comp = comp_dest(mp)) launch_save_components(ca, comp, s);
     };
+    bool table_counter_fresh = false;  // zero since the group's memset
     // builds the rows of chunk c into nbr (expand from the bitmap, or the
     // fill pass when there is no bitmap)
     auto build_chunk = [&](TableArgs& t, const RowChunk& c, uint32_t nasym) {
@@ -960,7 +998,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         t.unit_hi = c.u_hi;
         t.row_lo = c.r_lo;
         t.row_hi = c.r_hi;
-        CK(cudaMemsetAsync(t.tile_counter, 0, 4, s));
+        t.tile_counter = table_counter;
+        if (!table_counter_fresh) CK(cudaMemsetAsync(t.tile_counter, 0, 4, s));
+        table_counter_fresh = false;
         if (t.bitmap) {
             launch_expand(t, t.compact ? nb_expand16 : nb_expand32, s);
             if (nasym) launch_asym_flags(t, s);
@@ -974,10 +1014,38 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         chunks++;
     };
 
+    auto order_args = [&]() {
+        OrderArgs oa;
+        memset(&oa, 0, sizeof oa);
+        oa.x = x;
+        oa.y = y;
+        oa.gorig = gorig;
+        oa.pos = pos;
+        oa.gkey = gkey;
+        oa.n = n;
+        oa.gxy = gxy;
+        oa.glocal = glocal;
+        oa.gpos = gpos;
+        oa.mpb = mpb;
+        oa.mbb = (uint32_t)ds.mbb_size;
+        oa.gbox = gbox;
+        oa.cscan = cscan;
+        oa.clist = clist;
+        oa.ckey = ckey;
+        oa.ccx = ccx;
+        oa.tq = (uint32_t)tq;
+        oa.tiles = tiles;
+        oa.ptile = ptile;
+        oa.ntiles = d_ntiles;
+        oa.st = d_st;
+        return oa;
+    };
+
     for (const Group& gr : groups) {
         const double eps = gr.eps;
         const bool none = !(eps >= 0.0);  // negative or NaN epsilon: empty neighbourhoods
-        CK(cudaMemsetAsync(asym_n, 0, 4 * sizeof(uint32_t), s));
+        CK(cudaMemsetAsync(zeroed, 0, none ? zc.used - sort_zero_bytes(n, 32) : zc.used, s));
+        table_counter_fresh = true;
         uint64_t E = 0;
         GridParams g;
         bool clique = false;
@@ -1019,10 +1087,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             for (uint32_t i = 0; i < n; i++) iota[i] = i;
             CK(cudaMemcpyAsync(gorig, iota.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
             CK(cudaStreamSynchronize(s));
-            GridParams g1 = make_grid(hb, 1.0, 1);
-            g1.w = 1.0;
-            launch_grid_gather(x, y, gorig, pos, n, g1, gorig, gxy, glocal, gpos, s);
-            launch_point_boxes(gpos, n, mpb, ds.mbb_size, gbox, s);
+            OrderArgs oa = order_args();
+            oa.g = make_grid(hb, 1.0, 1);
+            oa.g.w = 1.0;
+            launch_gather(oa, s);
         } else {
             const size_t ta = tm.mark();
             const int r = o.cells_per_eps > 0 ? o.cells_per_eps : kCellsPerEps;
@@ -1049,10 +1117,14 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // so that the grid costs O(points + rows), not O(cells)
             g.sparse = g.ncells > 32ull * n + (1ull << 22) ? 1u : 0u;
             g.sub = isfinite(g.w) ? sub_bits(g.ncells) : 0u;
-            launch_grid_keys(x, y, n, g, gkey, gorig, s);
-            radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1) + 2 * (int)g.sub, scratch, s);
-            launch_grid_gather(x, y, gorig, pos, n, g, gkey, gxy, glocal, gpos, s);
-            launch_point_boxes(gpos, n, mpb, ds.mbb_size, gbox, s);
+            // the tuner needs the sorted grid before it can settle the tiles
+            const bool tune = o.tile_cells <= 0 && isfinite(g.w) && n >= kTuneMinPoints;
+            const int kbits = bits_for(g.ncells - 1) + 2 * (int)g.sub;
+            launch_grid_keys(x, y, n, g, kbits, skey, (uint32_t*)gz.sort, s);
+            radix_sort(skey, n, kbits, 2 * (int)g.sub, gz.sort, scratch, gkey, gorig, nullptr, d_st, s);
+            OrderArgs oa = order_args();
+            oa.g = g;
+            launch_order(oa, !tune, gz.order, s);
             auto build_cell_start = [&]() {
                 if (g.sparse) return;
                 if (g.ncells + 1 > cell_cap) {
@@ -1060,35 +1132,22 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                     cell_start = ar.get<uint32_t>(g.ncells + 1);
                     cell_cap = g.ncells + 1;
                 }
-                CK(cudaMemsetAsync(cell_start, 0xff, (g.ncells + 1) * 4, s));
-                launch_cell_marks(gkey, n, cell_start, g.ncells, s);
-                size_t need = suffix_min_u32_scratch_bytes(g.ncells + 1);
-                char* sm = need <= scr ? scratch : ar.get<char>(need);
-                suffix_min_u32(cell_start, g.ncells + 1, sm, s);
+                launch_cell_start(ckey, clist, cscan + n, n, g, cell_start, s);
             };
             build_cell_start();
-            // non-empty cells (clist) and the cell index of each cell's first point
-            launch_tile_flags(gkey, n, 1, 0xffffffffu, tflags, s);
-            scan_u32(tflags, cscan, n, scratch, s);
-            launch_tile_write(tflags, cscan, n, clist, s);
             if (g.sparse) {
                 if ((uint64_t)g.ncy + 1 > crow_cap) {
                     if (crow) ar.put(crow);
                     crow = ar.get<uint32_t>((size_t)g.ncy + 1);
                     crow_cap = (uint64_t)g.ncy + 1;
                 }
-                if (!ccx) ccx = ar.get<uint32_t>(n);
-                CK(cudaMemsetAsync(crow, 0xff, ((size_t)g.ncy + 1) * 4, s));
-                launch_cell_rows(gkey, clist, cscan + n, n, g, crow, ccx, s);
-                size_t need = suffix_min_u32_scratch_bytes((uint64_t)g.ncy + 1);
-                char* sm = need <= scr ? scratch : ar.get<char>(need);
-                suffix_min_u32(crow, (uint64_t)g.ncy + 1, sm, s);
+                launch_cell_rows(ckey, cscan + n, g, crow, s);
             }
             // tile shape: the cost model of choose_tile_cells on the grid's
             // own statistics (sampled non-empty cells); a new G only re-pads
             // the rows, so the keys are rewritten without sorting again (the
             // row directory of sparse grids does not depend on the padding)
-            if (o.tile_cells <= 0 && isfinite(g.w) && n >= kTuneMinPoints) {
+            if (tune) {
                 // decisions are kept per dataset (its buffers, size and box)
                 // and epsilon: a repeated call measures nothing
                 const TuneKey key{ds.x, ds.y, n, hb.minx, hb.maxx, hb.miny, hb.maxy, eps, r};
@@ -1125,7 +1184,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 if (G != g.G && g2.ncx == g.ncx && g2.ncy == g.ncy && g2.w == g.w) {
                     g2.sparse = g.sparse;
                     g2.sub = g.sub;
-                    launch_grid_rekey(gkey, n, g.ncx_pad, g2.ncx_pad, s);
+                    launch_grid_rekey(gkey, ckey, cscan + n, n, g.ncx_pad, g2.ncx_pad, s);
                     g = g2;
                     build_cell_start();
                     ep = make_eps(eps, g, hb, want_mixed);
@@ -1137,9 +1196,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 tile_cells_hist[lg]++;
             }
             const bool mixed = ep.mixed != 0;
-            launch_tile_flags(gkey, n, g.G, (uint32_t)tq, tflags, s);
-            scan_u32(tflags, tscan, n, scratch, s);
-            launch_tile_write(tflags, tscan, n, tiles, s);
+            if (tune) {
+                oa.g = g;
+                launch_tiles(oa, gz.tiles, s);
+            }
             // cells are cliques when two points of one cell always pass the
             // distance test without a box check: 2 w^2 below thr and tbox
             clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
@@ -1155,9 +1215,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ta_args.ep = d_ep;
             ta_args.mixed = mixed ? 1 : 0;
             ta_args.tiles = tiles;
-            ta_args.ntiles = tscan + n;
+            ta_args.ntiles = d_ntiles;
             ta_args.tile_end = 0xffffffffu;
-            ta_args.tile_counter = tile_counter;
+            ta_args.tile_counter = count_counter;
             ta_args.cell_start = cell_start;
             // compact entries are possible when the caller allows them and a
             // warp can hold the tile's row segments; their tile row ranges
@@ -1198,9 +1258,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // layout of the count pass's test bitmap (one word per query and
             // 32 candidates of its tile), which the table pass expands
             ta_args.unit_words = unit_words;
-            launch_tile_words(ta_args, tflags, tunits, nb_warps, s);
-            if (!no_rows) scan_u32_to_u64(tflags, tboff, n, scratch, s);
-            scan_u32(tunits, tuoff, n, scratch, s);
+            launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, d_nwords, d_nunits,
+                              gz.words, s);
             uint64_t bm_words = 0;
             uint32_t nunits = 0;
             uint32_t st_flags = 0;
@@ -1214,19 +1273,16 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 st_flags = (uint32_t)rec->take();
                 GraphCheck chk;
                 memset(&chk, 0, sizeof chk);
-                chk.c[0] = graph_cond(tuoff + n, kGcLe32, nunits);
+                chk.c[0] = graph_cond(d_nunits, kGcLe32, nunits);
                 chk.n = 1;
                 if (!no_rows) {
-                    chk.c[1] = graph_cond(tboff + n, kGcLe64, bm_words);
+                    chk.c[1] = graph_cond(d_nwords, kGcLe64, bm_words);
                     chk.c[2] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
                     chk.n = 3;
                 }
                 capture_checkpoint(*rec, s, chk);
             } else {
-                if (!no_rows)
-                    CK(cudaMemcpyAsync(ctx->h_pinned, tboff + n, 8, cudaMemcpyDeviceToHost, s));
-                CK(cudaMemcpyAsync((char*)ctx->h_pinned + 8, tuoff + n, 4,
-                                   cudaMemcpyDeviceToHost, s));
+                CK(cudaMemcpyAsync(ctx->h_pinned, d_totals, 16, cudaMemcpyDeviceToHost, s));
                 read_status(ctx, s);
                 status_before_count = *ctx->h_status;
                 if (!no_rows) memcpy(&bm_words, ctx->h_pinned, 8);
@@ -1241,11 +1297,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // 16-bit entries (positions within work units)
             compact = compact_ok;
             ta_args.compact = compact ? 1 : 0;
-            if (compact && !no_rows) {
-                if (!ptile) ptile = ar.get<uint32_t>(n);
-                ta_args.ptile = ptile;
-                launch_tile_owner(ta_args, ptile, nb_warps, s);
-            }
+            ta_args.ptile = ptile;
             // work units: (tile, chunk of unit_words bitmap words)
             if ((uint64_t)nunits + 1 > unit_cap) {
                 if (unit_tile) ar.put(unit_tile);
@@ -1256,12 +1308,11 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             }
             if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
             ta_args.tile_uoff = tuoff;
-            ta_args.nunits = tuoff + n;
+            ta_args.nunits = d_nunits;
             ta_args.unit_tile = unit_tile;
             ta_args.parts = no_rows ? nullptr : parts;
             ta_args.pair_sum = no_rows ? &d_st->pairs : nullptr;
-            launch_unit_list(ta_args, unit_tile, nb_warps, s);
-            CK(cudaMemsetAsync(deg, 0, (size_t)n * 4, s));
+            launch_unit_list(ta_args, unit_tile, s);
             ta_args.bitmap = nullptr;
             ta_args.tile_boff = tboff;
             if (no_rows) {
@@ -1298,12 +1349,15 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 launch_word_boxes(ta_args, s);
             }
             size_t tc = 0;
-            for (;;) {
-                CK(cudaMemsetAsync(tile_counter, 0, 4, s));
+            for (bool again = false;; again = true) {
+                if (again) {
+                    CK(cudaMemsetAsync(count_counter, 0, 4, s));
+                    CK(cudaMemsetAsync(gz.off, 0, scan_state_bytes(n), s));
+                }
                 launch_count(ta_args, nb_count, s);
                 CK(cudaGetLastError());
                 tc = tm.mark();
-                if (!no_rows) scan_u32_to_u64(deg, off, n, scratch, s);
+                if (!no_rows) scan_u32_to_u64(deg, off, n, gz.off, d_st, s);
                 if (capturing) break;
                 if (!no_rows)
                     CK(cudaMemcpyAsync(ctx->h_pinned, off + n, 8, cudaMemcpyDeviceToHost, s));
@@ -1395,7 +1449,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 nbr_cap_bytes = 0;
                 const int64_t budget = o.budget > 0 ? o.budget : (int64_t)(avail_bytes(ctx) * 0.9);
                 const uint64_t cap = (uint64_t)std::max<int64_t>(budget / (int64_t)esz, 1);
-                chunk_list = plan_row_chunks(ctx, tiles, tscan + n, tuoff, off, n, cap, s);
+                chunk_list = plan_row_chunks(ctx, tiles, d_ntiles, tuoff, off, n, cap, s);
                 uint64_t mx = 1;
                 for (const RowChunk& c : chunk_list) mx = std::max<uint64_t>(mx, c.e_hi - c.e_lo);
                 const size_t w = std::max<size_t>(words_for(mx), 1);
@@ -1446,8 +1500,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ca.seed = u.seed;
             ca.cstart = u.cstart;
             ca.best = u.best;
-            ca.cluster_no = u.cluster_no;
-            ca.pos_flag = u.pos_flag;
+            ca.bits = u.bits;
+            ca.brank = u.brank;
+            ca.nw = nw;
             ca.asym = asym;
             ca.asym_count = asym_n;
             ca.asym_cap = asym_cap;
@@ -1481,7 +1536,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 crng_cap = (size_t)n * nrows;
                 crng = ar.get<uint2>(crng_cap);
             }
-            if (!ccx) ccx = ar.get<uint32_t>(n);
             if (group_asym && want > cells_ws_slots) {
                 if (cells_ws) ar.put(cells_ws);
                 cells_ws = ar.get<uint32_t>(want * (resolve_scratch_bytes() / 4));
@@ -1548,7 +1602,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 if (chain) ca.minpts_prev = slots[si - 1].second;
                 launch_uf_init(ca, !chain, s);
                 if (!none) launch_uf_union(ca, nb_warps, s);
-                launch_uf_finish(ca, scratch, scratch + resolve_scratch_bytes(), s);
+                launch_uf_finish(ca, scratch, s);
                 if (!none) save_comp(ca, slots[si].second);
                 launch_border_and_write(ca, nb_warps, s);
                 CK(cudaGetLastError());
@@ -1570,7 +1624,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 }
             }
             for (size_t si = 0; si < cas.size(); si++) {
-                launch_uf_finish(cas[si], scratch, scratch + resolve_scratch_bytes(), s);
+                launch_uf_finish(cas[si], scratch, s);
                 save_comp(cas[si], slots[si].second);
             }
             for (const RowChunk& c : chunk_list) {
@@ -2301,14 +2355,21 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     Carve cv{base, kNoallocBytes, 0};
     DeviceStatus* st = cv.take<DeviceStatus>(1);
     BBox* d_bb = cv.take<BBox>(1);
-    const size_t scr = std::max({radix_sort_scratch_bytes(n), scan_u32_to_u64_scratch_bytes(n + 1),
-                                 bbox_scratch_bytes(n),
-                                 resolve_scratch_bytes() + scan_u32_scratch_bytes(n),
-                                 suffix_min_u32_scratch_bytes(kNoallocMaxCells + 1)});
-    char* scratch = cv.take<char>(scr);
+    uint32_t* resolve_ws = cv.take<uint32_t>(resolve_scratch_bytes() / 4);
+    ZeroCarve zm{nullptr, 0};
+    GroupZero(zm, n, false);
+    ZeroCarve zc{cv.take<char>(zm.used), 0};
+    const GroupZero gz(zc, n, false);
+    // the sorts' and the box's memory lies at the array's end: they are done
+    // before the table (or the cells' neighbour lists) takes that room
+    const size_t sort_zero = 256 + sort_zero_bytes(n, 32);
+    const size_t tail = (std::max(sort_scratch_bytes(n), bbox_scratch_bytes()) + 255) / 256 * 256;
+    char* const scratch = base + kNoallocBytes - tail;
+    char* const zeroed = scratch - (sort_zero + 255) / 256 * 256;
     // the array keeps the previous call's contents: clear what starts at zero
     CK(cudaMemsetAsync(st, 0, sizeof(DeviceStatus), s));
-    launch_bbox(x, y, n, d_bb, scratch, s);
+    CK(cudaMemsetAsync(zeroed, 0, 256 + sort_zero_bytes(n, kVisitBits), s));
+    launch_bbox(x, y, n, d_bb, scratch, (uint32_t*)zeroed, s);
     BBox bb;
     CK(cudaMemcpyAsync(&bb, d_bb, sizeof bb, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -2318,9 +2379,8 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* vkey = cv.take<uint32_t>(n);
     uint32_t* vorder = cv.take<uint32_t>(n);
     uint32_t* pos = cv.take<uint32_t>(n);
-    launch_visit_keys(x, y, n, d_bb, vkey, vorder, st, s);
-    radix_sort_pairs(vkey, vorder, n, bits_for(kVisitBins * kVisitBins - 1), scratch, s);
-    launch_invert(vorder, n, pos, s);
+    launch_visit_keys(x, y, n, d_bb, vkey, (uint32_t*)(zeroed + 256), st, s);
+    radix_sort(vkey, n, kVisitBits, 0, zeroed + 256, scratch, nullptr, vorder, pos, st, s);
     const uint32_t nmpb = (uint32_t)(((uint64_t)n + (uint32_t)mbb - 1) / (uint32_t)mbb);
     MpbBox* mpb = cv.take<MpbBox>(nmpb);
     launch_mpb_boxes(x, y, vorder, n, mbb, mpb, s);
@@ -2335,8 +2395,9 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* gpos = cv.take<uint32_t>(n);
     MpbBox* gbox = cv.take<MpbBox>(n);
     uint32_t* cell_start = cv.take<uint32_t>(g.ncells + 1);
-    uint32_t* tflags = cv.take<uint32_t>(n);
-    uint32_t* tscan = cv.take<uint32_t>((size_t)n + 1);
+    uint32_t* ckey = cv.take<uint32_t>(n);
+    uint32_t* ccx = cv.take<uint32_t>(n);
+    uint32_t* ptile = cv.take<uint32_t>(n);
     uint32_t* tiles = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* cscan = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* clist = cv.take<uint32_t>((size_t)n + 1);
@@ -2344,8 +2405,10 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* deg = cv.take<uint32_t>(n);
     unsigned long long* off = cv.take<unsigned long long>((size_t)n + 1);
     AsymPair* asym = cv.take<AsymPair>(kNoallocAsymCap);
-    uint32_t* asym_n = cv.take<uint32_t>(4);
-    uint32_t* tile_counter = asym_n + 1;
+    uint32_t* asym_n = gz.counts;
+    unsigned long long* d_totals = cv.take<unsigned long long>(4);
+    uint32_t* d_nunits = (uint32_t*)(d_totals + 1);
+    uint32_t* d_ntiles = (uint32_t*)(d_totals + 2);
     uint32_t* parent = cv.take<uint32_t>(n);
     uint32_t* seed = cv.take<uint32_t>(n);
     uint32_t* cstart = cv.take<uint32_t>(n);
@@ -2354,25 +2417,41 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* best = cv.take<uint32_t>(n);
     cv.take<uint32_t>(n);  // (cbest: both pieces, 8 bytes per cell)
     unsigned long long* cbest = (unsigned long long*)best;
-    uint32_t* cluster_no = cv.take<uint32_t>((size_t)n + 1);
-    uint32_t* pos_flag = cv.take<uint32_t>(n);
+    uint32_t* bits = cv.take<uint32_t>(start_words(n));
+    uint32_t* brank = cv.take<uint32_t>(start_words(n));
 
-    launch_grid_keys(x, y, n, g, gkey, gorig, s);
-    radix_sort_pairs(gkey, gorig, n, bits_for(g.ncells - 1) + 2 * (int)g.sub, scratch, s);
-    launch_grid_gather(x, y, gorig, pos, n, g, gkey, gxy, glocal, gpos, s);
-    launch_point_boxes(gpos, n, mpb, mbb, gbox, s);
-    CK(cudaMemsetAsync(cell_start, 0xff, (g.ncells + 1) * 4, s));
-    launch_cell_marks(gkey, n, cell_start, g.ncells, s);
-    suffix_min_u32(cell_start, g.ncells + 1, scratch, s);
-    const int tq = table_tile_queries();
-    launch_tile_flags(gkey, n, g.G, (uint32_t)tq, tflags, s);
-    scan_u32(tflags, tscan, n, scratch, s);
-    launch_tile_write(tflags, tscan, n, tiles, s);
-    launch_tile_flags(gkey, n, 1, 0xffffffffu, tflags, s);
-    scan_u32(tflags, cscan, n, scratch, s);
-    launch_tile_write(tflags, cscan, n, clist, s);
+    CK(cudaMemsetAsync(zc.base, 0, zc.used, s));
+    const int kbits = bits_for(g.ncells - 1) + 2 * (int)g.sub;
+    CK(cudaMemsetAsync(zeroed, 0, sort_zero_bytes(n, kbits), s));
+    launch_grid_keys(x, y, n, g, kbits, vkey, (uint32_t*)zeroed, s);
+    radix_sort(vkey, n, kbits, 2 * (int)g.sub, zeroed, scratch, gkey, gorig, nullptr, st, s);
+    OrderArgs oa;
+    memset(&oa, 0, sizeof oa);
+    oa.x = x;
+    oa.y = y;
+    oa.gorig = gorig;
+    oa.pos = pos;
+    oa.gkey = gkey;
+    oa.n = n;
+    oa.g = g;
+    oa.gxy = gxy;
+    oa.glocal = glocal;
+    oa.gpos = gpos;
+    oa.mpb = mpb;
+    oa.mbb = (uint32_t)mbb;
+    oa.gbox = gbox;
+    oa.cscan = cscan;
+    oa.clist = clist;
+    oa.ckey = ckey;
+    oa.ccx = ccx;
+    oa.tq = (uint32_t)table_tile_queries();
+    oa.tiles = tiles;
+    oa.ptile = ptile;
+    oa.ntiles = d_ntiles;
+    oa.st = st;
+    launch_order(oa, true, gz.order, s);
+    launch_cell_start(ckey, clist, cscan + n, n, g, cell_start, s);
     CK(cudaMemcpyAsync(d_ep, &ep, sizeof ep, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(asym_n, 0, 4 * sizeof(uint32_t), s));
 
     TableArgs ta;
     memset(&ta, 0, sizeof ta);
@@ -2380,9 +2459,9 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.ep = d_ep;
     ta.mixed = ep.mixed;
     ta.tiles = tiles;
-    ta.ntiles = tscan + n;
+    ta.ntiles = d_ntiles;
     ta.tile_end = 0xffffffffu;
-    ta.tile_counter = tile_counter;
+    ta.tile_counter = asym_n + 1;
     ta.cell_start = cell_start;
     ta.gkey = gkey;
     ta.glocal = glocal;
@@ -2396,52 +2475,46 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.asym_n = asym_n;
     ta.asym_cap = kNoallocAsymCap;
     ta.st = st;
-    ta.unit_words = kUnitWords;
+    ta.unit_words = kUnitWordsSmall;
     // work units of the count pass (no bitmap here: the fill pass writes the table)
-    uint32_t* twords = cv.take<uint32_t>(n);
-    uint32_t* tunits = cv.take<uint32_t>(n);
     uint32_t* tuoff = cv.take<uint32_t>((size_t)n + 1);
-    launch_tile_words(ta, twords, tunits, nsm * 8, s);
-    scan_u32(tunits, tuoff, n, scratch, s);
+    launch_tile_words(ta, nullptr, tuoff, d_totals, d_nunits, gz.words, s);
     uint32_t nunits = 0;
-    CK(cudaMemcpyAsync(&nunits, tuoff + n, 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(&nunits, d_nunits, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     uint32_t* unit_tile = cv.take<uint32_t>((size_t)nunits + 1);
     ta.tile_uoff = tuoff;
-    ta.nunits = tuoff + n;
+    ta.nunits = d_nunits;
     ta.unit_tile = unit_tile;
     ta.parts = nullptr;
     ta.bitmap = nullptr;
-    launch_unit_list(ta, unit_tile, nsm * 8, s);
-    CK(cudaMemsetAsync(deg, 0, (size_t)n * 4, s));
-    CK(cudaMemsetAsync(tile_counter, 0, 4, s));
+    launch_unit_list(ta, unit_tile, s);
     launch_count(ta, nsm * table_blocks_per_sm(false, ep.mixed != 0), s);
-    scan_u32_to_u64(deg, off, n, scratch, s);
+    scan_u32_to_u64(deg, off, n, gz.off, st, s);
     unsigned long long E = 0;
     DeviceStatus hs;
     CK(cudaMemcpyAsync(&E, off + n, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&hs, st, sizeof hs, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     check_flags(hs);
-    // the neighbour table has the rest of the array
-    const size_t room = (kNoallocBytes - cv.used) / sizeof(uint32_t);
+    // the limit on the neighbour pairs: what a table of 32-bit entries has
+    // beside 160 bytes per point, the cells and the one-way pairs
+    const size_t held = (size_t)n * 160 + (g.ncells + 1) * 4 +
+                        (size_t)kNoallocAsymCap * sizeof(AsymPair) + ((size_t)1 << 18);
+    const size_t room = held < kNoallocBytes ? (kNoallocBytes - held) / sizeof(uint32_t) : 0;
     if (E > room)
         throw VdbError{VDB_ERR_TOO_LARGE, "neighbour table exceeds the fixed scratch array"};
     uint32_t* nbr = nullptr;
     uint2* crng = nullptr;
-    uint32_t *ccx = nullptr, *bits = nullptr, *brank = nullptr;
     if (clique) {
         // cells that are cliques are labelled without the table: its room
-        // holds the cells' neighbour lists and the start bits
-        bits = cv.take<uint32_t>(start_words(n));
-        brank = cv.take<uint32_t>(start_words(n));
-        ccx = cv.take<uint32_t>(n);
+        // holds the cells' neighbour lists
         crng = cv.take<uint2>((size_t)n * (2 * ep.rho + 1));
     } else {
         nbr = cv.take<uint32_t>(E ? E : 1);
         ta.nbr = nbr;
         ta.off_base = 0;
-        CK(cudaMemsetAsync(tile_counter, 0, 4, s));
+        ta.tile_counter = asym_n + 2;
         launch_fill(ta, nsm * table_blocks_per_sm(true, ep.mixed != 0), s);
     }
     const int nb_warps = nsm * 8;
@@ -2479,13 +2552,13 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         ca.asym_count = asym_n;
         ca.asym_cap = kNoallocAsymCap;
         ca.st = st;
-        launch_cells(ca, 2 * ep.rho + 1, true, scratch, s);
+        launch_cells(ca, 2 * ep.rho + 1, true, resolve_ws, s);
     } else {
         ClusterArgs ca;
         memset(&ca, 0, sizeof ca);
         ca.n = n;
         ca.deg = deg;
-        ca.unit_words = kUnitWords;
+        ca.unit_words = kUnitWordsSmall;
         ca.minpts = minpts > 0x7fffffffu ? ~0ull : (unsigned long long)minpts;
         ca.minpts_prev = ~0ull;
         ca.off = off;
@@ -2498,8 +2571,9 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         ca.seed = seed;
         ca.cstart = cstart;
         ca.best = best;
-        ca.cluster_no = cluster_no;
-        ca.pos_flag = pos_flag;
+        ca.bits = bits;
+        ca.brank = brank;
+        ca.nw = start_words(n);
         ca.asym = asym;
         ca.asym_count = asym_n;
         ca.asym_cap = kNoallocAsymCap;
@@ -2509,7 +2583,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         ca.ep = d_ep;
         launch_uf_init(ca, true, s);
         launch_uf_union(ca, nb_warps, s);
-        launch_uf_finish(ca, scratch, scratch + resolve_scratch_bytes(), s);
+        launch_uf_finish(ca, resolve_ws, s);
         launch_border_and_write(ca, nb_warps, s);
     }
     CK(cudaGetLastError());

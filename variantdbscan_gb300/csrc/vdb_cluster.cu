@@ -67,15 +67,14 @@ __device__ __forceinline__ void uf_union(uint32_t* parent, uint32_t a, uint32_t 
     atomicOr(&st->flags, kStatUnionStall);
 }
 
-__global__ void uf_init_kernel(uint32_t n, int fresh, uint32_t* parent, uint32_t* seed,
-                               uint32_t* best, uint32_t* cstart, uint32_t* pos_flag) {
+__global__ void uf_init_kernel(ClusterArgs a, int fresh) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    if (fresh) parent[k] = k;
-    seed[k] = kNone;
-    best[k] = kNone;
-    cstart[k] = k;
-    pos_flag[k] = 0u;
+    if (k < a.nw) a.bits[k] = 0u;
+    if (k >= a.n) return;
+    if (fresh) a.parent[k] = k;
+    a.seed[k] = kNone;
+    a.best[k] = kNone;
+    a.cstart[k] = k;
 }
 
 // One warp per row.  From scratch, an edge (k, v) of two cores is united from
@@ -209,11 +208,79 @@ __global__ void resolve_kernel(ClusterArgs a, uint32_t* ws, uint32_t cap) {
     }
 }
 
+// Cluster numbers: a cluster's number is the rank of its start among the
+// starts (visit positions, one bit each).  rank[w] = starts before word w;
+// returns their number (one block; nw: start_words).
+constexpr int kRankThreads = 1024;
+constexpr int kRankItems = 8;
+__device__ uint32_t rank_bits(const uint32_t* __restrict__ bits, uint32_t* __restrict__ rank,
+                              uint32_t nw) {
+    __shared__ uint32_t s_tot[32];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t base = 0; base < nw; base += kRankThreads * kRankItems) {
+        const uint32_t w0 = base + threadIdx.x * kRankItems;
+        uint32_t c[kRankItems], sum = 0;
+        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
+        if (w0 < nw) {  // (nw is a multiple of kRankItems)
+            lo = reinterpret_cast<const uint4*>(bits + w0)[0];
+            hi = reinterpret_cast<const uint4*>(bits + w0)[1];
+        }
+        c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w;
+        c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
+#pragma unroll
+        for (int i = 0; i < kRankItems; i++) {
+            c[i] = __popc(c[i]);
+            sum += c[i];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, d);
+            if (lane >= (uint32_t)d) incl += t;
+        }
+        if (lane == 31) s_tot[wid] = incl;
+        __syncthreads();
+        uint32_t t = s_tot[lane], ti = t;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(kFull, ti, d);
+            if (lane >= (uint32_t)d) ti += o;
+        }
+        const uint32_t before = __shfl_sync(kFull, ti - t, (int)wid);
+        const uint32_t all = __shfl_sync(kFull, ti, 31);
+        uint32_t run = carry + before + incl - sum;
+#pragma unroll
+        for (int i = 0; i < kRankItems; i++) {
+            const uint32_t t2 = c[i];
+            c[i] = run;
+            run += t2;
+        }
+        if (w0 < nw) {
+            reinterpret_cast<uint4*>(rank + w0)[0] = make_uint4(c[0], c[1], c[2], c[3]);
+            reinterpret_cast<uint4*>(rank + w0)[1] = make_uint4(c[4], c[5], c[6], c[7]);
+        }
+        carry += all;
+        __syncthreads();
+    }
+    return carry;
+}
+// Label of the cluster that starts at visit position s.
+__device__ __forceinline__ uint32_t bit_label(const uint32_t* __restrict__ bits,
+                                              const uint32_t* __restrict__ rank, uint32_t s) {
+    return rank[s >> 5] + __popc(bits[s >> 5] & ((1u << (s & 31u)) - 1u)) + 1u;
+}
+
 __global__ void start_flags_kernel(ClusterArgs a) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n || !is_core(a.deg[k], a.minpts)) return;
     if (a.parent[k] == k && a.cstart[k] == k && VDB_GUARD(a.st, a.seed[k] < a.n, 12, a.seed[k]))
-        a.pos_flag[a.seed[k]] = 1u;
+        atomicOr(&a.bits[a.seed[k] >> 5], 1u << (a.seed[k] & 31u));
+}
+
+__global__ void __launch_bounds__(kRankThreads) rank_kernel(ClusterArgs a) {
+    const uint32_t k = rank_bits(a.bits, a.brank, a.nw);
+    if (threadIdx.x == 0 && k) atomicAdd(&a.st->clusters, (unsigned long long)k * a.copies);
 }
 
 __device__ __forceinline__ uint32_t start_time(const ClusterArgs& a, uint32_t u) {
@@ -280,14 +347,13 @@ __global__ void asym_push_kernel(ClusterArgs a) {
 __global__ void write_labels_kernel(ClusterArgs a) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
-    if (k == 0) atomicAdd(&a.st->clusters, (unsigned long long)a.cluster_no[a.n] * a.copies);
     uint32_t lab;
     if (is_core(a.deg[k], a.minpts)) {
         const uint32_t t = start_time(a, k);
-        lab = VDB_GUARD(a.st, t < a.n, 14, t) ? a.cluster_no[t] + 1u : 0u;
+        lab = VDB_GUARD(a.st, t < a.n, 14, t) ? bit_label(a.bits, a.brank, t) : 0u;
     } else {
         const uint32_t b = a.best[k];
-        lab = (b != kNone && b < a.gpos[k]) ? a.cluster_no[b] + 1u : 0u;
+        lab = (b != kNone && b < a.gpos[k]) ? bit_label(a.bits, a.brank, b) : 0u;
     }
     if (VDB_GUARD(a.st, a.gorig[k] < a.n, 13, a.gorig[k])) a.labels_out[a.gorig[k]] = lab;
 }
@@ -313,7 +379,6 @@ __global__ void cell_ranges_kernel(CellArgs a) {
     if (c >= ncl || r > 2u * rho) return;
     const uint32_t key = a.gkey[a.clist[c]];
     const int cy = (int)(key / a.g.ncx_pad), cx = (int)(key - (uint32_t)cy * a.g.ncx_pad);
-    if (r == rho && !a.g.sparse) a.ccx[c] = (uint32_t)cx;
     const int ry = cy + (int)r - (int)rho, reach = a.ep->reach[r];
     const uint32_t lo = (uint32_t)max(cx - reach, 0);
     const uint32_t hi = (uint32_t)min(cx + reach, (int)a.g.ncx - 1);
@@ -677,70 +742,16 @@ __global__ void cell_starts_kernel(CellArgs a) {
     a.cst[o + c] = s;
 }
 
-// brank[w] = cluster starts before word w of the slot's bits; the slot's
-// number of clusters (one block per slot).
-constexpr int kRankThreads = 1024;
-constexpr int kRankItems = 8;
+// The slots' ranks and numbers of clusters (one block per slot).
 __global__ void __launch_bounds__(kRankThreads) cell_rank_kernel(CellArgs a) {
-    __shared__ uint32_t s_tot[32];
     const int v = blockIdx.x;
-    const uint32_t* __restrict__ bits = a.bits + (size_t)v * a.nw;
-    uint32_t* rank = a.brank + (size_t)v * a.nw;
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t carry = 0;
-    for (uint32_t base = 0; base < a.nw; base += kRankThreads * kRankItems) {
-        const uint32_t w0 = base + threadIdx.x * kRankItems;
-        uint32_t c[kRankItems], sum = 0;
-        uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-        if (w0 < a.nw) {  // (nw is a multiple of kRankItems)
-            lo = reinterpret_cast<const uint4*>(bits + w0)[0];
-            hi = reinterpret_cast<const uint4*>(bits + w0)[1];
-        }
-        c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w;
-        c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
-#pragma unroll
-        for (int i = 0; i < kRankItems; i++) {
-            c[i] = __popc(c[i]);
-            sum += c[i];
-        }
-        uint32_t incl = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t t = __shfl_up_sync(kFull, incl, d);
-            if (lane >= (uint32_t)d) incl += t;
-        }
-        if (lane == 31) s_tot[wid] = incl;
-        __syncthreads();
-        uint32_t t = s_tot[lane], ti = t;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(kFull, ti, d);
-            if (lane >= (uint32_t)d) ti += o;
-        }
-        const uint32_t before = __shfl_sync(kFull, ti - t, (int)wid);
-        const uint32_t all = __shfl_sync(kFull, ti, 31);
-        uint32_t run = carry + before + incl - sum;
-#pragma unroll
-        for (int i = 0; i < kRankItems; i++) {
-            const uint32_t t2 = c[i];
-            c[i] = run;
-            run += t2;
-        }
-        if (w0 < a.nw) {
-            reinterpret_cast<uint4*>(rank + w0)[0] = make_uint4(c[0], c[1], c[2], c[3]);
-            reinterpret_cast<uint4*>(rank + w0)[1] = make_uint4(c[4], c[5], c[6], c[7]);
-        }
-        carry += all;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0 && carry)
-        atomicAdd(&a.st->clusters, (unsigned long long)carry * a.copies[v]);
+    const uint32_t k = rank_bits(a.bits + (size_t)v * a.nw, a.brank + (size_t)v * a.nw, a.nw);
+    if (threadIdx.x == 0 && k) atomicAdd(&a.st->clusters, (unsigned long long)k * a.copies[v]);
 }
 
 // Label of the cluster that starts at visit position s.
 __device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32_t s) {
-    const size_t w = (size_t)v * a.nw + (s >> 5);
-    return a.brank[w] + __popc(a.bits[w] & ((1u << (s & 31u)) - 1u)) + 1u;
+    return bit_label(a.bits + (size_t)v * a.nw, a.brank + (size_t)v * a.nw, s);
 }
 
 // Labels of the cores, and the saved components (comp[visit position] =
@@ -879,18 +890,16 @@ __global__ void cell_border_kernel(CellArgs a) {
 size_t resolve_scratch_bytes() { return (size_t)kResolveCap * 6 * sizeof(uint32_t); }
 
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s) {
-    if (a.n) VDB_COUNT_LAUNCH();
-    if (a.n)
-        uf_init_kernel<<<nblk(a.n), kThreads, 0, s>>>(a.n, fresh ? 1 : 0, a.parent, a.seed,
-                                                      a.best, a.cstart, a.pos_flag);
+    if (!a.n) return;
+    VDB_COUNT_LAUNCH();
+    uf_init_kernel<<<nblk(std::max(a.n, a.nw)), kThreads, 0, s>>>(a, fresh ? 1 : 0);
 }
 
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s) {
     if (a.row_hi > a.row_lo) { VDB_COUNT_LAUNCH(); uf_union_kernel<<<nblocks, kThreads, 0, s>>>(a); }
 }
 
-void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, void* scan_scratch,
-                      cudaStream_t s) {
+void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, cudaStream_t s) {
     if (!a.n) return;
     VDB_COUNT_LAUNCH();
     uf_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
@@ -898,7 +907,8 @@ void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, void* scan_scratch
     resolve_kernel<<<1, 32, 0, s>>>(a, (uint32_t*)resolve_ws, kResolveCap);
     VDB_COUNT_LAUNCH();
     start_flags_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    scan_u32(a.pos_flag, a.cluster_no, a.n, scan_scratch, s);
+    VDB_COUNT_LAUNCH();
+    rank_kernel<<<1, kRankThreads, 0, s>>>(a);
 }
 
 void launch_save_components(const ClusterArgs& a, uint32_t* comp, cudaStream_t s) {

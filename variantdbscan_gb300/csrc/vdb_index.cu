@@ -6,7 +6,7 @@
 //    cell keys, cell-ordered coordinates, cell start offsets and query tiles.
 #include <float.h>
 
-#include "vdb_internal.cuh"
+#include "vdb_lookback.cuh"
 
 namespace vdb {
 
@@ -16,36 +16,84 @@ constexpr int kThreads = 256;
 
 inline unsigned nblk(uint64_t n) { return (unsigned)((n + kThreads - 1) / kThreads); }
 
-// Bin key of src/main.cpp:491-540 evaluated with the same FP64 operations:
-// width = (max-min)*1.01, offset = -min (or fabs(min)), bin = floor(((x+offset)/width)*300).
-__global__ void visit_keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                  uint32_t n, const BBox* __restrict__ bb,
-                                  uint32_t* __restrict__ keys, uint32_t* __restrict__ idx,
-                                  DeviceStatus* st) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double minx = bb->minx, maxx = bb->maxx, miny = bb->miny, maxy = bb->maxy;
-    const double xw = __dmul_rn(__dsub_rn(maxx, minx), 1.01);
-    const double yw = __dmul_rn(__dsub_rn(maxy, miny), 1.01);
-    const double xo = (minx > 0) ? -minx : fabs(minx);
-    const double yo = (miny > 0) ? -miny : fabs(miny);
-    double fx = floor(__dmul_rn(__ddiv_rn(__dadd_rn(x[i], xo), xw), (double)kVisitBins));
-    double fy = floor(__dmul_rn(__ddiv_rn(__dadd_rn(y[i], yo), yw), (double)kVisitBins));
-    bool ok = fx >= 0.0 && fx <= (double)(kVisitBins - 1) && fy >= 0.0 &&
-              fy <= (double)(kVisitBins - 1);
-    if (!ok) {
-        atomicOr(&st->flags, kStatDegenerate);
-        fx = 0.0;
-        fy = 0.0;
+// Digit counts of a key in shared memory, added to the sort's histogram at
+// the end of the block.
+struct DigitCounts {
+    uint32_t c[kMaxPasses][kDigits];
+};
+__device__ __forceinline__ void counts_clear(DigitCounts& h, int passes) {
+    for (uint32_t i = threadIdx.x; i < (uint32_t)passes * kDigits; i += blockDim.x)
+        (&h.c[0][0])[i] = 0u;
+    __syncthreads();
+}
+__device__ __forceinline__ void counts_add(DigitCounts& h, int passes, uint32_t key) {
+    for (int p = 0; p < passes; p++)
+        atomicAdd(&h.c[p][(key >> (p * kDigitBits)) & (kDigits - 1u)], 1u);
+}
+__device__ __forceinline__ void counts_flush(DigitCounts& h, int passes, uint32_t* hist) {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < (uint32_t)passes * kDigits; i += blockDim.x) {
+        const uint32_t v = (&h.c[0][0])[i];
+        if (v) atomicAdd(&hist[i], v);
     }
-    keys[i] = (uint32_t)fx * kVisitBins + (uint32_t)fy;
-    idx[i] = i;
 }
 
-__global__ void invert_kernel(const uint32_t* __restrict__ order, uint32_t n,
-                              uint32_t* __restrict__ inv) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n && order[k] < n) inv[order[k]] = k;
+// floor(r) of a quotient that FP32 knows as r, within err: exact wherever r is
+// further than err from a whole number; *sure = 0 otherwise (and for NaN and
+// infinities), and the caller divides in FP64.  GB300 issues 2 FP64 lanes a
+// cycle per SM, and two divisions per point bounded the key kernels (1M
+// points: 54 us; 13 us with the filter).
+__device__ __forceinline__ float floor_if_sure(float r, float err, bool* sure) {
+    const float f = floorf(r);
+    *sure = r - f > err && r - f < 1.0f - err;
+    return f;
+}
+// usable FP32 factor (1 / w and 300 / w stay far from FP32's limits)
+__device__ __forceinline__ bool factor_ok(float v) { return v > 1e-30f && v < 1e30f; }
+
+// Bin key of src/main.cpp:491-540 with the same FP64 results:
+// width = (max-min)*1.01, offset = -min (or fabs(min)), bin = floor(((x+offset)/width)*300).
+// The FP32 quotient is off by less than 4 * 2^-24 of itself (conversion,
+// factor, product; the FP64 roundings of the exact sequence are far smaller),
+// which is below 1e-4 of a bin for bins up to 300; 1e-3 is required.
+__global__ void __launch_bounds__(kThreads) visit_keys_kernel(
+    const double* __restrict__ x, const double* __restrict__ y, uint32_t n,
+    const BBox* __restrict__ bb, uint32_t* __restrict__ keys, int passes,
+    uint32_t* __restrict__ hist, DeviceStatus* st) {
+    __shared__ DigitCounts s_h;
+    __shared__ double s_p[4];
+    __shared__ float s_f[2];
+    if (threadIdx.x < 2) {
+        const double mn = threadIdx.x ? bb->miny : bb->minx, mx = threadIdx.x ? bb->maxy : bb->maxx;
+        const double w = __dmul_rn(__dsub_rn(mx, mn), 1.01);
+        s_p[threadIdx.x] = w;
+        s_p[2 + threadIdx.x] = (mn > 0) ? -mn : fabs(mn);
+        s_f[threadIdx.x] = (float)((double)kVisitBins / w);
+    }
+    counts_clear(s_h, passes);
+    auto bin = [&](double v, int axis) {
+        const double a = __dadd_rn(v, s_p[2 + axis]);
+        const float r = (float)a * s_f[axis];
+        bool sure;
+        const float f = floor_if_sure(r, 1e-3f, &sure);
+        if (sure && factor_ok(s_f[axis]) && f >= 0.0f && f <= (float)(kVisitBins - 1)) return (double)f;
+        return floor(__dmul_rn(__ddiv_rn(a, s_p[axis]), (double)kVisitBins));
+    };
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        double fx = bin(x[i], 0), fy = bin(y[i], 1);
+        const bool ok = fx >= 0.0 && fx <= (double)(kVisitBins - 1) && fy >= 0.0 &&
+                        fy <= (double)(kVisitBins - 1);
+        if (!ok) {
+            atomicOr(&st->flags, kStatDegenerate);
+            fx = 0.0;
+            fy = 0.0;
+        }
+        const uint32_t key = (uint32_t)fx * kVisitBins + (uint32_t)fy;
+        keys[i] = key;
+        counts_add(s_h, passes, key);
+    }
+    counts_flush(s_h, passes, hist);
 }
 
 // One warp per box: the bounding box of visit positions [b*mbb, b*mbb+mbb)
@@ -82,105 +130,230 @@ __global__ void mpb_kernel(const double* __restrict__ x, const double* __restric
     if (lane == 0) boxes[b] = MpbBox{x0, x1, y0, y1};
 }
 
-// Cell of v and its subcell (of 2^sub per cell), which only orders the points
-// of a cell.
-__device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, uint32_t nc,
+// Cell of v, floor((v - v0) / w) in FP64, and its subcell (of 2^sub per cell),
+// which only orders the points of a cell.  FP32 decides where its quotient,
+// off by less than 4 * 2^-24 of itself, is surely between two whole numbers.
+__device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, float iw, uint32_t nc,
                                             uint32_t sub, uint32_t* sc) {
-    const double q = __ddiv_rn(__dsub_rn(v, v0), w);
+    const double a = __dsub_rn(v, v0);
+    const float r = (float)a * iw;
+    bool sure;
+    float f32 = floor_if_sure(r, 4e-7f * r + 1e-6f, &sure);
+    const float subs = (float)(1u << sub);
+    if (sure && factor_ok(iw) && f32 >= 0.0f && f32 < 8388608.0f && (uint32_t)f32 < nc) {
+        *sc = (uint32_t)fminf((r - f32) * subs, subs - 1.0f);
+        return (uint32_t)f32;
+    }
+    const double q = __ddiv_rn(a, w);
     double f = floor(q);
     if (!(f >= 0.0)) f = 0.0;
     if (f > (double)(nc - 1)) f = (double)(nc - 1);
-    const float r = (float)(q - f) * (float)(1u << sub);
-    *sc = (uint32_t)fminf(fmaxf(r, 0.f), (float)((1u << sub) - 1u));
+    *sc = (uint32_t)fminf(fmaxf((float)(q - f) * subs, 0.f), subs - 1.0f);
     return (uint32_t)f;
 }
 
-__global__ void grid_keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                 uint32_t n, GridParams g, uint32_t* __restrict__ keys,
-                                 uint32_t* __restrict__ idx) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t sx = 0, sy = 0;
-    uint32_t cx = cell_of(x[i], g.x0, g.w, g.ncx, g.sub, &sx);
-    uint32_t cy = cell_of(y[i], g.y0, g.w, g.ncy, g.sub, &sy);
-    uint32_t key = cy * g.ncx_pad + cx;
-    for (int b = (int)g.sub - 1; b >= 0; b--)
-        key = (key << 2) | (((sy >> b) & 1u) << 1) | ((sx >> b) & 1u);
-    keys[i] = key;
-    idx[i] = i;
-}
-
-// Cell-ordered copies: FP64 coordinates, FP32 coordinates relative to the own
-// cell's origin (the FP64 shift is exact up to one rounding; the FP32
-// conversion adds one more), and the visit position of every point.
-__global__ void grid_gather_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                                   const uint32_t* __restrict__ gorig,
-                                   const uint32_t* __restrict__ pos, uint32_t n, GridParams g,
-                                   uint32_t* __restrict__ gkey, double2* __restrict__ gxy,
-                                   float2* __restrict__ glocal, uint32_t* __restrict__ gpos) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    uint32_t o = gorig[k];
-    double xv = x[o], yv = y[o];
-    uint32_t key = gkey[k];
-    if (g.sub) {
-        key >>= 2u * g.sub;
-        gkey[k] = key;
+__global__ void __launch_bounds__(kThreads) grid_keys_kernel(
+    const double* __restrict__ x, const double* __restrict__ y, uint32_t n, GridParams g,
+    uint32_t* __restrict__ keys, int passes, uint32_t* __restrict__ hist) {
+    __shared__ DigitCounts s_h;
+    counts_clear(s_h, passes);
+    const float iw = (float)(1.0 / g.w);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        uint32_t sx = 0, sy = 0;
+        const uint32_t cx = cell_of(x[i], g.x0, g.w, iw, g.ncx, g.sub, &sx);
+        const uint32_t cy = cell_of(y[i], g.y0, g.w, iw, g.ncy, g.sub, &sy);
+        uint32_t key = cy * g.ncx_pad + cx;
+        for (int b = (int)g.sub - 1; b >= 0; b--)
+            key = (key << 2) | (((sy >> b) & 1u) << 1) | ((sx >> b) & 1u);
+        keys[i] = key;
+        counts_add(s_h, passes, key);
     }
-    uint32_t cy = key / g.ncx_pad, cx = key - cy * g.ncx_pad;
-    double ox = __dadd_rn(g.x0, __dmul_rn((double)cx, g.w));
-    double oy = __dadd_rn(g.y0, __dmul_rn((double)cy, g.w));
-    gxy[k] = make_double2(xv, yv);
-    glocal[k] = make_float2(__double2float_rn(__dsub_rn(xv, ox)),
-                            __double2float_rn(__dsub_rn(yv, oy)));
-    gpos[k] = pos[o];
+    counts_flush(s_h, passes, hist);
 }
 
-// cell_start[key] = first sorted index of each non-empty cell; the rest is
-// filled by a suffix-min so that empty cells point at the next non-empty one.
-__global__ void cell_marks_kernel(const uint32_t* __restrict__ gkey, uint32_t n,
-                                  uint32_t* __restrict__ cell_start, uint64_t ncells) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0) cell_start[ncells] = n;
-    if (k >= n) return;
-    if ((k == 0 || gkey[k] != gkey[k - 1]) && gkey[k] < ncells) cell_start[gkey[k]] = k;
+// Cell-ordered copies of point k: FP64 coordinates, FP32 coordinates relative
+// to the own cell's origin (the FP64 shift is exact up to one rounding; the
+// FP32 conversion adds one more), visit position and multiple-point box.
+__device__ __forceinline__ void gather_point(const OrderArgs& a, uint32_t k, uint32_t key) {
+    const uint32_t o = a.gorig[k];
+    const double xv = a.x[o], yv = a.y[o];
+    const uint32_t cy = key / a.g.ncx_pad, cx = key - cy * a.g.ncx_pad;
+    const double ox = __dadd_rn(a.g.x0, __dmul_rn((double)cx, a.g.w));
+    const double oy = __dadd_rn(a.g.y0, __dmul_rn((double)cy, a.g.w));
+    a.gxy[k] = make_double2(xv, yv);
+    a.glocal[k] = make_float2(__double2float_rn(__dsub_rn(xv, ox)),
+                              __double2float_rn(__dsub_rn(yv, oy)));
+    const uint32_t p = a.pos[o];
+    a.gpos[k] = p;
+    a.gbox[k] = a.mpb[p / a.mbb];
 }
 
-__global__ void tile_flags_kernel(const uint32_t* __restrict__ gkey, uint32_t n, uint32_t G,
-                                  uint32_t tq, uint32_t* __restrict__ flags) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    flags[k] = (k == 0 || (gkey[k] / G) != (gkey[k - 1] / G) || (k % tq) == 0) ? 1u : 0u;
-}
-
-__global__ void tile_write_kernel(const uint32_t* __restrict__ flags,
-                                  const uint32_t* __restrict__ scan, uint32_t n,
-                                  uint32_t* __restrict__ tiles) {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k == 0) tiles[scan[n]] = n;
-    if (k < n && flags[k]) tiles[scan[k]] = k;
-}
-
-__global__ void cell_rows_kernel(const uint32_t* __restrict__ gkey,
-                                 const uint32_t* __restrict__ clist,
-                                 const uint32_t* __restrict__ ncl, uint32_t n, uint32_t ncx_pad,
-                                 uint32_t ncy, uint32_t* __restrict__ crow,
-                                 uint32_t* __restrict__ ccx) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nc = *ncl;
-    if (c == 0) crow[ncy] = nc;
-    if (c >= nc || c >= n) return;
-    const uint32_t key = gkey[clist[c]];
-    const uint32_t cy = key / ncx_pad;
-    ccx[c] = key - cy * ncx_pad;
-    if (cy < ncy && (c == 0 || gkey[clist[c - 1]] / ncx_pad != cy)) crow[cy] = c;
-}
-
-__global__ void point_boxes_kernel(const uint32_t* __restrict__ gpos, uint32_t n,
-                                   const MpbBox* __restrict__ mpb, uint32_t mbb,
-                                   MpbBox* __restrict__ gbox) {
+__global__ void gather_kernel(OrderArgs a) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) gbox[k] = mpb[gpos[k] / mbb];
+    if (k < a.n) gather_point(a, k, k);
+}
+
+// One pass over the sorted keys: the gathers, and the first points of cells
+// and tiles compacted by a single-pass scan (both counts in one state word, 31
+// bits each).  A warp takes 32 * kOrderItems consecutive points.
+constexpr int kOrderItems = 4;
+constexpr uint32_t kOrderTile = kLookThreads * kOrderItems;
+template <bool CELLS, bool TILES>
+__global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookState ls) {
+    const uint32_t tile = lookback_ticket(ls);
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)tile * kOrderTile + wid * (32u * kOrderItems);
+    uint32_t key[kOrderItems], bc[kOrderItems], bt[kOrderItems];
+    unsigned long long mine = 0;  // cells | tiles << 31 of the warp
+#pragma unroll
+    for (int i = 0; i < kOrderItems; i++) {
+        const uint64_t k = base + 32u * i + lane;
+        const bool in = k < a.n;
+        key[i] = in ? a.gkey[k] : 0u;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, key[i], 1);
+        if (lane == 0 && in && k > 0) prev = a.gkey[k - 1];
+        const bool fc = in && (k == 0 || key[i] != prev);
+        const bool ft = in && (k == 0 || (TILES && (key[i] / a.g.G != prev / a.g.G ||
+                                                    (uint32_t)k % a.tq == 0u)));
+        bc[i] = CELLS ? __ballot_sync(0xffffffffu, fc) : 0u;
+        bt[i] = TILES ? __ballot_sync(0xffffffffu, ft) : 0u;
+        mine += (unsigned long long)__popc(bc[i]) | ((unsigned long long)__popc(bt[i]) << 31);
+    }
+    const unsigned long long before = block_lookback(lane == 31 ? mine : 0ull, tile, ls, a.st);
+    uint32_t c0 = (uint32_t)(before & 0x7fffffffull), t0 = (uint32_t)(before >> 31);
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int i = 0; i < kOrderItems; i++) {
+        const uint64_t k64 = base + 32u * i + lane;
+        const uint32_t k = (uint32_t)k64;
+        if (k64 < a.n) {
+            if (CELLS) {
+                const uint32_t c = c0 + __popc(bc[i] & lt);
+                const uint32_t fc = (bc[i] >> lane) & 1u;
+                if (!VDB_GUARD(a.st, c + fc <= a.n, 19, c)) return;
+                a.cscan[k] = c;
+                if (fc) {
+                    a.clist[c] = k;
+                    a.ckey[c] = key[i];
+                    a.ccx[c] = key[i] % a.g.ncx_pad;
+                }
+                if (k == a.n - 1) {
+                    a.cscan[a.n] = c + fc;
+                    a.clist[c + fc] = a.n;
+                }
+                gather_point(a, k, key[i]);
+            }
+            if (TILES) {
+                const uint32_t t = t0 + __popc(bt[i] & lt);
+                const uint32_t ft = (bt[i] >> lane) & 1u;
+                if (!VDB_GUARD(a.st, t + ft <= a.n && t + ft > 0u, 19, t)) return;
+                if (ft) a.tiles[t] = k;
+                a.ptile[k] = t + ft - 1u;
+                if (k == a.n - 1) {
+                    a.tiles[t + ft] = a.n;
+                    *a.ntiles = t + ft;
+                }
+            }
+        }
+        c0 += __popc(bc[i]);
+        t0 += __popc(bt[i]);
+    }
+}
+
+// First cell of ckey[0..ncl) with a key >= v: 33-ary search by a warp.
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* __restrict__ ckey,
+                                                     uint32_t ncl, uint64_t v) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = ncl;
+    while (hi > lo) {
+        const uint32_t len = hi - lo;
+        // probes lo + (len * (lane + 1)) / 33 are increasing and below hi
+        const uint32_t p = lo + (uint32_t)(((uint64_t)len * (lane + 1)) / 33u);
+        const uint32_t below = __ballot_sync(0xffffffffu, (uint64_t)ckey[p] < v);
+        const uint32_t nb = __popc(below);
+        if (nb < 32) hi = __shfl_sync(0xffffffffu, p, (int)nb);
+        if (nb > 0) lo = __shfl_sync(0xffffffffu, p, (int)nb - 1) + 1u;
+    }
+    return lo;
+}
+
+// Dense cell array, one block per kFillCells keys: the block finds its cells
+// among the sorted non-empty ones, drops their first points into shared memory
+// and fills every gap with the next cell's by a suffix minimum.  Each entry is
+// written once (26M cells: 31 us; memset, marks and a three-kernel suffix scan
+// took 170).
+constexpr int kFillItems = 16;
+constexpr uint32_t kFillCells = kThreads * kFillItems;
+__global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t* __restrict__ ckey,
+                                                              const uint32_t* __restrict__ clist,
+                                                              const uint32_t* __restrict__ nclp,
+                                                              uint32_t n, uint64_t entries,
+                                                              uint32_t* __restrict__ cell_start) {
+    __shared__ uint32_t s_v[kFillCells + kFillCells / kFillItems];  // 16 cells and a pad word
+    __shared__ uint32_t s_lim[2], s_warp[kThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const uint64_t c0 = (uint64_t)blockIdx.x * kFillCells;
+    const uint32_t ncl = *nclp;
+    if (wid < 2) {
+        const uint32_t b = warp_lower_bound(ckey, ncl, c0 + (wid ? kFillCells : 0u));
+        if (lane == 0) s_lim[wid] = b;
+    }
+    for (uint32_t i = tid; i < kFillCells + kFillCells / kFillItems; i += kThreads)
+        s_v[i] = 0xffffffffu;
+    __syncthreads();
+    const uint32_t lo = s_lim[0], hi = s_lim[1];
+    const uint32_t next = hi < ncl ? clist[hi] : n;
+    if (lo < hi) {
+        for (uint32_t i = lo + tid; i < hi; i += kThreads) {
+            const uint32_t j = (uint32_t)(ckey[i] - c0);
+            s_v[j + j / kFillItems] = clist[i];
+        }
+        __syncthreads();
+        uint32_t* mine = s_v + tid * (kFillItems + 1);
+        uint32_t m = 0xffffffffu;
+#pragma unroll
+        for (int i = 0; i < kFillItems; i++) m = min(m, mine[i]);
+        // smallest value after this thread's cells (first points ascend)
+        uint32_t suf = m;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_down_sync(0xffffffffu, suf, d);
+            if (lane + d < 32u) suf = min(suf, o);
+        }
+        if (lane == 0) s_warp[wid] = suf;
+        __syncthreads();
+        uint32_t after = __shfl_down_sync(0xffffffffu, suf, 1);
+        if (lane == 31) after = 0xffffffffu;
+        for (uint32_t w = wid + 1; w < kThreads / 32; w++) after = min(after, s_warp[w]);
+        after = min(after, next);
+#pragma unroll
+        for (int i = kFillItems - 1; i >= 0; i--) {
+            after = min(after, mine[i]);
+            mine[i] = after;
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < kFillCells; i += kThreads)
+            if (c0 + i < entries) cell_start[c0 + i] = s_v[i + i / kFillItems];
+    } else {
+        for (uint32_t i = tid; i < kFillCells; i += kThreads)
+            if (c0 + i < entries) cell_start[c0 + i] = next;
+    }
+}
+
+__global__ void cell_rows_kernel(const uint32_t* __restrict__ ckey,
+                                 const uint32_t* __restrict__ nclp, uint32_t ncx_pad, uint32_t ncy,
+                                 uint32_t* __restrict__ crow) {
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r > ncy) return;
+    const uint64_t v = (uint64_t)r * ncx_pad;
+    uint32_t b = 0, e = *nclp;
+    while (b < e) {
+        const uint32_t m = (b + e) >> 1;
+        if ((uint64_t)ckey[m] < v) b = m + 1;
+        else e = m;
+    }
+    crow[r] = b;
 }
 
 __global__ void tile_costs_kernel(GridParams g, const EpsParams* __restrict__ ep,
@@ -242,13 +415,18 @@ __global__ void tile_costs_kernel(GridParams g, const EpsParams* __restrict__ ep
         if (s_acc[i]) atomicAdd(&out[i], s_acc[i]);
 }
 
-__global__ void grid_rekey_kernel(uint32_t* __restrict__ gkey, uint32_t n, uint32_t from,
+__global__ void grid_rekey_kernel(uint32_t* __restrict__ gkey, uint32_t* __restrict__ ckey,
+                                  const uint32_t* __restrict__ ncl, uint32_t n, uint32_t from,
                                   uint32_t to) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t key = gkey[k];
     const uint32_t cy = key / from;
     gkey[k] = cy * to + (key - cy * from);
+    if (k < *ncl) {
+        const uint32_t ck = ckey[k], ry = ck / from;
+        ckey[k] = ry * to + (ck - ry * from);
+    }
 }
 
 }  // namespace
@@ -264,35 +442,23 @@ void launch_tile_costs(const GridParams& g, const EpsParams* ep, const uint32_t*
                                                         clist, ncl, n, out);
 }
 
-void launch_grid_rekey(uint32_t* gkey, uint32_t n, uint32_t ncx_pad_from, uint32_t ncx_pad_to,
-                       cudaStream_t s) {
+void launch_grid_rekey(uint32_t* gkey, uint32_t* ckey, const uint32_t* ncl, uint32_t n,
+                       uint32_t ncx_pad_from, uint32_t ncx_pad_to, cudaStream_t s) {
     if (!n || ncx_pad_from == ncx_pad_to) return;
     VDB_COUNT_LAUNCH();
-    grid_rekey_kernel<<<nblk(n), kThreads, 0, s>>>(gkey, n, ncx_pad_from, ncx_pad_to);
+    grid_rekey_kernel<<<nblk(n), kThreads, 0, s>>>(gkey, ckey, ncl, n, ncx_pad_from, ncx_pad_to);
 }
 
-void launch_point_boxes(const uint32_t* gpos, uint32_t n, const MpbBox* mpb, int mbb,
-                        MpbBox* gbox, cudaStream_t s) {
-    if (!n) return;
-    VDB_COUNT_LAUNCH();
-    point_boxes_kernel<<<nblk(n), kThreads, 0, s>>>(gpos, n, mpb, (uint32_t)mbb, gbox);
-}
-
-void launch_cell_rows(const uint32_t* gkey, const uint32_t* clist, const uint32_t* ncl,
-                      uint32_t n, const GridParams& g, uint32_t* crow, uint32_t* ccx,
-                      cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    cell_rows_kernel<<<nblk(n ? n : 1), kThreads, 0, s>>>(gkey, clist, ncl, n, g.ncx_pad, g.ncy,
-                                                         crow, ccx);
-}
+// Blocks of the key kernels: enough to fill the chip, and for large inputs
+// few enough that adding the digit counts up costs little.
+unsigned key_blocks(uint32_t n) { return std::min<unsigned>(nblk(n), 152u * 8u); }
 
 void launch_visit_keys(const double* x, const double* y, uint32_t n, const BBox* bb,
-                       uint32_t* keys, uint32_t* idx, DeviceStatus* st, cudaStream_t s) {
-    if (n) { VDB_COUNT_LAUNCH(); visit_keys_kernel<<<nblk(n), kThreads, 0, s>>>(x, y, n, bb, keys, idx, st); }
-}
-
-void launch_invert(const uint32_t* order, uint32_t n, uint32_t* inv, cudaStream_t s) {
-    if (n) { VDB_COUNT_LAUNCH(); invert_kernel<<<nblk(n), kThreads, 0, s>>>(order, n, inv); }
+                       uint32_t* keys, uint32_t* hist, DeviceStatus* st, cudaStream_t s) {
+    if (!n) return;
+    VDB_COUNT_LAUNCH();
+    visit_keys_kernel<<<key_blocks(n), kThreads, 0, s>>>(x, y, n, bb, keys, sort_passes(kVisitBits),
+                                                         hist, st);
 }
 
 void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, uint32_t n,
@@ -305,35 +471,53 @@ void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, 
     }
 }
 
-void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g,
-                      uint32_t* keys, uint32_t* idx, cudaStream_t s) {
-    if (n) { VDB_COUNT_LAUNCH(); grid_keys_kernel<<<nblk(n), kThreads, 0, s>>>(x, y, n, g, keys, idx); }
-}
-
-void launch_grid_gather(const double* x, const double* y, const uint32_t* gorig,
-                        const uint32_t* pos, uint32_t n, GridParams g, uint32_t* gkey,
-                        double2* gxy, float2* glocal, uint32_t* gpos, cudaStream_t s) {
-    if (n) VDB_COUNT_LAUNCH();
-    if (n)
-        grid_gather_kernel<<<nblk(n), kThreads, 0, s>>>(x, y, gorig, pos, n, g, gkey, gxy,
-                                                        glocal, gpos);
-}
-
-void launch_cell_marks(const uint32_t* gkey, uint32_t n, uint32_t* cell_start,
-                       uint64_t ncells, cudaStream_t s) {
+void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g, int bits,
+                      uint32_t* keys, uint32_t* hist, cudaStream_t s) {
+    if (!n) return;
     VDB_COUNT_LAUNCH();
-    cell_marks_kernel<<<nblk(n ? n : 1), kThreads, 0, s>>>(gkey, n, cell_start, ncells);
+    grid_keys_kernel<<<key_blocks(n), kThreads, 0, s>>>(x, y, n, g, keys, sort_passes(bits), hist);
 }
 
-void launch_tile_flags(const uint32_t* gkey, uint32_t n, uint32_t G, uint32_t tq,
-                       uint32_t* flags, cudaStream_t s) {
-    if (n) { VDB_COUNT_LAUNCH(); tile_flags_kernel<<<nblk(n), kThreads, 0, s>>>(gkey, n, G, tq, flags); }
+size_t order_state_bytes(uint32_t n) {
+    return look_state_bytes(((uint64_t)n + kOrderTile - 1) / kOrderTile);
 }
 
-void launch_tile_write(const uint32_t* flags, const uint32_t* scan, uint32_t n,
-                       uint32_t* tiles, cudaStream_t s) {
+void launch_order(const OrderArgs& a, bool with_tiles, void* zeroed, cudaStream_t s) {
+    if (!a.n) return;
+    const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
     VDB_COUNT_LAUNCH();
-    tile_write_kernel<<<nblk(n ? n : 1), kThreads, 0, s>>>(flags, scan, n, tiles);
+    if (with_tiles)
+        order_kernel<true, true><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
+    else
+        order_kernel<true, false><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
+}
+
+void launch_tiles(const OrderArgs& a, void* zeroed, cudaStream_t s) {
+    if (!a.n) return;
+    const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
+    VDB_COUNT_LAUNCH();
+    order_kernel<false, true><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
+}
+
+void launch_gather(const OrderArgs& a, cudaStream_t s) {
+    if (!a.n) return;
+    VDB_COUNT_LAUNCH();
+    gather_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+}
+
+void launch_cell_start(const uint32_t* ckey, const uint32_t* clist, const uint32_t* ncl,
+                       uint32_t n, const GridParams& g, uint32_t* cell_start, cudaStream_t s) {
+    const uint64_t entries = g.ncells + 1;
+    VDB_COUNT_LAUNCH();
+    cell_start_kernel<<<(unsigned)((entries + kFillCells - 1) / kFillCells), kThreads, 0, s>>>(
+        ckey, clist, ncl, n, entries, cell_start);
+}
+
+void launch_cell_rows(const uint32_t* ckey, const uint32_t* ncl, const GridParams& g,
+                      uint32_t* crow, cudaStream_t s) {
+    VDB_COUNT_LAUNCH();
+    cell_rows_kernel<<<nblk((uint64_t)g.ncy + 1), kThreads, 0, s>>>(ckey, ncl, g.ncx_pad, g.ncy,
+                                                                   crow);
 }
 
 }  // namespace vdb

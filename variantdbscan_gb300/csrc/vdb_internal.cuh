@@ -264,52 +264,86 @@ static __device__ __forceinline__ uint32_t decode_candidate(const TileSegs& sg, 
 }
 
 // ----------------------------------------------------------------- primitives
-// All launches go to `s`; temporaries come from the caller-provided scratch.
+// All launches go to `s`.  "zeroed" memory is zero at the launch and used up
+// by it.
 
 // Exclusive scan of n uint32 values into uint64 (out has n+1 entries; out[n] = total).
-size_t scan_u32_to_u64_scratch_bytes(uint64_t n);
-void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint64_t n, void* scratch,
-                     cudaStream_t s);
-// Exclusive scan of n uint32 values into uint32 (out has n+1 entries).
-size_t scan_u32_scratch_bytes(uint64_t n);
-void scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, void* scratch, cudaStream_t s);
-// Reverse inclusive min-scan in place: a[i] = min(a[i..n-1]).
-size_t suffix_min_u32_scratch_bytes(uint64_t n);
-void suffix_min_u32(uint32_t* a, uint64_t n, void* scratch, cudaStream_t s);
+size_t scan_state_bytes(uint32_t n);
+void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t n, void* zeroed,
+                     DeviceStatus* st, cudaStream_t s);
 
-// Stable LSD radix sort of (key, value) pairs on the low `bits` key bits.
-size_t radix_sort_scratch_bytes(uint32_t n);
-void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int bits, void* scratch,
-                      cudaStream_t s);
+// Stable LSD radix sort of keys and their indices on the low `bits` key bits.
+// zeroed: sort_zero_bytes, its first sort_passes(bits) * kDigits words holding
+// the keys' digit counts by the time of the call (the kernels that make the
+// keys count them).  okeys (may be null): the sorted keys >> drop; ovals: the
+// indices in key order; oinv (may be null): oinv[index] = its place.
+constexpr int kDigitBits = 9;
+constexpr uint32_t kDigits = 1u << kDigitBits;
+constexpr int kMaxPasses = 4;
+int sort_passes(int bits);
+size_t sort_zero_bytes(uint32_t n, int bits);
+size_t sort_scratch_bytes(uint32_t n);
+void radix_sort(const uint32_t* keys, uint32_t n, int bits, int drop, void* zeroed, void* scratch,
+                uint32_t* okeys, uint32_t* ovals, uint32_t* oinv, DeviceStatus* st,
+                cudaStream_t s);
 
 // ------------------------------------------------------------------ index
+// (zeroed: one word)
 void launch_bbox(const double* x, const double* y, uint32_t n, BBox* out, void* scratch,
-                 cudaStream_t s);
-size_t bbox_scratch_bytes(uint32_t n);
+                 uint32_t* zeroed, cudaStream_t s);
+size_t bbox_scratch_bytes();
+// keys and their digit counts (hist: sort_passes(17) * kDigits zeroed words)
+constexpr int kVisitBits = 17;
 void launch_visit_keys(const double* x, const double* y, uint32_t n, const BBox* bb,
-                       uint32_t* keys, uint32_t* idx, DeviceStatus* st, cudaStream_t s);
-void launch_invert(const uint32_t* order, uint32_t n, uint32_t* inv, cudaStream_t s);
+                       uint32_t* keys, uint32_t* hist, DeviceStatus* st, cudaStream_t s);
 void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, uint32_t n,
                       int mbb, MpbBox* boxes, cudaStream_t s);
-void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g,
-                      uint32_t* keys, uint32_t* idx, cudaStream_t s);
-// gbox[k] = mpb[gpos[k] / mbb]: the multiple-point box of cell-ordered point k
-void launch_point_boxes(const uint32_t* gpos, uint32_t n, const MpbBox* mpb, int mbb,
-                        MpbBox* gbox, cudaStream_t s);
-// (takes the subcell bits off gkey)
-void launch_grid_gather(const double* x, const double* y, const uint32_t* gorig,
-                        const uint32_t* pos, uint32_t n, GridParams g, uint32_t* gkey,
-                        double2* gxy, float2* glocal, uint32_t* gpos, cudaStream_t s);
-// Row directory of a sparse grid: ccx[c] = column of non-empty cell c,
-// crow[r] = first non-empty cell of row >= r (crow[ncy] = number of cells;
-// crow must hold 0xffffffff before the call, then is completed by a suffix min).
-void launch_cell_rows(const uint32_t* gkey, const uint32_t* clist, const uint32_t* ncl,
-                      uint32_t n, const GridParams& g, uint32_t* crow, uint32_t* ccx,
-                      cudaStream_t s);
-void launch_cell_marks(const uint32_t* gkey, uint32_t n, uint32_t* cell_start,
-                       uint64_t ncells, cudaStream_t s);
-void launch_tile_flags(const uint32_t* gkey, uint32_t n, uint32_t G, uint32_t tq,
-                       uint32_t* flags, cudaStream_t s);
+void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g, int bits,
+                      uint32_t* keys, uint32_t* hist, cudaStream_t s);
+
+// The cell order's arrays: per point the coordinates (gxy, FP32 relative to
+// the own cell: glocal), visit position and multiple-point box; the non-empty
+// cells (cscan[k]: cells that start before point k, clist: first points, ckey,
+// ccx: keys and columns; cscan[n] = their number, clist[number] = n) and, with
+// tiles, the tiles (tiles: first points, tiles[number] = n; ptile: tile of
+// every point; *ntiles).
+struct OrderArgs {
+    const double* x;
+    const double* y;
+    const uint32_t* gorig;
+    const uint32_t* pos;
+    const uint32_t* gkey;
+    uint32_t n;
+    GridParams g;
+    double2* gxy;
+    float2* glocal;
+    uint32_t* gpos;
+    const MpbBox* mpb;
+    uint32_t mbb;
+    MpbBox* gbox;
+    uint32_t* cscan;
+    uint32_t* clist;
+    uint32_t* ckey;
+    uint32_t* ccx;
+    uint32_t tq;                // points per tile at most
+    uint32_t* tiles;
+    uint32_t* ptile;
+    uint32_t* ntiles;
+    DeviceStatus* st;
+};
+size_t order_state_bytes(uint32_t n);
+void launch_order(const OrderArgs& a, bool with_tiles, void* zeroed, cudaStream_t s);
+// the tiles alone (another G)
+void launch_tiles(const OrderArgs& a, void* zeroed, cudaStream_t s);
+// gxy, glocal, gpos, gbox alone (no grid: an epsilon without neighbours)
+void launch_gather(const OrderArgs& a, cudaStream_t s);
+// cell_start[key] = first point of the first non-empty cell at or after key
+// (ncells + 1 entries)
+void launch_cell_start(const uint32_t* ckey, const uint32_t* clist, const uint32_t* ncl,
+                       uint32_t n, const GridParams& g, uint32_t* cell_start, cudaStream_t s);
+// crow[r] = first non-empty cell of row >= r (ncy + 1 entries; sparse grids)
+void launch_cell_rows(const uint32_t* ckey, const uint32_t* ncl, const GridParams& g,
+                      uint32_t* crow, cudaStream_t s);
 // Autotuner statistics of tile shapes: for each candidate G = 2^i (cells
 // per tile group), over the non-empty cells that start a group of G cells
 // among about kTuneSamples sampled cells (runs of kTuneRun consecutive
@@ -328,11 +362,8 @@ void launch_tile_costs(const GridParams& g, const EpsParams* ep, const uint32_t*
                        unsigned long long* out, cudaStream_t s);
 // Keys of grid `from` rewritten in the layout of grid `to` (same cells, other
 // padding of the rows: the cell order, hence the sort, is unchanged).
-void launch_grid_rekey(uint32_t* gkey, uint32_t n, uint32_t ncx_pad_from, uint32_t ncx_pad_to,
-                       cudaStream_t s);
-void launch_tile_write(const uint32_t* flags, const uint32_t* scan, uint32_t n,
-                       uint32_t* tiles, cudaStream_t s);
-
+void launch_grid_rekey(uint32_t* gkey, uint32_t* ckey, const uint32_t* ncl, uint32_t n,
+                       uint32_t ncx_pad_from, uint32_t ncx_pad_to, cudaStream_t s);
 // ------------------------------------------------------------------ tables
 struct TableArgs {
     GridParams g;
@@ -438,15 +469,15 @@ static __device__ __forceinline__ void walk_compact_row(
 void launch_count(const TableArgs& a, int nblocks, cudaStream_t s);
 void launch_word_boxes(const TableArgs& a, cudaStream_t s);
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s);
-void launch_tile_words(const TableArgs& a, uint32_t* words, uint32_t* units, int nblocks,
+size_t words_state_bytes(uint32_t n);
+void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
+                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
                        cudaStream_t s);
-void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, int nblocks, cudaStream_t s);
+void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, cudaStream_t s);
 // adds the hash of rows [row_lo, row_hi) of the table to st->table_hash
 // (gorig: input index of every cell-ordered point)
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s);
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s);
-// ptile[k] = t for the points [tiles[t], tiles[t+1]) of every tile t
-void launch_tile_owner(const TableArgs& a, uint32_t* ptile, int nblocks, cudaStream_t s);
 void launch_asym_flags(const TableArgs& a, cudaStream_t s);
 int table_block_threads();
 int table_tile_queries();
@@ -478,8 +509,9 @@ struct ClusterArgs {
     uint32_t* seed;             // per root: min visit position of its cores
     uint32_t* cstart;           // per root: root of the component that starts its cluster
     uint32_t* best;             // per point: earliest cluster start among adjacent cores
-    uint32_t* cluster_no;       // per visit position: clusters started before it (n+1)
-    uint32_t* pos_flag;         // per visit position: a cluster starts there
+    uint32_t* bits;             // visit positions at which clusters start
+    uint32_t* brank;            // starts before each word of bits
+    uint32_t nw;                // start_words(n)
     const AsymPair* asym;
     const uint32_t* asym_count;
     uint32_t asym_cap;
@@ -504,7 +536,7 @@ struct CellArgs {
     const EpsParams* ep;
     const uint32_t* cell_start;
     const uint32_t* crow;       // sparse grids: row directory (see cell_row_range)
-    uint32_t* ccx;              // column of every non-empty cell
+    const uint32_t* ccx;        // column of every non-empty cell
     uint2* crng;                // [2*rho+1][n] neighbour cells per row
     const uint32_t* clist;      // first point of every non-empty cell (ncl+1 entries)
     const uint32_t* ncl;        // device scalar
@@ -574,8 +606,7 @@ void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphCondition
 void launch_store_eps(EpsParams* dst, const EpsParams& v, cudaStream_t s);
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s);
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s);
-void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, void* scan_scratch,
-                      cudaStream_t s);
+void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, cudaStream_t s);
 void launch_border_and_write(const ClusterArgs& a, int nblocks, cudaStream_t s);
 // the two halves of launch_border_and_write: border pull over rows
 // [row_lo, row_hi) of the table held in nbr (from off_base), then the

@@ -1,0 +1,138 @@
+// Single-pass prefix sums (decoupled look-back, Merrill and Garland 2016): a
+// tile publishes its own sum, then adds up what the tiles before it have
+// published, back to the first that knows its whole prefix.  Tiles are taken
+// by ticket, so every tile before a running one has started.  A state is one
+// 64-bit word (two flag bits, 62 bits of sum), so a plain load sees both.
+// States and tickets are zero at the launch.
+#pragma once
+
+#include <algorithm>
+
+#include "vdb_internal.cuh"
+
+namespace vdb {
+
+constexpr int kLookThreads = 256;
+constexpr unsigned long long kLookSum = 1ull << 62;     // the tile's own sum
+constexpr unsigned long long kLookPrefix = 2ull << 62;  // the sum of all tiles up to this one
+constexpr unsigned long long kLookMask = (1ull << 62) - 1ull;
+// Polls of one state before the wait is given up (and reported as a failed
+// index guard): far above what a running tile takes to publish.
+constexpr int kLookPolls = 1 << 22;
+constexpr uint32_t kLookSite = 20;
+
+struct LookState {
+    uint32_t* ticket;
+    unsigned long long* tiles;
+};
+inline size_t look_state_bytes(uint64_t ntiles) { return 16 + (size_t)ntiles * 8; }
+inline LookState look_state(void* zeroed) {
+    return LookState{(uint32_t*)zeroed, (unsigned long long*)((char*)zeroed + 16)};
+}
+
+static __device__ __forceinline__ unsigned long long look_load(const unsigned long long* p) {
+    return *(const volatile unsigned long long*)p;
+}
+static __device__ __forceinline__ void look_store(unsigned long long* p, unsigned long long v) {
+    *(volatile unsigned long long*)p = v;
+}
+// A published state of *p (waits for it).
+static __device__ __forceinline__ unsigned long long look_wait(const unsigned long long* p,
+                                                               DeviceStatus* st) {
+    unsigned long long v = look_load(p);
+    for (int i = 0; (v >> 62) == 0ull && i < kLookPolls; i++) v = look_load(p);
+    if ((v >> 62) == 0ull) {
+        guard_fail(st, kLookSite, 0);
+        v = kLookPrefix;
+    }
+    return v;
+}
+
+// The block's tile (every thread).
+static __device__ __forceinline__ uint32_t lookback_ticket(LookState ls) {
+    __shared__ uint32_t s_ticket;
+    if (threadIdx.x == 0) s_ticket = atomicAdd(ls.ticket, 1u);
+    __syncthreads();
+    return s_ticket;
+}
+
+// Exclusive prefix of this thread's v over all tiles' threads (blocks of
+// kLookThreads; the first warp looks back, 32 tiles at a time).
+static __device__ __forceinline__ unsigned long long block_lookback(unsigned long long v,
+                                                                    uint32_t tile, LookState ls,
+                                                                    DeviceStatus* st) {
+    __shared__ unsigned long long s_sum[kLookThreads / 32];
+    __shared__ unsigned long long s_before;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __syncthreads();  // (a call before this one has read the shared words)
+    unsigned long long incl = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= (uint32_t)d) incl += t;
+    }
+    if (lane == 31) s_sum[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+        unsigned long long all = 0;
+#pragma unroll
+        for (int w = 0; w < kLookThreads / 32; w++) all += s_sum[w];
+        unsigned long long before = 0;
+        if (tile == 0) {
+            if (lane == 0) look_store(&ls.tiles[0], kLookPrefix | all);
+        } else {
+            if (lane == 0) look_store(&ls.tiles[tile], kLookSum | all);
+            for (int64_t b = (int64_t)tile - 1; b >= 0; b -= 32) {
+                const int64_t i = b - (int64_t)lane;
+                const unsigned long long s = i >= 0 ? look_wait(&ls.tiles[i], st) : kLookPrefix;
+                const uint32_t full = __ballot_sync(0xffffffffu, (s >> 62) == 2ull);
+                const uint32_t upto = full ? (uint32_t)__ffs(full) - 1u : 31u;
+                unsigned long long add = lane <= upto ? s & kLookMask : 0ull;
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xffffffffu, add, d);
+                before += add;
+                if (full) break;
+            }
+            if (lane == 0) look_store(&ls.tiles[tile], kLookPrefix | (before + all));
+        }
+        if (lane == 0) s_before = before;
+    }
+    __syncthreads();
+    unsigned long long r = s_before + incl - v;
+    for (uint32_t w = 0; w < wid; w++) r += s_sum[w];
+    return r;
+}
+
+// The same for one counter per thread: states of tile t at p[t * stride].
+static __device__ __forceinline__ unsigned long long digit_lookback(uint32_t v, uint32_t tile,
+                                                                    unsigned long long* p,
+                                                                    uint32_t stride,
+                                                                    DeviceStatus* st) {
+    if (tile == 0) {
+        look_store(p, kLookPrefix | v);
+        return 0;
+    }
+    look_store(p + (size_t)tile * stride, kLookSum | v);
+    unsigned long long before = 0;
+    for (int64_t t = (int64_t)tile - 1; t >= 0;) {
+        // four states at once: their loads overlap
+        unsigned long long s[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            s[j] = t - j >= 0 ? look_load(p + (size_t)(t - j) * stride) : kLookPrefix;
+        bool done = false;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (done) continue;
+            if ((s[j] >> 62) == 0ull) s[j] = look_wait(p + (size_t)(t - j) * stride, st);
+            before += s[j] & kLookMask;
+            done = (s[j] >> 62) == 2ull;
+        }
+        if (done) break;
+        t -= 4;
+    }
+    look_store(p + (size_t)tile * stride, kLookPrefix | (before + v));
+    return before;
+}
+
+}  // namespace vdb

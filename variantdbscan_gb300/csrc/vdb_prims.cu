@@ -1,289 +1,217 @@
-// Device primitives: block-decomposed scans, a stable LSD radix sort of
-// (key, value) pairs and the dataset bounding-box reduction.
+// Device primitives: single-pass scans, a stable LSD radix sort of (key, value)
+// pairs and the dataset bounding-box reduction.
 #include <float.h>
 
-#include "vdb_internal.cuh"
+#include "vdb_lookback.cuh"
 
 namespace vdb {
 
 std::atomic<unsigned long long> g_launches{0};
 
+// ------------------------------------------------------------------ scan
+//
+// One kernel: blocks take their tiles in order (a ticket), publish the tile's
+// sum and look back over the tiles before it (block_lookback), so the input is
+// read once and a scan is one launch.  With three kernels per scan the small
+// datasets' calls spent a third of their launches on scans.
+
 namespace {
 
-constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr uint32_t kScanTile = kLookThreads * kScanItems;
 
-struct OpSum {
-    template <class T>
-    __device__ static T apply(T a, T b) { return a + b; }
-    template <class T>
-    __device__ static T identity() { return T(0); }
-};
-struct OpMin {
-    template <class T>
-    __device__ static T apply(T a, T b) { return a < b ? a : b; }
-    template <class T>
-    __device__ static T identity() { return T(~T(0)); }
-};
-
-// Inclusive block scan of one value per thread; returns the inclusive prefix
-// and writes the block aggregate to *total.
-template <class T, class Op>
-__device__ T block_inclusive(T v, T* total) {
-    __shared__ T warp_tot[kScanThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kLookThreads) scan_kernel(const uint32_t* __restrict__ in,
+                                                            unsigned long long* __restrict__ out,
+                                                            uint32_t n, LookState ls,
+                                                            DeviceStatus* st) {
+    const uint32_t tile = lookback_ticket(ls);
+    const uint64_t base = (uint64_t)tile * kScanTile + threadIdx.x * kScanItems;
+    uint32_t v[kScanItems];
+    unsigned long long sum = 0;
+    if (base + kScanItems <= n) {
+        const uint4 a = *reinterpret_cast<const uint4*>(in + base);
+        const uint4 b = *reinterpret_cast<const uint4*>(in + base + 4);
+        v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+        v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        T o = __shfl_up_sync(0xffffffffu, v, d);
-        if (lane >= d) v = Op::apply(o, v);
+        for (int i = 0; i < kScanItems; i++) v[i] = base + i < n ? in[base + i] : 0u;
     }
-    if (lane == 31) warp_tot[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        T w = lane < kScanThreads / 32 ? warp_tot[lane] : Op::template identity<T>();
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            T o = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= d) w = Op::apply(o, w);
-        }
-        if (lane < kScanThreads / 32) warp_tot[lane] = w;
-    }
-    __syncthreads();
-    if (wid > 0) v = Op::apply(warp_tot[wid - 1], v);
-    *total = warp_tot[kScanThreads / 32 - 1];
-    __syncthreads();
-    return v;
-}
-
-// Exclusive block scan built on the inclusive one; *total = block aggregate.
-template <class T, class Op>
-__device__ T block_exclusive(T v, T* total) {
-    __shared__ T wl[kScanThreads / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    T inc = block_inclusive<T, Op>(v, total);
-    T prev = __shfl_up_sync(0xffffffffu, inc, 1);
-    if (lane == 31) wl[wid] = inc;
-    __syncthreads();
-    T exc = lane > 0 ? prev : (wid > 0 ? wl[wid - 1] : Op::template identity<T>());
-    __syncthreads();
-    return exc;
-}
-
-template <bool Rev>
-__device__ __forceinline__ uint64_t phys(uint64_t i, uint64_t n) { return Rev ? n - 1 - i : i; }
-
-template <class TIn, class TOut, class Op, bool Rev>
-__global__ void scan_reduce_kernel(const TIn* in, uint64_t n, TOut* part) {
-    uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-    TOut acc = Op::template identity<TOut>();
-    for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = base + (uint64_t)k * kScanThreads + threadIdx.x;
-        if (i < n) acc = Op::apply(acc, (TOut)in[phys<Rev>(i, n)]);
-    }
-    TOut tot;
-    block_inclusive<TOut, Op>(acc, &tot);
-    if (threadIdx.x == 0) part[blockIdx.x] = tot;
-}
-
-// Exclusive scan of the per-block aggregates (one block, loops with a carry).
-template <class TOut, class Op>
-__global__ void scan_parts_kernel(TOut* part, uint64_t nparts, TOut* total_out) {
-    TOut carry = Op::template identity<TOut>();
-    for (uint64_t b = 0; b < nparts; b += kScanThreads) {
-        uint64_t i = b + threadIdx.x;
-        TOut v = i < nparts ? part[i] : Op::template identity<TOut>();
-        TOut tot;
-        TOut exc = block_exclusive<TOut, Op>(v, &tot);
-        if (i < nparts) part[i] = Op::apply(carry, exc);
-        carry = Op::apply(carry, tot);
-    }
-    if (threadIdx.x == 0 && total_out) *total_out = carry;
-}
-
-template <class TIn, class TOut, class Op, bool Rev, bool Inclusive>
-__global__ void scan_apply_kernel(const TIn* in, uint64_t n, const TOut* part, TOut* out) {
-    uint64_t base = (uint64_t)blockIdx.x * kScanTile + (uint64_t)threadIdx.x * kScanItems;
-    TOut v[kScanItems];
-    TOut acc = Op::template identity<TOut>();
+    for (int i = 0; i < kScanItems; i++) sum += v[i];
+    unsigned long long run = block_lookback(sum, tile, ls, st);
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = base + k;
-        TOut x = i < n ? (TOut)in[phys<Rev>(i, n)] : Op::template identity<TOut>();
-        v[k] = x;
-        acc = Op::apply(acc, x);
+    for (int i = 0; i < kScanItems; i++) {
+        if (base + i < n) out[base + i] = run;
+        run += v[i];
+        if (base + i + 1 == n) out[n] = run;
     }
-    TOut tot;
-    TOut run = Op::apply(part[blockIdx.x], block_exclusive<TOut, Op>(acc, &tot));
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        uint64_t i = base + k;
-        if (Inclusive) run = Op::apply(run, v[k]);
-        if (i < n) out[phys<Rev>(i, n)] = run;
-        if (!Inclusive) run = Op::apply(run, v[k]);
-    }
-}
-
-uint64_t num_scan_blocks(uint64_t n) { return (n + kScanTile - 1) / kScanTile; }
-
-template <class TIn, class TOut, class Op, bool Rev, bool Inclusive>
-void scan_run(const TIn* in, TOut* out, uint64_t n, void* scratch, TOut* total_out,
-              cudaStream_t s) {
-    uint64_t nb = num_scan_blocks(n);
-    TOut* part = (TOut*)scratch;
-    if (nb == 0) {
-        VDB_COUNT_LAUNCH();
-        scan_parts_kernel<TOut, Op><<<1, kScanThreads, 0, s>>>(part, 0, total_out);
-        return;
-    }
-    VDB_COUNT_LAUNCH();
-    scan_reduce_kernel<TIn, TOut, Op, Rev><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, part);
-    VDB_COUNT_LAUNCH();
-    scan_parts_kernel<TOut, Op><<<1, kScanThreads, 0, s>>>(part, nb, total_out);
-    VDB_COUNT_LAUNCH();
-    scan_apply_kernel<TIn, TOut, Op, Rev, Inclusive>
-        <<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, part, out);
 }
 
 }  // namespace
 
-size_t scan_u32_to_u64_scratch_bytes(uint64_t n) { return (num_scan_blocks(n) + 1) * 8; }
-size_t scan_u32_scratch_bytes(uint64_t n) { return (num_scan_blocks(n) + 1) * 4; }
-size_t suffix_min_u32_scratch_bytes(uint64_t n) { return (num_scan_blocks(n) + 1) * 4; }
+size_t scan_state_bytes(uint32_t n) { return look_state_bytes((n + kScanTile - 1) / kScanTile); }
 
-void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint64_t n, void* scratch,
-                     cudaStream_t s) {
-    scan_run<uint32_t, unsigned long long, OpSum, false, false>(in, out, n, scratch, out + n, s);
-}
-
-void scan_u32(const uint32_t* in, uint32_t* out, uint64_t n, void* scratch, cudaStream_t s) {
-    scan_run<uint32_t, uint32_t, OpSum, false, false>(in, out, n, scratch, out + n, s);
-}
-
-void suffix_min_u32(uint32_t* a, uint64_t n, void* scratch, cudaStream_t s) {
-    scan_run<uint32_t, uint32_t, OpMin, true, true>(a, a, n, scratch, (uint32_t*)nullptr, s);
+void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t n, void* state,
+                     DeviceStatus* st, cudaStream_t s) {
+    if (!n) return;
+    const uint32_t nb = (n + kScanTile - 1) / kScanTile;
+    VDB_COUNT_LAUNCH();
+    scan_kernel<<<nb, kLookThreads, 0, s>>>(in, out, n, look_state(state), st);
 }
 
 // ------------------------------------------------------------------ radix sort
+//
+// Digits of 9 bits (27-bit keys take three passes, the 17 bits of the visit
+// order two).  The kernel that makes the keys also counts all their digits
+// (SortPlan::hist), so a pass is one kernel: a block ranks its tile's keys per
+// digit, looks back over the tiles before it, a thread per digit, and writes
+// every pair to its place.  Pairs travel as 8 bytes between passes; the last
+// pass writes the two arrays.  Measured on 1M keys of 25 bits: 3 launches and
+// 85 us against 20 launches and 140 us with separate histogram and scan
+// kernels per 8-bit digit.
 
 namespace {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortRounds = 16;                 // items per thread per tile
-constexpr int kSortRoundsSmall = 4;             // the same for sorts of <= 2^18 keys
-constexpr uint32_t kSortSmall = 1u << 18;
-constexpr int kRadix = 256;
+constexpr int kSortWarps = kDigits / 32;  // a thread per digit
 
-// Rounds per tile: small sorts take short tiles, so that their few blocks
-// become more blocks with a quarter of the serial rounds each.
-int sort_rounds(uint32_t n) { return n <= kSortSmall ? kSortRoundsSmall : kSortRounds; }
-
-__global__ void radix_hist_kernel(const uint32_t* keys, uint32_t n, int shift, uint32_t nblocks,
-                                  int rounds, uint32_t* hist) {
-    __shared__ uint32_t h[kRadix];
-    h[threadIdx.x] = 0;
+template <int ITEMS>
+__global__ void __launch_bounds__(kDigits) radix_pass_kernel(
+    const uint32_t* __restrict__ keys_in, const uint2* __restrict__ in, uint2* __restrict__ out,
+    uint32_t* __restrict__ okeys, uint32_t* __restrict__ ovals, uint32_t* __restrict__ oinv,
+    uint32_t n, int shift, int drop, const uint32_t* __restrict__ hist,
+    unsigned long long* __restrict__ state, uint32_t* __restrict__ ticket, DeviceStatus* st) {
+    __shared__ uint16_t s_cnt[kSortWarps][kDigits];
+    __shared__ uint32_t s_base[kDigits];
+    __shared__ uint32_t s_warp[kSortWarps];
+    __shared__ uint32_t s_tile;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    for (uint32_t i = tid; i < kSortWarps * kDigits / 2; i += kDigits)
+        reinterpret_cast<uint32_t*>(s_cnt)[i] = 0u;
+    if (tid == 0) s_tile = atomicAdd(ticket, 1u);
+    // first place of every digit: exclusive scan of the histogram
+    const uint32_t h = hist[tid];
+    uint32_t incl = h;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= (uint32_t)d) incl += v;
+    }
+    if (lane == 31) s_warp[wid] = incl;
     __syncthreads();
-    uint32_t base = blockIdx.x * (uint32_t)(kSortThreads * rounds);
-    for (int r = 0; r < rounds; r++) {
-        uint32_t i = base + r * kSortThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & (kRadix - 1)], 1u);
+    uint32_t gbase = incl - h;
+    for (uint32_t w = 0; w < wid; w++) gbase += s_warp[w];
+    const uint32_t tile = s_tile;
+    // a warp takes 32 * ITEMS consecutive keys; item i of lane l is number 32 i + l
+    const uint64_t seg = (uint64_t)tile * (kDigits * ITEMS) + wid * (32u * ITEMS);
+    uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const uint64_t k = seg + 32u * i + lane;
+        key[i] = val[i] = 0;
+        if (k < n) {
+            if (keys_in) {
+                key[i] = keys_in[k];
+                val[i] = (uint32_t)k;
+            } else {
+                const uint2 p = in[k];
+                key[i] = p.x;
+                val[i] = p.y;
+            }
+        }
+    }
+    const uint32_t lt = (1u << lane) - 1u;
+    uint16_t* cnt = s_cnt[wid];
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        const bool valid = seg + 32u * i + lane < n;
+        const uint32_t d = valid ? (key[i] >> shift) & (kDigits - 1u) : kDigits + lane;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        uint32_t b = 0;
+        if (valid) b = cnt[d];
+        __syncwarp();
+        if (valid && (peers & lt) == 0u) cnt[d] = (uint16_t)(b + __popc(peers));
+        __syncwarp();
+        rank[i] = b + __popc(peers & lt);
     }
     __syncthreads();
-    hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+    // thread = digit: the warps' counts become offsets within the tile
+    uint32_t total = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++) {
+        const uint32_t c = s_cnt[w][tid];
+        s_cnt[w][tid] = (uint16_t)total;
+        total += c;
+    }
+    s_base[tid] = gbase + (uint32_t)digit_lookback(total, tile, state + tid, kDigits, st);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; i++) {
+        if (seg + 32u * i + lane >= n) continue;
+        const uint32_t d = (key[i] >> shift) & (kDigits - 1u);
+        const uint32_t dst = s_base[d] + cnt[d] + rank[i];
+        if (dst >= n) continue;  // (only after a failed look-back, which is reported)
+        if (out) {
+            out[dst] = make_uint2(key[i], val[i]);
+        } else {
+            if (okeys) okeys[dst] = key[i] >> drop;
+            ovals[dst] = val[i];
+            if (oinv) oinv[val[i]] = dst;
+        }
+    }
 }
 
-// Stable scatter: inside a tile, items keep their order (rounds of 256
-// consecutive items; ranks within a warp from __match_any_sync, across warps
-// from a per-digit prefix over the warps).
-__global__ void radix_scatter_kernel(const uint32_t* keys, const uint32_t* vals, uint32_t n,
-                                     int shift, uint32_t nblocks, int rounds,
-                                     const uint32_t* hist_scan, uint32_t* okeys,
-                                     uint32_t* ovals) {
-    constexpr int W = kSortThreads / 32;
-    __shared__ uint32_t gbase[kRadix];
-    __shared__ uint32_t base[kRadix];
-    __shared__ uint32_t wcnt[W][kRadix];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    gbase[threadIdx.x] = hist_scan[threadIdx.x * nblocks + blockIdx.x];
-    base[threadIdx.x] = 0;
-    const uint32_t lt = (1u << lane) - 1u;
-    uint32_t tile = blockIdx.x * (uint32_t)(kSortThreads * rounds);
-    for (int r = 0; r < rounds; r++) {
-#pragma unroll
-        for (int w = 0; w < W; w++) wcnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        uint32_t i = tile + r * kSortThreads + threadIdx.x;
-        bool valid = i < n;
-        uint32_t k = valid ? keys[i] : 0u;
-        uint32_t v = valid ? vals[i] : 0u;
-        uint32_t d = valid ? ((k >> shift) & (kRadix - 1)) : (kRadix + lane);
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
-        uint32_t rank = __popc(peers & lt);
-        if (valid && rank == 0) wcnt[wid][d] = __popc(peers);
-        __syncthreads();
-        {
-            uint32_t acc = base[threadIdx.x];
-#pragma unroll
-            for (int w = 0; w < W; w++) {
-                uint32_t c = wcnt[w][threadIdx.x];
-                wcnt[w][threadIdx.x] = acc;
-                acc += c;
-            }
-            base[threadIdx.x] = acc;
-        }
-        __syncthreads();
-        if (valid) {
-            uint32_t dst = gbase[d] + wcnt[wid][d] + rank;
-            okeys[dst] = k;
-            ovals[dst] = v;
-        }
-        __syncthreads();
-    }
+// Keys per thread: short tiles for small sorts, so that they spread over the
+// chip (50k keys: 49 tiles of 1,024 instead of 13 of 4,096).
+int sort_items(uint32_t n) { return n <= (1u << 18) ? 2 : n <= (1u << 20) ? 8 : 16; }
+
+template <int ITEMS>
+void run_pass(uint32_t nb, const uint32_t* keys_in, const uint2* in, uint2* out, uint32_t* okeys,
+              uint32_t* ovals, uint32_t* oinv, uint32_t n, int shift, int drop,
+              const uint32_t* hist, unsigned long long* state, uint32_t* ticket, DeviceStatus* st,
+              cudaStream_t s) {
+    VDB_COUNT_LAUNCH();
+    radix_pass_kernel<ITEMS><<<nb, kDigits, 0, s>>>(keys_in, in, out, okeys, ovals, oinv, n, shift,
+                                                    drop, hist, state, ticket, st);
+}
+
+uint32_t sort_blocks(uint32_t n) {
+    const uint32_t tile = (uint32_t)(kDigits * sort_items(n));
+    return (uint32_t)(((uint64_t)n + tile - 1) / tile);
 }
 
 }  // namespace
 
-size_t radix_sort_scratch_bytes(uint32_t n) {
-    const uint64_t tile = (uint64_t)kSortThreads * sort_rounds(n);
-    uint64_t nb = ((uint64_t)n + tile - 1) / tile;
-    uint64_t h = nb * kRadix;
-    size_t b = 0;
-    b += (size_t)n * 8;                     // alternate key/value buffers
-    b += (h + 1) * 4 * 2;                   // histogram + its scan
-    b += scan_u32_scratch_bytes(h);
-    return b + 256;
-}
+// (keys of no bits are all equal: one pass puts every pair in its place)
+int sort_passes(int bits) { return std::max(1, (bits + kDigitBits - 1) / kDigitBits); }
 
-void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int bits, void* scratch,
-                      cudaStream_t s) {
-    if (n <= 1 || bits <= 0) return;
-    const int rounds = sort_rounds(n);
-    const uint32_t tile = (uint32_t)(kSortThreads * rounds);
-    uint32_t nb = (uint32_t)(((uint64_t)n + tile - 1) / tile);
-    uint64_t h = (uint64_t)nb * kRadix;
-    char* p = (char*)scratch;
-    uint32_t* k2 = (uint32_t*)p; p += (size_t)n * 4;
-    uint32_t* v2 = (uint32_t*)p; p += (size_t)n * 4;
-    uint32_t* hist = (uint32_t*)p; p += (h + 1) * 4;
-    uint32_t* hscan = (uint32_t*)p; p += (h + 1) * 4;
-    void* sscratch = p;
-    int passes = (bits + 7) / 8;
-    uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
-    for (int ps = 0; ps < passes; ps++) {
-        int shift = ps * 8;
-        VDB_COUNT_LAUNCH();
-        radix_hist_kernel<<<nb, kSortThreads, 0, s>>>(ka, n, shift, nb, rounds, hist);
-        scan_u32(hist, hscan, h, sscratch, s);
-        VDB_COUNT_LAUNCH();
-        radix_scatter_kernel<<<nb, kSortThreads, 0, s>>>(ka, va, n, shift, nb, rounds, hscan, kb,
-                                                         vb);
-        uint32_t* t;
-        t = ka; ka = kb; kb = t;
-        t = va; va = vb; vb = t;
-    }
-    if (ka != keys) {
-        cudaMemcpyAsync(keys, ka, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(vals, va, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);
+// zeroed memory of a sort: digit counts, tickets, look-back states
+size_t sort_zero_bytes(uint32_t n, int bits) {
+    const size_t p = (size_t)sort_passes(bits);
+    return p * kDigits * 4 + 256 + p * (size_t)sort_blocks(n) * kDigits * 8;
+}
+size_t sort_scratch_bytes(uint32_t n) { return (size_t)n * 16; }
+
+void radix_sort(const uint32_t* keys, uint32_t n, int bits, int drop, void* zeroed, void* scratch,
+                uint32_t* okeys, uint32_t* ovals, uint32_t* oinv, DeviceStatus* st,
+                cudaStream_t s) {
+    if (!n) return;
+    const int p = sort_passes(bits);
+    const uint32_t nb = sort_blocks(n);
+    uint32_t* hist = (uint32_t*)zeroed;
+    uint32_t* ticket = hist + (size_t)p * kDigits;
+    unsigned long long* state = (unsigned long long*)((char*)zeroed + (size_t)p * kDigits * 4 + 256);
+    uint2* buf[2] = {(uint2*)scratch, (uint2*)scratch + n};
+    const int items = sort_items(n);
+    for (int i = 0; i < p; i++) {
+        const bool last = i == p - 1;
+        const uint32_t* kin = i == 0 ? keys : nullptr;
+        const uint2* in = i == 0 ? nullptr : buf[(i - 1) & 1];
+        uint2* out = last ? nullptr : buf[i & 1];
+        auto pass = items == 2 ? run_pass<2> : items == 8 ? run_pass<8> : run_pass<16>;
+        pass(nb, kin, in, out, last ? okeys : nullptr, last ? ovals : nullptr, last ? oinv : nullptr,
+             n, i * kDigitBits, last ? drop : 0, hist + (size_t)i * kDigits,
+             state + (size_t)i * nb * kDigits, ticket + i, st, s);
     }
 }
 
@@ -318,6 +246,7 @@ __device__ BoxAcc box_block_reduce(BoxAcc v) {
         o.bad = __shfl_down_sync(0xffffffffu, v.bad, d);
         v = box_merge(v, o);
     }
+    __syncthreads();
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -326,9 +255,16 @@ __device__ BoxAcc box_block_reduce(BoxAcc v) {
     return v;
 }
 
-__global__ void bbox_partial_kernel(const double* x, const double* y, uint32_t n, BoxAcc* part) {
-    BoxAcc a{DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, 0u};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+// The block that finishes last (done, zero at the launch) merges the parts.
+__global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const double* __restrict__ x,
+                                                           const double* __restrict__ y,
+                                                           uint32_t n, BoxAcc* part,
+                                                           uint32_t* done, BBox* out) {
+    __shared__ bool s_last;
+    const BoxAcc none{DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, 0u};
+    BoxAcc a = none;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
         double xi = x[i], yi = y[i];
         if (!isfinite(xi) || !isfinite(yi)) a.bad = 1u;
         a.minx = fmin(a.minx, xi);
@@ -337,12 +273,19 @@ __global__ void bbox_partial_kernel(const double* x, const double* y, uint32_t n
         a.maxy = fmax(a.maxy, yi);
     }
     a = box_block_reduce(a);
-    if (threadIdx.x == 0) part[blockIdx.x] = a;
-}
-
-__global__ void bbox_final_kernel(const BoxAcc* part, int nparts, BBox* out) {
-    BoxAcc a{DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, 0u};
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) a = box_merge(a, part[i]);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = a;
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    a = none;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+        const volatile BoxAcc* p = part + i;
+        a = box_merge(a, BoxAcc{p->minx, p->maxx, p->miny, p->maxy, p->bad});
+    }
     a = box_block_reduce(a);
     if (threadIdx.x == 0) {
         // src/main.cpp:465-488: min starts at DBL_MAX, max at DBL_MIN
@@ -357,22 +300,17 @@ __global__ void bbox_final_kernel(const BoxAcc* part, int nparts, BBox* out) {
     }
 }
 
-constexpr int kBoxBlocks = 1024;
+constexpr int kBoxBlocks = 608;  // four per SM
 
 }  // namespace
 
-size_t bbox_scratch_bytes(uint32_t) { return sizeof(BoxAcc) * kBoxBlocks; }
+size_t bbox_scratch_bytes() { return sizeof(BoxAcc) * kBoxBlocks; }
 
 void launch_bbox(const double* x, const double* y, uint32_t n, BBox* out, void* scratch,
-                 cudaStream_t s) {
-    int nb = (int)((n + kBoxThreads - 1) / kBoxThreads);
-    if (nb > kBoxBlocks) nb = kBoxBlocks;
-    if (nb < 1) nb = 1;
-    BoxAcc* part = (BoxAcc*)scratch;
+                 uint32_t* zeroed, cudaStream_t s) {
+    const int nb = (int)std::max<uint32_t>(1u, std::min<uint32_t>(kBoxBlocks, (n + 511u) / 512u));
     VDB_COUNT_LAUNCH();
-    bbox_partial_kernel<<<nb, kBoxThreads, 0, s>>>(x, y, n, part);
-    VDB_COUNT_LAUNCH();
-    bbox_final_kernel<<<1, kBoxThreads, 0, s>>>(part, nb, out);
+    bbox_kernel<<<nb, kBoxThreads, 0, s>>>(x, y, n, (BoxAcc*)scratch, zeroed, out);
 }
 
 }  // namespace vdb

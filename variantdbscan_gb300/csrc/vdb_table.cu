@@ -33,7 +33,7 @@
 // afterwards from the asymmetric-pair list.  When the bitmap does not fit in
 // device memory, the fill kernel (blocks of kTT threads, kQPT queries each)
 // re-tests the candidates and writes the table directly.
-#include "vdb_internal.cuh"
+#include "vdb_lookback.cuh"
 
 namespace vdb {
 
@@ -1355,72 +1355,80 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
     if (lane == 0 && my_retest) atomicAdd(&a.st->retested, my_retest);
 }
 
-// Per tile (one warp per tile; lanes over rows): the bitmap size
-// ceil(C/32) words per query and the number of work units
-// ceil(ceil(C/32) / unit_words).  Tiles past the end write 0 so that scans
-// over n entries give the offsets.
-__global__ void tile_words_kernel(TableArgs a, uint32_t* words, uint32_t* units) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+// A thread per tile: its row segments (kept in trow_s/e where set), the words
+// of its test bitmap, ceil(C/32) per query, and its work units,
+// ceil(ceil(C/32) / unit_words); the offsets of both by a single-pass scan
+// (boff may be null: no bitmap).  Blocks past the last tile only clear their
+// part of deg.
+__global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
+    TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
+    unsigned long long* __restrict__ nwords, uint32_t* __restrict__ nunits, LookState lu,
+    LookState lw) {
+    const uint32_t tile = lookback_ticket(lu);
+    const uint32_t t = tile * kLookThreads + threadIdx.x;
+    if (t < a.n) a.deg[t] = 0u;
+    const uint32_t ntiles = *a.ntiles;
+    if (tile * kLookThreads >= ntiles) return;  // (the whole block)
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho, nrows = 2 * rho + 1;
-    const uint32_t ntiles = *a.ntiles;
-    for (uint64_t t = warp; t < a.n; t += nwarps) {
-        uint64_t w = 0;
-        uint32_t nu = 0;
+    unsigned long long w = 0;
+    uint32_t nu = 0;
+    if (t < ntiles) {
+        const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
+        const uint32_t key0 = a.gkey[qs];
+        const uint32_t cy = key0 / a.g.ncx_pad;
+        const uint32_t cx0 = (key0 - cy * a.g.ncx_pad) / a.g.G * a.g.G;
+        uint32_t c = 0;
+        for (int i = 0; i < nrows; i++) {
+            uint32_t st, len, base;
+            tile_row(a, ep, rho, cy, cx0, i, &st, &len, &base);
+            c += len;
+            if (a.trow_s) {
+                const unsigned long long k = (unsigned long long)t * (uint32_t)nrows + (uint32_t)i;
+                a.trow_s[k] = st;
+                a.trow_e[k] = st + len;
+            }
+        }
+        const uint32_t tw = (c + 31u) >> 5;
+        w = (unsigned long long)tw * (qe - qs);
+        nu = (tw + a.unit_words - 1) / a.unit_words;
+        if (w > 0xffffffffull) {
+            atomicOr(&a.st->flags, kStatBitmapTooLarge);
+            w = 0;
+        }
+    }
+    const uint32_t u0 = (uint32_t)block_lookback(nu, tile, lu, a.st);
+    if (t < ntiles) {
+        uoff[t] = u0;
+        if (t == ntiles - 1) {
+            uoff[ntiles] = u0 + nu;
+            *nunits = u0 + nu;
+        }
+    }
+    if (boff) {
+        const unsigned long long b0 = block_lookback(w, tile, lw, a.st);
         if (t < ntiles) {
-            const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
-            const uint32_t key0 = a.gkey[qs];
-            const uint32_t cy = key0 / a.g.ncx_pad;
-            const uint32_t cx0 = (key0 - cy * a.g.ncx_pad) / a.g.G * a.g.G;
-            uint32_t c = 0;
-            for (int i = lane; i < nrows; i += 32) {
-                uint32_t st, len, base;
-                tile_row(a, ep, rho, cy, cx0, i, &st, &len, &base);
-                c += len;
-                if (a.trow_s) {
-                    const unsigned long long k = t * (uint32_t)nrows + (uint32_t)i;
-                    a.trow_s[k] = st;
-                    a.trow_e[k] = st + len;
-                }
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) c += __shfl_down_sync(kFull, c, d);
-            const uint32_t tw = (c + 31u) >> 5;
-            w = (uint64_t)tw * (qe - qs);
-            nu = (tw + a.unit_words - 1) / a.unit_words;
-        }
-        if (lane == 0) {
-            if (w > 0xffffffffull) {
-                atomicOr(&a.st->flags, kStatBitmapTooLarge);
-                w = 0;
-            }
-            words[t] = (uint32_t)w;
-            units[t] = nu;
+            boff[t] = b0;
+            if (t == ntiles - 1) *nwords = b0 + w;
         }
     }
 }
 
-// ptile[k] = t for the points [tiles[t], tiles[t+1]) of every tile t.
-__global__ void tile_owner_kernel(TableArgs a, uint32_t* __restrict__ ptile) {
-    const uint32_t ntiles = *a.ntiles;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles;
-         t += gridDim.x * blockDim.x) {
-        const uint32_t qs = a.tiles[t], qe = min(a.tiles[t + 1], a.n);
-        for (uint32_t k = qs; k < qe; k++) ptile[k] = t;
-    }
-}
-
-// unit_tile[u] = t for the units [tile_uoff[t], tile_uoff[t+1]) of tile t.
+// unit_tile[u] = t for the units [tile_uoff[t], tile_uoff[t+1]) of tile t: a
+// thread per tile, long lists by the whole warp.
 __global__ void unit_list_kernel(TableArgs a, uint32_t* unit_tile) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     const uint32_t ntiles = *a.ntiles;
-    for (uint64_t t = warp; t < ntiles; t += nwarps) {
-        const uint32_t b = a.tile_uoff[t], e = a.tile_uoff[t + 1];
-        for (uint32_t u = b + lane; u < e; u += 32) unit_tile[u] = (uint32_t)t;
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t - lane >= ntiles) return;  // (whole warps)
+    const uint32_t b = t < ntiles ? a.tile_uoff[t] : 0u, e = t < ntiles ? a.tile_uoff[t + 1] : 0u;
+    if (e - b <= 8u)
+        for (uint32_t u = b; u < e; u++) unit_tile[u] = t;
+    for (uint32_t l = __ballot_sync(kFull, e - b > 8u); l; l &= l - 1u) {
+        const int src = __ffs(l) - 1;
+        const uint32_t bb = __shfl_sync(kFull, b, src), ee = __shfl_sync(kFull, e, src);
+        const uint32_t tt = t - lane + (uint32_t)src;
+        for (uint32_t u = bb + lane; u < ee; u += 32) unit_tile[u] = tt;
     }
 }
 
@@ -1557,15 +1565,25 @@ void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s) {
         table_kernel<false, true><<<nblocks, kTT, 0, s>>>(a);
 }
 
-void launch_tile_words(const TableArgs& a, uint32_t* words, uint32_t* units, int nblocks,
-                       cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    tile_words_kernel<<<nblocks, kTT, 0, s>>>(a, words, units);
+size_t words_state_bytes(uint32_t n) {
+    return 2 * ((look_state_bytes(((uint64_t)n + kLookThreads - 1) / kLookThreads) + 15) & ~(size_t)15);
 }
 
-void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, int nblocks, cudaStream_t s) {
+void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
+                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
+                       cudaStream_t s) {
+    if (!a.n) return;
+    const unsigned nb = (a.n + kLookThreads - 1) / kLookThreads;
     VDB_COUNT_LAUNCH();
-    unit_list_kernel<<<nblocks, kTT, 0, s>>>(a, unit_tile);
+    tile_words_kernel<<<nb, kLookThreads, 0, s>>>(
+        a, boff, uoff, nwords, nunits, look_state(zeroed),
+        look_state((char*)zeroed + words_state_bytes(a.n) / 2));
+}
+
+void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, cudaStream_t s) {
+    if (!a.n) return;
+    VDB_COUNT_LAUNCH();
+    unit_list_kernel<<<(a.n + kTT - 1) / kTT, kTT, 0, s>>>(a, unit_tile);
 }
 
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
@@ -1574,11 +1592,6 @@ void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
         expand16_kernel<<<nblocks, kXPB * 32, 0, s>>>(a);
     else
         expand_kernel<uint32_t><<<nblocks, kXPB * 32, 0, s>>>(a);
-}
-
-void launch_tile_owner(const TableArgs& a, uint32_t* ptile, int nblocks, cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    tile_owner_kernel<<<nblocks, kTT, 0, s>>>(a, ptile);
 }
 
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s) {
