@@ -460,33 +460,95 @@ __global__ void cell_best_kernel(CellArgs a) {
         atomicMax(&a.cbest[c], ((unsigned long long)mx << 32) | (uint32_t)~k);
 }
 
-// First unions of slot v: a thread per cell and row (its own and the next)
-// tests the points of largest degree of the cell and of its adjacent cells.
-// In dense regions that joins almost every pair of adjacent cells, so that
-// the search below finds most pairs already joined.
-__global__ void cell_near_kernel(CellArgs a, int v) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, dy = blockIdx.y;
-    if (c >= *a.ncl) return;
+// First unions: the points of largest degree of a cell and of an adjacent one
+// are tested.  In dense regions that joins almost every pair of adjacent
+// cells, so that the search below finds most pairs already joined.
+//
+// Along the rows (first slot only): a warp's run of cells that are joined to
+// their left neighbours points at its first cell, without atomics.
+__global__ void cell_runs_kernel(CellArgs a) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t ncl = *a.ncl;
+    if (c - lane >= ncl) return;  // (whole warps)
+    bool left = false;  // joined to cell c - 1
+    if (c < ncl && c > 0 && !a.continued) {
+        const uint32_t mp = a.mp[0];
+        const unsigned long long bA = a.cbest[c], bB = a.cbest[c - 1];
+        if (best_deg(bA) >= mp && best_deg(bB) >= mp) {
+            const uint32_t ku = best_point(bA), kv = best_point(bB);
+            if (ku < a.n && kv < a.n && a.ccx[c] == a.ccx[c - 1] + 1u &&
+                a.crng[(size_t)(uint32_t)a.ep->rho * a.n + c].x < c)
+                left = test_pair(a, pair_test(a), ku, kv, a.glocal[ku], a.glocal[kv], -1, 0) == 3u;
+        }
+    }
+    const uint32_t heads = ~__ballot_sync(kFull, left);
+    if (!left) return;
+    // the run's first cell in this warp, or the cell before the warp's
+    const uint32_t upto = heads & ((2u << lane) - 1u);
+    a.parent[c] = c - lane + (upto ? 31u - (uint32_t)__clz((int)upto) : 0u) - (upto ? 0u : 1u);
+}
+
+// From one row to the next (and along the rows where a run was not made): a
+// thread per cell looks at up to three adjacent cells.  Neighbouring lanes
+// mostly want the same two trees joined: one union per pair of roots and warp.
+constexpr int kNearLoads = 5;  // cells of two per eps: all the cells of a row within reach
+__global__ void __launch_bounds__(kThreads, 4) cell_near_kernel(CellArgs a, int v) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t dy = blockIdx.y ^ 1u;  // next row first
+    const uint32_t ncl = *a.ncl;
+    if (c - lane >= ncl) return;  // (whole warps)
     const uint32_t mp = a.mp[v];
-    const unsigned long long bA = a.cbest[c];
-    if (best_deg(bA) < mp) return;
     const uint32_t rho = (uint32_t)a.ep->rho;
-    const uint2 rg = a.crng[(size_t)(rho + dy) * a.n + c];
-    const int cx = (int)a.ccx[c];
-    const uint32_t ku = best_point(bA);
-    if (ku >= a.n) return;
     const PairTest t = pair_test(a);
-    const float2 pu = a.glocal[ku];
     uint32_t* parent = a.parent + (size_t)v * a.n;
-    for (uint32_t o = dy ? rg.x : c + 1; o < rg.y; o++) {
-        const int dx = (int)a.ccx[o] - cx;
-        if (dx > 1) break;
-        if (dx < -1) continue;
-        const unsigned long long bB = a.cbest[o];
-        if (best_deg(bB) < mp || parent[c] == parent[o]) continue;
-        const uint32_t kv = best_point(bB);
-        if (kv < a.n && test_pair(a, t, ku, kv, pu, a.glocal[kv], dx, (int)dy) == 3u)
-            uf_union(parent, c, o, a.st);
+    uint32_t o = 0, oe = 0, ku = 0;
+    int cx = 0;
+    float2 pu = make_float2(0.f, 0.f);
+    if (c < ncl && dy <= rho) {
+        const unsigned long long bA = a.cbest[c];
+        ku = best_point(bA);
+        if (best_deg(bA) >= mp && ku < a.n) {
+            const uint2 rg = a.crng[(size_t)(rho + dy) * a.n + c];
+            cx = (int)a.ccx[c];
+            pu = a.glocal[ku];
+            o = dy ? rg.x : c + 1;
+            oe = rg.y;
+        }
+    }
+    const uint32_t pc = o < oe ? parent[c] : 0u;
+    for (; __any_sync(kFull, o < oe); o = min(o + (uint32_t)kNearLoads, oe)) {
+        // a row's cells at once: their loads overlap
+        uint32_t want = 0;  // adjacent cells with cores and another parent
+        if (o < oe) {
+#pragma unroll
+            for (int j = 0; j < kNearLoads; j++) {
+                if (o + j >= oe) continue;
+                const int dx = (int)a.ccx[o + j] - cx;
+                if (best_deg(a.cbest[o + j]) >= mp && parent[o + j] != pc && dx >= -1 && dx <= 1)
+                    want |= 1u << j;
+            }
+        }
+        while (__any_sync(kFull, want != 0u)) {
+            uint32_t ra = 0, rb = 0;
+            bool join = want != 0u;
+            if (join) {
+                const uint32_t w = o + (uint32_t)__ffs(want) - 1u;
+                want &= want - 1u;
+                const uint32_t kv = best_point(a.cbest[w]);
+                join = kv < a.n && test_pair(a, t, ku, kv, pu, a.glocal[kv], (int)a.ccx[w] - cx,
+                                             (int)dy) == 3u;
+                if (join) {
+                    ra = uf_find(parent, c);
+                    rb = uf_find(parent, w);
+                    join = ra != rb;
+                }
+            }
+            const unsigned long long key =
+                join ? ((unsigned long long)max(ra, rb) << 32) | min(ra, rb) : ~0ull - lane;
+            const uint32_t same = __match_any_sync(kFull, key);
+            if (join && lane == (uint32_t)(__ffs(same) - 1)) uf_union(parent, ra, rb, a.st);
+            __syncwarp();
+        }
     }
 }
 
@@ -499,7 +561,7 @@ constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes
 // screens the roots and tests the pairs of next to empty cells itself; the
 // other pairs are searched by the whole warp, lanes over the point pairs (or,
 // for large cells, over the first cell's points within eps of the second).
-__global__ void cell_pairs_kernel(CellArgs a, int v) {
+__global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int v) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
     const uint32_t mp = a.mp[v];
@@ -528,16 +590,28 @@ __global__ void cell_pairs_kernel(CellArgs a, int v) {
             }
         }
     }
-    // every lane walks its row; each step's pairs that need more than a
-    // lane are then searched one after the other
-    while (__any_sync(kFull, o < oe)) {
+    // A row's cells are screened at once (their loads overlap): those with
+    // cores and another parent, as far as it is known, stay in `left`.
+    uint32_t left = 0;
+    const uint32_t o0 = o;
+    {
+        const uint32_t pc = c < ncl ? parent[c] : 0u;
+#pragma unroll 5
+        for (uint32_t j = 0; j < min(oe - o, 32u); j++)
+            if (best_deg(a.cbest[o + j]) >= mp && parent[o + j] != pc) left |= 1u << j;
+    }
+    // every lane takes the cells left in its row; each step's pairs that need
+    // more than a lane are then searched one after the other
+    while (__any_sync(kFull, left != 0u)) {
         bool need = false;
         uint32_t sB = 0, eB = 0;
         int dx = 0;
-        const uint32_t ob = o;
-        if (o < oe) {
+        uint32_t ob = 0;
+        if (left) {
+            ob = o = o0 + (uint32_t)__ffs(left) - 1u;
+            left &= left - 1u;
             const unsigned long long bB = a.cbest[o];
-            need = best_deg(bB) >= mp && uf_find(parent, c) != uf_find(parent, o);
+            need = uf_find(parent, c) != uf_find(parent, o);
             // cores in different components at the larger epsilon are not
             // connected at this one (its components refine those)
             if (need && comp && comp[a.gpos[best_point(bB)]] != compA) {
@@ -559,7 +633,6 @@ __global__ void cell_pairs_kernel(CellArgs a, int v) {
                     need = false;
                 }
             }
-            o++;
         }
         for (uint32_t todo = __ballot_sync(kFull, need); todo; todo &= todo - 1u) {
             const int src = __ffs(todo) - 1;
@@ -631,15 +704,16 @@ __global__ void cell_pairs_kernel(CellArgs a, int v) {
     if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
 }
 
-// Roots of slot v, which are also the next slot's start (a smaller minpts
-// keeps every core and every connection).
-__global__ void cell_flatten_kernel(CellArgs a, int v) {
+// Roots of slot v, after the first unions (so that the search tells joined
+// cells by one load) and after the search (last), when they are also the next
+// slot's start: a smaller minpts keeps every core and every connection.
+__global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= *a.ncl) return;
     uint32_t* parent = a.parent + (size_t)v * a.n;
     const uint32_t r = uf_find_ro(parent, c);
     parent[c] = r;
-    if (a.chain && v + 1 < a.m) parent[a.n + c] = r;
+    if (last && a.chain && v + 1 < a.m) parent[a.n + c] = r;
 }
 
 // seed[root] = first visit position among the component's cores (y: slot).
@@ -780,10 +854,11 @@ __global__ void cell_core_labels_kernel(CellArgs a) {
 // neighbour cells all belong to its own cell's cluster searches nothing, and
 // one surrounded by a single other cluster ends at the first core found.  A
 // start after p's own visit position cannot label it (p was visited first, as
-// noise).  A lane searches up to kLaneCores points itself; larger searches are
-// done by the warp, lanes over the cells' points.
+// noise).  The lanes of a warp search side by side while there are at most
+// kLaneCores points for each lane that searches; a few lanes' larger searches
+// are done by the warp one after the other, lanes over the cells' points.
 constexpr uint32_t kLaneCores = 16;
-__global__ void cell_border_kernel(CellArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) cell_border_kernel(CellArgs a) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t d = k < a.n ? a.deg[k] : kNone;
@@ -814,35 +889,48 @@ __global__ void cell_border_kernel(CellArgs a) {
         uint32_t floor_s = 0;  // starts below this one have been searched
         bool busy = border;
         while (__any_sync(kFull, busy)) {
-            // the earliest start that is left among the neighbour cells, and
-            // the points of its cells
-            uint32_t ms = kNone, npts = 0;
+            // the earliest start that is left among the neighbour cells
+            uint32_t ms = kNone;
             if (busy) {
                 const uint32_t lim = min(best, p);
                 for (int i = 0; i < nrows; i++) {
                     const uint2 rg = rng[(size_t)i * a.n];
-                    for (uint32_t o = rg.x; o < rg.y; o++) {
-                        const uint32_t st = cst[o];
-                        if (st >= lim || st < floor_s || st > ms) continue;
-                        if (st < ms) npts = 0;
-                        ms = st;
-                        npts += a.clist[o + 1] - a.clist[o];
+                    const uint32_t cnt = rg.y - rg.x;
+#pragma unroll 2
+                    for (uint32_t j = 0; j < cnt; j++) {
+                        const uint32_t st = cst[rg.x + j];
+                        ms = min(ms, st >= floor_s ? st : kNone);
                     }
                 }
-                if (ms == kNone) busy = false;
+                if (ms >= lim) {
+                    ms = kNone;
+                    busy = false;
+                }
+            }
+            if (!__any_sync(kFull, busy)) break;
+            // the points of its cells
+            uint32_t npts = 0;
+            if (busy) {
+                for (int i = 0; i < nrows; i++) {
+                    const uint2 rg = rng[(size_t)i * a.n];
+                    for (uint32_t o = rg.x; o < rg.y; o++)
+                        if (cst[o] == ms) npts += a.clist[o + 1] - a.clist[o];
+                }
             }
             bool hit = false;
-            const bool wide = busy && npts > kLaneCores;
+            const uint32_t searching = (uint32_t)__popc(__ballot_sync(kFull, busy));
+            const bool wide = busy && npts > kLaneCores * searching;
             if (busy && !wide) {
-                for (int i = 0; i < nrows && !hit; i++) {
-                    const uint2 rg = rng[(size_t)i * a.n];
+                for (int j = 0; j < nrows && !hit; j++) {
+                    const int dy = (j + 1) / 2 * ((j & 1) ? 1 : -1);  // nearest rows first
+                    const uint2 rg = rng[(size_t)(dy + rho) * a.n];
                     for (uint32_t o = rg.x; o < rg.y && !hit; o++) {
                         if (cst[o] != ms) continue;
                         const int dx = (int)a.ccx[o] - cx;
                         const uint32_t e = a.clist[o + 1];
                         for (uint32_t u = a.clist[o]; u < e && !hit; u++)
                             hit = a.deg[u] >= mp &&
-                                  (test_pair(a, t, k, u, loc, a.glocal[u], dx, i - rho) & 2u);
+                                  (test_pair(a, t, k, u, loc, a.glocal[u], dx, dy) & 2u);
                     }
                 }
             }
@@ -853,19 +941,55 @@ __global__ void cell_border_kernel(CellArgs a) {
                 const int cxx = __shfl_sync(kFull, cx, src);
                 const float2 l = make_float2(__shfl_sync(kFull, loc.x, src),
                                              __shfl_sync(kFull, loc.y, src));
+                // lanes over the rows' ranges, then over the cells: the cells
+                // with that start, each with its points
+                uint2 rg = make_uint2(0u, 0u);
+                if ((int)lane < nrows) rg = a.crng[(size_t)lane * a.n + cc];
+                uint32_t incl = rg.y - rg.x;
+#pragma unroll
+                for (int s1 = 1; s1 < 32; s1 <<= 1) {
+                    const uint32_t x = __shfl_up_sync(kFull, incl, s1);
+                    if ((int)lane >= s1) incl += x;
+                }
+                const uint32_t ncells = __shfl_sync(kFull, incl, 31);
                 bool found = false;
-                // nearest rows first
-                for (int j = 0; j < nrows && !found; j++) {
-                    const int dy = (j + 1) / 2 * ((j & 1) ? 1 : -1);
-                    const uint2 rg = a.crng[(size_t)(dy + rho) * a.n + cc];
-                    for (uint32_t o = rg.x; o < rg.y && !found; o++) {
-                        if (cst[o] != mss) continue;
-                        const int dx = (int)a.ccx[o] - cxx;
-                        const uint32_t b = a.clist[o], e = a.clist[o + 1];
-                        for (uint32_t u0 = b; u0 < e && !found; u0 += 32) {
+                for (uint32_t base = 0; base < ncells && !found; base += 32) {
+                    const uint32_t j = base + lane;
+                    uint32_t o = 0;
+                    int row = 0;
+                    for (int i = 0; i < nrows; i++) {
+                        const uint32_t ie = __shfl_sync(kFull, incl, i);
+                        const uint2 rr = make_uint2(__shfl_sync(kFull, rg.x, i),
+                                                    __shfl_sync(kFull, rg.y, i));
+                        if (j < ie && j >= ie - (rr.y - rr.x)) {
+                            o = rr.x + (j - (ie - (rr.y - rr.x)));
+                            row = i;
+                        }
+                    }
+                    const bool mine = j < ncells && cst[o] == mss;
+                    uint32_t b = 0, e = 0;
+                    int dx = 0;
+                    if (mine) {
+                        b = a.clist[o];
+                        e = a.clist[o + 1];
+                        dx = (int)a.ccx[o] - cxx;
+                    }
+                    // nearest cells first
+                    const int gx = max(abs(dx) - 1, 0), gy = max(abs(row - rho) - 1, 0);
+                    uint32_t left = __ballot_sync(kFull, mine);
+                    const uint32_t order = ((uint32_t)(gx * gx + gy * gy) << 5) | lane;
+                    while (left && !found) {
+                        const uint32_t pick =
+                            __reduce_min_sync(kFull, (left >> lane) & 1u ? order : kNone) & 31u;
+                        left &= ~(1u << pick);
+                        const uint32_t bb = __shfl_sync(kFull, b, (int)pick);
+                        const uint32_t ee = __shfl_sync(kFull, e, (int)pick);
+                        const int ox = __shfl_sync(kFull, dx, (int)pick);
+                        const int oy = __shfl_sync(kFull, row, (int)pick) - rho;
+                        for (uint32_t u0 = bb; u0 < ee && !found; u0 += 32) {
                             const uint32_t u = u0 + lane;
-                            const bool in = u < e && a.deg[u] >= mp &&
-                                            (test_pair(a, t, kk, u, l, a.glocal[u], dx, dy) & 2u);
+                            const bool in = u < ee && a.deg[u] >= mp &&
+                                            (test_pair(a, t, kk, u, l, a.glocal[u], ox, oy) & 2u);
                             found = __any_sync(kFull, in);
                         }
                     }
@@ -947,13 +1071,17 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     cell_ranges_kernel<<<dim3(nblk(a.n), (unsigned)nrows), kThreads, 0, s>>>(a);
     VDB_COUNT_LAUNCH();
     cell_best_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    VDB_COUNT_LAUNCH();
+    cell_runs_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
     for (int v = 0; v < a.m; v++) {
         VDB_COUNT_LAUNCH();
-        cell_near_kernel<<<dim3(nblk(a.n), nrows > 1 ? 2 : 1), kThreads, 0, s>>>(a, v);
+        cell_near_kernel<<<dim3(nblk(a.n), 2), kThreads, 0, s>>>(a, v);
+        VDB_COUNT_LAUNCH();
+        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v, 0);
         VDB_COUNT_LAUNCH();
         cell_pairs_kernel<<<dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, 0, s>>>(a, v);
         VDB_COUNT_LAUNCH();
-        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v);
+        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v, 1);
     }
     VDB_COUNT_LAUNCH();
     cell_seed_kernel<<<per_slot, kThreads, 0, s>>>(a);
