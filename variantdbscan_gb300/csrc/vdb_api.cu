@@ -542,9 +542,9 @@ double avail_bytes(vdb_context* ctx) {
     return ((double)fb + (double)ctx->pool.cached_free()) / ctx->mem_share;
 }
 
-// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi) = work units
-// [u_lo, u_hi), entries [e_lo, e_hi).  The whole table: t_hi = 0xffffffff and
-// u_hi = 0 (no limits).
+// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi), with the
+// entries [u_lo, u_hi) of the unit list, table entries [e_lo, e_hi).  The whole
+// table: t_hi = u_hi = 0xffffffff (no limits).
 struct RowChunk {
     uint32_t t_lo, t_hi, u_lo, u_hi, r_lo, r_hi;
     uint64_t e_lo, e_hi;
@@ -558,7 +558,7 @@ struct UfState {
 // Splits the table into row chunks of whole tiles holding at most cap
 // entries each (greedy, in tile order).
 std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, const uint32_t* tiles,
-                                      const uint32_t* ntiles_dev, const uint32_t* tuoff,
+                                      const uint32_t* ntiles_dev, const uint32_t* tloff,
                                       const unsigned long long* off, uint32_t n, uint64_t cap,
                                       cudaStream_t s) {
     uint32_t nt = 0;
@@ -568,7 +568,7 @@ std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, const uint32_t* tiles,
     std::vector<uint32_t> ht((size_t)nt + 1), hu((size_t)nt + 1);
     std::vector<unsigned long long> ho((size_t)n + 1);
     CK(cudaMemcpyAsync(ht.data(), tiles, ((size_t)nt + 1) * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(hu.data(), tuoff, ((size_t)nt + 1) * 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaMemcpyAsync(hu.data(), tloff, ((size_t)nt + 1) * 4, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(ho.data(), off, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (ht[nt] != n) throw VdbError{VDB_ERR_CUDA, "tile list does not end at n"};
@@ -921,10 +921,11 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* ccx = ar.get<uint32_t>(n);
     unsigned long long* tboff = ar.get<unsigned long long>((size_t)n + 1);
     uint32_t* tuoff = ar.get<uint32_t>((size_t)n + 1);
+    uint32_t* tloff = ar.get<uint32_t>((size_t)n + 1);
     float4* wbox = nullptr;  // boxes of runs of points
     uint32_t* bitmap = nullptr;
     uint64_t bitmap_cap = 0;
-    uint32_t* unit_tile = nullptr;
+    uint2* ulist = nullptr;
     uint32_t* parts = nullptr;
     uint64_t unit_cap = 0;
     uint32_t* nbr = nullptr;
@@ -1056,7 +1057,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         bool chunked = false;
         bool compact = false;  // 16-bit table entries for this group's table
         bool no_rows = false;  // labels only: the degrees are all that is needed
-        chunk_list.assign(1, RowChunk{0, 0xffffffffu, 0, 0, 0, n, 0, 0});
+        chunk_list.assign(1, RowChunk{0, 0xffffffffu, 0, 0xffffffffu, 0, n, 0, 0});
         table_marks.clear();
         // unique minpts of the group, largest first; a repeated minpts copies
         // the labels of the variant before it
@@ -1258,7 +1259,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // layout of the count pass's test bitmap (one word per query and
             // 32 candidates of its tile), which the table pass expands
             ta_args.unit_words = unit_words;
-            launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, d_nwords, d_nunits,
+            launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, tloff, d_nwords, d_nunits,
                               gz.words, s);
             uint64_t bm_words = 0;
             uint32_t nunits = 0;
@@ -1300,19 +1301,20 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ta_args.ptile = ptile;
             // work units: (tile, chunk of unit_words bitmap words)
             if ((uint64_t)nunits + 1 > unit_cap) {
-                if (unit_tile) ar.put(unit_tile);
+                if (ulist) ar.put(ulist);
                 if (parts) ar.put(parts);
                 unit_cap = (uint64_t)nunits + 1;
-                unit_tile = ar.get<uint32_t>(unit_cap);
+                ulist = ar.get<uint2>(unit_cap);
                 parts = nullptr;
             }
             if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
             ta_args.tile_uoff = tuoff;
+            ta_args.tile_loff = tloff;
             ta_args.nunits = d_nunits;
-            ta_args.unit_tile = unit_tile;
+            ta_args.ulist = ulist;
             ta_args.parts = no_rows ? nullptr : parts;
             ta_args.pair_sum = no_rows ? &d_st->pairs : nullptr;
-            launch_unit_list(ta_args, unit_tile, s);
+            launch_unit_list(ta_args, ulist, s);
             ta_args.bitmap = nullptr;
             ta_args.tile_boff = tboff;
             if (no_rows) {
@@ -1449,7 +1451,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 nbr_cap_bytes = 0;
                 const int64_t budget = o.budget > 0 ? o.budget : (int64_t)(avail_bytes(ctx) * 0.9);
                 const uint64_t cap = (uint64_t)std::max<int64_t>(budget / (int64_t)esz, 1);
-                chunk_list = plan_row_chunks(ctx, tiles, d_ntiles, tuoff, off, n, cap, s);
+                chunk_list = plan_row_chunks(ctx, tiles, d_ntiles, tloff, off, n, cap, s);
                 uint64_t mx = 1;
                 for (const RowChunk& c : chunk_list) mx = std::max<uint64_t>(mx, c.e_hi - c.e_lo);
                 const size_t w = std::max<size_t>(words_for(mx), 1);
@@ -2478,17 +2480,20 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.unit_words = kUnitWordsSmall;
     // work units of the count pass (no bitmap here: the fill pass writes the table)
     uint32_t* tuoff = cv.take<uint32_t>((size_t)n + 1);
-    launch_tile_words(ta, nullptr, tuoff, d_totals, d_nunits, gz.words, s);
+    uint32_t* tloff = cv.take<uint32_t>((size_t)n + 1);
+    launch_tile_words(ta, nullptr, tuoff, tloff, d_totals, d_nunits, gz.words, s);
     uint32_t nunits = 0;
     CK(cudaMemcpyAsync(&nunits, d_nunits, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    uint32_t* unit_tile = cv.take<uint32_t>((size_t)nunits + 1);
+    uint2* ulist = cv.take<uint2>((size_t)nunits + 1);
     ta.tile_uoff = tuoff;
+    ta.tile_loff = tloff;
     ta.nunits = d_nunits;
-    ta.unit_tile = unit_tile;
+    ta.ulist = ulist;
+    ta.ptile = ptile;
     ta.parts = nullptr;
     ta.bitmap = nullptr;
-    launch_unit_list(ta, unit_tile, s);
+    launch_unit_list(ta, ulist, s);
     launch_count(ta, nsm * table_blocks_per_sm(false, ep.mixed != 0), s);
     scan_u32_to_u64(deg, off, n, gz.off, st, s);
     unsigned long long E = 0;

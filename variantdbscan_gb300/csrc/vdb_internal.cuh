@@ -402,16 +402,19 @@ struct TableArgs {
     uint32_t* bitmap;               // count pass: per-tile test bitmaps (nullptr: none)
     const unsigned long long* tile_boff;  // first bitmap word of each tile
     // work units of the count and table passes: (tile, chunk of unit_words
-    // bitmap words); unit u belongs to tile unit_tile[u], chunk u - tile_uoff[tile]
+    // bitmap words); tile t has the units tile_uoff[t]..tile_uoff[t+1].  Warps
+    // take the units of ulist (unit, tile), which leaves out those of small
+    // tiles; tile t's are tile_loff[t]..tile_loff[t+1] of it.
     uint32_t unit_words;            // kUnitWords or kUnitWordsSmall
-    const uint32_t* unit_tile;
+    const uint2* ulist;
     const uint32_t* tile_uoff;
-    const uint32_t* nunits;         // device scalar
+    const uint32_t* tile_loff;
+    const uint32_t* nunits;         // device: units, units in ulist
     uint32_t* parts;                // per unit and query slot: neighbours in that chunk
     unsigned long long* pair_sum;   // count pass: adds the neighbours counted (nullptr: not)
-    // one row chunk of the table (zero: the whole table): the fill pass takes
-    // tiles from tile_lo on, the expand pass units [unit_lo, unit_hi), and the
-    // asymmetric flags touch rows [row_lo, row_hi) only
+    // one row chunk of the table: the fill pass takes tiles from tile_lo on,
+    // the expand pass entries [unit_lo, unit_hi) of ulist, and the small tiles
+    // and the asymmetric flags touch rows [row_lo, row_hi) only
     uint32_t tile_lo;
     uint32_t unit_lo, unit_hi;
     uint32_t row_lo, row_hi;
@@ -471,9 +474,9 @@ void launch_word_boxes(const TableArgs& a, cudaStream_t s);
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s);
 size_t words_state_bytes(uint32_t n);
 void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
-                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
-                       cudaStream_t s);
-void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, cudaStream_t s);
+                       uint32_t* loff, unsigned long long* nwords, uint32_t* nunits,
+                       void* zeroed, cudaStream_t s);
+void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s);
 // adds the hash of rows [row_lo, row_hi) of the table to st->table_hash
 // (gorig: input index of every cell-ordered point)
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s);

@@ -214,6 +214,156 @@ __global__ void word_boxes_kernel(TableArgs a) {
     a.wbox[i] = b;
 }
 
+// Tiles of few queries and candidates are not worth a warp: its chain of
+// dependent loads (unit, tile, segments, candidates) is the same for a tile of
+// one query as for 64.  They are counted and expanded by a thread per point
+// instead, which keeps 32 such chains in flight per warp.  Up to kSmallCand
+// candidates the thread's serial tests stay shorter than that chain (1M
+// uniform points, 3 epsilons: count 2,385 -> 310 us, expand 2,510 -> 65 us).
+constexpr uint32_t kSmallCand = 128;
+constexpr uint32_t kSmallQueries = 8;
+// FP64 tests: only up to one word of candidates, and never fused.  A warp with
+// lane = candidate keeps the FP64 pipe as busy as threads of unequal lists do
+// (100k-point sweep: 2.8 ms against 3.1 with 128, 3.7 fused).
+constexpr uint32_t kSmallCand64 = 32;
+// Inputs of at most so many points: the first blocks of the count and expand
+// kernels take the small tiles before they join the others (a launch of their
+// own would add its whole latency, 15 to 30 us, to calls of 300).  Larger ones
+// get a kernel of their own, at twice the warps per SM.
+constexpr uint32_t kSmallFused = 1u << 17;
+
+// Count pass of point k of a small tile: FP32 tests on coordinates relative to
+// the point's own cell (FP64 inside the band, or for every pair), candidates
+// in the tile's order, the loads of four at a time.  A block's threads take
+// consecutive points.
+template <bool MIXED>
+__device__ void small_count(const TableArgs& a, uint32_t k) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t t = 0;
+    bool mine = false;
+    if (k < a.n) {
+        t = a.ptile[k];
+        mine = a.tile_loff[t + 1] == a.tile_loff[t];
+    }
+    if (!__any_sync(kFull, mine)) return;
+    uint32_t cnt = 0, retest = 0, g = 0;
+    if (mine) {
+        const EpsParams* __restrict__ ep = a.ep;
+        const float lo = ep->lo32, hi = ep->hi32, wf = (float)a.g.w;
+        const int rho = ep->rho, nrows = 2 * rho + 1;
+        const uint32_t qs = a.tiles[t], Q = a.tiles[t + 1] - qs;
+        const uint32_t key = a.gkey[k];
+        const uint32_t key0 = a.gkey[qs], cy = key0 / a.g.ncx_pad;
+        const uint32_t cx0 = (key0 - cy * a.g.ncx_pad) / a.g.G * a.g.G;
+        const float2 q = a.glocal[k];
+        uint32_t* const bm = a.bitmap ? a.bitmap + a.tile_boff[t] + (k - qs) : nullptr;
+        uint32_t word = 0;
+        for (int i = 0; i < nrows; i++) {
+            uint32_t st, len, base;
+            tile_row(a, ep, rho, cy, cx0, i, &st, &len, &base, t);
+            const uint32_t own = key + (uint32_t)((i - rho) * (int)a.g.ncx_pad);
+            const float dyw = __fmul_rn((float)(i - rho), wf);
+            for (uint32_t j0 = st; j0 < st + len; j0 += 4) {
+                const uint32_t m = min(4u, st + len - j0);
+                float2 c[4];
+                uint32_t ck[4];
+                if (MIXED) {
+#pragma unroll
+                    for (uint32_t b = 0; b < 4; b++) {
+                        const uint32_t j = j0 + min(b, m - 1u);
+                        c[b] = a.glocal[j];
+                        ck[b] = a.gkey[j];
+                    }
+                }
+#pragma unroll
+                for (uint32_t b = 0; b < 4; b++) {
+                    if (b >= m) break;
+                    bool in = false, band = true;
+                    if (MIXED) {
+                        const float dx =
+                            __fsub_rn(q.x, __fmaf_rn((float)(int)(ck[b] - own), wf, c[b].x));
+                        const float dy = __fsub_rn(q.y, __fadd_rn(c[b].y, dyw));
+                        const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                        in = d2 < lo;
+                        band = !in && d2 <= hi;
+                    }
+                    if (band) {
+                        const uint32_t j = j0 + b;
+                        const uint32_t r = exact_pair(a.gxy[k], a.gxy[j], k, j,
+                                                      exact_bounds(ep->eps, ep->thr, ep->tbox), a.gbox);
+                        retest += MIXED ? 1u : 0u;
+                        in = (r & 1u) != 0u;
+                        record_one_way(a, k, j, r);
+                    }
+                    if (in) {
+                        word |= 1u << (g & 31u);
+                        cnt++;
+                    }
+                    if ((g & 31u) == 31u) {
+                        if (bm) bm[(unsigned long long)(g >> 5) * Q] = word;
+                        word = 0;
+                    }
+                    g++;
+                }
+            }
+        }
+        if ((g & 31u) && bm) bm[(unsigned long long)(g >> 5) * Q] = word;
+        a.deg[k] = cnt;
+        if (a.parts) a.parts[(unsigned long long)a.tile_uoff[t] * kUnitQ + (k - qs)] = cnt;
+    }
+    const uint32_t tests = __reduce_add_sync(kFull, g), again = __reduce_add_sync(kFull, retest);
+    const uint32_t pairs = __reduce_add_sync(kFull, cnt);
+    if (lane == 0) {
+        atomicAdd(&a.st->candidates, (unsigned long long)tests);
+        if (again) atomicAdd(&a.st->retested, (unsigned long long)again);
+        if (a.pair_sum) atomicAdd(a.pair_sum, (unsigned long long)pairs);
+    }
+}
+
+template <bool MIXED>
+__global__ void __launch_bounds__(kTT) small_count_kernel(TableArgs a) {
+    small_count<MIXED>(a, blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+// Table row of point k of a small tile.
+template <typename E>
+__device__ void small_expand(const TableArgs& a, uint32_t k) {
+    const uint32_t t = a.ptile[k];
+    if (a.tile_loff[t + 1] != a.tile_loff[t]) return;
+    const uint32_t qs = a.tiles[t], Q = a.tiles[t + 1] - qs;
+    const uint32_t* __restrict__ bm = a.bitmap + a.tile_boff[t] + (k - qs);
+    E* dst = reinterpret_cast<E*>(a.nbr) + (a.off[k] - a.off_base);
+    E* const end = reinterpret_cast<E*>(a.nbr) + (a.off[k + 1] - a.off_base);
+    const int rho = a.ep->rho, nrows = 2 * rho + 1;
+    const uint32_t key0 = a.gkey[qs], cy = key0 / a.g.ncx_pad;
+    const uint32_t cx0 = (key0 - cy * a.g.ncx_pad) / a.g.G * a.g.G;
+    // 32-bit entries: the segment that holds the position
+    int row = -1;
+    uint32_t st = 0, before = 0, after = 0;
+    for (uint32_t w = 0; dst < end && w < kSmallCand / 32; w++) {
+        for (uint32_t m = bm[(unsigned long long)w * Q]; m && dst < end; m &= m - 1u) {
+            const uint32_t g = w * 32u + (uint32_t)__ffs(m) - 1u;
+            if (sizeof(E) == 2) {
+                *dst++ = (E)g;
+            } else {
+                while (g >= after && row + 1 < nrows) {
+                    uint32_t len, base;
+                    before = after;
+                    tile_row(a, a.ep, rho, cy, cx0, ++row, &st, &len, &base, t);
+                    after = before + len;
+                }
+                *dst++ = (E)(st + (g - before));
+            }
+        }
+    }
+}
+
+template <typename E>
+__global__ void __launch_bounds__(kTT) small_expand_kernel(TableArgs a) {
+    const uint32_t k = a.row_lo + blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < a.row_hi) small_expand<E>(a, k);
+}
+
 // Count pass over work units (tile, chunk of unit_words*32 candidates): adds
 // each query's neighbours in the chunk to deg, records them in parts (for the
 // table pass) and, when a.bitmap is set, stores the chunk's test bitmap
@@ -243,7 +393,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
     const float wf = (float)a.g.w;
-    const uint32_t nunits = *a.nunits;
+    const uint32_t nlist = a.nunits[1];
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     const float fnan = __int_as_float(0x7fc00000);
     const double dnan = __longlong_as_double(0x7ff8000000000000ll);
@@ -253,12 +403,18 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
         s_madd[wib][lane + 32] = 0u;
     }
 
+    if (MIXED && a.n <= kSmallFused)
+        for (uint32_t k0 = blockIdx.x * (kWPB * 32u); k0 < a.n; k0 += gridDim.x * (kWPB * 32u))
+            small_count<MIXED>(a, k0 + threadIdx.x);
+
     for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nunits) break;
-        const uint32_t t = a.unit_tile[u];
+        if (u >= nlist) break;
+        const uint2 ut = a.ulist[u];
+        u = ut.x;
+        const uint32_t t = ut.y;
         const uint32_t chunk = u - a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ)) {
@@ -746,8 +902,12 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
     const float wf = (float)a.g.w;
-    // units of the row chunk (all units when unit_hi is 0)
-    const uint32_t nunits = a.unit_hi ? min(*a.nunits, a.unit_hi) : *a.nunits;
+    const uint32_t nlist = min(a.nunits[1], a.unit_hi);  // the row chunk's part of the list
+    if (a.n <= kSmallFused)
+        for (uint64_t k = a.row_lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.row_hi;
+             k += (uint64_t)gridDim.x * blockDim.x)
+            small_expand<E>(a, (uint32_t)k);
+    __syncwarp();
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     uint32_t par = 0;        // staging buffer of the next query
     uint32_t pending = 0;    // bit b: a copy from buffer b may still be reading it
@@ -758,8 +918,10 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
         uint32_t u = 0;
         if (lane == 0) u = a.unit_lo + atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nunits) break;
-        const uint32_t t = a.unit_tile[u];
+        if (u >= nlist) break;
+        const uint2 ut = a.ulist[u];
+        u = ut.x;
+        const uint32_t t = ut.y;
         const uint32_t u0 = a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ && u0 <= u)) {
@@ -951,7 +1113,12 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
-    const uint32_t nunits = a.unit_hi ? min(*a.nunits, a.unit_hi) : *a.nunits;
+    const uint32_t nlist = min(a.nunits[1], a.unit_hi);
+    if (a.n <= kSmallFused)
+        for (uint64_t k = a.row_lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.row_hi;
+             k += (uint64_t)gridDim.x * blockDim.x)
+            small_expand<E>(a, (uint32_t)k);
+    __syncwarp();
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     uint32_t pending = 0;    // nonzero: a copy from this half's buffer may be reading it
     const uint32_t stage_s = (uint32_t)__cvta_generic_to_shared(&s_stage[wib][0][0]);
@@ -960,8 +1127,10 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
         uint32_t u = 0;
         if (lane == 0) u = a.unit_lo + atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nunits) break;
-        const uint32_t t = a.unit_tile[u];
+        if (u >= nlist) break;
+        const uint2 ut = a.ulist[u];
+        u = ut.x;
+        const uint32_t t = ut.y;
         const uint32_t u0 = a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ && u0 <= u)) {
@@ -1357,13 +1526,14 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
 
 // A thread per tile: its row segments (kept in trow_s/e where set), the words
 // of its test bitmap, ceil(C/32) per query, and its work units,
-// ceil(ceil(C/32) / unit_words); the offsets of both by a single-pass scan
-// (boff may be null: no bitmap).  Blocks past the last tile only clear their
-// part of deg.
+// ceil(ceil(C/32) / unit_words); the offsets of both, and of the units that
+// warps take (those of tiles that are not small), by a single-pass scan (boff
+// may be null: no bitmap).  Blocks past the last tile only clear their part of
+// deg.
 __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
-    unsigned long long* __restrict__ nwords, uint32_t* __restrict__ nunits, LookState lu,
-    LookState lw) {
+    uint32_t* __restrict__ loff, unsigned long long* __restrict__ nwords,
+    uint32_t* __restrict__ nunits, LookState lu, LookState lw) {
     const uint32_t tile = lookback_ticket(lu);
     const uint32_t t = tile * kLookThreads + threadIdx.x;
     if (t < a.n) a.deg[t] = 0u;
@@ -1372,7 +1542,7 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho, nrows = 2 * rho + 1;
     unsigned long long w = 0;
-    uint32_t nu = 0;
+    uint32_t nu = 0, nl = 0;
     if (t < ntiles) {
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         const uint32_t key0 = a.gkey[qs];
@@ -1392,17 +1562,23 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
         const uint32_t tw = (c + 31u) >> 5;
         w = (unsigned long long)tw * (qe - qs);
         nu = (tw + a.unit_words - 1) / a.unit_words;
+        nl = c <= (a.mixed ? kSmallCand : kSmallCand64) && qe - qs <= kSmallQueries ? 0u : nu;
         if (w > 0xffffffffull) {
             atomicOr(&a.st->flags, kStatBitmapTooLarge);
             w = 0;
         }
     }
-    const uint32_t u0 = (uint32_t)block_lookback(nu, tile, lu, a.st);
+    const unsigned long long un =
+        block_lookback(nu | ((unsigned long long)nl << 31), tile, lu, a.st);
     if (t < ntiles) {
+        const uint32_t u0 = (uint32_t)(un & 0x7fffffffull), l0 = (uint32_t)(un >> 31);
         uoff[t] = u0;
+        loff[t] = l0;
         if (t == ntiles - 1) {
             uoff[ntiles] = u0 + nu;
-            *nunits = u0 + nu;
+            loff[ntiles] = l0 + nl;
+            nunits[0] = u0 + nu;
+            nunits[1] = l0 + nl;
         }
     }
     if (boff) {
@@ -1414,21 +1590,26 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     }
 }
 
-// unit_tile[u] = t for the units [tile_uoff[t], tile_uoff[t+1]) of tile t: a
-// thread per tile, long lists by the whole warp.
-__global__ void unit_list_kernel(TableArgs a, uint32_t* unit_tile) {
+// ulist: (unit, tile) of the units that warps take: a thread per tile, long
+// lists by the whole warp.
+__global__ void unit_list_kernel(TableArgs a, uint2* ulist) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ntiles = *a.ntiles;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t - lane >= ntiles) return;  // (whole warps)
-    const uint32_t b = t < ntiles ? a.tile_uoff[t] : 0u, e = t < ntiles ? a.tile_uoff[t + 1] : 0u;
+    uint32_t b = 0, e = 0, u0 = 0;
+    if (t < ntiles) {
+        b = a.tile_loff[t];
+        e = a.tile_loff[t + 1];
+        u0 = a.tile_uoff[t];
+    }
     if (e - b <= 8u)
-        for (uint32_t u = b; u < e; u++) unit_tile[u] = t;
+        for (uint32_t i = b; i < e; i++) ulist[i] = make_uint2(u0 + (i - b), t);
     for (uint32_t l = __ballot_sync(kFull, e - b > 8u); l; l &= l - 1u) {
         const int src = __ffs(l) - 1;
         const uint32_t bb = __shfl_sync(kFull, b, src), ee = __shfl_sync(kFull, e, src);
-        const uint32_t tt = t - lane + (uint32_t)src;
-        for (uint32_t u = bb + lane; u < ee; u += 32) unit_tile[u] = tt;
+        const uint32_t uu = __shfl_sync(kFull, u0, src), tt = t - lane + (uint32_t)src;
+        for (uint32_t i = bb + lane; i < ee; i += 32) ulist[i] = make_uint2(uu + (i - bb), tt);
     }
 }
 
@@ -1544,6 +1725,14 @@ int table_tile_queries() {
 }
 
 void launch_count(const TableArgs& a, int nblocks, cudaStream_t s) {
+    if (!a.mixed || a.n > kSmallFused) {
+        const unsigned nb = (a.n + kTT - 1) / kTT;
+        VDB_COUNT_LAUNCH();
+        if (a.mixed)
+            small_count_kernel<true><<<nb, kTT, 0, s>>>(a);
+        else
+            small_count_kernel<false><<<nb, kTT, 0, s>>>(a);
+    }
     VDB_COUNT_LAUNCH();
     if (a.mixed)
         count_kernel<true><<<nblocks, kWPB * 32, 0, s>>>(a);
@@ -1570,23 +1759,32 @@ size_t words_state_bytes(uint32_t n) {
 }
 
 void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
-                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
+                       uint32_t* loff, unsigned long long* nwords, uint32_t* nunits, void* zeroed,
                        cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (a.n + kLookThreads - 1) / kLookThreads;
     VDB_COUNT_LAUNCH();
     tile_words_kernel<<<nb, kLookThreads, 0, s>>>(
-        a, boff, uoff, nwords, nunits, look_state(zeroed),
+        a, boff, uoff, loff, nwords, nunits, look_state(zeroed),
         look_state((char*)zeroed + words_state_bytes(a.n) / 2));
 }
 
-void launch_unit_list(const TableArgs& a, uint32_t* unit_tile, cudaStream_t s) {
+void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s) {
     if (!a.n) return;
     VDB_COUNT_LAUNCH();
-    unit_list_kernel<<<(a.n + kTT - 1) / kTT, kTT, 0, s>>>(a, unit_tile);
+    unit_list_kernel<<<(a.n + kTT - 1) / kTT, kTT, 0, s>>>(a, ulist);
 }
 
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
+    if (a.n > kSmallFused && a.row_hi > a.row_lo) {
+        const unsigned nb = (a.row_hi - a.row_lo + kTT - 1) / kTT;
+        VDB_COUNT_LAUNCH();
+        if (a.compact)
+            small_expand_kernel<uint16_t><<<nb, kTT, 0, s>>>(a);
+        else
+            small_expand_kernel<uint32_t><<<nb, kTT, 0, s>>>(a);
+    }
+    if (a.unit_hi <= a.unit_lo && a.n > kSmallFused) return;
     VDB_COUNT_LAUNCH();
     if (a.compact)
         expand16_kernel<<<nblocks, kXPB * 32, 0, s>>>(a);
