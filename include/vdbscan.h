@@ -117,9 +117,9 @@ typedef struct {
                                components at a larger epsilon (and a smaller or equal
                                minpts) are not searched: both only save work, the labels
                                are those of a from-scratch run */
-    int32_t tile_cells;     /* grid cells per tile group of the neighbour search (1, 2, 4,
-                               8, 16); 0 = autotuned per table from a lane-slot cost model
-                               of the grid's own occupancy (sampled cells) */
+    int32_t tile_cells;     /* grid cells per tile group of the neighbour search (1 to 64);
+                               0 = the library's choice: 2 on grids of more than two cells
+                               per point, else 1 */
     int32_t unit_candidates; /* candidates of a tile per work unit of the neighbour search
                                (1024, 2048 or 4096); 0 = 1024 for datasets of fewer than
                                2^18 points (a table with few units is bounded by its

@@ -97,26 +97,10 @@ struct Pool {
 
 }  // namespace
 
-// Tile-shape decision of one table: dataset buffers, size and bounding box,
-// epsilon and cells per epsilon.
-struct TuneKey {
-    const void *x, *y;
-    uint32_t n;
-    double minx, maxx, miny, maxy, eps;
-    int r;
-    bool operator<(const TuneKey& o) const {
-        return std::tie(x, y, n, minx, maxx, miny, maxy, eps, r) <
-               std::tie(o.x, o.y, o.n, o.minx, o.maxx, o.miny, o.maxy, o.eps, o.r);
-    }
-};
-
 struct GraphEntry;
 
 struct vdb_context {
     std::vector<GraphEntry*> graphs;         // captured calls (vdb_options.graph), oldest first
-    std::map<TuneKey, uint32_t> tune_cache;  // autotuned tiles per table
-    std::mutex tune_mu;
-    vdb_context* tune_owner = nullptr;       // workers share their caller's cache
     int device = 0;
     int nsm = 1;
     cudaStream_t stream = nullptr;
@@ -295,11 +279,10 @@ struct ZeroCarve {
 // The zeroed memory of one epsilon: look-back states and counters.
 struct GroupZero {
     uint32_t* counts;   // asym_n, count and expand tile counters
-    void *sort, *order, *tiles, *words, *off;
+    void *sort, *order, *words, *off;
     GroupZero(ZeroCarve& z, uint32_t n, bool with_sort) {
         counts = (uint32_t*)z.take(4 * sizeof(uint32_t));
         order = z.take(order_state_bytes(n));
-        tiles = z.take(order_state_bytes(n));
         words = z.take(words_state_bytes(n));
         off = z.take(scan_state_bytes(n));
         sort = with_sort ? z.take(sort_zero_bytes(n, 32)) : nullptr;
@@ -397,7 +380,7 @@ struct Options {
     int table_hash = 0;
     int entry_bytes = 0;  // 0 / 2: compact entries where they fit; 4: always 32-bit
     bool reuse = true;    // labellings start from earlier variants' components
-    int tile_cells = 0;   // cells per tile group G; 0 = autotuned per table
+    int tile_cells = 0;   // cells per tile group G; 0 = default_tile_cells
     int unit_words = 0;   // work-unit size in bitmap words; 0 = by dataset size
     bool graph = false;   // repeated calls replayed as one CUDA graph
 };
@@ -437,48 +420,26 @@ struct Group {
 // tile scans 25 cells of (eps/2)^2, 1.99x the disc's area, against 2.86x for
 // cells of width eps.  Three cells per eps scan 1.6x the disc but multiply the
 // cell pairs the clustering searches (measured slower at every eps of the
-// variant sweep and the lattice), so the cell size is a fixed choice and the
-// tile shape is the tuned one (choose_tile_cells).
+// variant sweep and the lattice), so the cell size is a fixed choice.
 constexpr int kCellsPerEps = 2;
 
-// Tile-shape autotuner.  A tile is up to 64 consecutive cell-ordered points of
-// one group of G cells of a grid row; its candidates are the cells within
-// reach of the whole group.  Larger groups put more queries in a tile (sparse
-// grids leave most of a warp's 64 query slots empty with G = 1) at the price
-// of more candidates per query.  The cost of shape G is modelled from the
-// statistics of launch_tile_costs, measured on the grid itself:
-//   lane-slot tests  C * 32 * ceil(P/32)  x kCostSlot   (count and expand
-//                                                         passes scale with it)
-//   tiles            ceil(P/64)           x kCostTile   (per-tile fixed work)
-// The weights are a non-negative least-squares fit of the count + expand time
-// of single tables measured for every G on 17 tables (2M-point sweep at 4 eps,
-// 1M uniform points at 4 eps, blob datasets of 2e4-4e5 points at 3 eps, each
-// G timed 3 times); a bitmap-word term fitted to zero weight and was dropped.
-// The fitted model picks the fastest shape on every table of >= 4e5 points
-// and recovers 97% of the time the best shapes save over G = 1; below about
-// 1e5 points the shapes differ by a few percent and the model's picks are no
-// better than G = 1, so small datasets keep G = 1 (kTuneMinPoints).  A shape
-// replaces G = 1 only when it models at least 5% cheaper.  The statistics come
-// from about 65,536 sampled non-empty cells in runs of 64 (launch_tile_costs),
-// which track the exact sums within a few percent on the tables above.
-constexpr double kCostSlot = 6.9e-13, kCostTile = 2.8e-9;  // seconds
-constexpr uint32_t kTuneMinPoints = 131072;
+// Tile groups: a tile is up to 64 consecutive cell-ordered points of one group
+// of G cells of a grid row; its candidates are the cells within reach of the
+// whole group.  Larger groups put more queries in a tile and more candidates
+// before each of them.  Since tiles of few queries no longer leave lanes idle
+// (they are tested lane = candidate, or by a thread per point), one and two
+// cells are within 3% of the best shape on every table measured (1M uniform
+// points, 400k and 1M sweeps, 100k and 400k mixtures, 2M lattice, eps 0.05 to
+// 1.5), and 8 or 16 cost 10 to 35% more there.  Two cells win slightly where
+// most cells are empty (1M sweep, eps 0.1: 0.766 against 0.763 ms of count and
+// table; 400k uniform 3% less), one where they are not (eps 0.4: 2.45 against
+// 2.52 ms), so the line lies at half a point per cell.
+uint32_t default_tile_cells(uint32_t n, uint64_t ncells) {
+    return (uint64_t)n * 2 < ncells ? 2u : 1u;
+}
+
 constexpr uint32_t kBoxPoints = 1u << 15;        // word boxes from this many points on
 constexpr uint32_t kSmallUnitPoints = 1u << 18;  // smaller work units below this many points
-
-uint32_t choose_tile_cells(const unsigned long long* sums) {
-    double best = 0.0, base = 0.0;
-    uint32_t G = 1;
-    for (int i = 0; i < kTuneShapes; i++) {
-        const double c = kCostSlot * (double)sums[2 * i] + kCostTile * (double)sums[2 * i + 1];
-        if (i == 0) base = best = c;
-        else if (c < best) {
-            best = c;
-            G = 1u << i;
-        }
-    }
-    return best < 0.95 * base ? G : 1u;
-}
 
 // Worker streams of a multi-dataset call: datasets run concurrently so that
 // one dataset's host waits and small grids are covered by the others, but
@@ -720,7 +681,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         throw VdbError{VDB_ERR_INVALID_ARG, "null pointer"};
     if (ds.mbb_size <= 0) throw VdbError{VDB_ERR_INVALID_ARG, "MBBsize must be positive"};
     if (o.tile_cells < 0 || o.tile_cells > 64)
-        throw VdbError{VDB_ERR_INVALID_ARG, "tile_cells must be 0 (autotuned) or 1..64"};
+        throw VdbError{VDB_ERR_INVALID_ARG, "tile_cells must be 0 (the library's choice) or 1..64"};
     if (o.unit_words != 0 && o.unit_words != (int)kUnitWordsSmall && o.unit_words != 64 &&
         o.unit_words != (int)kUnitWords)
         throw VdbError{VDB_ERR_INVALID_ARG, "unit_candidates must be 0, 1024, 2048 or 4096"};
@@ -905,7 +866,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* d_nunits = (uint32_t*)(d_totals + 1);     // work units
     uint32_t* d_ntiles = (uint32_t*)(d_totals + 2);
     EpsParams* d_ep = ar.get<EpsParams>(1);
-    unsigned long long* tune_sums = ar.get<unsigned long long>(2 * kTuneShapes);
     uint32_t tile_cells_hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // tables per log2(G)
     uint32_t* gkey = ar.get<uint32_t>(n);
     uint32_t* gorig = ar.get<uint32_t>(n);
@@ -1107,9 +1067,13 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 ep.reach[0] = 0;
                 ep.mixed = 0;
             } else {
-                // tile groups of G cells: fixed by the caller, or 1 until the
-                // autotuner below has measured the grid
                 g = make_grid(hb, eps / r, o.tile_cells > 0 ? (uint32_t)o.tile_cells : 1u);
+                if (o.tile_cells <= 0 && default_tile_cells(n, g.ncells) > 1u) {
+                    // (a padding that would exceed the cell limit coarsens the
+                    // cells: such a shape is not taken)
+                    const GridParams g2 = make_grid(hb, eps / r, default_tile_cells(n, g.ncells));
+                    if (g2.ncx == g.ncx && g2.ncy == g.ncy && g2.w == g.w) g = g2;
+                }
                 ep = make_eps(eps, g, hb, want_mixed);
             }
             // grid
@@ -1118,25 +1082,20 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // so that the grid costs O(points + rows), not O(cells)
             g.sparse = g.ncells > 32ull * n + (1ull << 22) ? 1u : 0u;
             g.sub = isfinite(g.w) ? sub_bits(g.ncells) : 0u;
-            // the tuner needs the sorted grid before it can settle the tiles
-            const bool tune = o.tile_cells <= 0 && isfinite(g.w) && n >= kTuneMinPoints;
             const int kbits = bits_for(g.ncells - 1) + 2 * (int)g.sub;
             launch_grid_keys(x, y, n, g, kbits, skey, (uint32_t*)gz.sort, s);
             radix_sort(skey, n, kbits, 2 * (int)g.sub, gz.sort, scratch, gkey, gorig, nullptr, d_st, s);
             OrderArgs oa = order_args();
             oa.g = g;
-            launch_order(oa, !tune, gz.order, s);
-            auto build_cell_start = [&]() {
-                if (g.sparse) return;
+            launch_order(oa, gz.order, s);
+            if (!g.sparse) {
                 if (g.ncells + 1 > cell_cap) {
                     if (cell_start) ar.put(cell_start);
                     cell_start = ar.get<uint32_t>(g.ncells + 1);
                     cell_cap = g.ncells + 1;
                 }
                 launch_cell_start(ckey, clist, cscan + n, n, g, cell_start, s);
-            };
-            build_cell_start();
-            if (g.sparse) {
+            } else {
                 if ((uint64_t)g.ncy + 1 > crow_cap) {
                     if (crow) ar.put(crow);
                     crow = ar.get<uint32_t>((size_t)g.ncy + 1);
@@ -1144,63 +1103,12 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 }
                 launch_cell_rows(ckey, cscan + n, g, crow, s);
             }
-            // tile shape: the cost model of choose_tile_cells on the grid's
-            // own statistics (sampled non-empty cells); a new G only re-pads
-            // the rows, so the keys are rewritten without sorting again (the
-            // row directory of sparse grids does not depend on the padding)
-            if (tune) {
-                // decisions are kept per dataset (its buffers, size and box)
-                // and epsilon: a repeated call measures nothing
-                const TuneKey key{ds.x, ds.y, n, hb.minx, hb.maxx, hb.miny, hb.maxy, eps, r};
-                vdb_context* tc = ctx->tune_owner ? ctx->tune_owner : ctx;
-                uint32_t G = 0;
-                {
-                    std::lock_guard<std::mutex> lk(tc->tune_mu);
-                    auto it = tc->tune_cache.find(key);
-                    if (it != tc->tune_cache.end()) G = it->second;
-                }
-                if (G == 0) {
-                    if (capturing)
-                        throw VdbError{VDB_ERR_CUDA, "graph capture: tile shape not recorded"};
-                    memcpy(ctx->h_pinned, &ep, sizeof ep);
-                    CK(cudaMemcpyAsync(d_ep, ctx->h_pinned, sizeof ep, cudaMemcpyHostToDevice, s));
-                    CK(cudaMemsetAsync(tune_sums, 0, 2 * kTuneShapes * sizeof(unsigned long long),
-                                       s));
-                    launch_tile_costs(g, d_ep, gkey, cell_start, crow, ccx, clist, cscan + n, n,
-                                      tune_sums, s);
-                    char* hs = (char*)ctx->h_pinned + 2048;
-                    CK(cudaMemcpyAsync(hs, tune_sums, 2 * kTuneShapes * sizeof(unsigned long long),
-                                       cudaMemcpyDeviceToHost, s));
-                    CK(cudaStreamSynchronize(s));
-                    unsigned long long sums[2 * kTuneShapes];
-                    memcpy(sums, hs, sizeof sums);
-                    G = choose_tile_cells(sums);
-                    std::lock_guard<std::mutex> lk(tc->tune_mu);
-                    if (tc->tune_cache.size() >= 4096) tc->tune_cache.clear();
-                    tc->tune_cache[key] = G;
-                }
-                GridParams g2 = make_grid(hb, eps / r, G);
-                // (a padding that would exceed the cell limit coarsens the
-                // cells: such a shape is not taken)
-                if (G != g.G && g2.ncx == g.ncx && g2.ncy == g.ncy && g2.w == g.w) {
-                    g2.sparse = g.sparse;
-                    g2.sub = g.sub;
-                    launch_grid_rekey(gkey, ckey, cscan + n, n, g.ncx_pad, g2.ncx_pad, s);
-                    g = g2;
-                    build_cell_start();
-                    ep = make_eps(eps, g, hb, want_mixed);
-                }
-            }
             if (isfinite(g.w)) {
                 int lg = 0;
                 while ((1u << lg) < g.G && lg < 7) lg++;
                 tile_cells_hist[lg]++;
             }
             const bool mixed = ep.mixed != 0;
-            if (tune) {
-                oa.g = g;
-                launch_tiles(oa, gz.tiles, s);
-            }
             // cells are cliques when two points of one cell always pass the
             // distance test without a box check: 2 w^2 below thr and tbox
             clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
@@ -1805,7 +1713,6 @@ void run_concurrent(vdb_context* ctx, const vdb_dataset* ds, int nds, const Opti
     }
     for (int i = 0; i < nw; i++) {
         ctx->workers[i]->mem_share = nw;
-        ctx->workers[i]->tune_owner = ctx;
     }
     cudaEvent_t ready = nullptr;
     CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
@@ -2451,7 +2358,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     oa.ptile = ptile;
     oa.ntiles = d_ntiles;
     oa.st = st;
-    launch_order(oa, true, gz.order, s);
+    launch_order(oa, gz.order, s);
     launch_cell_start(ckey, clist, cscan + n, n, g, cell_start, s);
     CK(cudaMemcpyAsync(d_ep, &ep, sizeof ep, cudaMemcpyHostToDevice, s));
 

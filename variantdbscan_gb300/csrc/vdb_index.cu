@@ -199,7 +199,6 @@ __global__ void gather_kernel(OrderArgs a) {
 // bits each).  A warp takes 32 * kOrderItems consecutive points.
 constexpr int kOrderItems = 4;
 constexpr uint32_t kOrderTile = kLookThreads * kOrderItems;
-template <bool CELLS, bool TILES>
 __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookState ls) {
     const uint32_t tile = lookback_ticket(ls);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -214,10 +213,10 @@ __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookSt
         uint32_t prev = __shfl_up_sync(0xffffffffu, key[i], 1);
         if (lane == 0 && in && k > 0) prev = a.gkey[k - 1];
         const bool fc = in && (k == 0 || key[i] != prev);
-        const bool ft = in && (k == 0 || (TILES && (key[i] / a.g.G != prev / a.g.G ||
-                                                    (uint32_t)k % a.tq == 0u)));
-        bc[i] = CELLS ? __ballot_sync(0xffffffffu, fc) : 0u;
-        bt[i] = TILES ? __ballot_sync(0xffffffffu, ft) : 0u;
+        const bool ft = in && (k == 0 || key[i] / a.g.G != prev / a.g.G ||
+                               (uint32_t)k % a.tq == 0u);
+        bc[i] = __ballot_sync(0xffffffffu, fc);
+        bt[i] = __ballot_sync(0xffffffffu, ft);
         mine += (unsigned long long)__popc(bc[i]) | ((unsigned long long)__popc(bt[i]) << 31);
     }
     const unsigned long long before = block_lookback(lane == 31 ? mine : 0ull, tile, ls, a.st);
@@ -228,33 +227,24 @@ __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookSt
         const uint64_t k64 = base + 32u * i + lane;
         const uint32_t k = (uint32_t)k64;
         if (k64 < a.n) {
-            if (CELLS) {
-                const uint32_t c = c0 + __popc(bc[i] & lt);
-                const uint32_t fc = (bc[i] >> lane) & 1u;
-                if (!VDB_GUARD(a.st, c + fc <= a.n, 19, c)) return;
-                a.cscan[k] = c;
-                if (fc) {
-                    a.clist[c] = k;
-                    a.ckey[c] = key[i];
-                    a.ccx[c] = key[i] % a.g.ncx_pad;
-                }
-                if (k == a.n - 1) {
-                    a.cscan[a.n] = c + fc;
-                    a.clist[c + fc] = a.n;
-                }
-                gather_point(a, k, key[i]);
+            const uint32_t c = c0 + __popc(bc[i] & lt), t = t0 + __popc(bt[i] & lt);
+            const uint32_t fc = (bc[i] >> lane) & 1u, ft = (bt[i] >> lane) & 1u;
+            if (!VDB_GUARD(a.st, c + fc <= a.n && t + ft <= a.n && t + ft > 0u, 19, c)) return;
+            a.cscan[k] = c;
+            if (fc) {
+                a.clist[c] = k;
+                a.ckey[c] = key[i];
+                a.ccx[c] = key[i] % a.g.ncx_pad;
             }
-            if (TILES) {
-                const uint32_t t = t0 + __popc(bt[i] & lt);
-                const uint32_t ft = (bt[i] >> lane) & 1u;
-                if (!VDB_GUARD(a.st, t + ft <= a.n && t + ft > 0u, 19, t)) return;
-                if (ft) a.tiles[t] = k;
-                a.ptile[k] = t + ft - 1u;
-                if (k == a.n - 1) {
-                    a.tiles[t + ft] = a.n;
-                    *a.ntiles = t + ft;
-                }
+            if (ft) a.tiles[t] = k;
+            a.ptile[k] = t + ft - 1u;
+            if (k == a.n - 1) {
+                a.cscan[a.n] = c + fc;
+                a.clist[c + fc] = a.n;
+                a.tiles[t + ft] = a.n;
+                *a.ntiles = t + ft;
             }
+            gather_point(a, k, key[i]);
         }
         c0 += __popc(bc[i]);
         t0 += __popc(bt[i]);
@@ -356,98 +346,7 @@ __global__ void cell_rows_kernel(const uint32_t* __restrict__ ckey,
     crow[r] = b;
 }
 
-__global__ void tile_costs_kernel(GridParams g, const EpsParams* __restrict__ ep,
-                                  const uint32_t* __restrict__ gkey,
-                                  const uint32_t* __restrict__ cell_start,
-                                  const uint32_t* __restrict__ crow,
-                                  const uint32_t* __restrict__ ccx,
-                                  const uint32_t* __restrict__ clist,
-                                  const uint32_t* __restrict__ ncl, uint32_t n,
-                                  unsigned long long* __restrict__ out) {
-    __shared__ unsigned long long s_acc[2 * kTuneShapes];
-    for (int i = threadIdx.x; i < 2 * kTuneShapes; i += blockDim.x) s_acc[i] = 0ull;
-    __syncthreads();
-    const uint32_t nc = min(*ncl, n);
-    const int rho = ep->rho;
-    // sampled cells: about kTuneSamples of them, in runs of kTuneRun
-    // consecutive non-empty cells spread evenly over all of them (a regular
-    // stride of single cells would alias with the period G of the groups of
-    // dense rows and count some shapes' groups more often than others)
-    const uint64_t per = ((uint64_t)nc + kTuneSamples - 1) / kTuneSamples;
-    const uint64_t stride = per ? per : 1;
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t c = (t / kTuneRun) * kTuneRun * stride + t % kTuneRun;
-    if (c < nc) {
-        const uint32_t key = gkey[clist[c]];
-        const uint32_t cy = key / g.ncx_pad, cx = key - cy * g.ncx_pad;
-        uint32_t pcy = 0xffffffffu, pcx = 0;
-        if (c > 0) {
-            const uint32_t pk = gkey[clist[c - 1]];
-            pcy = pk / g.ncx_pad;
-            pcx = pk - pcy * g.ncx_pad;
-        }
-#pragma unroll 1
-        for (int i = 0; i < kTuneShapes; i++) {
-            const uint32_t G = 1u << i;
-            if (pcy == cy && pcx / G == cx / G) continue;  // not the group's first cell
-            const uint32_t gx0 = cx / G * G;
-            const uint32_t gx1 = min(gx0 + G - 1, g.ncx - 1);
-            uint32_t s0, e0;
-            cell_row_range(g, cell_start, crow, ccx, clist, cy, gx0, gx1, &s0, &e0);
-            const unsigned long long P = e0 - s0;
-            unsigned long long C = 0;
-            for (int r = 0; r <= 2 * rho; r++) {
-                const int ry = (int)cy + r - rho;
-                if (ry < 0 || ry >= (int)g.ncy) continue;
-                const int reach = ep->reach[r];
-                const uint32_t lo = (uint32_t)max((int)gx0 - reach, 0);
-                const uint32_t hi = (uint32_t)min((int)gx1 + reach, (int)g.ncx - 1);
-                uint32_t s1, e1;
-                cell_row_range(g, cell_start, crow, ccx, clist, (uint32_t)ry, lo, hi, &s1, &e1);
-                C += e1 - s1;
-            }
-            atomicAdd(&s_acc[2 * i], C * 32ull * ((P + 31) / 32));
-            atomicAdd(&s_acc[2 * i + 1], (P + 63) / 64);
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 2 * kTuneShapes; i += blockDim.x)
-        if (s_acc[i]) atomicAdd(&out[i], s_acc[i]);
-}
-
-__global__ void grid_rekey_kernel(uint32_t* __restrict__ gkey, uint32_t* __restrict__ ckey,
-                                  const uint32_t* __restrict__ ncl, uint32_t n, uint32_t from,
-                                  uint32_t to) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t key = gkey[k];
-    const uint32_t cy = key / from;
-    gkey[k] = cy * to + (key - cy * from);
-    if (k < *ncl) {
-        const uint32_t ck = ckey[k], ry = ck / from;
-        ckey[k] = ry * to + (ck - ry * from);
-    }
-}
-
 }  // namespace
-
-void launch_tile_costs(const GridParams& g, const EpsParams* ep, const uint32_t* gkey,
-                       const uint32_t* cell_start, const uint32_t* crow, const uint32_t* ccx,
-                       const uint32_t* clist, const uint32_t* ncl, uint32_t n,
-                       unsigned long long* out, cudaStream_t s) {
-    if (!n) return;
-    const uint64_t threads = (uint64_t)kTuneSamples + kTuneRun;
-    VDB_COUNT_LAUNCH();
-    tile_costs_kernel<<<nblk(threads), kThreads, 0, s>>>(g, ep, gkey, cell_start, crow, ccx,
-                                                        clist, ncl, n, out);
-}
-
-void launch_grid_rekey(uint32_t* gkey, uint32_t* ckey, const uint32_t* ncl, uint32_t n,
-                       uint32_t ncx_pad_from, uint32_t ncx_pad_to, cudaStream_t s) {
-    if (!n || ncx_pad_from == ncx_pad_to) return;
-    VDB_COUNT_LAUNCH();
-    grid_rekey_kernel<<<nblk(n), kThreads, 0, s>>>(gkey, ckey, ncl, n, ncx_pad_from, ncx_pad_to);
-}
 
 // Blocks of the key kernels: enough to fill the chip, and for large inputs
 // few enough that adding the digit counts up costs little.
@@ -482,21 +381,11 @@ size_t order_state_bytes(uint32_t n) {
     return look_state_bytes(((uint64_t)n + kOrderTile - 1) / kOrderTile);
 }
 
-void launch_order(const OrderArgs& a, bool with_tiles, void* zeroed, cudaStream_t s) {
+void launch_order(const OrderArgs& a, void* zeroed, cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
     VDB_COUNT_LAUNCH();
-    if (with_tiles)
-        order_kernel<true, true><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
-    else
-        order_kernel<true, false><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
-}
-
-void launch_tiles(const OrderArgs& a, void* zeroed, cudaStream_t s) {
-    if (!a.n) return;
-    const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
-    VDB_COUNT_LAUNCH();
-    order_kernel<false, true><<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
+    order_kernel<<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
 }
 
 void launch_gather(const OrderArgs& a, cudaStream_t s) {

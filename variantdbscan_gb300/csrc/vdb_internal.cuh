@@ -304,8 +304,8 @@ void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g
 // The cell order's arrays: per point the coordinates (gxy, FP32 relative to
 // the own cell: glocal), visit position and multiple-point box; the non-empty
 // cells (cscan[k]: cells that start before point k, clist: first points, ckey,
-// ccx: keys and columns; cscan[n] = their number, clist[number] = n) and, with
-// tiles, the tiles (tiles: first points, tiles[number] = n; ptile: tile of
+// ccx: keys and columns; cscan[n] = their number, clist[number] = n) and the
+// tiles (tiles: first points, tiles[number] = n; ptile: tile of
 // every point; *ntiles).
 struct OrderArgs {
     const double* x;
@@ -332,9 +332,7 @@ struct OrderArgs {
     DeviceStatus* st;
 };
 size_t order_state_bytes(uint32_t n);
-void launch_order(const OrderArgs& a, bool with_tiles, void* zeroed, cudaStream_t s);
-// the tiles alone (another G)
-void launch_tiles(const OrderArgs& a, void* zeroed, cudaStream_t s);
+void launch_order(const OrderArgs& a, void* zeroed, cudaStream_t s);
 // gxy, glocal, gpos, gbox alone (no grid: an epsilon without neighbours)
 void launch_gather(const OrderArgs& a, cudaStream_t s);
 // cell_start[key] = first point of the first non-empty cell at or after key
@@ -344,26 +342,6 @@ void launch_cell_start(const uint32_t* ckey, const uint32_t* clist, const uint32
 // crow[r] = first non-empty cell of row >= r (ncy + 1 entries; sparse grids)
 void launch_cell_rows(const uint32_t* ckey, const uint32_t* ncl, const GridParams& g,
                       uint32_t* crow, cudaStream_t s);
-// Autotuner statistics of tile shapes: for each candidate G = 2^i (cells
-// per tile group), over the non-empty cells that start a group of G cells
-// among about kTuneSamples sampled cells (runs of kTuneRun consecutive
-// non-empty cells spread evenly over the grid's non-empty cells):
-// out[2i] += candidate tests in lane slots (C * 32 * ceil(P/32)),
-// out[2i+1] += tiles (ceil(P/64)), with P the group's points and C its
-// candidates (cells within reach of the group in rows cy-rho..cy+rho).  Cell
-// structures of the grid g (any G), keys in its layout; out must hold
-// 2*kTuneShapes zeroed u64.
-constexpr int kTuneShapes = 5;   // G = 1, 2, 4, 8, 16
-constexpr uint32_t kTuneSamples = 65536;
-constexpr uint32_t kTuneRun = 64;
-void launch_tile_costs(const GridParams& g, const EpsParams* ep, const uint32_t* gkey,
-                       const uint32_t* cell_start, const uint32_t* crow, const uint32_t* ccx,
-                       const uint32_t* clist, const uint32_t* ncl, uint32_t n,
-                       unsigned long long* out, cudaStream_t s);
-// Keys of grid `from` rewritten in the layout of grid `to` (same cells, other
-// padding of the rows: the cell order, hence the sort, is unchanged).
-void launch_grid_rekey(uint32_t* gkey, uint32_t* ckey, const uint32_t* ncl, uint32_t n,
-                       uint32_t ncx_pad_from, uint32_t ncx_pad_to, cudaStream_t s);
 // ------------------------------------------------------------------ tables
 struct TableArgs {
     GridParams g;

@@ -249,6 +249,7 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
     uint32_t cnt = 0, retest = 0, g = 0;
     if (mine) {
         const EpsParams* __restrict__ ep = a.ep;
+        const ExactBounds xb = exact_bounds(ep->eps, ep->thr, ep->tbox);
         const float lo = ep->lo32, hi = ep->hi32, wf = (float)a.g.w;
         const int rho = ep->rho, nrows = 2 * rho + 1;
         const uint32_t qs = a.tiles[t], Q = a.tiles[t + 1] - qs;
@@ -263,48 +264,48 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
             tile_row(a, ep, rho, cy, cx0, i, &st, &len, &base, t);
             const uint32_t own = key + (uint32_t)((i - rho) * (int)a.g.ncx_pad);
             const float dyw = __fmul_rn((float)(i - rho), wf);
-            for (uint32_t j0 = st; j0 < st + len; j0 += 4) {
-                const uint32_t m = min(4u, st + len - j0);
-                float2 c[4];
-                uint32_t ck[4];
+            for (uint32_t j0 = st; j0 < st + len; j0 += 32) {
+                const uint32_t m = min(32u, st + len - j0);
+                uint32_t in = 0, band = MIXED ? 0u : (m == 32u ? kFull : (1u << m) - 1u);
                 if (MIXED) {
+                    for (uint32_t b0 = 0; b0 < m; b0 += 4) {
+                        float2 c[4];
+                        uint32_t ck[4];
 #pragma unroll
-                    for (uint32_t b = 0; b < 4; b++) {
-                        const uint32_t j = j0 + min(b, m - 1u);
-                        c[b] = a.glocal[j];
-                        ck[b] = a.gkey[j];
+                        for (uint32_t b = 0; b < 4; b++) {
+                            const uint32_t j = j0 + min(b0 + b, m - 1u);
+                            c[b] = a.glocal[j];
+                            ck[b] = a.gkey[j];
+                        }
+#pragma unroll
+                        for (uint32_t b = 0; b < 4; b++) {
+                            const float dx =
+                                __fsub_rn(q.x, __fmaf_rn((float)(int)(ck[b] - own), wf, c[b].x));
+                            const float dy = __fsub_rn(q.y, __fadd_rn(c[b].y, dyw));
+                            const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+                            if (b0 + b < m) {
+                                if (d2 < lo) in |= 1u << (b0 + b);
+                                else if (d2 <= hi) band |= 1u << (b0 + b);
+                            }
+                        }
                     }
                 }
-#pragma unroll
-                for (uint32_t b = 0; b < 4; b++) {
-                    if (b >= m) break;
-                    bool in = false, band = true;
-                    if (MIXED) {
-                        const float dx =
-                            __fsub_rn(q.x, __fmaf_rn((float)(int)(ck[b] - own), wf, c[b].x));
-                        const float dy = __fsub_rn(q.y, __fadd_rn(c[b].y, dyw));
-                        const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
-                        in = d2 < lo;
-                        band = !in && d2 <= hi;
-                    }
-                    if (band) {
-                        const uint32_t j = j0 + b;
-                        const uint32_t r = exact_pair(a.gxy[k], a.gxy[j], k, j,
-                                                      exact_bounds(ep->eps, ep->thr, ep->tbox), a.gbox);
-                        retest += MIXED ? 1u : 0u;
-                        in = (r & 1u) != 0u;
-                        record_one_way(a, k, j, r);
-                    }
-                    if (in) {
-                        word |= 1u << (g & 31u);
-                        cnt++;
-                    }
-                    if ((g & 31u) == 31u) {
-                        if (bm) bm[(unsigned long long)(g >> 5) * Q] = word;
-                        word = 0;
-                    }
-                    g++;
+                // (the lanes' re-tests run side by side)
+                for (; band; band &= band - 1u) {
+                    const uint32_t b = (uint32_t)__ffs(band) - 1u, j = j0 + b;
+                    const uint32_t r = exact_pair(a.gxy[k], a.gxy[j], k, j, xb, a.gbox);
+                    retest += MIXED ? 1u : 0u;
+                    if (r & 1u) in |= 1u << b;
+                    record_one_way(a, k, j, r);
                 }
+                cnt += (uint32_t)__popc(in);
+                const uint32_t sh = g & 31u;
+                word |= in << sh;
+                if (sh + m >= 32u) {
+                    if (bm) bm[(unsigned long long)(g >> 5) * Q] = word;
+                    word = sh ? in >> (32u - sh) : 0u;
+                }
+                g += m;
             }
         }
         if ((g & 31u) && bm) bm[(unsigned long long)(g >> 5) * Q] = word;
@@ -503,6 +504,10 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
             __syncwarp();
         } else if (Q <= kLaneCand) {
             float4* sq = s_relp[wib];
+            uint16_t* rq = s_rq[wib];
+            uint32_t* madd = s_madd[wib];
+            uint32_t* ids = s_id[wib];
+            static_assert(kLaneCand * 4 <= kWQ, "the accepted bits' words");
             if ((uint32_t)lane < Q) {
                 const float q2 = __fmaf_rn(qx[0], qx[0], __fmul_rn(qy[0], qy[0]));
                 sq[lane] = make_float4(qx[0], qy[0], -0.5f * __fsub_rn(q2, L), 0.f);
@@ -510,8 +515,8 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
             __syncwarp();
             for (uint32_t cb = cbeg; cb < cend; cb += kWC) {
                 // this lane's four candidates (words s = 0..3)
+                __syncwarp();  // (ids of the candidates before have been read)
                 unsigned long long X[2], Y[2], H[2];
-                uint32_t id[4];
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     float rx[2], ry[2], hc[2];
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                     for (int e = 0; e < 2; e++) {
                         const uint32_t g = cb + 32u * (2 * h + e) + (uint32_t)lane;
                         rx[e] = ry[e] = hc[e] = fnan;
-                        id[2 * h + e] = 0;
+                        uint32_t id = 0;
                         if (g < cend) {
                             int i;
                             const uint32_t k = tile_candidate(rows.start, rows.off, nrows, g, &i);
@@ -529,16 +534,17 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                                 rx[e] = __fmaf_rn((float)dcx, wf, loc.x);
                                 ry[e] = __fadd_rn(loc.y, rows.dyw[i]);
                                 hc[e] = 0.5f * __fmaf_rn(rx[e], rx[e], __fmul_rn(ry[e], ry[e]));
-                                id[2 * h + e] = k;
+                                id = k;
                             }
                         }
+                        ids[32 * (2 * h + e) + lane] = id;
                     }
                     X[h] = f2_pack(rx[0], rx[1]);
                     Y[h] = f2_pack(ry[0], ry[1]);
                     H[h] = f2_pack(hc[0], hc[1]);
                 }
                 const uint32_t nwv = (min((uint32_t)kWC, cend - cb) + 31u) >> 5;
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
+                uint32_t w[4] = {0u, 0u, 0u, 0u}, amb[4] = {0u, 0u, 0u, 0u};
                 for (uint32_t q = 0; q < Q; q++) {
                     const float4 Qv = sq[q];
                     const unsigned long long qxx = f2_pack(Qv.x, Qv.x), qyy = f2_pack(Qv.y, Qv.y),
@@ -550,27 +556,65 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                         const unsigned long long s =
                             f2_sub(H[h], f2_fma(qxx, X[h], f2_fma(qyy, Y[h], nh)));
                         const unsigned long long nwm = f2_sub(s, w2p);
-                        bool in0 = (int)(uint32_t)s < 0, in1 = (int)(uint32_t)(s >> 32) < 0;
+                        const bool in0 = (int)(uint32_t)s < 0, in1 = (int)(uint32_t)(s >> 32) < 0;
                         const bool b0 = !in0 && (int)(uint32_t)nwm < 0;
                         const bool b1 = !in1 && (int)(uint32_t)(nwm >> 32) < 0;
-                        if (__any_sync(kFull, b0 || b1)) {
-#pragma unroll
-                            for (int e = 0; e < 2; e++) {
-                                if (e ? b1 : b0) {
-                                    const uint32_t k = id[2 * h + e];
-                                    const uint32_t r = exact_pair(sqd[q], a.gxy[k], qs + q, k, xb, a.gbox);
-                                    my_retest++;
-                                    (e ? in1 : in0) = (r & 1u) != 0u;
-                                    record_one_way(a, qs + q, k, r);
-                                }
-                            }
-                        }
                         const uint32_t m0 = __ballot_sync(kFull, in0), m1 = __ballot_sync(kFull, in1);
                         if ((uint32_t)lane == q) {
                             w[2 * h] = m0;
                             w[2 * h + 1] = m1;
                         }
+                        if (__any_sync(kFull, b0 || b1)) {
+                            const uint32_t a0 = __ballot_sync(kFull, b0), a1 = __ballot_sync(kFull, b1);
+                            if ((uint32_t)lane == q) {
+                                amb[2 * h] = a0;
+                                amb[2 * h + 1] = a1;
+                            }
+                        }
                     }
+                }
+                // pairs in the band, queued as below (entries: query, candidate)
+                if (__any_sync(kFull, (amb[0] | amb[1] | amb[2] | amb[3]) != 0u)) {
+                    const uint32_t c =
+                        __popc(amb[0]) + __popc(amb[1]) + __popc(amb[2]) + __popc(amb[3]);
+                    uint32_t incl = c;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const uint32_t v = __shfl_up_sync(kFull, incl, d);
+                        if (lane >= d) incl += v;
+                    }
+                    const uint32_t excl = incl - c, total = __shfl_sync(kFull, incl, 31);
+                    for (uint32_t pb = 0; pb < total; pb += kRQ) {
+                        uint32_t idx = excl;
+#pragma unroll
+                        for (int s = 0; s < 4; s++) {
+                            for (uint32_t bits = amb[s]; bits; bits &= bits - 1u, idx++) {
+                                if (idx >= pb && idx < pb + kRQ)
+                                    rq[idx - pb] = (uint16_t)(((uint32_t)lane << 7) | (32u * s) |
+                                                              (uint32_t)(__ffs(bits) - 1));
+                            }
+                        }
+                        __syncwarp();
+                        const uint32_t ne = min((uint32_t)kRQ, total - pb);
+                        for (uint32_t e = lane; e < ne; e += 32) {
+                            const uint32_t ent = rq[e], q = ent >> 7, jj = ent & 127u;
+                            const uint32_t kq = ids[jj];
+                            const uint32_t r =
+                                exact_pair(sqd[q], a.gxy[kq], qs + q, kq, xb, a.gbox);
+                            my_retest++;
+                            if (r & 1u) atomicOr(&madd[q * 4 + (jj >> 5)], 1u << (jj & 31u));
+                            record_one_way(a, qs + q, kq, r);
+                        }
+                        __syncwarp();
+                    }
+                    if ((uint32_t)lane < Q) {
+#pragma unroll
+                        for (int s = 0; s < 4; s++) {
+                            w[s] |= madd[lane * 4 + s];
+                            madd[lane * 4 + s] = 0u;
+                        }
+                    }
+                    __syncwarp();
                 }
                 if ((uint32_t)lane < Q) {
                     const unsigned long long wrow = bm0 + (unsigned long long)(cb >> 5) * Q + (uint32_t)lane;
