@@ -410,6 +410,13 @@ struct Timer {
     }
 };
 
+// Plain launches while it lives (stream capture).
+struct PlainLaunches {
+    const bool before;
+    explicit PlainLaunches(bool on) : before(g_plain_launch) { g_plain_launch = before || on; }
+    ~PlainLaunches() { g_plain_launch = before; }
+};
+
 struct Group {
     double eps;
     std::vector<std::pair<uint32_t, uint32_t>> vars;  // (minpts, variant index), minpts desc
@@ -700,6 +707,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     Timer tm(s, capturing);
     DeviceStatus* const d_st = capturing ? rec->d_status : ctx->d_status;
     const unsigned long long launches0 = g_launches.load();
+    PlainLaunches plain(capturing);
     if (capturing) capture_top(*rec, s);
     const size_t t0 = tm.mark();
     const bool host = o.location == VDB_LOC_HOST;

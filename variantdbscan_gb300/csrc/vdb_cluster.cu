@@ -68,6 +68,7 @@ __device__ __forceinline__ void uf_union(uint32_t* parent, uint32_t a, uint32_t 
 }
 
 __global__ void uf_init_kernel(ClusterArgs a, int fresh) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < a.nw) a.bits[k] = 0u;
     if (k >= a.n) return;
@@ -82,6 +83,7 @@ __global__ void uf_init_kernel(ClusterArgs a, int fresh) {
 // larger minpts, only rows of the new cores are read and all their core
 // neighbours are united.
 __global__ void uf_union_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -126,6 +128,7 @@ __device__ __forceinline__ uint32_t uf_find_ro(const uint32_t* parent, uint32_t 
 }
 
 __global__ void save_components_kernel(ClusterArgs a, uint32_t* __restrict__ comp) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
     const uint32_t p = a.gpos[k];
@@ -134,6 +137,7 @@ __global__ void save_components_kernel(ClusterArgs a, uint32_t* __restrict__ com
 }
 
 __global__ void uf_flatten_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n || !is_core(a.deg[k], a.minpts)) return;
     const uint32_t r = uf_find_ro(a.parent, k);
@@ -147,6 +151,7 @@ __global__ void uf_flatten_kernel(ClusterArgs a) {
 // Directed core-core edges between different components (single thread; the
 // list is empty unless the box rule broke the symmetry of a core pair).
 __global__ void resolve_kernel(ClusterArgs a, uint32_t* ws, uint32_t cap) {
+    pdl_sync();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     uint32_t na = *a.asym_count;
     if (na > a.asym_cap) na = a.asym_cap;
@@ -272,6 +277,7 @@ __device__ __forceinline__ uint32_t bit_label(const uint32_t* __restrict__ bits,
 }
 
 __global__ void start_flags_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n || !is_core(a.deg[k], a.minpts)) return;
     if (a.parent[k] == k && a.cstart[k] == k && VDB_GUARD(a.st, a.seed[k] < a.n, 12, a.seed[k]))
@@ -279,6 +285,7 @@ __global__ void start_flags_kernel(ClusterArgs a) {
 }
 
 __global__ void __launch_bounds__(kRankThreads) rank_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t k = rank_bits(a.bits, a.brank, a.nw);
     if (threadIdx.x == 0 && k) atomicAdd(&a.st->clusters, (unsigned long long)k * a.copies);
 }
@@ -291,6 +298,7 @@ __device__ __forceinline__ uint32_t start_time(const ClusterArgs& a, uint32_t u)
 // neighbours that hold the point in their own neighbourhood.  (32 registers:
 // the launch's 8 blocks of 256 threads per SM all stay resident.)
 __global__ void __launch_bounds__(kThreads, 8) border_pull_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -326,6 +334,7 @@ __global__ void __launch_bounds__(kThreads, 8) border_pull_kernel(ClusterArgs a)
 // In-edges that the non-core row does not list: pairs accepted only towards
 // the non-core point.
 __global__ void asym_push_kernel(ClusterArgs a) {
+    pdl_sync();
     uint32_t na = *a.asym_count;
     if (na > a.asym_cap) na = a.asym_cap;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < na;
@@ -345,6 +354,7 @@ __global__ void asym_push_kernel(ClusterArgs a) {
 }
 
 __global__ void write_labels_kernel(ClusterArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
     uint32_t lab;
@@ -373,6 +383,7 @@ __global__ void write_labels_kernel(ClusterArgs a) {
 // grids by binary search), so that the kernels below walk lists of cells that
 // exist instead of probing every offset.
 __global__ void cell_ranges_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t rho = (uint32_t)a.ep->rho;
     const uint32_t ncl = *a.ncl;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
@@ -436,6 +447,7 @@ __device__ __forceinline__ uint32_t test_pair(const CellArgs& a, const PairTest&
 // Start state of all slots: every cell its own root in the first slot's
 // forest (the others copy their predecessor's), no seeds, no cluster starts.
 __global__ void cells_init_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < a.nw)
         for (int v = 0; v < a.m; v++) a.bits[(size_t)v * a.nw + k] = 0u;
@@ -449,6 +461,7 @@ __global__ void cells_init_kernel(CellArgs a) {
 }
 
 __global__ void cell_best_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = k < a.n;
     const uint32_t c = in ? a.cscan[k + 1] - 1u : kNone;
@@ -467,6 +480,7 @@ __global__ void cell_best_kernel(CellArgs a) {
 // Along the rows (first slot only): a warp's run of cells that are joined to
 // their left neighbours points at its first cell, without atomics.
 __global__ void cell_runs_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
     if (c - lane >= ncl) return;  // (whole warps)
@@ -493,6 +507,7 @@ __global__ void cell_runs_kernel(CellArgs a) {
 // mostly want the same two trees joined: one union per pair of roots and warp.
 constexpr int kNearLoads = 5;  // cells of two per eps: all the cells of a row within reach
 __global__ void __launch_bounds__(kThreads, 4) cell_near_kernel(CellArgs a, int v) {
+    pdl_sync();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const uint32_t dy = blockIdx.y ^ 1u;  // next row first
     const uint32_t ncl = *a.ncl;
@@ -562,6 +577,7 @@ constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes
 // other pairs are searched by the whole warp, lanes over the point pairs (or,
 // for large cells, over the first cell's points within eps of the second).
 __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int v) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
     const uint32_t mp = a.mp[v];
@@ -708,6 +724,7 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
 // cells by one load) and after the search (last), when they are also the next
 // slot's start: a smaller minpts keeps every core and every connection.
 __global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
+    pdl_sync();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= *a.ncl) return;
     uint32_t* parent = a.parent + (size_t)v * a.n;
@@ -718,6 +735,7 @@ __global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
 
 // seed[root] = first visit position among the component's cores (y: slot).
 __global__ void cell_seed_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const int v = blockIdx.y;
     if (k >= a.n || a.deg[k] < a.mp[v]) return;
@@ -735,6 +753,7 @@ __global__ void cell_seed_kernel(CellArgs a) {
 // thread per slot; run only when the table has one-way pairs): the components
 // that an earlier cluster's expansion absorbs take its start as their seed.
 __global__ void cell_resolve_kernel(CellArgs a, uint32_t* ws, uint32_t cap) {
+    pdl_sync();
     if (threadIdx.x != 0) return;
     const int v = blockIdx.x;
     const uint32_t mp = a.mp[v];
@@ -802,6 +821,7 @@ __global__ void cell_resolve_kernel(CellArgs a, uint32_t* ws, uint32_t cap) {
 // cst = visit position at which the cluster of the cell's cores starts (kNone:
 // no cores); the starts' bits (y: slot).
 __global__ void cell_starts_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const int v = blockIdx.y;
     if (c >= *a.ncl) return;
@@ -818,6 +838,7 @@ __global__ void cell_starts_kernel(CellArgs a) {
 
 // The slots' ranks and numbers of clusters (one block per slot).
 __global__ void __launch_bounds__(kRankThreads) cell_rank_kernel(CellArgs a) {
+    pdl_sync();
     const int v = blockIdx.x;
     const uint32_t k = rank_bits(a.bits + (size_t)v * a.nw, a.brank + (size_t)v * a.nw, a.nw);
     if (threadIdx.x == 0 && k) atomicAdd(&a.st->clusters, (unsigned long long)k * a.copies[v]);
@@ -831,6 +852,7 @@ __device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32
 // Labels of the cores, and the saved components (comp[visit position] =
 // cluster start of the core there, kNone for other points).
 __global__ void cell_core_labels_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n) return;
     const uint32_t d = a.deg[k], c = a.cscan[k + 1] - 1u, o = a.gorig[k], p = a.gpos[k];
@@ -859,6 +881,7 @@ __global__ void cell_core_labels_kernel(CellArgs a) {
 // are done by the warp one after the other, lanes over the cells' points.
 constexpr uint32_t kLaneCores = 16;
 __global__ void __launch_bounds__(kThreads, 5) cell_border_kernel(CellArgs a) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t d = k < a.n ? a.deg[k] : kNone;
@@ -1015,44 +1038,35 @@ size_t resolve_scratch_bytes() { return (size_t)kResolveCap * 6 * sizeof(uint32_
 
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    uf_init_kernel<<<nblk(std::max(a.n, a.nw)), kThreads, 0, s>>>(a, fresh ? 1 : 0);
+    launch(uf_init_kernel, nblk(std::max(a.n, a.nw)), kThreads, s, a, fresh ? 1 : 0);
 }
 
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s) {
-    if (a.row_hi > a.row_lo) { VDB_COUNT_LAUNCH(); uf_union_kernel<<<nblocks, kThreads, 0, s>>>(a); }
+    if (a.row_hi > a.row_lo) { launch(uf_union_kernel, nblocks, kThreads, s, a); }
 }
 
 void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    uf_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    resolve_kernel<<<1, 32, 0, s>>>(a, (uint32_t*)resolve_ws, kResolveCap);
-    VDB_COUNT_LAUNCH();
-    start_flags_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    rank_kernel<<<1, kRankThreads, 0, s>>>(a);
+    launch(uf_flatten_kernel, nblk(a.n), kThreads, s, a);
+    launch(resolve_kernel, 1, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);
+    launch(start_flags_kernel, nblk(a.n), kThreads, s, a);
+    launch(rank_kernel, 1, kRankThreads, s, a);
 }
 
 void launch_save_components(const ClusterArgs& a, uint32_t* comp, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    save_components_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, comp);
+    launch(save_components_kernel, nblk(a.n), kThreads, s, a, comp);
 }
 
 void launch_border_pull(const ClusterArgs& a, int nblocks, cudaStream_t s) {
     if (a.row_hi <= a.row_lo) return;
-    VDB_COUNT_LAUNCH();
-    border_pull_kernel<<<nblocks, kThreads, 0, s>>>(a);
+    launch(border_pull_kernel, nblocks, kThreads, s, a);
 }
 
 void launch_label_write(const ClusterArgs& a, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    asym_push_kernel<<<64, kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    write_labels_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    launch(asym_push_kernel, 64, kThreads, s, a);
+    launch(write_labels_kernel, nblk(a.n), kThreads, s, a);
 }
 
 void launch_border_and_write(const ClusterArgs& a, int nblocks, cudaStream_t s) {
@@ -1065,38 +1079,24 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
                   cudaStream_t s) {
     if (!a.n) return;
     const dim3 per_slot(nblk(a.n), (unsigned)a.m);
-    VDB_COUNT_LAUNCH();
-    cells_init_kernel<<<nblk(std::max(a.n, a.nw)), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_ranges_kernel<<<dim3(nblk(a.n), (unsigned)nrows), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_best_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_runs_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    launch(cells_init_kernel, nblk(std::max(a.n, a.nw)), kThreads, s, a);
+    launch(cell_ranges_kernel, dim3(nblk(a.n), (unsigned)nrows), kThreads, s, a);
+    launch(cell_best_kernel, nblk(a.n), kThreads, s, a);
+    launch(cell_runs_kernel, nblk(a.n), kThreads, s, a);
     for (int v = 0; v < a.m; v++) {
-        VDB_COUNT_LAUNCH();
-        cell_near_kernel<<<dim3(nblk(a.n), 2), kThreads, 0, s>>>(a, v);
-        VDB_COUNT_LAUNCH();
-        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v, 0);
-        VDB_COUNT_LAUNCH();
-        cell_pairs_kernel<<<dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, 0, s>>>(a, v);
-        VDB_COUNT_LAUNCH();
-        cell_flatten_kernel<<<nblk(a.n), kThreads, 0, s>>>(a, v, 1);
+        launch(cell_near_kernel, dim3(nblk(a.n), 2), kThreads, s, a, v);
+        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v, 0);
+        launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, s, a, v);
+        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v, 1);
     }
-    VDB_COUNT_LAUNCH();
-    cell_seed_kernel<<<per_slot, kThreads, 0, s>>>(a);
+    launch(cell_seed_kernel, per_slot, kThreads, s, a);
     if (one_way) {
-        VDB_COUNT_LAUNCH();
-        cell_resolve_kernel<<<a.m, 32, 0, s>>>(a, (uint32_t*)resolve_ws, kResolveCap);
+        launch(cell_resolve_kernel, a.m, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);
     }
-    VDB_COUNT_LAUNCH();
-    cell_starts_kernel<<<per_slot, kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_rank_kernel<<<a.m, kRankThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_core_labels_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
-    VDB_COUNT_LAUNCH();
-    cell_border_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    launch(cell_starts_kernel, per_slot, kThreads, s, a);
+    launch(cell_rank_kernel, a.m, kRankThreads, s, a);
+    launch(cell_core_labels_kernel, nblk(a.n), kThreads, s, a);
+    launch(cell_border_kernel, nblk(a.n), kThreads, s, a);
 }
 
 }  // namespace vdb

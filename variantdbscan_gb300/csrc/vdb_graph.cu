@@ -10,6 +10,7 @@ namespace {
 
 __global__ void graph_check_kernel(GraphCheck chk, uint32_t* bad,
                                    cudaGraphConditionalHandle next) {
+    pdl_sync();
     if (threadIdx.x != 0) return;
     // an earlier checkpoint failed: everything after it is skipped
     bool ok = *bad == 0u;
@@ -46,6 +47,7 @@ __global__ void graph_check_kernel(GraphCheck chk, uint32_t* bad,
 }
 
 __global__ void store_eps_kernel(EpsParams* dst, EpsParams v) {
+    pdl_sync();
     if (threadIdx.x == 0 && blockIdx.x == 0) *dst = v;
 }
 
@@ -53,13 +55,11 @@ __global__ void store_eps_kernel(EpsParams* dst, EpsParams v) {
 
 void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphConditionalHandle next,
                         cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    graph_check_kernel<<<1, 32, 0, s>>>(chk, bad, next);
+    launch(graph_check_kernel, 1, 32, s, chk, bad, next);
 }
 
 void launch_store_eps(EpsParams* dst, const EpsParams& v, cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    store_eps_kernel<<<1, 32, 0, s>>>(dst, v);
+    launch(store_eps_kernel, 1, 32, s, dst, v);
 }
 
 }  // namespace vdb

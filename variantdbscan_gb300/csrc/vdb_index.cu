@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(kThreads) visit_keys_kernel(
     const double* __restrict__ x, const double* __restrict__ y, uint32_t n,
     const BBox* __restrict__ bb, uint32_t* __restrict__ keys, int passes,
     uint32_t* __restrict__ hist, DeviceStatus* st) {
+    pdl_sync();
     __shared__ DigitCounts s_h;
     __shared__ double s_p[4];
     __shared__ float s_f[2];
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(kThreads) visit_keys_kernel(
 __global__ void mpb_kernel(const double* __restrict__ x, const double* __restrict__ y,
                            const uint32_t* __restrict__ vorder, uint32_t n, int mbb,
                            uint32_t nboxes, MpbBox* __restrict__ boxes) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t b = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b >= nboxes) return;  // (whole warps)
@@ -155,6 +157,7 @@ __device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, float
 __global__ void __launch_bounds__(kThreads) grid_keys_kernel(
     const double* __restrict__ x, const double* __restrict__ y, uint32_t n, GridParams g,
     uint32_t* __restrict__ keys, int passes, uint32_t* __restrict__ hist) {
+    pdl_sync();
     __shared__ DigitCounts s_h;
     counts_clear(s_h, passes);
     const float iw = (float)(1.0 / g.w);
@@ -190,6 +193,7 @@ __device__ __forceinline__ void gather_point(const OrderArgs& a, uint32_t k, uin
 }
 
 __global__ void gather_kernel(OrderArgs a) {
+    pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < a.n) gather_point(a, k, k);
 }
@@ -200,6 +204,7 @@ __global__ void gather_kernel(OrderArgs a) {
 constexpr int kOrderItems = 4;
 constexpr uint32_t kOrderTile = kLookThreads * kOrderItems;
 __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookState ls) {
+    pdl_sync();
     const uint32_t tile = lookback_ticket(ls);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint64_t base = (uint64_t)tile * kOrderTile + wid * (32u * kOrderItems);
@@ -280,6 +285,7 @@ __global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t* __
                                                               const uint32_t* __restrict__ nclp,
                                                               uint32_t n, uint64_t entries,
                                                               uint32_t* __restrict__ cell_start) {
+    pdl_sync();
     __shared__ uint32_t s_v[kFillCells + kFillCells / kFillItems];  // 16 cells and a pad word
     __shared__ uint32_t s_lim[2], s_warp[kThreads / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -334,6 +340,7 @@ __global__ void __launch_bounds__(kThreads) cell_start_kernel(const uint32_t* __
 __global__ void cell_rows_kernel(const uint32_t* __restrict__ ckey,
                                  const uint32_t* __restrict__ nclp, uint32_t ncx_pad, uint32_t ncy,
                                  uint32_t* __restrict__ crow) {
+    pdl_sync();
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r > ncy) return;
     const uint64_t v = (uint64_t)r * ncx_pad;
@@ -355,8 +362,7 @@ unsigned key_blocks(uint32_t n) { return std::min<unsigned>(nblk(n), 152u * 8u);
 void launch_visit_keys(const double* x, const double* y, uint32_t n, const BBox* bb,
                        uint32_t* keys, uint32_t* hist, DeviceStatus* st, cudaStream_t s) {
     if (!n) return;
-    VDB_COUNT_LAUNCH();
-    visit_keys_kernel<<<key_blocks(n), kThreads, 0, s>>>(x, y, n, bb, keys, sort_passes(kVisitBits),
+    launch(visit_keys_kernel, key_blocks(n), kThreads, s, x, y, n, bb, keys, sort_passes(kVisitBits),
                                                          hist, st);
 }
 
@@ -364,8 +370,7 @@ void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, 
                       int mbb, MpbBox* boxes, cudaStream_t s) {
     uint32_t nb = (uint32_t)(((uint64_t)n + (uint32_t)mbb - 1) / (uint32_t)mbb);
     if (nb) {
-        VDB_COUNT_LAUNCH();
-        mpb_kernel<<<nblk((uint64_t)nb * 32u), kThreads, 0, s>>>(x, y, vorder, n, mbb, nb,
+        launch(mpb_kernel, nblk((uint64_t)nb * 32u), kThreads, s, x, y, vorder, n, mbb, nb,
                                                                   boxes);
     }
 }
@@ -373,8 +378,7 @@ void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, 
 void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g, int bits,
                       uint32_t* keys, uint32_t* hist, cudaStream_t s) {
     if (!n) return;
-    VDB_COUNT_LAUNCH();
-    grid_keys_kernel<<<key_blocks(n), kThreads, 0, s>>>(x, y, n, g, keys, sort_passes(bits), hist);
+    launch(grid_keys_kernel, key_blocks(n), kThreads, s, x, y, n, g, keys, sort_passes(bits), hist);
 }
 
 size_t order_state_bytes(uint32_t n) {
@@ -384,28 +388,23 @@ size_t order_state_bytes(uint32_t n) {
 void launch_order(const OrderArgs& a, void* zeroed, cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
-    VDB_COUNT_LAUNCH();
-    order_kernel<<<nb, kLookThreads, 0, s>>>(a, look_state(zeroed));
+    launch(order_kernel, nb, kLookThreads, s, a, look_state(zeroed));
 }
 
 void launch_gather(const OrderArgs& a, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    gather_kernel<<<nblk(a.n), kThreads, 0, s>>>(a);
+    launch(gather_kernel, nblk(a.n), kThreads, s, a);
 }
 
 void launch_cell_start(const uint32_t* ckey, const uint32_t* clist, const uint32_t* ncl,
                        uint32_t n, const GridParams& g, uint32_t* cell_start, cudaStream_t s) {
     const uint64_t entries = g.ncells + 1;
-    VDB_COUNT_LAUNCH();
-    cell_start_kernel<<<(unsigned)((entries + kFillCells - 1) / kFillCells), kThreads, 0, s>>>(
-        ckey, clist, ncl, n, entries, cell_start);
+    launch(cell_start_kernel, (unsigned)((entries + kFillCells - 1) / kFillCells), kThreads, s, ckey, clist, ncl, n, entries, cell_start);
 }
 
 void launch_cell_rows(const uint32_t* ckey, const uint32_t* ncl, const GridParams& g,
                       uint32_t* crow, cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    cell_rows_kernel<<<nblk((uint64_t)g.ncy + 1), kThreads, 0, s>>>(ckey, ncl, g.ncx_pad, g.ncy,
+    launch(cell_rows_kernel, nblk((uint64_t)g.ncy + 1), kThreads, s, ckey, ncl, g.ncx_pad, g.ncy,
                                                                    crow);
 }
 

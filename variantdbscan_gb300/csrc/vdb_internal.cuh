@@ -13,7 +13,33 @@ namespace vdb {
 
 // Kernels launched by this library since it was loaded.
 extern std::atomic<unsigned long long> g_launches;
-#define VDB_COUNT_LAUNCH() (::vdb::g_launches.fetch_add(1, std::memory_order_relaxed))
+
+// Launches go out with programmatic stream serialization: a kernel may be
+// scheduled while the one before it still runs, and every kernel begins with
+// pdl_sync(), which waits until that one has completed and its writes are
+// visible (so the order of the work is the stream's), then lets the next one
+// be scheduled.  A chain of small kernels thus does not pay each launch's
+// latency in turn.  Not while a stream is captured (the thread's g_plain_launch;
+// the graph's nodes depend on whole kernels).
+extern thread_local bool g_plain_launch;
+static __device__ __forceinline__ void pdl_sync() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... P, class... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = g_plain_launch ? 0 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
 constexpr int kVisitBins = 300;          // src/main.cpp:107 (binDataset(&dataPoints, 300, ...))
 constexpr int kMaxRows = 65;             // neighbour rows per tile: 2*rho+1 <= 65

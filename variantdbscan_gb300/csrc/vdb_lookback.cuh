@@ -104,6 +104,7 @@ static __device__ __forceinline__ unsigned long long block_lookback(unsigned lon
 }
 
 // The same for one counter per thread: states of tile t at p[t * stride].
+constexpr int kDigitLooks = 8;
 static __device__ __forceinline__ unsigned long long digit_lookback(uint32_t v, uint32_t tile,
                                                                     unsigned long long* p,
                                                                     uint32_t stride,
@@ -115,21 +116,21 @@ static __device__ __forceinline__ unsigned long long digit_lookback(uint32_t v, 
     look_store(p + (size_t)tile * stride, kLookSum | v);
     unsigned long long before = 0;
     for (int64_t t = (int64_t)tile - 1; t >= 0;) {
-        // four states at once: their loads overlap
-        unsigned long long s[4];
+        // many states at once: their loads overlap
+        unsigned long long s[kDigitLooks];
 #pragma unroll
-        for (int j = 0; j < 4; j++)
+        for (int j = 0; j < kDigitLooks; j++)
             s[j] = t - j >= 0 ? look_load(p + (size_t)(t - j) * stride) : kLookPrefix;
         bool done = false;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
+        for (int j = 0; j < kDigitLooks; j++) {
             if (done) continue;
             if ((s[j] >> 62) == 0ull) s[j] = look_wait(p + (size_t)(t - j) * stride, st);
             before += s[j] & kLookMask;
             done = (s[j] >> 62) == 2ull;
         }
         if (done) break;
-        t -= 4;
+        t -= kDigitLooks;
     }
     look_store(p + (size_t)tile * stride, kLookPrefix | (before + v));
     return before;

@@ -7,6 +7,7 @@
 namespace vdb {
 
 std::atomic<unsigned long long> g_launches{0};
+thread_local bool g_plain_launch = false;
 
 // ------------------------------------------------------------------ scan
 //
@@ -24,6 +25,7 @@ __global__ void __launch_bounds__(kLookThreads) scan_kernel(const uint32_t* __re
                                                             unsigned long long* __restrict__ out,
                                                             uint32_t n, LookState ls,
                                                             DeviceStatus* st) {
+    pdl_sync();
     const uint32_t tile = lookback_ticket(ls);
     const uint64_t base = (uint64_t)tile * kScanTile + threadIdx.x * kScanItems;
     uint32_t v[kScanItems];
@@ -56,8 +58,7 @@ void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t n, vo
                      DeviceStatus* st, cudaStream_t s) {
     if (!n) return;
     const uint32_t nb = (n + kScanTile - 1) / kScanTile;
-    VDB_COUNT_LAUNCH();
-    scan_kernel<<<nb, kLookThreads, 0, s>>>(in, out, n, look_state(state), st);
+    launch(scan_kernel, nb, kLookThreads, s, in, out, n, look_state(state), st);
 }
 
 // ------------------------------------------------------------------ radix sort
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kDigits) radix_pass_kernel(
     uint32_t* __restrict__ okeys, uint32_t* __restrict__ ovals, uint32_t* __restrict__ oinv,
     uint32_t n, int shift, int drop, const uint32_t* __restrict__ hist,
     unsigned long long* __restrict__ state, uint32_t* __restrict__ ticket, DeviceStatus* st) {
+    pdl_sync();
     __shared__ uint16_t s_cnt[kSortWarps][kDigits];
     __shared__ uint32_t s_base[kDigits];
     __shared__ uint32_t s_warp[kSortWarps];
@@ -170,8 +172,7 @@ void run_pass(uint32_t nb, const uint32_t* keys_in, const uint2* in, uint2* out,
               uint32_t* ovals, uint32_t* oinv, uint32_t n, int shift, int drop,
               const uint32_t* hist, unsigned long long* state, uint32_t* ticket, DeviceStatus* st,
               cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    radix_pass_kernel<ITEMS><<<nb, kDigits, 0, s>>>(keys_in, in, out, okeys, ovals, oinv, n, shift,
+    launch(radix_pass_kernel<ITEMS>, nb, kDigits, s, keys_in, in, out, okeys, ovals, oinv, n, shift,
                                                     drop, hist, state, ticket, st);
 }
 
@@ -260,6 +261,7 @@ __global__ void __launch_bounds__(kBoxThreads) bbox_kernel(const double* __restr
                                                            const double* __restrict__ y,
                                                            uint32_t n, BoxAcc* part,
                                                            uint32_t* done, BBox* out) {
+    pdl_sync();
     __shared__ bool s_last;
     const BoxAcc none{DBL_MAX, -DBL_MAX, DBL_MAX, -DBL_MAX, 0u};
     BoxAcc a = none;
@@ -309,8 +311,7 @@ size_t bbox_scratch_bytes() { return sizeof(BoxAcc) * kBoxBlocks; }
 void launch_bbox(const double* x, const double* y, uint32_t n, BBox* out, void* scratch,
                  uint32_t* zeroed, cudaStream_t s) {
     const int nb = (int)std::max<uint32_t>(1u, std::min<uint32_t>(kBoxBlocks, (n + 511u) / 512u));
-    VDB_COUNT_LAUNCH();
-    bbox_kernel<<<nb, kBoxThreads, 0, s>>>(x, y, n, (BoxAcc*)scratch, zeroed, out);
+    launch(bbox_kernel, nb, kBoxThreads, s, x, y, n, (BoxAcc*)scratch, zeroed, out);
 }
 
 }  // namespace vdb

@@ -194,6 +194,7 @@ constexpr uint32_t kLaneCand = 16;
 constexpr uint32_t kBoxCand = 2048;
 constexpr uint32_t kBoxRun = 36;
 __global__ void word_boxes_kernel(TableArgs a) {
+    pdl_sync();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k0 = 4u * i;
     if (k0 >= a.n) return;
@@ -323,6 +324,7 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
 
 template <bool MIXED>
 __global__ void __launch_bounds__(kTT) small_count_kernel(TableArgs a) {
+    pdl_sync();
     small_count<MIXED>(a, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -361,6 +363,7 @@ __device__ void small_expand(const TableArgs& a, uint32_t k) {
 
 template <typename E>
 __global__ void __launch_bounds__(kTT) small_expand_kernel(TableArgs a) {
+    pdl_sync();
     const uint32_t k = a.row_lo + blockIdx.x * blockDim.x + threadIdx.x;
     if (k < a.row_hi) small_expand<E>(a, k);
 }
@@ -371,6 +374,7 @@ __global__ void __launch_bounds__(kTT) small_expand_kernel(TableArgs a) {
 // ([word][query] words; bit j of word w: candidate 32w+j is a neighbour).
 template <bool MIXED>
 __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
+    pdl_sync();
     __shared__ WarpRows s_rows[kWPB];
     __shared__ uint32_t s_id[kWPB][MIXED ? kWC : 1];
     // lane = query: candidate pairs (x_a, x_b, y_a, y_b); lane = candidate:
@@ -928,6 +932,7 @@ __device__ __forceinline__ void bulk_copy_to_global(void* gdst, const void* ssrc
 
 template <typename E>
 __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
+    pdl_sync();
     constexpr uint32_t kVec = XFmt<E>::kVec, kSec = XFmt<E>::kSec, kStage = XFmt<E>::kStage;
     constexpr bool kCompact = sizeof(E) == 2;
     static_assert(kWXW == 16, "the query slot layout holds 16 words");
@@ -1141,6 +1146,7 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
 // more of the kernel's dependency latency (2M sweep: 34.7 ms of tables against
 // 40.3 with two buffers per half at 6 blocks).
 __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
+    pdl_sync();
     using E = uint16_t;
     constexpr uint32_t kVec = XFmt<E>::kVec, kSec = XFmt<E>::kSec, kStage = XFmt<E>::kStage;
     static_assert(kWXW == 16, "the query slot layout holds 16 words");
@@ -1328,6 +1334,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
 
 template <bool MIXED, bool FILL>
 __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
+    pdl_sync();
     __shared__ float2 s_rel[kChunk];
     __shared__ double2 s_xy[kChunk];
     __shared__ uint32_t s_id[kChunk];
@@ -1578,6 +1585,7 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
     uint32_t* __restrict__ loff, unsigned long long* __restrict__ nwords,
     uint32_t* __restrict__ nunits, LookState lu, LookState lw) {
+    pdl_sync();
     const uint32_t tile = lookback_ticket(lu);
     const uint32_t t = tile * kLookThreads + threadIdx.x;
     if (t < a.n) a.deg[t] = 0u;
@@ -1637,6 +1645,7 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
 // ulist: (unit, tile) of the units that warps take: a thread per tile, long
 // lists by the whole warp.
 __global__ void unit_list_kernel(TableArgs a, uint2* ulist) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ntiles = *a.ntiles;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1671,6 +1680,7 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long x) {
 // entries q of row p of mix64(p << 32 | q), plus a constant for entries
 // flagged one-way, p and q input indices.
 __global__ void table_hash_kernel(TableArgs a, const uint32_t* __restrict__ gorig) {
+    pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -1707,6 +1717,7 @@ __global__ void table_hash_kernel(TableArgs a, const uint32_t* __restrict__ gori
 // recorded them): b in row a when dir == 1, a in row b when dir == 2.  Rows are
 // sorted by neighbour index.
 __global__ void asym_flags_kernel(TableArgs a) {
+    pdl_sync();
     uint32_t na = *a.asym_n;
     if (na > a.asym_cap) na = a.asym_cap;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < na;
@@ -1771,31 +1782,27 @@ int table_tile_queries() {
 void launch_count(const TableArgs& a, int nblocks, cudaStream_t s) {
     if (!a.mixed || a.n > kSmallFused) {
         const unsigned nb = (a.n + kTT - 1) / kTT;
-        VDB_COUNT_LAUNCH();
         if (a.mixed)
-            small_count_kernel<true><<<nb, kTT, 0, s>>>(a);
+            launch(small_count_kernel<true>, nb, kTT, s, a);
         else
-            small_count_kernel<false><<<nb, kTT, 0, s>>>(a);
+            launch(small_count_kernel<false>, nb, kTT, s, a);
     }
-    VDB_COUNT_LAUNCH();
     if (a.mixed)
-        count_kernel<true><<<nblocks, kWPB * 32, 0, s>>>(a);
+        launch(count_kernel<true>, nblocks, kWPB * 32, s, a);
     else
-        count_kernel<false><<<nblocks, kWPB * 32, 0, s>>>(a);
+        launch(count_kernel<false>, nblocks, kWPB * 32, s, a);
 }
 
 void launch_word_boxes(const TableArgs& a, cudaStream_t s) {
     const uint32_t nb = (a.n + 3u) / 4u;
-    VDB_COUNT_LAUNCH();
-    word_boxes_kernel<<<(nb + kTT - 1) / kTT, kTT, 0, s>>>(a);
+    launch(word_boxes_kernel, (nb + kTT - 1) / kTT, kTT, s, a);
 }
 
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
     if (a.mixed)
-        table_kernel<true, true><<<nblocks, kTT, 0, s>>>(a);
+        launch(table_kernel<true, true>, nblocks, kTT, s, a);
     else
-        table_kernel<false, true><<<nblocks, kTT, 0, s>>>(a);
+        launch(table_kernel<false, true>, nblocks, kTT, s, a);
 }
 
 size_t words_state_bytes(uint32_t n) {
@@ -1807,44 +1814,37 @@ void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* u
                        cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (a.n + kLookThreads - 1) / kLookThreads;
-    VDB_COUNT_LAUNCH();
-    tile_words_kernel<<<nb, kLookThreads, 0, s>>>(
-        a, boff, uoff, loff, nwords, nunits, look_state(zeroed),
+    launch(tile_words_kernel, nb, kLookThreads, s, a, boff, uoff, loff, nwords, nunits, look_state(zeroed),
         look_state((char*)zeroed + words_state_bytes(a.n) / 2));
 }
 
 void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s) {
     if (!a.n) return;
-    VDB_COUNT_LAUNCH();
-    unit_list_kernel<<<(a.n + kTT - 1) / kTT, kTT, 0, s>>>(a, ulist);
+    launch(unit_list_kernel, (a.n + kTT - 1) / kTT, kTT, s, a, ulist);
 }
 
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
     if (a.n > kSmallFused && a.row_hi > a.row_lo) {
         const unsigned nb = (a.row_hi - a.row_lo + kTT - 1) / kTT;
-        VDB_COUNT_LAUNCH();
         if (a.compact)
-            small_expand_kernel<uint16_t><<<nb, kTT, 0, s>>>(a);
+            launch(small_expand_kernel<uint16_t>, nb, kTT, s, a);
         else
-            small_expand_kernel<uint32_t><<<nb, kTT, 0, s>>>(a);
+            launch(small_expand_kernel<uint32_t>, nb, kTT, s, a);
     }
     if (a.unit_hi <= a.unit_lo && a.n > kSmallFused) return;
-    VDB_COUNT_LAUNCH();
     if (a.compact)
-        expand16_kernel<<<nblocks, kXPB * 32, 0, s>>>(a);
+        launch(expand16_kernel, nblocks, kXPB * 32, s, a);
     else
-        expand_kernel<uint32_t><<<nblocks, kXPB * 32, 0, s>>>(a);
+        launch(expand_kernel<uint32_t>, nblocks, kXPB * 32, s, a);
 }
 
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s) {
     if (a.row_hi <= a.row_lo) return;
-    VDB_COUNT_LAUNCH();
-    table_hash_kernel<<<nblocks, kTT, 0, s>>>(a, gorig);
+    launch(table_hash_kernel, nblocks, kTT, s, a, gorig);
 }
 
 void launch_asym_flags(const TableArgs& a, cudaStream_t s) {
-    VDB_COUNT_LAUNCH();
-    asym_flags_kernel<<<64, kTT, 0, s>>>(a);
+    launch(asym_flags_kernel, 64, kTT, s, a);
 }
 
 int table_blocks_per_sm(bool fill, bool mixed) {
