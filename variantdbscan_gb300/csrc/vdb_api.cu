@@ -440,7 +440,8 @@ constexpr int kCellsPerEps = 2;
 // 1.5), and 8 or 16 cost 10 to 35% more there.  Two cells win slightly where
 // most cells are empty (1M sweep, eps 0.1: 0.766 against 0.763 ms of count and
 // table; 400k uniform 3% less), one where they are not (eps 0.4: 2.45 against
-// 2.52 ms), so the line lies at half a point per cell.
+// 2.52 ms), so the line lies at half a point per cell.  FP64 tests keep one
+// cell: their time is the number of candidates (100k sweep: 2.8 against 3.4 ms).
 uint32_t default_tile_cells(uint32_t n, uint64_t ncells) {
     return (uint64_t)n * 2 < ncells ? 2u : 1u;
 }
@@ -1076,7 +1077,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 ep.mixed = 0;
             } else {
                 g = make_grid(hb, eps / r, o.tile_cells > 0 ? (uint32_t)o.tile_cells : 1u);
-                if (o.tile_cells <= 0 && default_tile_cells(n, g.ncells) > 1u) {
+                if (o.tile_cells <= 0 && want_mixed && default_tile_cells(n, g.ncells) > 1u) {
                     // (a padding that would exceed the cell limit coarsens the
                     // cells: such a shape is not taken)
                     const GridParams g2 = make_grid(hb, eps / r, default_tile_cells(n, g.ncells));

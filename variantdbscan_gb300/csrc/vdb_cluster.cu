@@ -377,39 +377,6 @@ __global__ void write_labels_kernel(ClusterArgs a) {
 // minpts of one epsilon (slots, largest minpts first) share the kernels that
 // do not depend on one another.
 
-// Neighbour cells: crng[i * n + c] = the non-empty cells [x, y) of row
-// i - rho within reach of cell c, ccx[c] = the column of cell c.  One thread
-// per cell and row looks them up once for all slots and kernels (in sparse
-// grids by binary search), so that the kernels below walk lists of cells that
-// exist instead of probing every offset.
-__global__ void cell_ranges_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t rho = (uint32_t)a.ep->rho;
-    const uint32_t ncl = *a.ncl;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
-    if (c >= ncl || r > 2u * rho) return;
-    const uint32_t key = a.gkey[a.clist[c]];
-    const int cy = (int)(key / a.g.ncx_pad), cx = (int)(key - (uint32_t)cy * a.g.ncx_pad);
-    const int ry = cy + (int)r - (int)rho, reach = a.ep->reach[r];
-    const uint32_t lo = (uint32_t)max(cx - reach, 0);
-    const uint32_t hi = (uint32_t)min(cx + reach, (int)a.g.ncx - 1);
-    uint2 out = make_uint2(0u, 0u);
-    if (ry >= 0 && ry < (int)a.g.ncy) {
-        if (a.g.sparse) {
-            const uint32_t re = a.crow[ry + 1];
-            out.x = cx_lower_bound(a.ccx, a.crow[ry], re, lo);
-            out.y = out.x;
-            while (out.y < re && a.ccx[out.y] <= hi) out.y++;
-        } else {
-            const uint32_t base = (uint32_t)ry * a.g.ncx_pad;
-            out.x = a.cscan[a.cell_start[base + lo]];
-            out.y = a.cscan[a.cell_start[base + hi + 1]];
-        }
-    }
-    if (!VDB_GUARD(a.st, out.x <= out.y && out.y <= ncl, 16, out.y)) out = make_uint2(0u, 0u);
-    a.crng[(size_t)r * a.n + c] = out;
-}
-
 // cbest[c] = largest degree of the cell (high word) and the first point that
 // has it (complemented, low word): the cell has cores at minpts m iff the
 // high word is >= m, and that point is one of them.
@@ -444,20 +411,50 @@ __device__ __forceinline__ uint32_t test_pair(const CellArgs& a, const PairTest&
     return exact_pair(a.gxy[ku], a.gxy[kv], ku, kv, t.xb, a.gbox);
 }
 
-// Start state of all slots: every cell its own root in the first slot's
-// forest (the others copy their predecessor's), no seeds, no cluster starts.
-__global__ void cells_init_kernel(CellArgs a) {
+// Neighbour cells: crng[i * n + c] = the non-empty cells [x, y) of row
+// i - rho within reach of cell c, ccx[c] = the column of cell c.  One thread
+// per cell and row looks them up once for all slots and kernels (in sparse
+// grids by binary search), so that the kernels below walk lists of cells that
+// exist instead of probing every offset.
+//
+// The middle row's threads also set the slots' start state: no seeds, no
+// cluster starts, every cell its own root in the first slot.
+__global__ void cell_setup_kernel(CellArgs a) {
     pdl_sync();
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < a.nw)
-        for (int v = 0; v < a.m; v++) a.bits[(size_t)v * a.nw + k] = 0u;
-    if (k >= a.n) return;
-    a.cbest[k] = 0ull;
-    for (int v = 0; v < a.m; v++) {
-        const size_t o = (size_t)v * a.n + k;
-        a.seed[o] = kNone;
-        if (v == 0 ? !a.continued : !a.chain) a.parent[o] = k;
+    if (blockIdx.y == (uint32_t)a.ep->rho) {
+        const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+        if (k < a.nw)
+            for (int v = 0; v < a.m; v++) a.bits[(size_t)v * a.nw + k] = 0u;
+        if (k < a.n) {
+            a.cbest[k] = 0ull;
+            if (!a.continued) a.parent[k] = k;
+            for (int v = 0; v < a.m; v++) a.seed[(size_t)v * a.n + k] = kNone;
+        }
     }
+    const uint32_t rho = (uint32_t)a.ep->rho;
+    const uint32_t ncl = *a.ncl;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+    if (c >= ncl || r > 2u * rho) return;
+    const uint32_t key = a.gkey[a.clist[c]];
+    const int cy = (int)(key / a.g.ncx_pad), cx = (int)(key - (uint32_t)cy * a.g.ncx_pad);
+    const int ry = cy + (int)r - (int)rho, reach = a.ep->reach[r];
+    const uint32_t lo = (uint32_t)max(cx - reach, 0);
+    const uint32_t hi = (uint32_t)min(cx + reach, (int)a.g.ncx - 1);
+    uint2 out = make_uint2(0u, 0u);
+    if (ry >= 0 && ry < (int)a.g.ncy) {
+        if (a.g.sparse) {
+            const uint32_t re = a.crow[ry + 1];
+            out.x = cx_lower_bound(a.ccx, a.crow[ry], re, lo);
+            out.y = out.x;
+            while (out.y < re && a.ccx[out.y] <= hi) out.y++;
+        } else {
+            const uint32_t base = (uint32_t)ry * a.g.ncx_pad;
+            out.x = a.cscan[a.cell_start[base + lo]];
+            out.y = a.cscan[a.cell_start[base + hi + 1]];
+        }
+    }
+    if (!VDB_GUARD(a.st, out.x <= out.y && out.y <= ncl, 16, out.y)) out = make_uint2(0u, 0u);
+    a.crng[(size_t)r * a.n + c] = out;
 }
 
 __global__ void cell_best_kernel(CellArgs a) {
@@ -477,33 +474,65 @@ __global__ void cell_best_kernel(CellArgs a) {
 // are tested.  In dense regions that joins almost every pair of adjacent
 // cells, so that the search below finds most pairs already joined.
 //
-// Along the rows (first slot only): a warp's run of cells that are joined to
-// their left neighbours points at its first cell, without atomics.
-__global__ void cell_runs_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    const uint32_t ncl = *a.ncl;
-    if (c - lane >= ncl) return;  // (whole warps)
-    bool left = false;  // joined to cell c - 1
-    if (c < ncl && c > 0 && !a.continued) {
-        const uint32_t mp = a.mp[0];
-        const unsigned long long bA = a.cbest[c], bB = a.cbest[c - 1];
-        if (best_deg(bA) >= mp && best_deg(bB) >= mp) {
-            const uint32_t ku = best_point(bA), kv = best_point(bB);
-            if (ku < a.n && kv < a.n && a.ccx[c] == a.ccx[c - 1] + 1u &&
-                a.crng[(size_t)(uint32_t)a.ep->rho * a.n + c].x < c)
-                left = test_pair(a, pair_test(a), ku, kv, a.glocal[ku], a.glocal[kv], -1, 0) == 3u;
+// Hooks: a cell that has cores for the first time in slot v is a tree of its
+// own and nobody else writes its parent, so it can be hung under an earlier
+// cell without atomics: under the first cell of the run of joined cells that
+// it ends (within the warp), else under a joined cell of the row before.
+// Returns cell c's parent (whole warps; old: its parent so far).
+__device__ __forceinline__ uint32_t hook_parent(const CellArgs& a, const PairTest& t, uint32_t c,
+                                                bool in, uint32_t mp, uint32_t mp_before,
+                                                uint32_t old) {
+    const uint32_t lane = threadIdx.x & 31;
+    const int rho = a.ep->rho;
+    const unsigned long long bA = in ? a.cbest[c] : 0ull;
+    const uint32_t ku = best_point(bA);
+    const bool fresh = in && best_deg(bA) >= mp && best_deg(bA) < mp_before && ku < a.n;
+    bool left = false;
+    int cx = 0;
+    float2 pu = make_float2(0.f, 0.f);
+    if (fresh) {
+        cx = (int)a.ccx[c];
+        pu = a.glocal[ku];
+        if (c > 0) {
+            const unsigned long long bB = a.cbest[c - 1];
+            const uint32_t kv = best_point(bB);
+            if (best_deg(bB) >= mp && kv < a.n && (int)a.ccx[c - 1] + 1 == cx &&
+                a.crng[(size_t)rho * a.n + c].x < c)  // (the same row)
+                left = test_pair(a, t, ku, kv, pu, a.glocal[kv], -1, 0) == 3u;
         }
     }
     const uint32_t heads = ~__ballot_sync(kFull, left);
-    if (!left) return;
-    // the run's first cell in this warp, or the cell before the warp's
-    const uint32_t upto = heads & ((2u << lane) - 1u);
-    a.parent[c] = c - lane + (upto ? 31u - (uint32_t)__clz((int)upto) : 0u) - (upto ? 0u : 1u);
+    if (!fresh) return old;
+    if (left) {
+        // the run's first cell in this warp, or the cell before the warp's
+        const uint32_t upto = heads & ((2u << lane) - 1u);
+        return upto ? c - lane + 31u - (uint32_t)__clz((int)upto) : c - lane - 1u;
+    }
+    if (rho >= 1) {
+        const uint2 rg = a.crng[(size_t)(rho - 1) * a.n + c];
+        for (uint32_t o = rg.x; o < rg.y; o++) {
+            const int dx = (int)a.ccx[o] - cx;
+            const unsigned long long bB = a.cbest[o];
+            const uint32_t kv = best_point(bB);
+            if (dx >= -1 && dx <= 1 && o < c && best_deg(bB) >= mp && kv < a.n &&
+                test_pair(a, t, ku, kv, pu, a.glocal[kv], dx, -1) == 3u)
+                return o;
+        }
+    }
+    return old;
 }
 
-// From one row to the next (and along the rows where a run was not made): a
-// thread per cell looks at up to three adjacent cells.  Neighbouring lanes
+__global__ void cell_hook_kernel(CellArgs a) {
+    pdl_sync();
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t ncl = *a.ncl;
+    if (c - lane >= ncl || a.continued) return;  // (whole warps)
+    const uint32_t p = hook_parent(a, pair_test(a), c, c < ncl, a.mp[0], kNone, c);
+    if (c < ncl) a.parent[c] = p;
+}
+
+// The other adjacent cells, of the next row and along the row: a thread per
+// cell and row looks at up to three of them.  Neighbouring lanes
 // mostly want the same two trees joined: one union per pair of roots and warp.
 constexpr int kNearLoads = 5;  // cells of two per eps: all the cells of a row within reach
 __global__ void __launch_bounds__(kThreads, 4) cell_near_kernel(CellArgs a, int v) {
@@ -722,15 +751,24 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
 
 // Roots of slot v, after the first unions (so that the search tells joined
 // cells by one load) and after the search (last), when they are also the next
-// slot's start: a smaller minpts keeps every core and every connection.
+// slot's start: a smaller minpts keeps every core and every connection, and
+// its new cells are hooked.
 __global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
     pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= *a.ncl) return;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t ncl = *a.ncl;
+    if (c - lane >= ncl) return;  // (whole warps)
     uint32_t* parent = a.parent + (size_t)v * a.n;
-    const uint32_t r = uf_find_ro(parent, c);
-    parent[c] = r;
-    if (last && a.chain && v + 1 < a.m) parent[a.n + c] = r;
+    uint32_t r = 0;
+    if (c < ncl) {
+        r = uf_find_ro(parent, c);
+        parent[c] = r;
+    }
+    if (last && v + 1 < a.m) {
+        const uint32_t p = hook_parent(a, pair_test(a), c, c < ncl, a.mp[v + 1],
+                                       a.chain ? a.mp[v] : kNone, a.chain ? r : c);
+        if (c < ncl) parent[a.n + c] = p;
+    }
 }
 
 // seed[root] = first visit position among the component's cores (y: slot).
@@ -849,26 +887,9 @@ __device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32
     return bit_label(a.bits + (size_t)v * a.nw, a.brank + (size_t)v * a.nw, s);
 }
 
-// Labels of the cores, and the saved components (comp[visit position] =
-// cluster start of the core there, kNone for other points).
-__global__ void cell_core_labels_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n) return;
-    const uint32_t d = a.deg[k], c = a.cscan[k + 1] - 1u, o = a.gorig[k], p = a.gpos[k];
-    if (!VDB_GUARD(a.st, c < a.n && o < a.n && p < a.n, 13, o)) return;
-    for (int v = 0; v < a.m; v++) {
-        const bool core = d >= a.mp[v];
-        uint32_t s = kNone;
-        if (core) {
-            s = a.cst[(size_t)v * a.n + c];
-            if (VDB_GUARD(a.st, s < a.n, 14, s)) a.labels[v][o] = start_label(a, v, s);
-        }
-        if (a.comp_out[v]) a.comp_out[v][p] = s;
-    }
-}
-
-// Labels of the points that are not core, a thread per point.  Such a point p
+// Labels, a thread per point and slot (y), and the saved components
+// (comp[visit position] = cluster start of the core there, kNone for other
+// points).  A core has its cell's cluster.  A point p that is not core
 // takes the earliest cluster start among the cores u with p in N(u): the
 // start of its own cell if that has cores (a clique), or of a neighbour cell
 // if one of that cell's cores lists p.  Only neighbour cells whose start is
@@ -880,35 +901,40 @@ __global__ void cell_core_labels_kernel(CellArgs a) {
 // kLaneCores points for each lane that searches; a few lanes' larger searches
 // are done by the warp one after the other, lanes over the cells' points.
 constexpr uint32_t kLaneCores = 16;
-__global__ void __launch_bounds__(kThreads, 5) cell_border_kernel(CellArgs a) {
+__global__ void __launch_bounds__(kThreads, 5) cell_labels_kernel(CellArgs a) {
     pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t d = k < a.n ? a.deg[k] : kNone;
-    if (!__any_sync(kFull, d < a.mp[0])) return;  // (slots in descending minpts: all cores)
-    const PairTest t = pair_test(a);
-    const int rho = a.ep->rho, nrows = 2 * rho + 1;
-    uint32_t c = 0, p = 0, out = 0;
-    int cx = 0;
-    float2 loc = make_float2(0.f, 0.f);
-    bool ok = d < a.mp[0];
-    if (ok) {
+    const int v = blockIdx.y;
+    const uint32_t mp = a.mp[v];
+    const uint32_t* __restrict__ cst = a.cst + (size_t)v * a.n;
+    uint32_t c = 0, p = 0, out = 0, best = 0;
+    bool border = false;
+    if (k < a.n) {
+        const uint32_t d = a.deg[k];
         c = a.cscan[k + 1] - 1u;
         p = a.gpos[k];
         out = a.gorig[k];
-        ok = VDB_GUARD(a.st, c < a.n && out < a.n, 13, out);
+        if (VDB_GUARD(a.st, c < a.n && out < a.n && p < a.n, 13, out)) {
+            best = cst[c];
+            border = d < mp;
+            if (!border) {
+                if (VDB_GUARD(a.st, best < a.n, 14, best)) a.labels[v][out] = start_label(a, v, best);
+            }
+            if (a.comp_out[v]) a.comp_out[v][p] = border ? kNone : best;
+        }
     }
-    if (ok) {
+    if (!__any_sync(kFull, border)) return;
+    const PairTest t = pair_test(a);
+    const int rho = a.ep->rho, nrows = 2 * rho + 1;
+    int cx = 0;
+    float2 loc = make_float2(0.f, 0.f);
+    if (border) {
         cx = (int)a.ccx[c];
         loc = a.glocal[k];
     }
     const uint2* __restrict__ rng = a.crng + c;  // row i: rng[i * n]
-    for (int v = 0; v < a.m; v++) {
-        const uint32_t mp = a.mp[v];
-        const bool border = ok && d < mp;
-        if (!__any_sync(kFull, border)) break;  // (nor at a smaller minpts)
-        const uint32_t* __restrict__ cst = a.cst + (size_t)v * a.n;
-        uint32_t best = border ? cst[c] : 0u;
+    {
         uint32_t floor_s = 0;  // starts below this one have been searched
         bool busy = border;
         while (__any_sync(kFull, busy)) {
@@ -1079,10 +1105,9 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
                   cudaStream_t s) {
     if (!a.n) return;
     const dim3 per_slot(nblk(a.n), (unsigned)a.m);
-    launch(cells_init_kernel, nblk(std::max(a.n, a.nw)), kThreads, s, a);
-    launch(cell_ranges_kernel, dim3(nblk(a.n), (unsigned)nrows), kThreads, s, a);
+    launch(cell_setup_kernel, dim3(nblk(std::max(a.n, a.nw)), (unsigned)nrows), kThreads, s, a);
     launch(cell_best_kernel, nblk(a.n), kThreads, s, a);
-    launch(cell_runs_kernel, nblk(a.n), kThreads, s, a);
+    launch(cell_hook_kernel, nblk(a.n), kThreads, s, a);
     for (int v = 0; v < a.m; v++) {
         launch(cell_near_kernel, dim3(nblk(a.n), 2), kThreads, s, a, v);
         launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v, 0);
@@ -1095,8 +1120,7 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     }
     launch(cell_starts_kernel, per_slot, kThreads, s, a);
     launch(cell_rank_kernel, a.m, kRankThreads, s, a);
-    launch(cell_core_labels_kernel, nblk(a.n), kThreads, s, a);
-    launch(cell_border_kernel, nblk(a.n), kThreads, s, a);
+    launch(cell_labels_kernel, per_slot, kThreads, s, a);
 }
 
 }  // namespace vdb
