@@ -44,10 +44,16 @@ struct Pool {
         const size_t g = (size_t)2 << 20;
         return (b + g - 1) / g * g;
     }
+    // the largest cached block that serves b bytes: up to twice their size for
+    // small ones (the datasets of a batch reuse one another's buffers whatever
+    // worker gets them), a quarter more for large ones
+    static size_t fits(size_t b) {
+        return b + std::max(b / 4, std::min(b, (size_t)64 << 20)) + ((size_t)4 << 20);
+    }
     void* get(size_t bytes, cudaError_t* err) {
         size_t b = round(bytes ? bytes : 1);
         auto it = free_blocks.lower_bound(b);
-        if (it != free_blocks.end() && it->first <= b + b / 4 + ((size_t)4 << 20)) {
+        if (it != free_blocks.end() && it->first <= fits(b)) {
             void* p = it->second;
             free_blocks.erase(it);
             return p;
@@ -108,6 +114,9 @@ struct vdb_context {
     Pool pool;
     std::string err;
     cudaEvent_t box_ready = nullptr;   // the bounding box has reached h_pinned
+    std::vector<cudaEvent_t> events;   // timing events that no call is using
+    int blocks_count[2] = {0, 0}, blocks_fill[2] = {0, 0};  // resident blocks per SM of the
+    int blocks_expand[2] = {0, 0};     // count and fill (FP64, mixed), expand (32, 16 bits) kernels
     DeviceStatus* d_status = nullptr;  // device status block, read back through h_status
     DeviceStatus* h_status = nullptr;  // pinned host mirror
     void* h_pinned = nullptr;          // pinned staging (EpsParams, scalars)
@@ -130,6 +139,10 @@ struct VdbError {
         if (e_ != cudaSuccess)                                                           \
             throw VdbError{VDB_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
     } while (0)
+
+// Buffers up to this size are taken without weighing them against the free
+// memory first (a question to the driver of 5 to 10 us).
+constexpr size_t kSmallAlloc = (size_t)64 << 20;
 
 // Allocations of one call, returned to the context pool when it ends.
 // The bytes it holds (as the pool rounds them) and their peak: the call's
@@ -171,6 +184,16 @@ struct Arena {
         cur += ctx->pool.sizes[p];
         peak = std::max(peak, cur);
         return (T*)p;
+    }
+    // The same for up to kSmallAlloc bytes, nullptr where there is no room.
+    template <class T>
+    T* get_small(size_t count) {
+        if (count * sizeof(T) > kSmallAlloc) return nullptr;
+        try {
+            return get<T>(count);
+        } catch (const VdbError&) {
+            return nullptr;
+        }
     }
     void put(void* p) {
         if (keep) {
@@ -278,7 +301,7 @@ struct ZeroCarve {
 };
 // The zeroed memory of one epsilon: look-back states and counters.
 struct GroupZero {
-    uint32_t* counts;   // asym_n, count and expand tile counters
+    uint32_t* counts;   // next unit of the count pass, of the table pass
     void *sort, *order, *words, *off;
     GroupZero(ZeroCarve& z, uint32_t n, bool with_sort) {
         counts = (uint32_t*)z.take(4 * sizeof(uint32_t));
@@ -385,22 +408,31 @@ struct Options {
     bool graph = false;   // repeated calls replayed as one CUDA graph
 };
 
+// Times of a call's phases; its events come from the context and go back to it.
 struct Timer {
+    vdb_context* ctx;
     std::vector<cudaEvent_t> evs;
     cudaStream_t s;
     bool off;  // no events (stream capture into conditional bodies takes none)
-    explicit Timer(cudaStream_t st, bool off_ = false) : s(st), off(off_) {}
+    Timer(vdb_context* c, bool off_) : ctx(c), s(c->stream), off(off_) {}
     ~Timer() {
         for (auto e : evs)
-            if (e) cudaEventDestroy(e);
+            if (e) ctx->events.push_back(e);
     }
     size_t mark() {
         cudaEvent_t e = nullptr;
         if (!off) {
-            CK(cudaEventCreate(&e));
+            if (ctx->events.empty()) {
+                CK(cudaEventCreate(&e));
+            } else {
+                e = ctx->events.back();
+                ctx->events.pop_back();
+            }
+            evs.push_back(e);
             CK(cudaEventRecord(e, s));
+        } else {
+            evs.push_back(e);
         }
-        evs.push_back(e);
         return evs.size() - 1;
     }
     double ms(size_t a, size_t b) {
@@ -705,7 +737,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     const bool recording = rec && !rec->capture;
     Arena local_ar(ctx);
     Arena& ar = capturing ? *rec->ar : local_ar;
-    Timer tm(s, capturing);
+    Timer tm(ctx, capturing);
     DeviceStatus* const d_st = capturing ? rec->d_status : ctx->d_status;
     const unsigned long long launches0 = g_launches.load();
     PlainLaunches plain(capturing);
@@ -867,13 +899,12 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     AsymPair* asym = ar.get<AsymPair>(asym_cap);
     ZeroCarve zc{zeroed, 0};
     const GroupZero gz(zc, n, true);
-    uint32_t* asym_n = gz.counts;
-    uint32_t* count_counter = asym_n + 1;  // next unit of the count pass
-    uint32_t* table_counter = asym_n + 2;  // next unit (tile) of the table pass
-    unsigned long long* d_totals = ar.get<unsigned long long>(4);
-    unsigned long long* d_nwords = d_totals;            // bitmap words
-    uint32_t* d_nunits = (uint32_t*)(d_totals + 1);     // work units
-    uint32_t* d_ntiles = (uint32_t*)(d_totals + 2);
+    uint32_t* count_counter = gz.counts;      // next unit of the count pass
+    uint32_t* table_counter = gz.counts + 1;  // next unit (tile) of the table pass
+    uint32_t* asym_n = &d_st->asym_n;
+    unsigned long long* d_nwords = &d_st->nwords;
+    uint32_t* d_nunits = &d_st->nunits;
+    uint32_t* d_ntiles = &d_st->ntiles;
     EpsParams* d_ep = ar.get<EpsParams>(1);
     uint32_t tile_cells_hist[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // tables per log2(G)
     uint32_t* gkey = ar.get<uint32_t>(n);
@@ -909,10 +940,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
 
     const bool want_mixed = o.precision == VDB_PRECISION_MIXED;
     const int tq = table_tile_queries();
-    const int nb_count = ctx->nsm * table_blocks_per_sm(false, want_mixed);
-    const int nb_fill = ctx->nsm * table_blocks_per_sm(true, want_mixed);
-    const int nb_expand16 = ctx->nsm * expand_blocks_per_sm(true);
-    const int nb_expand32 = ctx->nsm * expand_blocks_per_sm(false);
+    const int nb_count = ctx->nsm * ctx->blocks_count[want_mixed];
+    const int nb_fill = ctx->nsm * ctx->blocks_fill[want_mixed];
+    const int nb_expand16 = ctx->nsm * ctx->blocks_expand[1];
+    const int nb_expand32 = ctx->nsm * ctx->blocks_expand[0];
     const int nb_warps = ctx->nsm * 8;
     uint64_t pairs = 0, asym_total = 0, entry_bytes = 0;
     uint32_t compact_tables = 0;
@@ -1050,6 +1081,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // not captured)
             if (capturing) throw VdbError{VDB_ERR_CUDA, "graph capture: path not captured"};
             if (recording) rec->graphable = false;
+            CK(cudaMemsetAsync(asym_n, 0, sizeof(uint32_t), s));
             CK(cudaMemsetAsync(deg, 0, (size_t)n * 4, s));
             CK(cudaMemsetAsync(off, 0, ((size_t)n + 1) * 8, s));
             // grid order = input order
@@ -1121,12 +1153,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // cells are cliques when two points of one cell always pass the
             // distance test without a box check: 2 w^2 below thr and tbox
             clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
-            if (capturing) {
-                launch_store_eps(d_ep, ep, s);
-            } else {
-                memcpy(ctx->h_pinned, &ep, sizeof ep);
-                CK(cudaMemcpyAsync(d_ep, ctx->h_pinned, sizeof ep, cudaMemcpyHostToDevice, s));
-            }
+            launch_store_eps(d_ep, ep, s);
             const size_t tb = tm.mark();
 
             ta_args.g = g;
@@ -1200,11 +1227,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 }
                 capture_checkpoint(*rec, s, chk);
             } else {
-                CK(cudaMemcpyAsync(ctx->h_pinned, d_totals, 16, cudaMemcpyDeviceToHost, s));
                 read_status(ctx, s);
                 status_before_count = *ctx->h_status;
-                if (!no_rows) memcpy(&bm_words, ctx->h_pinned, 8);
-                memcpy(&nunits, (char*)ctx->h_pinned + 8, 4);
+                if (!no_rows) bm_words = ctx->h_status->nwords;
+                nunits = ctx->h_status->nunits;
                 st_flags = ctx->h_status->flags & kStatBitmapTooLarge;
                 if (recording) {
                     rec->put(bm_words);
@@ -1252,11 +1278,11 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                     // the test bitmap is kept when it fits 35% of the memory
                     // (and the caller's table budget); else the fill pass
                     // re-tests the candidates instead
-                    double cap = 0.35 * avail_bytes(ctx);
-                    if (o.budget > 0) cap = std::min(cap, (double)o.budget);
-                    if ((double)bm_words * 4.0 <= cap) {
-                        bitmap = ar.get<uint32_t>(bm_words ? bm_words : 1);
-                        bitmap_cap = bm_words;
+                    if (o.budget <= 0 || (double)bm_words * 4.0 <= (double)o.budget) {
+                        bitmap = ar.get_small<uint32_t>(bm_words ? bm_words : 1);
+                        if (!bitmap && (double)bm_words * 4.0 <= 0.35 * avail_bytes(ctx))
+                            bitmap = ar.get<uint32_t>(bm_words ? bm_words : 1);
+                        if (bitmap) bitmap_cap = bm_words;
                     }
                 }
                 if (bitmap && bm_words <= bitmap_cap) ta_args.bitmap = bitmap;
@@ -1278,16 +1304,12 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 tc = tm.mark();
                 if (!no_rows) scan_u32_to_u64(deg, off, n, gz.off, d_st, s);
                 if (capturing) break;
-                if (!no_rows)
-                    CK(cudaMemcpyAsync(ctx->h_pinned, off + n, 8, cudaMemcpyDeviceToHost, s));
-                CK(cudaMemcpyAsync((char*)ctx->h_pinned + 8, asym_n, 4, cudaMemcpyDeviceToHost, s));
                 read_status(ctx, s);
                 if (!(ctx->h_status->flags & kStatAsymOverflow)) break;
                 if (recording) rec->graphable = false;  // (the re-count is not captured)
                 // more one-way pairs than the list holds: grow it past the
                 // counted number and run the count pass again
-                uint32_t want = 0;
-                memcpy(&want, (char*)ctx->h_pinned + 8, 4);
+                const uint32_t want = ctx->h_status->asym_n;
                 uint64_t cap2 = (uint64_t)asym_cap * 2;
                 while (cap2 < (uint64_t)want + want / 4) cap2 *= 2;
                 if (cap2 > 0x7fffffffull)
@@ -1318,9 +1340,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 capture_checkpoint(*rec, s, chk);
             } else {
                 check_flags(*ctx->h_status);
-                if (no_rows) E = ctx->h_status->pairs - status_before_count.pairs;
-                else memcpy(&E, ctx->h_pinned, 8);
-                memcpy(&group_asym, (char*)ctx->h_pinned + 8, 4);
+                E = no_rows ? ctx->h_status->pairs - status_before_count.pairs
+                            : ctx->h_status->entries;
+                group_asym = ctx->h_status->asym_n;
                 if (recording) {
                     rec->put(E);
                     rec->put(group_asym);
@@ -1344,16 +1366,16 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 nbr = nullptr;
                 nbr_cap_bytes = 0;
                 // (a captured call was recorded unchunked: its table fits)
-                const int64_t budget = o.budget > 0 ? o.budget
-                                       : capturing  ? INT64_MAX
-                                                    : (int64_t)(avail_bytes(ctx) * 0.9);
-                if ((int64_t)(Erows * esz) <= budget) {
-                    const size_t w = std::max<size_t>(words_for(Erows), 1);
-                    nbr = ar.get<uint32_t>(w);
-                    nbr_cap_bytes = w * 4;
-                } else {
-                    chunked = true;
+                const size_t w = std::max<size_t>(words_for(Erows), 1);
+                if (o.budget <= 0 && !capturing) nbr = ar.get_small<uint32_t>(w);
+                if (!nbr) {
+                    const int64_t budget = o.budget > 0 ? o.budget
+                                           : capturing  ? INT64_MAX
+                                                        : (int64_t)(avail_bytes(ctx) * 0.9);
+                    if ((int64_t)(Erows * esz) <= budget) nbr = ar.get<uint32_t>(w);
                 }
+                if (nbr) nbr_cap_bytes = w * 4;
+                else chunked = true;
             }
             if (chunked && capturing)
                 throw VdbError{VDB_ERR_CUDA, "graph capture: chunked table not captured"};
@@ -1580,12 +1602,13 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         rec->launches = g_launches.load() - launches0;
         return;
     }
+    CK(cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(DeviceStatus),
+                       cudaMemcpyDeviceToHost, s));
     if (host) {
         CK(cudaMemcpyAsync(ds.labels, labels, (size_t)n * V * 4, cudaMemcpyDeviceToHost, s));
     }
     const size_t tend = tm.mark();
     CK(cudaStreamSynchronize(s));
-    read_status(ctx, s);
     check_flags(*ctx->h_status);
     for (const GroupSpan& gs : group_spans) {
         double in_cluster_tables = 0;
@@ -1676,6 +1699,11 @@ int init_context(vdb_context* ctx, void* stream) {
     }
     if (cudaEventCreateWithFlags(&ctx->box_ready, cudaEventDisableTiming) != cudaSuccess)
         return VDB_ERR_CUDA;
+    for (int i = 0; i < 2; i++) {
+        ctx->blocks_count[i] = table_blocks_per_sm(false, i != 0);
+        ctx->blocks_fill[i] = table_blocks_per_sm(true, i != 0);
+        ctx->blocks_expand[i] = expand_blocks_per_sm(i != 0);
+    }
     if (cudaMalloc(&ctx->d_status, sizeof(DeviceStatus)) != cudaSuccess) return VDB_ERR_NOMEM;
     if (cudaMallocHost(&ctx->h_status, sizeof(DeviceStatus)) != cudaSuccess) return VDB_ERR_NOMEM;
     ctx->h_pinned_bytes = 4096;
@@ -2170,6 +2198,7 @@ void vdb_context_destroy(vdb_context* ctx) {
     ctx->workers.clear();
     ctx->pool.release_all();
     if (ctx->box_ready) cudaEventDestroy(ctx->box_ready);
+    for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
@@ -2323,10 +2352,9 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t* deg = cv.take<uint32_t>(n);
     unsigned long long* off = cv.take<unsigned long long>((size_t)n + 1);
     AsymPair* asym = cv.take<AsymPair>(kNoallocAsymCap);
-    uint32_t* asym_n = gz.counts;
-    unsigned long long* d_totals = cv.take<unsigned long long>(4);
-    uint32_t* d_nunits = (uint32_t*)(d_totals + 1);
-    uint32_t* d_ntiles = (uint32_t*)(d_totals + 2);
+    uint32_t* asym_n = &st->asym_n;
+    uint32_t* d_nunits = &st->nunits;
+    uint32_t* d_ntiles = &st->ntiles;
     uint32_t* parent = cv.take<uint32_t>(n);
     uint32_t* seed = cv.take<uint32_t>(n);
     uint32_t* cstart = cv.take<uint32_t>(n);
@@ -2379,7 +2407,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.tiles = tiles;
     ta.ntiles = d_ntiles;
     ta.tile_end = 0xffffffffu;
-    ta.tile_counter = asym_n + 1;
+    ta.tile_counter = gz.counts;
     ta.cell_start = cell_start;
     ta.gkey = gkey;
     ta.glocal = glocal;
@@ -2397,7 +2425,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     // work units of the count pass (no bitmap here: the fill pass writes the table)
     uint32_t* tuoff = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* tloff = cv.take<uint32_t>((size_t)n + 1);
-    launch_tile_words(ta, nullptr, tuoff, tloff, d_totals, d_nunits, gz.words, s);
+    launch_tile_words(ta, nullptr, tuoff, tloff, &st->nwords, d_nunits, gz.words, s);
     uint32_t nunits = 0;
     CK(cudaMemcpyAsync(&nunits, d_nunits, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -2412,12 +2440,11 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     launch_unit_list(ta, ulist, s);
     launch_count(ta, nsm * table_blocks_per_sm(false, ep.mixed != 0), s);
     scan_u32_to_u64(deg, off, n, gz.off, st, s);
-    unsigned long long E = 0;
     DeviceStatus hs;
-    CK(cudaMemcpyAsync(&E, off + n, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(&hs, st, sizeof hs, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     check_flags(hs);
+    const unsigned long long E = hs.entries;
     // the limit on the neighbour pairs: what a table of 32-bit entries has
     // beside 160 bytes per point, the cells and the one-way pairs
     const size_t held = (size_t)n * 160 + (g.ncells + 1) * 4 +
@@ -2435,7 +2462,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         nbr = cv.take<uint32_t>(E ? E : 1);
         ta.nbr = nbr;
         ta.off_base = 0;
-        ta.tile_counter = asym_n + 2;
+        ta.tile_counter = gz.counts + 1;
         launch_fill(ta, nsm * table_blocks_per_sm(true, ep.mixed != 0), s);
     }
     const int nb_warps = nsm * 8;

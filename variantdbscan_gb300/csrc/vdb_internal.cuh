@@ -79,7 +79,13 @@ struct DeviceStatus {
     unsigned long long table_hash; // hash of the tables built (vdb_stats.table_hash)
     unsigned long long reuse_skips; // cell pairs not searched: different components at a
                                     // larger epsilon
-    unsigned long long pairs;      // neighbour pairs counted (graph replays only)
+    unsigned long long pairs;      // neighbour pairs counted (graph replays, labels-only calls)
+    // sizes of the current epsilon, which the host reads back with the rest
+    unsigned long long nwords;     // words of the test bitmap
+    unsigned long long entries;    // entries of the neighbour table
+    uint32_t nunits, nlist;        // work units; those that warps take
+    uint32_t ntiles;
+    uint32_t asym_n;               // one-way pairs recorded
 };
 
 // Index guards: a data-derived index outside its array is recorded (site and
@@ -293,7 +299,8 @@ static __device__ __forceinline__ uint32_t decode_candidate(const TileSegs& sg, 
 // All launches go to `s`.  "zeroed" memory is zero at the launch and used up
 // by it.
 
-// Exclusive scan of n uint32 values into uint64 (out has n+1 entries; out[n] = total).
+// Exclusive scan of n uint32 values into uint64 (out has n+1 entries; out[n] =
+// st->entries = total).
 size_t scan_state_bytes(uint32_t n);
 void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t n, void* zeroed,
                      DeviceStatus* st, cudaStream_t s);

@@ -46,7 +46,10 @@ __global__ void __launch_bounds__(kLookThreads) scan_kernel(const uint32_t* __re
     for (int i = 0; i < kScanItems; i++) {
         if (base + i < n) out[base + i] = run;
         run += v[i];
-        if (base + i + 1 == n) out[n] = run;
+        if (base + i + 1 == n) {
+            out[n] = run;
+            st->entries = run;
+        }
     }
 }
 

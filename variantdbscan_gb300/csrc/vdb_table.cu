@@ -1580,7 +1580,7 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
 // ceil(ceil(C/32) / unit_words); the offsets of both, and of the units that
 // warps take (those of tiles that are not small), by a single-pass scan (boff
 // may be null: no bitmap).  Blocks past the last tile only clear their part of
-// deg.
+// deg (and the one-way pairs' counter).
 __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
     uint32_t* __restrict__ loff, unsigned long long* __restrict__ nwords,
@@ -1589,6 +1589,7 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     const uint32_t tile = lookback_ticket(lu);
     const uint32_t t = tile * kLookThreads + threadIdx.x;
     if (t < a.n) a.deg[t] = 0u;
+    if (t == 0) *a.asym_n = 0u;
     const uint32_t ntiles = *a.ntiles;
     if (tile * kLookThreads >= ntiles) return;  // (the whole block)
     const EpsParams* __restrict__ ep = a.ep;
