@@ -285,7 +285,7 @@ int bits_for(uint64_t v) {
 // of the sort: they order the points of a cell, nothing depends on them.
 uint32_t sub_bits(uint64_t ncells) {
     const int kb = bits_for(ncells - 1);
-    return (uint32_t)std::min(3, (std::min(32, sort_passes(kb) * kDigitBits) - kb) / 2);
+    return (uint32_t)std::min(4, (std::min(32, sort_passes(kb) * kDigitBits) - kb) / 2);
 }
 
 // Zeroed device memory, carved in 256-byte pieces: first measured (base null),

@@ -154,6 +154,28 @@ __device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, float
     return (uint32_t)f;
 }
 
+// Place of subcell (x, y) along the Hilbert curve over 2^sub x 2^sub subcells:
+// from the coarsest quadrant down, each level turned the way the curve enters
+// it.  Every run of the curve is connected, so a run of points has a small box
+// (along the Z order every second step is a diagonal or a jump).
+__device__ __forceinline__ uint32_t curve_index(uint32_t x, uint32_t y, uint32_t sub) {
+    uint32_t d = 0;
+    for (int b = (int)sub - 1; b >= 0; b--) {
+        const uint32_t rx = (x >> b) & 1u, ry = (y >> b) & 1u;
+        d = (d << 2) | ((3u * rx) ^ ry);
+        if (!ry) {
+            if (rx) {
+                x = ~x;
+                y = ~y;
+            }
+            const uint32_t t = x;
+            x = y;
+            y = t;
+        }
+    }
+    return d;
+}
+
 __global__ void __launch_bounds__(kThreads) grid_keys_kernel(
     const double* __restrict__ x, const double* __restrict__ y, uint32_t n, GridParams g,
     uint32_t* __restrict__ keys, int passes, uint32_t* __restrict__ hist) {
@@ -167,8 +189,7 @@ __global__ void __launch_bounds__(kThreads) grid_keys_kernel(
         const uint32_t cx = cell_of(x[i], g.x0, g.w, iw, g.ncx, g.sub, &sx);
         const uint32_t cy = cell_of(y[i], g.y0, g.w, iw, g.ncy, g.sub, &sy);
         uint32_t key = cy * g.ncx_pad + cx;
-        for (int b = (int)g.sub - 1; b >= 0; b--)
-            key = (key << 2) | (((sy >> b) & 1u) << 1) | ((sx >> b) & 1u);
+        key = (key << (2u * g.sub)) | curve_index(sx, sy, g.sub);
         keys[i] = key;
         counts_add(s_h, passes, key);
     }

@@ -119,7 +119,7 @@ struct GridParams {
     // 1: many more cells than points - a row directory of the non-empty
     //    cells (crow, ccx, clist) replaces it
     uint32_t sparse;
-    // points are sorted by cell and, within a cell, along a Morton curve of
+    // points are sorted by cell and, within a cell, along a Hilbert curve of
     // 2^sub x 2^sub subcells (neighbours in the order are near each other)
     uint32_t sub;
 };

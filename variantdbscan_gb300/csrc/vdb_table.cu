@@ -1132,6 +1132,70 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// A full round of a 16-bit table: all 512 candidates of the round's 16 words
+// are neighbours of every query (in dense cells most entries come in such
+// rounds: the words' boxes lie inside eps of the whole tile).  All rows then
+// get the same run of ids, at their own places: lane = query writes the entries
+// carried from its last round and those up to the next 16-byte boundary, and
+// copies the rest straight from one of eight staged runs, the one that starts
+// with the id that falls on the boundary.  Four runs at a time fit the slots'
+// memory.  cur: the row's place of id0, nc entries are carried before it; the
+// row is written up to its last 32-byte boundary (last: up to its end) and the
+// entries after that are carried.
+__device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* slots,
+                                        uint16_t* carry, bool wrow, uint32_t id0, bool last,
+                                        unsigned long long cur, uint32_t nc, int lane) {
+    constexpr uint32_t kRun = kWXW * 32u;
+    static_assert(4u * kRun * sizeof(uint16_t) <= 32u * kXS * sizeof(uint32_t), "four runs fit");
+    const unsigned long long wcur = cur - nc, end = cur + kRun;
+    const unsigned long long A = (cur + 7ull) & ~7ull;
+    const unsigned long long wto = last ? end : end & ~15ull;
+    const unsigned long long B = wto & ~7ull;
+    const uint32_t first = (uint32_t)(A - cur);  // entries of the run before A
+    if (wrow) {
+        const uint32_t n0 = (uint32_t)(A - wcur);
+        auto entry = [&](uint32_t i) {
+            return i < nc ? (uint32_t)carry[i] : id0 + (i - nc);
+        };
+        if (((uint32_t)wcur & 7u) == 0u) {
+            for (uint32_t i = 0; i < n0; i += 8) {
+                uint4 v;
+                v.x = entry(i) | (entry(i + 1) << 16);
+                v.y = entry(i + 2) | (entry(i + 3) << 16);
+                v.z = entry(i + 4) | (entry(i + 5) << 16);
+                v.w = entry(i + 6) | (entry(i + 7) << 16);
+                *reinterpret_cast<uint4*>(nbr + wcur + i) = v;
+            }
+        } else {
+            for (uint32_t i = 0; i < n0; i++) nbr[wcur + i] = (uint16_t)entry(i);
+        }
+        for (unsigned long long i = B; i < wto; i++) nbr[i] = (uint16_t)(id0 + (uint32_t)(i - cur));
+        for (unsigned long long i = wto; i < end; i++)
+            carry[i - wto] = (uint16_t)(id0 + (uint32_t)(i - cur));
+    }
+#pragma unroll 1
+    for (uint32_t b = 0; b < 2; b++) {
+        const bool mine = wrow && (first >> 2) == b;
+        if (!__any_sync(kFull, mine)) continue;
+        if (b) {  // the first four runs have been read
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+        }
+        for (uint32_t v = (uint32_t)lane; v < kRun / 2; v += 32) {
+            const uint32_t run = v / (kRun / 8), at = v % (kRun / 8);
+            const uint32_t x = id0 + 4u * b + run + 8u * at;
+            const uint32_t two = x * 0x10001u + 0x10000u;  // x, x + 1
+            reinterpret_cast<uint4*>(slots)[run * (kRun / 8) + at] =
+                make_uint4(two, two + 0x20002u, two + 0x40004u, two + 0x60006u);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (mine && B > A)
+            bulk_copy_to_global(nbr + A, slots + (first & 3u) * (kRun / 2),
+                                (uint32_t)(B - A) * (uint32_t)sizeof(uint16_t));
+    }
+}
+
 // 16-bit tables: two queries per pass.  The round's words are transposed
 // into the query slots as above (lane = query); then lanes 0-15 expand one
 // query of a pair and lanes 16-31 the other, lane j of a half taking bits j
@@ -1171,6 +1235,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     __syncwarp();
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     uint32_t pending = 0;    // nonzero: a copy from this half's buffer may be reading it
+    uint32_t slot_copies = 0;  // nonzero: copies of a full round may be reading the slots
     const uint32_t stage_s = (uint32_t)__cvta_generic_to_shared(&s_stage[wib][0][0]);
 
     for (;;) {
@@ -1221,16 +1286,44 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
             const uint32_t* bw = a.bitmap + bm0 + (unsigned long long)w0 * Q;
             for (uint32_t qh = 0; qh < Q; qh += 32) {
                 const uint32_t q = qh + (uint32_t)lane;
-                __syncwarp();  // the previous slots have been read
                 const bool wrow = qh == 0 ? v0 : v1;
                 uint32_t todo = __ballot_sync(kFull, wrow);
-                if (wrow) {
-                    uint32_t wd[kWXW], pm[kWXW];
+                const unsigned long long cur = qh == 0 ? cur0 : cur1;
+                const uint32_t nc = qh == 0 ? nc0 : nc1;
+                uint32_t wd[kWXW], all = kFull, any = 0u;
 #pragma unroll
-                    for (int s = 0; s < kWXW; s++)
-                        wd[s] = ((uint32_t)s < nw) ? __ldg(bw + (unsigned long long)s * Q + q) : 0u;
-                    const unsigned long long cur = qh == 0 ? cur0 : cur1;
-                    const uint32_t nc = qh == 0 ? nc0 : nc1;
+                for (int s = 0; s < kWXW; s++) {
+                    wd[s] = (wrow && (uint32_t)s < nw) ? __ldg(bw + (unsigned long long)s * Q + q) : 0u;
+                    all &= wd[s];
+                    any |= wd[s];
+                }
+                // an empty round of all queries changes nothing (the last one
+                // still writes what was carried)
+                if (__all_sync(kFull, any == 0u && (!last || nc == 0u))) continue;
+                if (slot_copies) {
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    pending = 0;
+                    slot_copies = 0;
+                }
+                __syncwarp();  // the previous slots have been read
+                if (__all_sync(kFull, !wrow || all == kFull)) {
+                    full_round(nbr, slots, s_carry[wib][qh + lane], wrow, (w0 - wbeg) * 32u, last,
+                               cur, nc, lane);
+                    pending = 0;
+                    slot_copies = 1;
+                    const unsigned long long end = cur + kWXW * 32u;
+                    const uint32_t left = last ? 0u : (uint32_t)end & (kSec - 1u);
+                    if (qh == 0) {
+                        cur0 = end;
+                        nc0 = left;
+                    } else {
+                        cur1 = end;
+                        nc1 = left;
+                    }
+                    continue;
+                }
+                if (wrow) {
+                    uint32_t pm[kWXW];
                     const unsigned long long wcur = cur - nc;
                     uint32_t acc = ((uint32_t)wcur & (kVec - 1u)) + nc;
                     // the k-th query of todo is expanded in pass k / 2 by half
@@ -1329,7 +1422,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
             }
         }
     }
-    if (hj == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 template <bool MIXED, bool FILL>
