@@ -927,6 +927,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint64_t bitmap_cap = 0;
     uint2* ulist = nullptr;
     uint32_t* parts = nullptr;
+    uint2* wflags = nullptr;
     uint64_t unit_cap = 0;
     uint32_t* nbr = nullptr;
     size_t nbr_cap_bytes = 0;
@@ -1246,11 +1247,15 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             if ((uint64_t)nunits + 1 > unit_cap) {
                 if (ulist) ar.put(ulist);
                 if (parts) ar.put(parts);
+                if (wflags) ar.put(wflags);
+                wflags = nullptr;
                 unit_cap = (uint64_t)nunits + 1;
                 ulist = ar.get<uint2>(unit_cap);
                 parts = nullptr;
             }
             if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
+            if (!wflags && compact && !no_rows) wflags = ar.get<uint2>(unit_cap * (unit_words / 32));
+            ta_args.wflags = compact && !no_rows ? wflags : nullptr;
             ta_args.tile_uoff = tuoff;
             ta_args.tile_loff = tloff;
             ta_args.nunits = d_nunits;

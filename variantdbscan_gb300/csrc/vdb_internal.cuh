@@ -422,6 +422,8 @@ struct TableArgs {
     const uint32_t* tile_loff;
     const uint32_t* nunits;         // device: units, units in ulist
     uint32_t* parts;                // per unit and query slot: neighbours in that chunk
+    uint2* wflags;                  // per unit and block of 32 words: words wholly inside eps of
+                                    // the tile, wholly outside (16-bit tables; else null)
     unsigned long long* pair_sum;   // count pass: adds the neighbours counted (nullptr: not)
     // one row chunk of the table: the fill pass takes tiles from tile_lo on,
     // the expand pass entries [unit_lo, unit_hi) of ulist, and the small tiles

@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
             sqd[lane + 32 * q] = qd;
         }
         const bool two = Q > 32;  // second query slot used by some lane
+        bool settled = false;     // the unit's words settled by their boxes have been recorded
         // the float above w (w > 0)
         const float wup = __uint_as_float(__float_as_uint(wq) + 1u);
         const unsigned long long w2p = f2_pack(wup, wup);
@@ -647,6 +648,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                 nhq2[q] = f2_pack(nhq, nhq);
             }
             const bool boxes = a.wbox && C >= kBoxCand;
+            if (boxes) settled = true;
             float bx0 = 0.f, bx1 = 0.f, by0 = 0.f, by1 = 0.f;  // the queries' box (fmin/fmax skip NaN)
             float pad = 0.f;  // more than the roundings of a box's edges (16 of them)
             if (boxes) {
@@ -691,6 +693,9 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                     }
                     const uint32_t mi = __ballot_sync(kFull, in), mo = __ballot_sync(kFull, out);
                     todo &= ~(mi | mo);
+                    if (a.wflags && lane == 0)
+                        a.wflags[(unsigned long long)u * (a.unit_words / 32u) + (wb - (cbeg >> 5)) / 32u] =
+                            make_uint2(mi, mo);
                     const uint32_t add = __reduce_add_sync(kFull, in ? g1 - g0 : 0u);
                     if (qk[0] < qe) cnt[0] += add;
                     if (qk[1] < qe) cnt[1] += add;
@@ -849,6 +854,8 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                 }
             }
         }
+        if (a.wflags && !settled && (uint32_t)lane < a.unit_words / 32u)
+            a.wflags[(unsigned long long)u * (a.unit_words / 32u) + lane] = make_uint2(0u, 0u);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             if (qk[q] < qe) {
@@ -1132,10 +1139,22 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// A full round of a 16-bit table: all 512 candidates of the round's 16 words
-// are neighbours of every query (in dense cells most entries come in such
-// rounds: the words' boxes lie inside eps of the whole tile).  All rows then
-// get the same run of ids, at their own places: lane = query writes the entries
+// The words of a block of 32 (the first is word w0 of the tile's, of C
+// candidates) that a 16-bit table's rows get as runs: full words (inside, as
+// the count pass flagged them) in a row of three or more.  Shorter runs cost
+// less among the words that are expanded; the tile's last word, if it has
+// fewer than 32 candidates, is no full one.  Within a unit, a row holds the
+// other words' entries first, in order, then the runs'.
+__device__ __forceinline__ uint32_t full_runs(uint32_t inside, uint32_t w0, uint32_t C) {
+    const uint32_t whole = (C >> 5) > w0 ? (C >> 5) - w0 : 0u;  // words of 32 candidates
+    const uint32_t F = whole >= 32u ? inside : inside & ((1u << whole) - 1u);
+    const uint32_t starts = F & (F >> 1) & (F >> 2);
+    return starts | (starts << 1) | (starts << 2);
+}
+
+// A run of full words of a 16-bit table (len candidates, up to 16 words): all
+// are neighbours of every query, their boxes lie inside eps of the whole tile.
+// All rows get the same run of ids, at their own places: lane = query writes the entries
 // carried from its last round and those up to the next 16-byte boundary, and
 // copies the rest straight from one of eight staged runs, the one that starts
 // with the id that falls on the boundary.  Four runs at a time fit the slots'
@@ -1143,13 +1162,13 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
 // row is written up to its last 32-byte boundary (last: up to its end) and the
 // entries after that are carried.
 __device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* slots,
-                                        uint16_t* carry, bool wrow, uint32_t id0, bool last,
+                                        uint16_t* carry, bool wrow, uint32_t id0, uint32_t len, bool last,
                                         unsigned long long cur, uint32_t nc, int lane) {
     constexpr uint32_t kRun = kWXW * 32u;
     static_assert(4u * kRun * sizeof(uint16_t) <= 32u * kXS * sizeof(uint32_t), "four runs fit");
-    const unsigned long long wcur = cur - nc, end = cur + kRun;
+    const unsigned long long wcur = cur - nc, end = cur + len;
     const unsigned long long A = (cur + 7ull) & ~7ull;
-    const unsigned long long wto = last ? end : end & ~15ull;
+    const unsigned long long wto = last ? end : end & ~15ull;  // (at least A: len >= 64)
     const unsigned long long B = wto & ~7ull;
     const uint32_t first = (uint32_t)(A - cur);  // entries of the run before A
     if (wrow) {
@@ -1218,6 +1237,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     __shared__ __align__(16) uint32_t s_slot[kXPB][32 * kXS];
     __shared__ __align__(16) E s_stage[kXPB][2][kStage];
     __shared__ E s_carry[kXPB][kWQ][kSec];
+    __shared__ __align__(16) uint8_t s_list[kXPB][kUnitWords];
     E* const nbr = reinterpret_cast<E*>(a.nbr);
 
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1276,54 +1296,64 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
             if (v0) cur0 += a.parts[(unsigned long long)uu * kUnitQ + lane];
             if (v1) cur1 += a.parts[(unsigned long long)uu * kUnitQ + lane + 32];
         }
-        uint32_t nc0 = 0, nc1 = 0;
-        for (uint32_t w0 = wbeg; w0 < wend; w0 += kWXW) {
-            const uint32_t nw = min((uint32_t)kWXW, wend - w0);
-            const bool last = w0 + kWXW >= wend;
-            // position in the unit of bit hj of the round's word s (bit hj + 16:
-            // + 16); bits past the candidates are never set
-            const uint32_t idbase = (w0 - wbeg) * 32u + hj;
-            const uint32_t* bw = a.bitmap + bm0 + (unsigned long long)w0 * Q;
-            for (uint32_t qh = 0; qh < Q; qh += 32) {
-                const uint32_t q = qh + (uint32_t)lane;
-                const bool wrow = qh == 0 ? v0 : v1;
-                uint32_t todo = __ballot_sync(kFull, wrow);
-                const unsigned long long cur = qh == 0 ? cur0 : cur1;
-                const uint32_t nc = qh == 0 ? nc0 : nc1;
-                uint32_t wd[kWXW], all = kFull, any = 0u;
+        // The unit's words in blocks of 32 (lane b: block b): first those to
+        // expand, then the runs of full words.
+        uint32_t mix = 0u, run = 0u;
+        if ((uint32_t)lane * 32u < wend - wbeg) {
+            const uint32_t w0 = wbeg + 32u * (uint32_t)lane;
+            const uint2 f = a.wflags[(unsigned long long)u * (a.unit_words / 32u) + lane];
+            const uint32_t nwb = min(32u, wend - w0);
+            run = full_runs(f.x, w0, C);
+            mix = (nwb == 32u ? kFull : (1u << nwb) - 1u) & ~f.y & ~run;
+        }
+        uint8_t* const list = s_list[wib];
+        uint32_t nmix = 0;
+        __syncwarp();  // (the list before has been read)
 #pragma unroll
-                for (int s = 0; s < kWXW; s++) {
-                    wd[s] = (wrow && (uint32_t)s < nw) ? __ldg(bw + (unsigned long long)s * Q + q) : 0u;
-                    all &= wd[s];
-                    any |= wd[s];
-                }
-                // an empty round of all queries changes nothing (the last one
-                // still writes what was carried)
-                if (__all_sync(kFull, any == 0u && (!last || nc == 0u))) continue;
+        for (uint32_t b = 0; b < kUnitWords / 32u; b++) {
+            const uint32_t m = __shfl_sync(kFull, mix, (int)b);
+            if ((m >> lane) & 1u)
+                list[nmix + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(32u * b + (uint32_t)lane);
+            nmix += (uint32_t)__popc(m);
+        }
+        __syncwarp();
+        const uint32_t run_blocks = __ballot_sync(kFull, run != 0u);
+        const uint32_t* bw = a.bitmap + bm0 + (unsigned long long)wbeg * Q;
+        for (uint32_t qh = 0; qh < Q; qh += 32) {
+            const uint32_t q = qh + (uint32_t)lane;
+            const bool wrow = qh == 0 ? v0 : v1;
+            unsigned long long cur = qh == 0 ? cur0 : cur1;
+            uint32_t nc = 0;
+            for (uint32_t r0 = 0; r0 < nmix; r0 += kWXW) {
+                uint32_t todo = __ballot_sync(kFull, wrow);
+                const uint32_t nw = min((uint32_t)kWXW, nmix - r0);
+                const bool last = r0 + kWXW >= nmix && run_blocks == 0u;
                 if (slot_copies) {
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     pending = 0;
                     slot_copies = 0;
                 }
                 __syncwarp();  // the previous slots have been read
-                if (__all_sync(kFull, !wrow || all == kFull)) {
-                    full_round(nbr, slots, s_carry[wib][qh + lane], wrow, (w0 - wbeg) * 32u, last,
-                               cur, nc, lane);
-                    pending = 0;
-                    slot_copies = 1;
-                    const unsigned long long end = cur + kWXW * 32u;
-                    const uint32_t left = last ? 0u : (uint32_t)end & (kSec - 1u);
-                    if (qh == 0) {
-                        cur0 = end;
-                        nc0 = left;
-                    } else {
-                        cur1 = end;
-                        nc1 = left;
-                    }
-                    continue;
+                // the round's words, and the ids of bit hj of words 2i (low
+                // half) and 2i + 1 (bit hj + 16: + 16): positions in the unit
+                uint32_t l4[4];
+                {
+                    const uint4 v = *reinterpret_cast<const uint4*>(list + r0);
+                    l4[0] = v.x; l4[1] = v.y; l4[2] = v.z; l4[3] = v.w;
+                }
+                uint32_t ids2[kWXW / 2];
+#pragma unroll
+                for (int i = 0; i < kWXW / 2; i++) {
+                    const uint32_t pair = l4[i >> 1] >> (16 * (i & 1));
+                    ids2[i] = ((pair & 127u) * 32u + hj) | ((((pair >> 8) & 127u) * 32u + hj) << 16);
                 }
                 if (wrow) {
-                    uint32_t pm[kWXW];
+                    uint32_t wd[kWXW], pm[kWXW];
+#pragma unroll
+                    for (int s = 0; s < kWXW; s++) {
+                        const uint32_t at = (l4[s >> 2] >> (8 * (s & 3))) & 127u;
+                        wd[s] = (uint32_t)s < nw ? __ldg(bw + (unsigned long long)at * Q + q) : 0u;
+                    }
                     const unsigned long long wcur = cur - nc;
                     uint32_t acc = ((uint32_t)wcur & (kVec - 1u)) + nc;
                     // the k-th query of todo is expanded in pass k / 2 by half
@@ -1348,13 +1378,8 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
                         sl[4 + v] = make_uint4(pm[4 * v], pm[4 * v + 1], pm[4 * v + 2], pm[4 * v + 3]);
                     }
                     sl[8] = make_uint4((uint32_t)wcur, (uint32_t)(wcur >> 32), nstage, nc | (nwrite << 4));
-                    if (qh == 0) {
-                        cur0 = end;
-                        nc0 = nstage - nwrite;
-                    } else {
-                        cur1 = end;
-                        nc1 = nstage - nwrite;
-                    }
+                    cur = end;
+                    nc = nstage - nwrite;
                 }
                 __syncwarp();
                 while (todo) {
@@ -1390,7 +1415,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
 #pragma unroll
                         for (int wi = 0; wi < kWXW; wi++) {
                             const uint32_t xa = W[wi] << lsh_a, xb = W[wi] << lsh_b;
-                            const uint32_t id = idbase + 32u * (uint32_t)wi;
+                            const uint32_t id = (wi & 1) ? ids2[wi >> 1] >> 16 : ids2[wi >> 1];
                             st_shared_if_neg((int)xa, P[wi] + (uint32_t)sizeof(E) * __popc(xa), (E)id);
                             st_shared_if_neg((int)xb, P[wi] + (uint32_t)sizeof(E) * __popc(xb),
                                              (E)(id + 16u));
@@ -1418,6 +1443,27 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
                         }
                         if (hj < nstage - nwrite) carry[hj] = sb[nwrite + hj];
                     }
+                }
+            }
+            __syncwarp();  // (the carries have been written)
+            for (uint32_t bl = run_blocks; bl; bl &= bl - 1u) {
+                const uint32_t b = (uint32_t)__ffs(bl) - 1u;
+                for (uint32_t rem = __shfl_sync(kFull, run, (int)b); rem;) {
+                    const uint32_t w = (uint32_t)__ffs(rem) - 1u;
+                    // (32 words of a run: ffs(0) - 1 is larger than any)
+                    const uint32_t k = min((uint32_t)__ffs(~(rem >> w)) - 1u, (uint32_t)kWXW);
+                    rem &= ~(((1u << k) - 1u) << w);
+                    if (slot_copies) {
+                        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                        pending = 0;
+                    }
+                    __syncwarp();
+                    const bool last = rem == 0u && (bl & (bl - 1u)) == 0u;
+                    full_round(nbr, slots, s_carry[wib][qh + lane], wrow, (32u * b + w) * 32u, 32u * k,
+                               last, cur, nc, lane);
+                    slot_copies = 1;
+                    cur += 32u * k;
+                    nc = last ? 0u : (uint32_t)cur & (kSec - 1u);
                 }
             }
         }
@@ -1839,7 +1885,15 @@ __global__ void asym_flags_kernel(TableArgs a) {
             const uint32_t c = g / (a.unit_words * 32u), pos = g % (a.unit_words * 32u);
             if (!VDB_GUARD(a.st, g != 0xffffffffu && c < nu && slot < kUnitQ, 5, target)) continue;
             for (uint32_t u = u0; u < u0 + c; u++) lo += a.parts[(unsigned long long)u * kUnitQ + slot];
-            hi = lo + a.parts[(unsigned long long)(u0 + c) * kUnitQ + slot];
+            // (a one-way pair was tested: it is not in the runs that follow the
+            // unit's other entries)
+            uint32_t in_runs = 0;
+            if (a.wflags && a.tile_loff[t + 1] != a.tile_loff[t])
+                for (uint32_t b = 0; b < a.unit_words / 32u; b++)
+                    in_runs += 32u * (uint32_t)__popc(full_runs(
+                                         a.wflags[(unsigned long long)(u0 + c) * (a.unit_words / 32u) + b].x,
+                                         c * a.unit_words + 32u * b, before));
+            hi = lo + a.parts[(unsigned long long)(u0 + c) * kUnitQ + slot] - in_runs;
             if (hi > end) hi = end;
             if (lo > hi) lo = hi;
             const unsigned long long seg_end = hi;
