@@ -121,9 +121,9 @@ typedef struct {
                                0 = the library's choice: 2 on grids of more than two cells
                                per point, else 1 */
     int32_t unit_candidates; /* candidates of a tile per work unit of the neighbour search
-                               (1024, 2048 or 4096); 0 = 1024 for datasets of fewer than
-                               2^18 points (a table with few units is bounded by its
-                               longest unit), else 4096.  Labels and tables do not
+                               (1024, 2048 or 4096); 0 = the library's choice by the
+                               table's work, 512 to 4096 (a table with few units is
+                               bounded by its longest unit).  Labels and tables do not
                                depend on it */
     int32_t graph;          /* nonzero: replay repeated calls as one CUDA graph.  The first
                                call with given datasets (buffers, sizes, variants) and

@@ -478,8 +478,23 @@ uint32_t default_tile_cells(uint32_t n, uint64_t ncells) {
     return (uint64_t)n * 2 < ncells ? 2u : 1u;
 }
 
+constexpr uint32_t kSmallTilePoints = 1u << 17;  // tiles of 32 queries below this many points
 constexpr uint32_t kBoxPoints = 1u << 15;        // word boxes from this many points on
-constexpr uint32_t kSmallUnitPoints = 1u << 18;  // smaller work units below this many points
+
+// Candidates per work unit, in bitmap words.  A table with few units takes as
+// long as its longest ones, and the expand pass packs its rounds better in long
+// ones; points x points per cell measures a table's work.  Count + table, ms,
+// with units of 32 / 64 / 128 words: 1M sweep eps 0.1 (0.04M) 0.61 / 0.67 / 0.69,
+// eps 0.2 (0.15M) 1.06 / 1.08 / 1.13, eps 0.4 (0.6M) 2.04 / 1.98 / 1.99, eps 0.8
+// (2.5M) 4.34 / 4.17 / 4.04; 2M lattice eps 0.05 (0.04M) 1.69 / 1.85 / 2.07, eps
+// 0.25 (1.0M) 2.89 / 2.79 / 2.81; 400k mixture eps 0.8 (0.4M) 0.75 / 0.77 / 0.84.
+// Small inputs, whole calls with 16 / 32 words: 50k 383 / 409 us, 60k x 16 variants
+// 1.71 / 1.76 ms, FP64 100k sweep 3.82 / 4.23 ms.
+uint32_t default_unit_words(uint32_t n, uint64_t ncells) {
+    if (n < kSmallTilePoints) return kUnitWordsTiny;
+    const double work = (double)n * (double)n / (double)ncells;
+    return work < 0.5e6 ? kUnitWordsSmall : work < 1.5e6 ? 64u : kUnitWords;
+}
 
 // Worker streams of a multi-dataset call: datasets run concurrently so that
 // one dataset's host waits and small grids are covered by the others, but
@@ -725,11 +740,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     if (o.unit_words != 0 && o.unit_words != (int)kUnitWordsSmall && o.unit_words != 64 &&
         o.unit_words != (int)kUnitWords)
         throw VdbError{VDB_ERR_INVALID_ARG, "unit_candidates must be 0, 1024, 2048 or 4096"};
-    // work units: 1024 candidates for datasets below 2^18 points (few units:
-    // the longest one bounds the count and expand passes), else 4096
-    const uint32_t unit_words = o.unit_words > 0 ? (uint32_t)o.unit_words
-                                : n < kSmallUnitPoints ? kUnitWordsSmall
-                                                       : kUnitWords;
     if (n > 0x7fffffffu) throw VdbError{VDB_ERR_TOO_LARGE, "more than 2^31-1 points"};
 
     // graph replay: recording a direct run, or capturing one from its record
@@ -940,7 +950,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     size_t trow_cap = 0;
 
     const bool want_mixed = o.precision == VDB_PRECISION_MIXED;
-    const int tq = table_tile_queries();
+    // (small inputs: tiles of 32, twice as many and half as long)
+    const int tq = n < kSmallTilePoints ? table_tile_queries() / 2 : table_tile_queries();
     const int nb_count = ctx->nsm * ctx->blocks_count[want_mixed];
     const int nb_fill = ctx->nsm * ctx->blocks_fill[want_mixed];
     const int nb_expand16 = ctx->nsm * ctx->blocks_expand[1];
@@ -1057,6 +1068,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         uint32_t group_asym = 0;
         bool chunked = false;
         bool compact = false;  // 16-bit table entries for this group's table
+        uint32_t unit_words = kUnitWordsSmall;
         bool no_rows = false;  // labels only: the degrees are all that is needed
         chunk_list.assign(1, RowChunk{0, 0xffffffffu, 0, 0xffffffffu, 0, n, 0, 0});
         table_marks.clear();
@@ -1203,6 +1215,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ta_args.st = d_st;
             // layout of the count pass's test bitmap (one word per query and
             // 32 candidates of its tile), which the table pass expands
+            unit_words = o.unit_words > 0 ? (uint32_t)o.unit_words : default_unit_words(n, g.ncells);
             ta_args.unit_words = unit_words;
             launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, tloff, d_nwords, d_nunits,
                               gz.words, s);
@@ -1254,7 +1267,9 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 parts = nullptr;
             }
             if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
-            if (!wflags && compact && !no_rows) wflags = ar.get<uint2>(unit_cap * (unit_words / 32));
+            // (sized for any unit size: a later epsilon may take larger units)
+            if (!wflags && compact && !no_rows)
+                wflags = ar.get<uint2>(unit_cap * flag_blocks(kUnitWords));
             ta_args.wflags = compact && !no_rows ? wflags : nullptr;
             ta_args.tile_uoff = tuoff;
             ta_args.tile_loff = tloff;
@@ -2395,7 +2410,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     oa.clist = clist;
     oa.ckey = ckey;
     oa.ccx = ccx;
-    oa.tq = (uint32_t)table_tile_queries();
+    oa.tq = (uint32_t)table_tile_queries() / 2;
     oa.tiles = tiles;
     oa.ptile = ptile;
     oa.ntiles = d_ntiles;
@@ -2426,7 +2441,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.asym_n = asym_n;
     ta.asym_cap = kNoallocAsymCap;
     ta.st = st;
-    ta.unit_words = kUnitWordsSmall;
+    ta.unit_words = kUnitWordsTiny;
     // work units of the count pass (no bitmap here: the fill pass writes the table)
     uint32_t* tuoff = cv.take<uint32_t>((size_t)n + 1);
     uint32_t* tloff = cv.take<uint32_t>((size_t)n + 1);
@@ -2511,7 +2526,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         memset(&ca, 0, sizeof ca);
         ca.n = n;
         ca.deg = deg;
-        ca.unit_words = kUnitWordsSmall;
+        ca.unit_words = kUnitWordsTiny;
         ca.minpts = minpts > 0x7fffffffu ? ~0ull : (unsigned long long)minpts;
         ca.minpts_prev = ~0ull;
         ca.off = off;

@@ -221,16 +221,22 @@ __global__ void gather_kernel(OrderArgs a) {
 
 // One pass over the sorted keys: the gathers, and the first points of cells
 // and tiles compacted by a single-pass scan (both counts in one state word, 31
-// bits each).  A warp takes 32 * kOrderItems consecutive points.
-constexpr int kOrderItems = 4;
+// bits each).  A warp takes 32 * kOrderItems consecutive points.  The tiles of a
+// group of cells start every tq points from the group's first point (found by
+// looking back for the last group start): cut at multiples of tq of the point
+// index instead, a cell of 30 points was two tiles half of the time.
+constexpr int kOrderItems = 2;
 constexpr uint32_t kOrderTile = kLookThreads * kOrderItems;
-__global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookState ls) {
+__global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookState ls,
+                                                             unsigned long long* marks) {
     pdl_sync();
+    __shared__ uint32_t s_last[kLookThreads / 32];  // 1 + the warp's last group start, or 0
+    __shared__ uint32_t s_in;
     const uint32_t tile = lookback_ticket(ls);
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint64_t base = (uint64_t)tile * kOrderTile + wid * (32u * kOrderItems);
     uint32_t key[kOrderItems], bc[kOrderItems], bt[kOrderItems];
-    unsigned long long mine = 0;  // cells | tiles << 31 of the warp
+    uint32_t last = 0;
 #pragma unroll
     for (int i = 0; i < kOrderItems; i++) {
         const uint64_t k = base + 32u * i + lane;
@@ -238,11 +244,29 @@ __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookSt
         key[i] = in ? a.gkey[k] : 0u;
         uint32_t prev = __shfl_up_sync(0xffffffffu, key[i], 1);
         if (lane == 0 && in && k > 0) prev = a.gkey[k - 1];
-        const bool fc = in && (k == 0 || key[i] != prev);
-        const bool ft = in && (k == 0 || key[i] / a.g.G != prev / a.g.G ||
-                               (uint32_t)k % a.tq == 0u);
-        bc[i] = __ballot_sync(0xffffffffu, fc);
-        bt[i] = __ballot_sync(0xffffffffu, ft);
+        bc[i] = __ballot_sync(0xffffffffu, in && (k == 0 || key[i] != prev));
+        bt[i] = __ballot_sync(0xffffffffu, in && (k == 0 || key[i] / a.g.G != prev / a.g.G));
+        if (bt[i]) last = (uint32_t)base + 32u * i + 32u - (uint32_t)__clz((int)bt[i]);
+    }
+    if (lane == 0) s_last[wid] = last;
+    __syncthreads();
+    if (wid == 0) {
+        uint32_t mine = lane < kLookThreads / 32 ? s_last[lane] : 0u;
+        mine = __reduce_max_sync(0xffffffffu, mine);
+        const uint32_t in = (uint32_t)warp_last_mark(mine, tile, marks, a.st);
+        if (lane == 0) s_in = in;
+    }
+    __syncthreads();
+    uint32_t start = s_in;
+    for (uint32_t w = 0; w < wid; w++) start = max(start, s_last[w]);
+    unsigned long long mine = 0;  // cells | tiles << 31 of the warp
+#pragma unroll
+    for (int i = 0; i < kOrderItems; i++) {
+        const uint64_t k = base + 32u * i + lane;
+        const uint32_t upto = bt[i] & ((2u << lane) - 1u);
+        const uint32_t s1 = upto ? (uint32_t)base + 32u * i + 32u - (uint32_t)__clz((int)upto) : start;
+        if (bt[i]) start = (uint32_t)base + 32u * i + 32u - (uint32_t)__clz((int)bt[i]);
+        bt[i] = __ballot_sync(0xffffffffu, k < a.n && ((uint32_t)k + 1u - s1) % a.tq == 0u);
         mine += (unsigned long long)__popc(bc[i]) | ((unsigned long long)__popc(bt[i]) << 31);
     }
     const unsigned long long before = block_lookback(lane == 31 ? mine : 0ull, tile, ls, a.st);
@@ -403,13 +427,15 @@ void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g
 }
 
 size_t order_state_bytes(uint32_t n) {
-    return look_state_bytes(((uint64_t)n + kOrderTile - 1) / kOrderTile);
+    const uint64_t nb = ((uint64_t)n + kOrderTile - 1) / kOrderTile;
+    return look_state_bytes(nb) + nb * 8;
 }
 
 void launch_order(const OrderArgs& a, void* zeroed, cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (unsigned)(((uint64_t)a.n + kOrderTile - 1) / kOrderTile);
-    launch(order_kernel, nb, kLookThreads, s, a, look_state(zeroed));
+    launch(order_kernel, nb, kLookThreads, s, a, look_state(zeroed),
+           (unsigned long long*)((char*)zeroed + look_state_bytes(nb)));
 }
 
 void launch_gather(const OrderArgs& a, cudaStream_t s) {

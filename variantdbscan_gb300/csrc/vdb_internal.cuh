@@ -46,7 +46,7 @@ constexpr int kMaxRows = 65;             // neighbour rows per tile: 2*rho+1 <= 
 constexpr uint32_t kAsymFlag = 0x80000000u;  // neighbour-table entry accepted in one direction only
 constexpr uint32_t kIdMask = 0x7fffffffu;
 // Compact tables: 16-bit entries.  A row lists its neighbours work unit by
-// work unit (units of 1024 to 4096 candidates of the row's tile, in
+// work unit (units of 512 to 4096 candidates of the row's tile, in
 // order; the count pass's per-unit counts give each unit's share of the row);
 // an entry holds the neighbour's position within its unit's candidates (12
 // bits) and, in the top bit, the one-way flag.  Positions map to cell-ordered
@@ -416,7 +416,7 @@ struct TableArgs {
     // bitmap words); tile t has the units tile_uoff[t]..tile_uoff[t+1].  Warps
     // take the units of ulist (unit, tile), which leaves out those of small
     // tiles; tile t's are tile_loff[t]..tile_loff[t+1] of it.
-    uint32_t unit_words;            // kUnitWords or kUnitWordsSmall
+    uint32_t unit_words;            // bitmap words per unit (default_unit_words)
     const uint2* ulist;
     const uint32_t* tile_uoff;
     const uint32_t* tile_loff;
@@ -432,12 +432,16 @@ struct TableArgs {
     uint32_t unit_lo, unit_hi;
     uint32_t row_lo, row_hi;
 };
-// Work units hold 4096 candidates of a tile (kUnitWords bitmap words) or, for
-// small datasets, 1024 (kUnitWordsSmall): a warp's longest unit bounds the
-// count and expand passes of a table with few units.  Compact entries are
-// positions within a unit (12 bits) either way.
+// Work units hold up to 4096 candidates of a tile (kUnitWords bitmap words;
+// compact entries are positions within a unit, 12 bits), down to 512
+// (kUnitWordsTiny) for tables of few units (default_unit_words).
 constexpr uint32_t kUnitWords = 128;
 constexpr uint32_t kUnitWordsSmall = 32;
+constexpr uint32_t kUnitWordsTiny = 16;
+// Entries of wflags per unit.
+static __host__ __device__ __forceinline__ uint32_t flag_blocks(uint32_t unit_words) {
+    return (unit_words + 31u) / 32u;
+}
 constexpr uint32_t kUnitQ = 64;        // query slots per unit (tiles hold <= 64 queries)
 
 // Walks row k of a compact table (nb16, the row's entries [row0, row1)) unit

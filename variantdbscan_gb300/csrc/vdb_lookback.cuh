@@ -103,6 +103,29 @@ static __device__ __forceinline__ unsigned long long block_lookback(unsigned lon
     return r;
 }
 
+// The last mark before this tile, by the same scheme (warp 0 of the block; the
+// result in every lane): mine = the tile's last mark, 0 if it has none.  A
+// tile with a mark of its own answers for all before it; the first has one.
+static __device__ __forceinline__ unsigned long long warp_last_mark(unsigned long long mine,
+                                                                    uint32_t tile,
+                                                                    unsigned long long* tiles,
+                                                                    DeviceStatus* st) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane == 0) look_store(&tiles[tile], (mine ? kLookPrefix : kLookSum) | mine);
+    unsigned long long found = 0;
+    for (int64_t b = (int64_t)tile - 1; b >= 0; b -= 32) {
+        const int64_t i = b - (int64_t)lane;
+        const unsigned long long s = i >= 0 ? look_wait(&tiles[i], st) : kLookSum;
+        const uint32_t full = __ballot_sync(0xffffffffu, (s >> 62) == 2ull);
+        if (full) {
+            found = __shfl_sync(0xffffffffu, s & kLookMask, __ffs(full) - 1);
+            break;
+        }
+    }
+    if (lane == 0 && !mine) look_store(&tiles[tile], kLookPrefix | found);
+    return found;
+}
+
 // The same for one counter per thread: states of tile t at p[t * stride].
 constexpr int kDigitLooks = 8;
 static __device__ __forceinline__ unsigned long long digit_lookback(uint32_t v, uint32_t tile,

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                     const uint32_t mi = __ballot_sync(kFull, in), mo = __ballot_sync(kFull, out);
                     todo &= ~(mi | mo);
                     if (a.wflags && lane == 0)
-                        a.wflags[(unsigned long long)u * (a.unit_words / 32u) + (wb - (cbeg >> 5)) / 32u] =
+                        a.wflags[(unsigned long long)u * flag_blocks(a.unit_words) + (wb - (cbeg >> 5)) / 32u] =
                             make_uint2(mi, mo);
                     const uint32_t add = __reduce_add_sync(kFull, in ? g1 - g0 : 0u);
                     if (qk[0] < qe) cnt[0] += add;
@@ -854,8 +854,8 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                 }
             }
         }
-        if (a.wflags && !settled && (uint32_t)lane < a.unit_words / 32u)
-            a.wflags[(unsigned long long)u * (a.unit_words / 32u) + lane] = make_uint2(0u, 0u);
+        if (a.wflags && !settled && (uint32_t)lane < flag_blocks(a.unit_words))
+            a.wflags[(unsigned long long)u * flag_blocks(a.unit_words) + lane] = make_uint2(0u, 0u);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
             if (qk[q] < qe) {
@@ -1301,7 +1301,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
         uint32_t mix = 0u, run = 0u;
         if ((uint32_t)lane * 32u < wend - wbeg) {
             const uint32_t w0 = wbeg + 32u * (uint32_t)lane;
-            const uint2 f = a.wflags[(unsigned long long)u * (a.unit_words / 32u) + lane];
+            const uint2 f = a.wflags[(unsigned long long)u * flag_blocks(a.unit_words) + lane];
             const uint32_t nwb = min(32u, wend - w0);
             run = full_runs(f.x, w0, C);
             mix = (nwb == 32u ? kFull : (1u << nwb) - 1u) & ~f.y & ~run;
@@ -1889,9 +1889,9 @@ __global__ void asym_flags_kernel(TableArgs a) {
             // unit's other entries)
             uint32_t in_runs = 0;
             if (a.wflags && a.tile_loff[t + 1] != a.tile_loff[t])
-                for (uint32_t b = 0; b < a.unit_words / 32u; b++)
+                for (uint32_t b = 0; b < flag_blocks(a.unit_words); b++)
                     in_runs += 32u * (uint32_t)__popc(full_runs(
-                                         a.wflags[(unsigned long long)(u0 + c) * (a.unit_words / 32u) + b].x,
+                                         a.wflags[(unsigned long long)(u0 + c) * flag_blocks(a.unit_words) + b].x,
                                          c * a.unit_words + 32u * b, before));
             hi = lo + a.parts[(unsigned long long)(u0 + c) * kUnitQ + slot] - in_runs;
             if (hi > end) hi = end;
