@@ -470,10 +470,6 @@ __global__ void cell_best_kernel(CellArgs a) {
         atomicMax(&a.cbest[c], ((unsigned long long)mx << 32) | (uint32_t)~k);
 }
 
-// First unions: the points of largest degree of a cell and of an adjacent one
-// are tested.  In dense regions that joins almost every pair of adjacent
-// cells, so that the search below finds most pairs already joined.
-//
 // Hooks: a cell that has cores for the first time in slot v is a tree of its
 // own and nobody else writes its parent, so it can be hung under an earlier
 // cell without atomics: under the first cell of the run of joined cells that
@@ -531,81 +527,20 @@ __global__ void cell_hook_kernel(CellArgs a) {
     if (c < ncl) a.parent[c] = p;
 }
 
-// The other adjacent cells, of the next row and along the row: a thread per
-// cell and row looks at up to three of them.  Neighbouring lanes
-// mostly want the same two trees joined: one union per pair of roots and warp.
-constexpr int kNearLoads = 5;  // cells of two per eps: all the cells of a row within reach
-__global__ void __launch_bounds__(kThreads, 4) cell_near_kernel(CellArgs a, int v) {
-    pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    const uint32_t dy = blockIdx.y ^ 1u;  // next row first
-    const uint32_t ncl = *a.ncl;
-    if (c - lane >= ncl) return;  // (whole warps)
-    const uint32_t mp = a.mp[v];
-    const uint32_t rho = (uint32_t)a.ep->rho;
-    const PairTest t = pair_test(a);
-    uint32_t* parent = a.parent + (size_t)v * a.n;
-    uint32_t o = 0, oe = 0, ku = 0;
-    int cx = 0;
-    float2 pu = make_float2(0.f, 0.f);
-    if (c < ncl && dy <= rho) {
-        const unsigned long long bA = a.cbest[c];
-        ku = best_point(bA);
-        if (best_deg(bA) >= mp && ku < a.n) {
-            const uint2 rg = a.crng[(size_t)(rho + dy) * a.n + c];
-            cx = (int)a.ccx[c];
-            pu = a.glocal[ku];
-            o = dy ? rg.x : c + 1;
-            oe = rg.y;
-        }
-    }
-    const uint32_t pc = o < oe ? parent[c] : 0u;
-    for (; __any_sync(kFull, o < oe); o = min(o + (uint32_t)kNearLoads, oe)) {
-        // a row's cells at once: their loads overlap
-        uint32_t want = 0;  // adjacent cells with cores and another parent
-        if (o < oe) {
-#pragma unroll
-            for (int j = 0; j < kNearLoads; j++) {
-                if (o + j >= oe) continue;
-                const int dx = (int)a.ccx[o + j] - cx;
-                if (best_deg(a.cbest[o + j]) >= mp && parent[o + j] != pc && dx >= -1 && dx <= 1)
-                    want |= 1u << j;
-            }
-        }
-        while (__any_sync(kFull, want != 0u)) {
-            uint32_t ra = 0, rb = 0;
-            bool join = want != 0u;
-            if (join) {
-                const uint32_t w = o + (uint32_t)__ffs(want) - 1u;
-                want &= want - 1u;
-                const uint32_t kv = best_point(a.cbest[w]);
-                join = kv < a.n && test_pair(a, t, ku, kv, pu, a.glocal[kv], (int)a.ccx[w] - cx,
-                                             (int)dy) == 3u;
-                if (join) {
-                    ra = uf_find(parent, c);
-                    rb = uf_find(parent, w);
-                    join = ra != rb;
-                }
-            }
-            const unsigned long long key =
-                join ? ((unsigned long long)max(ra, rb) << 32) | min(ra, rb) : ~0ull - lane;
-            const uint32_t same = __match_any_sync(kFull, key);
-            if (join && lane == (uint32_t)(__ffs(same) - 1)) uf_union(parent, ra, rb, a.st);
-            __syncwarp();
-        }
-    }
-}
-
 constexpr uint32_t kLanePairs = 4;     // cells of at most so many point pairs: one lane
 constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes over the pairs
 
-// Remaining unions of slot v: every pair of cells within reach whose roots
-// still differ is searched for one core-core pair accepted in both
-// directions.  A lane takes a cell and one row of its half neighbourhood; it
-// screens the roots and tests the pairs of next to empty cells itself; the
-// other pairs are searched by the whole warp, lanes over the point pairs (or,
-// for large cells, over the first cell's points within eps of the second).
-__global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int v) {
+// Unions of slot v: every pair of cells within reach whose roots differ is
+// searched for one core-core pair accepted in both directions.  A lane takes a
+// cell and one row of its half neighbourhood: it screens the roots and tests
+// the cells' points of largest degree (and all pairs of next to empty cells);
+// only then the pairs that are still apart are searched by the whole warp,
+// lanes over the point pairs (or, for large cells, over the first cell's points
+// within eps of the second).  The searches are the expensive part, and after
+// the cheap unions few are left.  The clustering of the 2M sweep at eps 0.2 took
+// 0.88 ms with the cheap unions and a flatten as kernels before it, 0.67 like
+// this; 1M uniform points at eps 0.05 0.50 -> 0.41 ms.
+__global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a, int v) {
     pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
@@ -614,16 +549,18 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
     const double eps = a.ep->eps;
     const float near2 = (float)(eps * eps * (1.0 + 0x1p-8));
     const float wf = t.wf;
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, dy = blockIdx.y;
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t dy = (blockIdx.y + 1u) % gridDim.y;  // (the next row's many pairs first)
     if (c - lane >= ncl) return;  // (whole warps)
     uint32_t* parent = a.parent + (size_t)v * a.n;
     const uint32_t* __restrict__ comp = a.comp_prev[v];
     uint32_t skipped = 0;  // cell pairs of different components at a larger epsilon
-    uint32_t o = 0, oe = 0, sA = 0, eA = 0, compA = kNone;
+    uint32_t o = 0, oe = 0, sA = 0, eA = 0, compA = kNone, ku = 0;
     int cx = 0;
     if (c < ncl) {
         const unsigned long long bA = a.cbest[c];
-        if (best_deg(bA) >= mp) {
+        ku = best_point(bA);
+        if (best_deg(bA) >= mp && ku < a.n) {
             const uint2 rg = a.crng[(size_t)((uint32_t)a.ep->rho + dy) * a.n + c];
             o = dy ? rg.x : c + 1;
             oe = rg.y;
@@ -631,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
                 cx = (int)a.ccx[c];
                 sA = a.clist[c];
                 eA = a.clist[c + 1];
-                if (comp) compA = comp[a.gpos[best_point(bA)]];
+                if (comp) compA = comp[a.gpos[ku]];
             }
         }
     }
@@ -642,41 +579,69 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
     {
         const uint32_t pc = c < ncl ? parent[c] : 0u;
 #pragma unroll 5
-        for (uint32_t j = 0; j < min(oe - o, 32u); j++)
+        for (uint32_t j = 0; j < (o < oe ? min(oe - o, 32u) : 0u); j++)
             if (best_deg(a.cbest[o + j]) >= mp && parent[o + j] != pc) left |= 1u << j;
     }
-    // every lane takes the cells left in its row; each step's pairs that need
-    // more than a lane are then searched one after the other
+    // Every lane takes the cells left in its row: the cells' points of largest
+    // degree first, which in dense regions mostly pair, or all points of next
+    // to empty cells.  `hard` keeps the pairs that need a search.
+    uint32_t hard = 0;
     while (__any_sync(kFull, left != 0u)) {
-        bool need = false;
-        uint32_t sB = 0, eB = 0;
-        int dx = 0;
-        uint32_t ob = 0;
+        bool join = false;
+        uint32_t ra = 0, rb = 0;
         if (left) {
-            ob = o = o0 + (uint32_t)__ffs(left) - 1u;
+            const uint32_t j = (uint32_t)__ffs(left) - 1u;
+            o = o0 + j;
             left &= left - 1u;
             const unsigned long long bB = a.cbest[o];
-            need = uf_find(parent, c) != uf_find(parent, o);
+            const uint32_t kv = best_point(bB);
+            ra = uf_find(parent, c);
+            rb = uf_find(parent, o);
             // cores in different components at the larger epsilon are not
             // connected at this one (its components refine those)
-            if (need && comp && comp[a.gpos[best_point(bB)]] != compA) {
-                need = false;
-                skipped++;
-            }
-            if (need) {
-                sB = a.clist[o];
-                eB = a.clist[o + 1];
-                dx = (int)a.ccx[o] - cx;
-                if ((uint64_t)(eA - sA) * (eB - sB) <= kLanePairs) {
-                    for (uint32_t u = sA; u < eA && need; u++)
-                        for (uint32_t w = sB; w < eB && need; w++)
-                            if (a.deg[u] >= mp && a.deg[w] >= mp &&
-                                test_pair(a, t, u, w, a.glocal[u], a.glocal[w], dx, (int)dy) == 3u) {
-                                uf_union(parent, c, o, a.st);
-                                need = false;
-                            }
-                    need = false;
+            const bool apart = ra != rb && comp && kv < a.n && comp[a.gpos[kv]] != compA;
+            if (apart) skipped++;
+            if (ra != rb && !apart && kv < a.n) {
+                const int dx = (int)a.ccx[o] - cx;
+                join = test_pair(a, t, ku, kv, a.glocal[ku], a.glocal[kv], dx, (int)dy) == 3u;
+                if (!join) {
+                    const uint32_t sB = a.clist[o], eB = a.clist[o + 1];
+                    if ((uint64_t)(eA - sA) * (eB - sB) <= kLanePairs) {
+                        for (uint32_t u = sA; u < eA && !join; u++)
+                            for (uint32_t w = sB; w < eB && !join; w++)
+                                join = a.deg[u] >= mp && a.deg[w] >= mp &&
+                                       test_pair(a, t, u, w, a.glocal[u], a.glocal[w], dx,
+                                                 (int)dy) == 3u;
+                    } else {
+                        hard |= 1u << j;
+                    }
                 }
+            }
+        }
+        // neighbouring lanes mostly want the same two trees joined: one union
+        // per pair of roots and warp
+        if (__any_sync(kFull, join)) {
+            const unsigned long long key =
+                join ? ((unsigned long long)max(ra, rb) << 32) | min(ra, rb) : ~0ull - lane;
+            const uint32_t same = __match_any_sync(kFull, key);
+            if (join && lane == (uint32_t)(__ffs(same) - 1)) uf_union(parent, ra, rb, a.st);
+            __syncwarp();
+        }
+    }
+    // the others, if their roots still differ, by the whole warp one after the
+    // other
+    while (__any_sync(kFull, hard != 0u)) {
+        bool need = false;
+        uint32_t sB = 0, eB = 0, ob = 0;
+        int dx = 0;
+        if (hard) {
+            ob = o0 + (uint32_t)__ffs(hard) - 1u;
+            hard &= hard - 1u;
+            need = uf_find(parent, c) != uf_find(parent, ob);
+            if (need) {
+                sB = a.clist[ob];
+                eB = a.clist[ob + 1];
+                dx = (int)a.ccx[ob] - cx;
             }
         }
         for (uint32_t todo = __ballot_sync(kFull, need); todo; todo &= todo - 1u) {
@@ -749,11 +714,9 @@ __global__ void __launch_bounds__(kThreads, 5) cell_pairs_kernel(CellArgs a, int
     if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
 }
 
-// Roots of slot v, after the first unions (so that the search tells joined
-// cells by one load) and after the search (last), when they are also the next
-// slot's start: a smaller minpts keeps every core and every connection, and
-// its new cells are hooked.
-__global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
+// Roots of slot v, which are also the next slot's start: a smaller minpts keeps
+// every core and every connection, and its new cells are hooked.
+__global__ void cell_flatten_kernel(CellArgs a, int v) {
     pdl_sync();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
@@ -764,7 +727,7 @@ __global__ void cell_flatten_kernel(CellArgs a, int v, int last) {
         r = uf_find_ro(parent, c);
         parent[c] = r;
     }
-    if (last && v + 1 < a.m) {
+    if (v + 1 < a.m) {
         const uint32_t p = hook_parent(a, pair_test(a), c, c < ncl, a.mp[v + 1],
                                        a.chain ? a.mp[v] : kNone, a.chain ? r : c);
         if (c < ncl) parent[a.n + c] = p;
@@ -901,7 +864,7 @@ __device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32
 // kLaneCores points for each lane that searches; a few lanes' larger searches
 // are done by the warp one after the other, lanes over the cells' points.
 constexpr uint32_t kLaneCores = 16;
-__global__ void __launch_bounds__(kThreads, 5) cell_labels_kernel(CellArgs a) {
+__global__ void __launch_bounds__(kThreads, 8) cell_labels_kernel(CellArgs a) {
     pdl_sync();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1109,10 +1072,8 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     launch(cell_best_kernel, nblk(a.n), kThreads, s, a);
     launch(cell_hook_kernel, nblk(a.n), kThreads, s, a);
     for (int v = 0; v < a.m; v++) {
-        launch(cell_near_kernel, dim3(nblk(a.n), 2), kThreads, s, a, v);
-        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v, 0);
         launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, s, a, v);
-        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v, 1);
+        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v);
     }
     launch(cell_seed_kernel, per_slot, kThreads, s, a);
     if (one_way) {
