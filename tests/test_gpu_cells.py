@@ -67,3 +67,25 @@ def test_sparse_cells_over_a_wide_box(ctx, vdb, orc):
     x[:6000] = rng.normal(700, 2, 6000)
     y[:6000] = rng.normal(700, 2, 6000)
     _check(ctx, vdb, orc, x, y, np.array([0.3, 0.3, 5.0]), np.array([4, 12, 3], np.uint32))
+
+
+@pytest.mark.parametrize("entry_bytes", [2, 4])
+@pytest.mark.parametrize("share", [1, 2, 3, 300])
+def test_row_chunks_of_a_budget(ctx, vdb, orc, share, entry_bytes):
+    # 2 chunks up to hundreds (more than one plan holds), and rows of a tile
+    # that do not fit a chunk
+    rng = np.random.default_rng(5)
+    n = 40011
+    x, y = rng.uniform(0, 40, n), rng.uniform(0, 40, n)
+    eps, mp = np.array([0.4, 0.4]), np.array([9, 14], np.uint32)
+    kw = dict(entry_bytes=entry_bytes, table_hash=True)
+    item = vdb.BatchItem(x, y, eps, mp, 70)
+    whole, sw = ctx.run([item], **kw)
+    np.testing.assert_array_equal(whole[0], orc.variants(x, y, eps, mp, 70))
+    out, st = ctx.run([item], budget=(sw["entry_bytes"] - 1) // share, **kw)
+    np.testing.assert_array_equal(out[0], whole[0])
+    assert st["table_hash"] == sw["table_hash"] == orc.table_hash(x, y, 0.4, 70) & M64
+    assert st["table_chunks"] > share
+    with pytest.raises(vdb.VDBError) as e:
+        ctx.run([item], budget=2, **kw)
+    assert e.value.code == -4  # no memory: the rows of one tile exceed the budget

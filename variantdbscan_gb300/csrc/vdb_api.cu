@@ -558,14 +558,6 @@ double avail_bytes(vdb_context* ctx) {
     return ((double)fb + (double)ctx->pool.cached_free()) / ctx->mem_share;
 }
 
-// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi), with the
-// entries [u_lo, u_hi) of the unit list, table entries [e_lo, e_hi).  The whole
-// table: t_hi = u_hi = 0xffffffff (no limits).
-struct RowChunk {
-    uint32_t t_lo, t_hi, u_lo, u_hi, r_lo, r_hi;
-    uint64_t e_lo, e_hi;
-};
-
 // Union-find state of one variant.
 struct UfState {
     uint32_t *parent, *seed, *cstart, *best, *bits, *brank;
@@ -573,32 +565,26 @@ struct UfState {
 
 // Splits the table into row chunks of whole tiles holding at most cap
 // entries each (greedy, in tile order).
-std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, const uint32_t* tiles,
+std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, Arena& ar, const uint32_t* tiles,
                                       const uint32_t* ntiles_dev, const uint32_t* tloff,
                                       const unsigned long long* off, uint32_t n, uint64_t cap,
                                       cudaStream_t s) {
-    uint32_t nt = 0;
-    CK(cudaMemcpyAsync(ctx->h_pinned, ntiles_dev, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    memcpy(&nt, ctx->h_pinned, 4);
-    std::vector<uint32_t> ht((size_t)nt + 1), hu((size_t)nt + 1);
-    std::vector<unsigned long long> ho((size_t)n + 1);
-    CK(cudaMemcpyAsync(ht.data(), tiles, ((size_t)nt + 1) * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(hu.data(), tloff, ((size_t)nt + 1) * 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ho.data(), off, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    if (ht[nt] != n) throw VdbError{VDB_ERR_CUDA, "tile list does not end at n"};
+    static_assert(sizeof(ChunkPlan) <= 4096, "the plan fits the pinned buffer");
     std::vector<RowChunk> out;
-    uint32_t t = 0;
-    while (t < nt) {
-        const uint64_t e0 = ho[ht[t]];
-        uint32_t t1 = t;
-        while (t1 < nt && ho[ht[t1 + 1]] - e0 <= cap) t1++;
-        if (t1 == t)
+    ChunkPlan* d = (ChunkPlan*)ar.get<uint64_t>(sizeof(ChunkPlan) / 8);
+    ChunkPlan h;
+    do {
+        launch_plan_chunks(tiles, ntiles_dev, tloff, off, n, cap, out.empty() ? 0u : h.next, d, s);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(ctx->h_pinned, d, sizeof h, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        memcpy(&h, ctx->h_pinned, sizeof h);
+        if (h.refused == 2) throw VdbError{VDB_ERR_CUDA, "tile list does not end at n"};
+        if (h.refused || (h.n == 0 && h.next < h.ntiles))
             throw VdbError{VDB_ERR_NOMEM, "the rows of one tile exceed the table budget"};
-        out.push_back(RowChunk{t, t1, hu[t], hu[t1], ht[t], ht[t1], e0, ho[ht[t1]]});
-        t = t1;
-    }
+        out.insert(out.end(), h.list, h.list + h.n);
+    } while (h.next < h.ntiles);
+    ar.put(d);
     if (out.empty()) out.push_back(RowChunk{0, 0, 0, 0, 0, 0, 0, 0});
     return out;
 }
@@ -1410,7 +1396,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 nbr_cap_bytes = 0;
                 const int64_t budget = o.budget > 0 ? o.budget : (int64_t)(avail_bytes(ctx) * 0.9);
                 const uint64_t cap = (uint64_t)std::max<int64_t>(budget / (int64_t)esz, 1);
-                chunk_list = plan_row_chunks(ctx, tiles, d_ntiles, tloff, off, n, cap, s);
+                chunk_list = plan_row_chunks(ctx, ar, tiles, d_ntiles, tloff, off, n, cap, s);
                 uint64_t mx = 1;
                 for (const RowChunk& c : chunk_list) mx = std::max<uint64_t>(mx, c.e_hi - c.e_lo);
                 const size_t w = std::max<size_t>(words_for(mx), 1);

@@ -499,6 +499,27 @@ void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s);
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s);
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s);
 void launch_asym_flags(const TableArgs& a, cudaStream_t s);
+
+// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi), with the
+// entries [u_lo, u_hi) of the unit list, table entries [e_lo, e_hi).  The whole
+// table: t_hi = u_hi = 0xffffffff (no limits).
+struct RowChunk {
+    uint32_t t_lo, t_hi, u_lo, u_hi, r_lo, r_hi;
+    uint64_t e_lo, e_hi;
+};
+constexpr uint32_t kPlanChunks = 64;
+struct ChunkPlan {
+    uint32_t n;       // chunks listed here
+    uint32_t next;    // first tile after them
+    uint32_t ntiles;
+    uint32_t refused; // 1: a tile's rows exceed the cap, 2: the tile list does not end at n
+    RowChunk list[kPlanChunks];
+};
+// The next (up to kPlanChunks) row chunks from tile t0: whole tiles, at most cap
+// entries each, greedy in tile order.
+void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tloff,
+                        const unsigned long long* off, uint32_t n, uint64_t cap, uint32_t t0,
+                        ChunkPlan* plan, cudaStream_t s);
 int table_block_threads();
 int table_tile_queries();
 int table_blocks_per_sm(bool fill, bool mixed);

@@ -1853,6 +1853,51 @@ __global__ void table_hash_kernel(TableArgs a, const uint32_t* __restrict__ gori
     if (lane == 0 && acc) atomicAdd(&a.st->table_hash, acc);
 }
 
+// Row chunks by one warp: each ends at the last tile whose rows still fit, found
+// by a 32-way search over the row offsets (4 rounds of two dependent loads for a
+// million tiles), so that the host reads a few hundred bytes of plan.  Copying
+// the tiles and the n + 1 row offsets to the host for the same loop there held up
+// each chunked table of 2M points by 1.4 ms.
+__global__ void plan_chunks_kernel(const uint32_t* __restrict__ tiles,
+                                   const uint32_t* __restrict__ ntiles,
+                                   const uint32_t* __restrict__ tloff,
+                                   const unsigned long long* __restrict__ off, uint32_t n,
+                                   uint64_t cap, uint32_t t0, ChunkPlan* plan) {
+    pdl_sync();
+    const uint32_t lane = threadIdx.x;
+    const uint32_t nt = *ntiles;
+    uint32_t t = t0, k = 0;
+    uint32_t refused = nt > n || tiles[nt] != n ? 2u : 0u;
+    while (!refused && t < nt && k < kPlanChunks) {
+        const unsigned long long e0 = off[tiles[t]];
+        uint32_t lo = t, hi = nt;  // the chunk's end: the last tile bound in [lo, hi] that fits
+        while (lo < hi) {
+            const uint64_t step = ((uint64_t)(hi - lo) + 31) / 32;
+            const uint32_t probe = (uint32_t)min((uint64_t)lo + (lane + 1) * step, (uint64_t)hi);
+            const uint32_t fit =
+                (uint32_t)__popc(__ballot_sync(kFull, off[tiles[probe]] - e0 <= cap));
+            const uint64_t base = lo;
+            lo = (uint32_t)min(base + fit * step, (uint64_t)hi);
+            if (fit < 32) hi = max(lo, (uint32_t)min(base + (fit + 1) * step, (uint64_t)hi) - 1u);
+        }
+        if (lo == t) {
+            refused = 1;
+        } else {
+            if (lane == 0)
+                plan->list[k] = RowChunk{t,         lo, tloff[t], tloff[lo], tiles[t], tiles[lo],
+                                         e0, off[tiles[lo]]};
+            k++;
+            t = lo;
+        }
+    }
+    if (lane == 0) {
+        plan->n = k;
+        plan->next = t;
+        plan->ntiles = nt;
+        plan->refused = refused;
+    }
+}
+
 // Flags the table entries accepted in one direction only (the count pass
 // recorded them): b in row a when dir == 1, a in row b when dir == 2.  Rows are
 // sorted by neighbour index.
@@ -1993,6 +2038,12 @@ void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, c
 
 void launch_asym_flags(const TableArgs& a, cudaStream_t s) {
     launch(asym_flags_kernel, 64, kTT, s, a);
+}
+
+void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tloff,
+                        const unsigned long long* off, uint32_t n, uint64_t cap, uint32_t t0,
+                        ChunkPlan* plan, cudaStream_t s) {
+    launch(plan_chunks_kernel, 1, 32, s, tiles, ntiles, tloff, off, n, cap, t0, plan);
 }
 
 int table_blocks_per_sm(bool fill, bool mixed) {
