@@ -312,6 +312,24 @@ struct GroupZero {
     }
 };
 
+// The parts of a distance test that are the same for all its threads.  Worked
+// out by each thread, the square root and the FP64 comparisons kept the SMs'
+// narrow FP64 pipe busy for 62% of the label kernel's time on sparse data
+// (1M uniform points, three epsilons: the whole call 3.0 -> 2.5 ms without).
+void finish_eps(EpsParams& p, const GridParams& g) {
+    auto ordered = [](double v) {
+        int64_t b = v == 0.0 ? 0 : -1;
+        if (v > 0.0) memcpy(&b, &v, sizeof b);
+        return (long long)b;
+    };
+    p.xb.eps = p.eps;
+    p.xb.thr = ordered(p.thr);
+    p.xb.tbox = ordered(p.tbox);
+    p.xb.ax = ordered(sqrt(p.tbox));
+    p.wf = (float)g.w;
+    p.near2 = (float)(p.eps * p.eps * (1.0 + 0x1p-8));
+}
+
 // Distance-test parameters of eps on grid g.  Cells (i, j) relative to a query
 // cell are scanned when their nearest points can be within eps:
 // (max(|i|-1,0)^2 + max(|j|-1,0)^2) * w^2 <= eps^2 (1 + 2^-16).  The margin
@@ -1152,6 +1170,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // cells are cliques when two points of one cell always pass the
             // distance test without a box check: 2 w^2 below thr and tbox
             clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
+            finish_eps(ep, g);
             launch_store_eps(d_ep, ep, s);
             const size_t tb = tm.mark();
 
@@ -2340,7 +2359,8 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
 
     GridParams g = make_grid(hb, eps / kCellsPerEps, 1, kNoallocMaxCells);
     g.sub = sub_bits(g.ncells);
-    const EpsParams ep = make_eps(eps, g, hb, true);
+    EpsParams ep = make_eps(eps, g, hb, true);
+    finish_eps(ep, g);
     uint32_t* gkey = cv.take<uint32_t>(n);
     uint32_t* gorig = cv.take<uint32_t>(n);
     double2* gxy = cv.take<double2>(n);

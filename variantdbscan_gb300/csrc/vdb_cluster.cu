@@ -393,8 +393,8 @@ __device__ __forceinline__ PairTest pair_test(const CellArgs& a) {
     t.mixed = a.ep->mixed != 0;
     t.lo = a.ep->lo32;
     t.hi = a.ep->hi32;
-    t.wf = (float)a.g.w;
-    t.xb = exact_bounds(a.ep->eps, a.ep->thr, a.ep->tbox);
+    t.wf = a.ep->wf;
+    t.xb = a.ep->xb;
     return t;
 }
 // bit0: v in N(u), bit1: u in N(v), for points ku and kv whose cells lie
@@ -546,8 +546,7 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a, int
     const uint32_t ncl = *a.ncl;
     const uint32_t mp = a.mp[v];
     const PairTest t = pair_test(a);
-    const double eps = a.ep->eps;
-    const float near2 = (float)(eps * eps * (1.0 + 0x1p-8));
+    const float near2 = a.ep->near2;
     const float wf = t.wf;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t dy = (blockIdx.y + 1u) % gridDim.y;  // (the next row's many pairs first)

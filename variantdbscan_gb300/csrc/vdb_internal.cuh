@@ -157,11 +157,24 @@ static __device__ __forceinline__ void cell_row_range(const GridParams& g,
     }
 }
 
+// Bounds of the exact predicate as ordered integers.  For doubles >= +0 the
+// order of the values is the order of their bit patterns read as integers, so
+// the predicate compares d2 and |d| with integer instructions and leaves
+// GB300's narrow FP64 pipe to the subtractions and products.  A negative or
+// NaN bound becomes -1, which no value passes (as with the FP64 comparison).
+struct ExactBounds {
+    double eps;
+    long long thr, tbox, ax;  // thr, tbox and ax_in = sqrt(tbox), ordered
+};
+
 // Distance test of one epsilon.
 struct EpsParams {
     double eps;
     double thr;     // largest double t with sqrt(t) <= eps
     double tbox;    // d2 <= tbox guarantees the candidate lies in the query box
+    ExactBounds xb; // of eps, thr and tbox
+    float wf;       // the cells' width, FP32
+    float near2;    // eps^2 (1 + 2^-8), FP32
     float lo32;     // FP32 d2 < lo32: neighbour (no FP64 re-test)
     float hi32;     // FP32 d2 > hi32: not a neighbour
     // count pass filter on the quadratic form nS = |c|^2/2 + (|q|^2 - L32)/2 - q.c
@@ -204,27 +217,6 @@ static __device__ __forceinline__ bool box_overlap(MpbBox m, double px, double p
     const double x0 = __dsub_rn(px, eps), x1 = __dadd_rn(px, eps);
     const double y0 = __dsub_rn(py, eps), y1 = __dadd_rn(py, eps);
     return !(x0 > m.x1 || m.x0 > x1 || y0 > m.y1 || m.y0 > y1);
-}
-
-// Bounds of the exact predicate as ordered integers.  For doubles >= +0 the
-// order of the values is the order of their bit patterns read as integers, so
-// the predicate compares d2 and |d| with integer instructions and leaves
-// GB300's narrow FP64 pipe to the subtractions and products.  A negative or
-// NaN bound becomes -1, which no value passes (as with the FP64 comparison).
-struct ExactBounds {
-    double eps;
-    long long thr, tbox, ax;  // thr, tbox and ax_in = sqrt(tbox), ordered
-};
-static __device__ __forceinline__ long long ordered_bits(double v) {
-    return v > 0.0 ? __double_as_longlong(v) : (v == 0.0 ? 0ll : -1ll);
-}
-static __device__ __forceinline__ ExactBounds exact_bounds(double eps, double thr, double tbox) {
-    ExactBounds b;
-    b.eps = eps;
-    b.thr = ordered_bits(thr);
-    b.tbox = ordered_bits(tbox);
-    b.ax = ordered_bits(sqrt(tbox));
-    return b;
 }
 
 // Exact predicate in both directions: bit0 = q in N(p), bit1 = p in N(q).

@@ -200,7 +200,7 @@ __global__ void word_boxes_kernel(TableArgs a) {
     if (k0 >= a.n) return;
     const uint32_t key0 = a.gkey[k0], cy0 = key0 / a.g.ncx_pad;
     const uint32_t e = min(k0 + kBoxRun, a.n);
-    const float wf = (float)a.g.w;
+    const float wf = a.ep->wf;
     float4 b = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
     if (a.gkey[e - 1] / a.g.ncx_pad == cy0) {
         for (uint32_t k = k0; k < e; k++) {
@@ -250,8 +250,8 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
     uint32_t cnt = 0, retest = 0, g = 0;
     if (mine) {
         const EpsParams* __restrict__ ep = a.ep;
-        const ExactBounds xb = exact_bounds(ep->eps, ep->thr, ep->tbox);
-        const float lo = ep->lo32, hi = ep->hi32, wf = (float)a.g.w;
+        const ExactBounds xb = ep->xb;
+        const float lo = ep->lo32, hi = ep->hi32, wf = a.ep->wf;
         const int rho = ep->rho, nrows = 2 * rho + 1;
         const uint32_t qs = a.tiles[t], Q = a.tiles[t + 1] - qs;
         const uint32_t key = a.gkey[k];
@@ -393,11 +393,11 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
     WarpRows& rows = s_rows[wib];
     double2* sqd = s_qd[wib];
     const EpsParams* __restrict__ ep = a.ep;
-    const ExactBounds xb = exact_bounds(ep->eps, ep->thr, ep->tbox);
+    const ExactBounds xb = ep->xb;
     const float L = ep->L32, wq = ep->w32;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
-    const float wf = (float)a.g.w;
+    const float wf = a.ep->wf;
     const uint32_t nlist = a.nunits[1];
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     const float fnan = __int_as_float(0x7fc00000);
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
-    const float wf = (float)a.g.w;
+    const float wf = a.ep->wf;
     const uint32_t nlist = min(a.nunits[1], a.unit_hi);  // the row chunk's part of the list
     if (a.n <= kSmallFused)
         for (uint64_t k = a.row_lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.row_hi;
@@ -1487,11 +1487,11 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
     const uint32_t lt = (1u << lane) - 1u;
     const EpsParams* __restrict__ ep = a.ep;
     const double eps = ep->eps, thr = ep->thr, tbox = ep->tbox;
-    const ExactBounds xb = exact_bounds(eps, thr, tbox);
+    const ExactBounds xb = ep->xb;
     const float lo = ep->lo32, hi = ep->hi32;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
-    const float wf = (float)a.g.w;
+    const float wf = a.ep->wf;
     const uint32_t tile_end = a.tile_end != 0xffffffffu ? a.tile_end : *a.ntiles;
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     unsigned long long my_retest = 0;
