@@ -89,3 +89,21 @@ def test_row_chunks_of_a_budget(ctx, vdb, orc, share, entry_bytes):
     with pytest.raises(vdb.VDBError) as e:
         ctx.run([item], budget=2, **kw)
     assert e.value.code == -4  # no memory: the rows of one tile exceed the budget
+
+
+@pytest.mark.parametrize("shift", [-9.0, -1.0, 0.0])
+@pytest.mark.parametrize("n", [1, 33, 255, 257, 1025, 70001])
+def test_boxes_of_signed_coordinates(ctx, vdb, orc, n, shift):
+    # negative coordinates only, of both signs, and zeros of both signs; the
+    # box's corners are the last points
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0, 2, n) + shift, rng.uniform(0, 1, n) + shift
+    x[: n // 4], y[n // 4 : n // 3] = 0.0, -0.0
+    x[-1], y[-1] = 2.5 + shift, 1.5 + shift
+    x[n // 2], y[n // 2] = shift - 0.5, shift - 0.5
+    eps, mp = np.array([20.0 / np.sqrt(n) if n < 1000 else 0.01]), np.array([4], np.uint32)
+    _check(ctx, vdb, orc, x, y, eps, mp)
+    for bad in (np.nan, np.inf, -np.inf):
+        x[-1] = bad
+        with pytest.raises(vdb.VDBError):
+            ctx.run([vdb.BatchItem(x, y, eps, mp, 70)])

@@ -109,27 +109,24 @@ __global__ void mpb_kernel(const double* __restrict__ x, const double* __restric
     const uint64_t s = b * (uint32_t)mbb;
     uint64_t e = s + (uint32_t)mbb;
     if (e > n) e = n;
-    double x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;
+    // (ordered keys; a minimum is the complement of the complements' maximum)
+    unsigned long long x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+#pragma unroll 2
     for (uint64_t k = s + lane; k < e; k += 32) {
         const uint32_t o = vorder[k];
-        const double xv = x[o], yv = y[o];
-        if (xv < x0) x0 = xv;
-        if (xv > x1) x1 = xv;
-        if (yv < y0) y0 = yv;
-        if (yv > y1) y1 = yv;
+        const unsigned long long kx = ordered_key(x[o]), ky = ordered_key(y[o]);
+        x0 = max(x0, ~kx);
+        x1 = max(x1, kx);
+        y0 = max(y0, ~ky);
+        y1 = max(y1, ky);
     }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        const double a0 = __shfl_xor_sync(0xffffffffu, x0, d);
-        const double a1 = __shfl_xor_sync(0xffffffffu, x1, d);
-        const double b0 = __shfl_xor_sync(0xffffffffu, y0, d);
-        const double b1 = __shfl_xor_sync(0xffffffffu, y1, d);
-        if (a0 < x0) x0 = a0;
-        if (a1 > x1) x1 = a1;
-        if (b0 < y0) y0 = b0;
-        if (b1 > y1) y1 = b1;
-    }
-    if (lane == 0) boxes[b] = MpbBox{x0, x1, y0, y1};
+    x0 = warp_max_u64(x0);
+    x1 = warp_max_u64(x1);
+    y0 = warp_max_u64(y0);
+    y1 = warp_max_u64(y1);
+    if (lane == 0)
+        boxes[b] = MpbBox{ordered_value(~x0), ordered_value(x1), ordered_value(~y0),
+                          ordered_value(y1)};
 }
 
 // Cell of v, floor((v - v0) / w) in FP64, and its subcell (of 2^sub per cell),

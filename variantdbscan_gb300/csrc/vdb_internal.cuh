@@ -157,6 +157,25 @@ static __device__ __forceinline__ void cell_row_range(const GridParams& g,
     }
 }
 
+// Doubles as unsigned integers of the same order (-0 just below +0), and back.
+// Minima and maxima are taken of these: GB300's FP64 pipe takes 16 cycles for a
+// warp's comparison, the integer pipe less than 2.
+static __device__ __forceinline__ unsigned long long ordered_key(double v) {
+    const long long b = __double_as_longlong(v);
+    return (unsigned long long)(b ^ ((b >> 63) | (long long)0x8000000000000000ull));
+}
+static __device__ __forceinline__ double ordered_value(unsigned long long k) {
+    const long long b = (long long)k;
+    return __longlong_as_double(b ^ (~(b >> 63) | (long long)0x8000000000000000ull));
+}
+// The largest of a warp's values (every lane, the result in all lanes).
+static __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, (uint32_t)(v >> 32));
+    const uint32_t lo =
+        __reduce_max_sync(0xffffffffu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0u);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
 // Bounds of the exact predicate as ordered integers.  For doubles >= +0 the
 // order of the values is the order of their bit patterns read as integers, so
 // the predicate compares d2 and |d| with integer instructions and leaves
