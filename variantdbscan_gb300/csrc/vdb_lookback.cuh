@@ -56,51 +56,83 @@ static __device__ __forceinline__ uint32_t lookback_ticket(LookState ls) {
     return s_ticket;
 }
 
-// Exclusive prefix of this thread's v over all tiles' threads (blocks of
-// kLookThreads; the first warp looks back, 32 tiles at a time).
+// One warp: what the tiles before this one add up to (every lane), all being
+// this tile's own sum; 32 tiles are looked at at a time.
+static __device__ __forceinline__ unsigned long long warp_lookback(unsigned long long all,
+                                                                   uint32_t tile,
+                                                                   unsigned long long* tiles,
+                                                                   DeviceStatus* st) {
+    const uint32_t lane = threadIdx.x & 31;
+    unsigned long long before = 0;
+    if (tile == 0) {
+        if (lane == 0) look_store(&tiles[0], kLookPrefix | all);
+        return 0;
+    }
+    if (lane == 0) look_store(&tiles[tile], kLookSum | all);
+    for (int64_t b = (int64_t)tile - 1; b >= 0; b -= 32) {
+        const int64_t i = b - (int64_t)lane;
+        const unsigned long long s = i >= 0 ? look_wait(&tiles[i], st) : kLookPrefix;
+        const uint32_t full = __ballot_sync(0xffffffffu, (s >> 62) == 2ull);
+        const uint32_t upto = full ? (uint32_t)__ffs(full) - 1u : 31u;
+        unsigned long long add = lane <= upto ? s & kLookMask : 0ull;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xffffffffu, add, d);
+        before += add;
+        if (full) break;
+    }
+    if (lane == 0) look_store(&tiles[tile], kLookPrefix | (before + all));
+    return before;
+}
+
+// Exclusive prefixes of this thread's K values v[] over all tiles' threads, in
+// place (blocks of kLookThreads).  Warp i looks back for value i, so that
+// several sums wait side by side.  (Once per kernel: the shared words are not
+// guarded against a second call.)
+template <int K>
+static __device__ __forceinline__ void block_lookbacks(unsigned long long (&v)[K], uint32_t tile,
+                                                       unsigned long long* const (&tiles)[K],
+                                                       DeviceStatus* st) {
+    static_assert(K <= kLookThreads / 32, "a warp for each value");
+    __shared__ unsigned long long s_sum[K][kLookThreads / 32];
+    __shared__ unsigned long long s_before[K];
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long incl[K];
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        incl[i] = v[i];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, incl[i], d);
+            if (lane >= (uint32_t)d) incl[i] += t;
+        }
+        if (lane == 31) s_sum[i][wid] = incl[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        if (wid != (uint32_t)i) continue;
+        unsigned long long all = 0;
+#pragma unroll
+        for (int w = 0; w < kLookThreads / 32; w++) all += s_sum[i][w];
+        const unsigned long long before = warp_lookback(all, tile, tiles[i], st);
+        if (lane == 0) s_before[i] = before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < K; i++) {
+        v[i] = s_before[i] + incl[i] - v[i];
+        for (uint32_t w = 0; w < wid; w++) v[i] += s_sum[i][w];
+    }
+}
+
+// The same for one value.
 static __device__ __forceinline__ unsigned long long block_lookback(unsigned long long v,
                                                                     uint32_t tile, LookState ls,
                                                                     DeviceStatus* st) {
-    __shared__ unsigned long long s_sum[kLookThreads / 32];
-    __shared__ unsigned long long s_before;
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();  // (a call before this one has read the shared words)
-    unsigned long long incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= (uint32_t)d) incl += t;
-    }
-    if (lane == 31) s_sum[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        unsigned long long all = 0;
-#pragma unroll
-        for (int w = 0; w < kLookThreads / 32; w++) all += s_sum[w];
-        unsigned long long before = 0;
-        if (tile == 0) {
-            if (lane == 0) look_store(&ls.tiles[0], kLookPrefix | all);
-        } else {
-            if (lane == 0) look_store(&ls.tiles[tile], kLookSum | all);
-            for (int64_t b = (int64_t)tile - 1; b >= 0; b -= 32) {
-                const int64_t i = b - (int64_t)lane;
-                const unsigned long long s = i >= 0 ? look_wait(&ls.tiles[i], st) : kLookPrefix;
-                const uint32_t full = __ballot_sync(0xffffffffu, (s >> 62) == 2ull);
-                const uint32_t upto = full ? (uint32_t)__ffs(full) - 1u : 31u;
-                unsigned long long add = lane <= upto ? s & kLookMask : 0ull;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xffffffffu, add, d);
-                before += add;
-                if (full) break;
-            }
-            if (lane == 0) look_store(&ls.tiles[tile], kLookPrefix | (before + all));
-        }
-        if (lane == 0) s_before = before;
-    }
-    __syncthreads();
-    unsigned long long r = s_before + incl - v;
-    for (uint32_t w = 0; w < wid; w++) r += s_sum[w];
-    return r;
+    unsigned long long k[1] = {v};
+    unsigned long long* const t[1] = {ls.tiles};
+    block_lookbacks<1>(k, tile, t, st);
+    return k[0];
 }
 
 // The last mark before this tile, by the same scheme (warp 0 of the block; the

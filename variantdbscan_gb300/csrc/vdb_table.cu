@@ -1714,6 +1714,80 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
     if (lane == 0 && my_retest) atomicAdd(&a.st->retested, my_retest);
 }
 
+// Candidate ranges [st[j], en[j]) of kRowBatch rows i0 + j of a tile at cells
+// cy, cx0 .. cx0 + G - 1.  The rows' loads, and in sparse grids the steps of
+// their searches, are side by side: one after the other they were most of the
+// tile-words pass.
+constexpr int kRowBatch = 5;
+__device__ __forceinline__ void tile_rows(const TableArgs& a, const EpsParams* __restrict__ ep,
+                                          int rho, int nrows, uint32_t cy, uint32_t cx0, int i0,
+                                          uint32_t (&st)[kRowBatch], uint32_t (&en)[kRowBatch]) {
+    uint32_t lo[kRowBatch], hi[kRowBatch];  // columns [lo, hi]
+    bool on[kRowBatch];
+#pragma unroll
+    for (int j = 0; j < kRowBatch; j++) {
+        const int i = i0 + j, ry = (int)cy + i - rho;
+        on[j] = i < nrows && ry >= 0 && ry < (int)a.g.ncy;
+        const int reach = on[j] ? ep->reach[i] : 0;
+        lo[j] = (uint32_t)max((int)cx0 - reach, 0);
+        hi[j] = (uint32_t)min((int)(cx0 + a.g.G - 1) + reach, (int)a.g.ncx - 1);
+        st[j] = en[j] = 0;
+    }
+    if (!a.g.sparse) {
+#pragma unroll
+        for (int j = 0; j < kRowBatch; j++) {
+            if (!on[j]) continue;
+            const uint32_t base = (uint32_t)((int)cy + i0 + j - rho) * a.g.ncx_pad;
+            st[j] = a.cell_start[base + lo[j]];
+            en[j] = a.cell_start[base + hi[j] + 1];
+        }
+    } else {
+        uint32_t b[kRowBatch], len[kRowBatch], re[kRowBatch];
+        bool left = false;
+#pragma unroll
+        for (int j = 0; j < kRowBatch; j++) {
+            const uint32_t ry = on[j] ? (uint32_t)((int)cy + i0 + j - rho) : 0u;
+            b[j] = a.crow[ry];
+            re[j] = a.crow[ry + 1];
+            len[j] = on[j] ? re[j] - b[j] : 0u;
+            left |= len[j] != 0u;
+        }
+        while (left) {
+            left = false;
+#pragma unroll
+            for (int j = 0; j < kRowBatch; j++) {
+                const uint32_t half = len[j] >> 1;
+                if (len[j]) {
+                    if (a.ccx[b[j] + half] < lo[j]) {
+                        b[j] += half + 1;
+                        len[j] -= half + 1;
+                    } else {
+                        len[j] = half;
+                    }
+                }
+                left |= len[j] != 0u;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kRowBatch; j++) {
+            if (!on[j]) continue;
+            uint32_t e = b[j];
+            if (hi[j] - lo[j] <= 16u)
+                while (e < re[j] && a.ccx[e] <= hi[j]) e++;
+            else
+                e = cx_lower_bound(a.ccx, e, re[j], hi[j] + 1);
+            st[j] = a.clist[b[j]];
+            en[j] = a.clist[e];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < kRowBatch; j++) {
+        if (!VDB_GUARD(a.st, st[j] <= en[j] && en[j] <= a.n, 2,
+                       ((unsigned long long)st[j] << 32) | en[j]))
+            st[j] = en[j] = 0;
+    }
+}
+
 // A thread per tile: its row segments (kept in trow_s/e where set), the words
 // of its test bitmap, ceil(C/32) per query, and its work units,
 // ceil(ceil(C/32) / unit_words); the offsets of both, and of the units that
@@ -1741,14 +1815,18 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
         const uint32_t cy = key0 / a.g.ncx_pad;
         const uint32_t cx0 = (key0 - cy * a.g.ncx_pad) / a.g.G * a.g.G;
         uint32_t c = 0;
-        for (int i = 0; i < nrows; i++) {
-            uint32_t st, len, base;
-            tile_row(a, ep, rho, cy, cx0, i, &st, &len, &base);
-            c += len;
-            if (a.trow_s) {
-                const unsigned long long k = (unsigned long long)t * (uint32_t)nrows + (uint32_t)i;
-                a.trow_s[k] = st;
-                a.trow_e[k] = st + len;
+        for (int i0 = 0; i0 < nrows; i0 += kRowBatch) {
+            uint32_t st[kRowBatch], en[kRowBatch];
+            tile_rows(a, ep, rho, nrows, cy, cx0, i0, st, en);
+#pragma unroll
+            for (int j = 0; j < kRowBatch; j++) {
+                c += en[j] - st[j];
+                if (a.trow_s && i0 + j < nrows) {
+                    const unsigned long long k =
+                        (unsigned long long)t * (uint32_t)nrows + (uint32_t)(i0 + j);
+                    a.trow_s[k] = st[j];
+                    a.trow_e[k] = en[j];
+                }
             }
         }
         const uint32_t tw = (c + 31u) >> 5;
@@ -1760,24 +1838,20 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
             w = 0;
         }
     }
-    const unsigned long long un =
-        block_lookback(nu | ((unsigned long long)nl << 31), tile, lu, a.st);
+    unsigned long long before[2] = {nu | ((unsigned long long)nl << 31), boff ? w : 0ull};
+    unsigned long long* const states[2] = {lu.tiles, lw.tiles};
+    block_lookbacks<2>(before, tile, states, a.st);
     if (t < ntiles) {
-        const uint32_t u0 = (uint32_t)(un & 0x7fffffffull), l0 = (uint32_t)(un >> 31);
+        const uint32_t u0 = (uint32_t)(before[0] & 0x7fffffffull), l0 = (uint32_t)(before[0] >> 31);
         uoff[t] = u0;
         loff[t] = l0;
+        if (boff) boff[t] = before[1];
         if (t == ntiles - 1) {
             uoff[ntiles] = u0 + nu;
             loff[ntiles] = l0 + nl;
             nunits[0] = u0 + nu;
             nunits[1] = l0 + nl;
-        }
-    }
-    if (boff) {
-        const unsigned long long b0 = block_lookback(w, tile, lw, a.st);
-        if (t < ntiles) {
-            boff[t] = b0;
-            if (t == ntiles - 1) *nwords = b0 + w;
+            if (boff) *nwords = before[1] + w;
         }
     }
 }
