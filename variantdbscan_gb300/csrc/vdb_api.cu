@@ -1141,10 +1141,16 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             g.sparse = g.ncells > 32ull * n + (1ull << 22) ? 1u : 0u;
             g.sub = isfinite(g.w) ? sub_bits(g.ncells) : 0u;
             const int kbits = bits_for(g.ncells - 1) + 2 * (int)g.sub;
-            launch_grid_keys(x, y, n, g, kbits, skey, (uint32_t*)gz.sort, s);
+            finish_eps(ep, g);
+            launch_grid_keys(x, y, n, g, kbits, skey, (uint32_t*)gz.sort, ep, d_ep, s);
             radix_sort(skey, n, kbits, 2 * (int)g.sub, gz.sort, scratch, gkey, gorig, nullptr, d_st, s);
+            // cells are cliques when two points of one cell always pass the
+            // distance test without a box check: 2 w^2 below thr and tbox
+            clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
+            if (clique && !cbest) cbest = ar.get<unsigned long long>(n);
             OrderArgs oa = order_args();
             oa.g = g;
+            oa.cbest = clique ? cbest : nullptr;
             launch_order(oa, gz.order, s);
             if (!g.sparse) {
                 if (g.ncells + 1 > cell_cap) {
@@ -1167,11 +1173,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 tile_cells_hist[lg]++;
             }
             const bool mixed = ep.mixed != 0;
-            // cells are cliques when two points of one cell always pass the
-            // distance test without a box check: 2 w^2 below thr and tbox
-            clique = isfinite(g.w) && 2.0 * g.w * g.w * (1.0 + 0x1p-20) <= std::min(ep.thr, ep.tbox);
-            finish_eps(ep, g);
-            launch_store_eps(d_ep, ep, s);
             const size_t tb = tm.mark();
 
             ta_args.g = g;
@@ -1282,6 +1283,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ta_args.ulist = ulist;
             ta_args.parts = no_rows ? nullptr : parts;
             ta_args.pair_sum = no_rows ? &d_st->pairs : nullptr;
+            if (mixed && n >= kBoxPoints) {
+                if (!wbox) wbox = ar.get<float4>((n + 3u) / 4u);
+                ta_args.wbox = wbox;
+            }
             launch_unit_list(ta_args, ulist, s);
             ta_args.bitmap = nullptr;
             ta_args.tile_boff = tboff;
@@ -1313,11 +1318,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 if (bitmap && bm_words <= bitmap_cap) ta_args.bitmap = bitmap;
             }
             if (recording && !no_rows) rec->put(ta_args.bitmap ? 1 : 0);
-            if (mixed && n >= kBoxPoints) {
-                if (!wbox) wbox = ar.get<float4>((n + 3u) / 4u);
-                ta_args.wbox = wbox;
-                launch_word_boxes(ta_args, s);
-            }
             size_t tc = 0;
             for (bool again = false;; again = true) {
                 if (again) {
@@ -1495,7 +1495,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 cells_buf = ar.get<uint32_t>(want * (3 * n8 + 2 * (size_t)nw));
                 cells_slots = want;
             }
-            if (!cbest) cbest = ar.get<unsigned long long>(n);
             const int nrows = 2 * ep.rho + 1;
             if ((size_t)n * nrows > crng_cap) {
                 if (crng) ar.put(crng);
@@ -2395,7 +2394,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     CK(cudaMemsetAsync(zc.base, 0, zc.used, s));
     const int kbits = bits_for(g.ncells - 1) + 2 * (int)g.sub;
     CK(cudaMemsetAsync(zeroed, 0, sort_zero_bytes(n, kbits), s));
-    launch_grid_keys(x, y, n, g, kbits, vkey, (uint32_t*)zeroed, s);
+    launch_grid_keys(x, y, n, g, kbits, vkey, (uint32_t*)zeroed, ep, d_ep, s);
     radix_sort(vkey, n, kbits, 2 * (int)g.sub, zeroed, scratch, gkey, gorig, nullptr, st, s);
     OrderArgs oa;
     memset(&oa, 0, sizeof oa);
@@ -2420,10 +2419,10 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     oa.tiles = tiles;
     oa.ptile = ptile;
     oa.ntiles = d_ntiles;
+    oa.cbest = clique ? cbest : nullptr;
     oa.st = st;
     launch_order(oa, gz.order, s);
     launch_cell_start(ckey, clist, cscan + n, n, g, cell_start, s);
-    CK(cudaMemcpyAsync(d_ep, &ep, sizeof ep, cudaMemcpyHostToDevice, s));
 
     TableArgs ta;
     memset(&ta, 0, sizeof ta);

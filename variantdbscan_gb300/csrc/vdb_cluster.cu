@@ -218,8 +218,7 @@ __global__ void resolve_kernel(ClusterArgs a, uint32_t* ws, uint32_t cap) {
 // returns their number (one block; nw: start_words).
 constexpr int kRankThreads = 1024;
 constexpr int kRankItems = 8;
-__device__ uint32_t rank_bits(const uint32_t* __restrict__ bits, uint32_t* __restrict__ rank,
-                              uint32_t nw) {
+__device__ uint32_t rank_bits(const uint32_t* bits, uint32_t* __restrict__ rank, uint32_t nw) {
     __shared__ uint32_t s_tot[32];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t carry = 0;
@@ -228,8 +227,9 @@ __device__ uint32_t rank_bits(const uint32_t* __restrict__ bits, uint32_t* __res
         uint32_t c[kRankItems], sum = 0;
         uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
         if (w0 < nw) {  // (nw is a multiple of kRankItems)
-            lo = reinterpret_cast<const uint4*>(bits + w0)[0];
-            hi = reinterpret_cast<const uint4*>(bits + w0)[1];
+            // (from L2: other blocks of this kernel may have set them)
+            lo = __ldcg(reinterpret_cast<const uint4*>(bits + w0));
+            hi = __ldcg(reinterpret_cast<const uint4*>(bits + w0) + 1);
         }
         c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w;
         c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
@@ -418,18 +418,27 @@ __device__ __forceinline__ uint32_t test_pair(const CellArgs& a, const PairTest&
 // exist instead of probing every offset.
 //
 // The middle row's threads also set the slots' start state: no seeds, no
-// cluster starts, every cell its own root in the first slot.
+// cluster starts, every cell its own root in the first slot; and each cell's
+// largest degree with its point (cbest, zero before).
 __global__ void cell_setup_kernel(CellArgs a) {
     pdl_sync();
     if (blockIdx.y == (uint32_t)a.ep->rho) {
         const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
         if (k < a.nw)
             for (int v = 0; v < a.m; v++) a.bits[(size_t)v * a.nw + k] = 0u;
-        if (k < a.n) {
-            a.cbest[k] = 0ull;
+        const bool in = k < a.n;
+        if (k < (uint32_t)a.m) a.st->starts_done[k] = 0u;
+        if (in) {
             if (!a.continued) a.parent[k] = k;
             for (int v = 0; v < a.m; v++) a.seed[(size_t)v * a.n + k] = kNone;
         }
+        const uint32_t c = in ? a.cscan[k + 1] - 1u : kNone;
+        const uint32_t d = in ? a.deg[k] : 0u;
+        const uint32_t same = __match_any_sync(kFull, c);
+        const uint32_t mx = __reduce_max_sync(same, d);
+        const uint32_t first = __reduce_min_sync(same, d == mx ? k : kNone);
+        if (in && first == k && VDB_GUARD(a.st, c < a.n, 15, c))
+            atomicMax(&a.cbest[c], ((unsigned long long)mx << 32) | (uint32_t)~k);
     }
     const uint32_t rho = (uint32_t)a.ep->rho;
     const uint32_t ncl = *a.ncl;
@@ -455,19 +464,6 @@ __global__ void cell_setup_kernel(CellArgs a) {
     }
     if (!VDB_GUARD(a.st, out.x <= out.y && out.y <= ncl, 16, out.y)) out = make_uint2(0u, 0u);
     a.crng[(size_t)r * a.n + c] = out;
-}
-
-__global__ void cell_best_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool in = k < a.n;
-    const uint32_t c = in ? a.cscan[k + 1] - 1u : kNone;
-    const uint32_t d = in ? a.deg[k] : 0u;
-    const uint32_t same = __match_any_sync(kFull, c);
-    const uint32_t mx = __reduce_max_sync(same, d);
-    const uint32_t first = __reduce_min_sync(same, d == mx ? k : kNone);
-    if (in && first == k && VDB_GUARD(a.st, c < a.n, 15, c))
-        atomicMax(&a.cbest[c], ((unsigned long long)mx << 32) | (uint32_t)~k);
 }
 
 // Hooks: a cell that has cores for the first time in slot v is a tree of its
@@ -819,28 +815,34 @@ __global__ void cell_resolve_kernel(CellArgs a, uint32_t* ws, uint32_t cap) {
 }
 
 // cst = visit position at which the cluster of the cell's cores starts (kNone:
-// no cores); the starts' bits (y: slot).
-__global__ void cell_starts_kernel(CellArgs a) {
+// no cores); the starts' bits (y: slot).  The slot's last block ranks the bits
+// and counts the clusters.
+__global__ void __launch_bounds__(kRankThreads) cell_starts_kernel(CellArgs a) {
     pdl_sync();
+    __shared__ bool s_last;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const int v = blockIdx.y;
-    if (c >= *a.ncl) return;
-    const size_t o = (size_t)v * a.n;
-    uint32_t s = kNone;
-    if (best_deg(a.cbest[c]) >= a.mp[v]) {
-        const uint32_t r = a.parent[o + c];
-        s = r < a.n ? a.seed[o + r] : kNone;
-        if (!VDB_GUARD(a.st, s < a.n, 12, s)) s = kNone;
-        else if (r == c) atomicOr(&a.bits[(size_t)v * a.nw + (s >> 5)], 1u << (s & 31u));
+    uint32_t* const bits = a.bits + (size_t)v * a.nw;
+    if (c < *a.ncl) {
+        const size_t o = (size_t)v * a.n;
+        uint32_t s = kNone;
+        if (best_deg(a.cbest[c]) >= a.mp[v]) {
+            const uint32_t r = a.parent[o + c];
+            s = r < a.n ? a.seed[o + r] : kNone;
+            if (!VDB_GUARD(a.st, s < a.n, 12, s)) s = kNone;
+            else if (r == c) atomicOr(&bits[s >> 5], 1u << (s & 31u));
+        }
+        a.cst[o + c] = s;
     }
-    a.cst[o + c] = s;
-}
-
-// The slots' ranks and numbers of clusters (one block per slot).
-__global__ void __launch_bounds__(kRankThreads) cell_rank_kernel(CellArgs a) {
-    pdl_sync();
-    const int v = blockIdx.x;
-    const uint32_t k = rank_bits(a.bits + (size_t)v * a.nw, a.brank + (size_t)v * a.nw, a.nw);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(&a.st->starts_done[v], 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t k = rank_bits(bits, a.brank + (size_t)v * a.nw, a.nw);
     if (threadIdx.x == 0 && k) atomicAdd(&a.st->clusters, (unsigned long long)k * a.copies[v]);
 }
 
@@ -1068,7 +1070,6 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     if (!a.n) return;
     const dim3 per_slot(nblk(a.n), (unsigned)a.m);
     launch(cell_setup_kernel, dim3(nblk(std::max(a.n, a.nw)), (unsigned)nrows), kThreads, s, a);
-    launch(cell_best_kernel, nblk(a.n), kThreads, s, a);
     launch(cell_hook_kernel, nblk(a.n), kThreads, s, a);
     for (int v = 0; v < a.m; v++) {
         launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, s, a, v);
@@ -1078,8 +1079,8 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     if (one_way) {
         launch(cell_resolve_kernel, a.m, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);
     }
-    launch(cell_starts_kernel, per_slot, kThreads, s, a);
-    launch(cell_rank_kernel, a.m, kRankThreads, s, a);
+    launch(cell_starts_kernel, dim3((a.n + kRankThreads - 1) / kRankThreads, (unsigned)a.m),
+           kRankThreads, s, a);
     launch(cell_labels_kernel, per_slot, kThreads, s, a);
 }
 

@@ -46,20 +46,11 @@ __global__ void graph_check_kernel(GraphCheck chk, uint32_t* bad,
     cudaGraphSetConditional(next, ok ? 1u : 0u);
 }
 
-__global__ void store_eps_kernel(EpsParams* dst, EpsParams v) {
-    pdl_sync();
-    if (threadIdx.x == 0 && blockIdx.x == 0) *dst = v;
-}
-
 }  // namespace
 
 void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphConditionalHandle next,
                         cudaStream_t s) {
     launch(graph_check_kernel, 1, 32, s, chk, bad, next);
-}
-
-void launch_store_eps(EpsParams* dst, const EpsParams& v, cudaStream_t s) {
-    launch(store_eps_kernel, 1, 32, s, dst, v);
 }
 
 }  // namespace vdb

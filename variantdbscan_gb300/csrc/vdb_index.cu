@@ -175,10 +175,12 @@ __device__ __forceinline__ uint32_t curve_index(uint32_t x, uint32_t y, uint32_t
 
 __global__ void __launch_bounds__(kThreads) grid_keys_kernel(
     const double* __restrict__ x, const double* __restrict__ y, uint32_t n, GridParams g,
-    uint32_t* __restrict__ keys, int passes, uint32_t* __restrict__ hist) {
+    uint32_t* __restrict__ keys, int passes, uint32_t* __restrict__ hist, EpsParams ep,
+    EpsParams* __restrict__ ep_out) {
     pdl_sync();
     __shared__ DigitCounts s_h;
     counts_clear(s_h, passes);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *ep_out = ep;
     const float iw = (float)(1.0 / g.w);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
@@ -291,6 +293,7 @@ __global__ void __launch_bounds__(kLookThreads) order_kernel(OrderArgs a, LookSt
                 a.tiles[t + ft] = a.n;
                 *a.ntiles = t + ft;
             }
+            if (a.cbest) a.cbest[k] = 0ull;
             gather_point(a, k, key[i]);
         }
         c0 += __popc(bc[i]);
@@ -418,9 +421,11 @@ void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, 
 }
 
 void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g, int bits,
-                      uint32_t* keys, uint32_t* hist, cudaStream_t s) {
+                      uint32_t* keys, uint32_t* hist, const EpsParams& ep, EpsParams* ep_out,
+                      cudaStream_t s) {
     if (!n) return;
-    launch(grid_keys_kernel, key_blocks(n), kThreads, s, x, y, n, g, keys, sort_passes(bits), hist);
+    launch(grid_keys_kernel, key_blocks(n), kThreads, s, x, y, n, g, keys, sort_passes(bits), hist,
+           ep, ep_out);
 }
 
 size_t order_state_bytes(uint32_t n) {

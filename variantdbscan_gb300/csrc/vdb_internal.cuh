@@ -86,6 +86,7 @@ struct DeviceStatus {
     uint32_t nunits, nlist;        // work units; those that warps take
     uint32_t ntiles;
     uint32_t asym_n;               // one-way pairs recorded
+    uint32_t starts_done[8];       // blocks done per slot of cell_starts_kernel
 };
 
 // Index guards: a data-derived index outside its array is recorded (site and
@@ -342,8 +343,10 @@ void launch_visit_keys(const double* x, const double* y, uint32_t n, const BBox*
                        uint32_t* keys, uint32_t* hist, DeviceStatus* st, cudaStream_t s);
 void launch_mpb_boxes(const double* x, const double* y, const uint32_t* vorder, uint32_t n,
                       int mbb, MpbBox* boxes, cudaStream_t s);
+// (the epsilon's parameters are left at ep_out for the kernels that follow)
 void launch_grid_keys(const double* x, const double* y, uint32_t n, GridParams g, int bits,
-                      uint32_t* keys, uint32_t* hist, cudaStream_t s);
+                      uint32_t* keys, uint32_t* hist, const EpsParams& ep, EpsParams* ep_out,
+                      cudaStream_t s);
 
 // The cell order's arrays: per point the coordinates (gxy, FP32 relative to
 // the own cell: glocal), visit position and multiple-point box; the non-empty
@@ -373,6 +376,7 @@ struct OrderArgs {
     uint32_t* tiles;
     uint32_t* ptile;
     uint32_t* ntiles;
+    unsigned long long* cbest;  // cleared (n words) for cell_setup_kernel; may be null
     DeviceStatus* st;
 };
 size_t order_state_bytes(uint32_t n);
@@ -409,7 +413,7 @@ struct TableArgs {
     const uint32_t* gkey;
     const float2* glocal;
     const double2* gxy;
-    float4* wbox;               // boxes of runs of points (launch_word_boxes), (n+3)/4; may be null
+    float4* wbox;               // boxes of runs of points (launch_unit_list), (n+3)/4; may be null
     const uint32_t* gpos;
     const MpbBox* gbox;         // multiple-point box of each cell-ordered point
     uint32_t n;
@@ -498,7 +502,6 @@ static __device__ __forceinline__ void walk_compact_row(
     }
 }
 void launch_count(const TableArgs& a, int nblocks, cudaStream_t s);
-void launch_word_boxes(const TableArgs& a, cudaStream_t s);
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s);
 size_t words_state_bytes(uint32_t n);
 void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
@@ -655,7 +658,6 @@ void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphCondition
                         cudaStream_t s);
 // *dst = v by a kernel (a captured host-to-device copy would read the host
 // buffer at replay time).
-void launch_store_eps(EpsParams* dst, const EpsParams& v, cudaStream_t s);
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s);
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s);
 void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, cudaStream_t s);

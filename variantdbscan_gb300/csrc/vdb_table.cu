@@ -193,9 +193,7 @@ constexpr uint32_t kLaneCand = 16;
 // a box wholly inside or outside eps settles 64 x 32 pairs without a test.
 constexpr uint32_t kBoxCand = 2048;
 constexpr uint32_t kBoxRun = 36;
-__global__ void word_boxes_kernel(TableArgs a) {
-    pdl_sync();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void word_box(const TableArgs& a, uint32_t i) {
     const uint32_t k0 = 4u * i;
     if (k0 >= a.n) return;
     const uint32_t key0 = a.gkey[k0], cy0 = key0 / a.g.ncx_pad;
@@ -1857,12 +1855,18 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
 }
 
 // ulist: (unit, tile) of the units that warps take: a thread per tile, long
-// lists by the whole warp.
-__global__ void unit_list_kernel(TableArgs a, uint2* ulist) {
+// lists by the whole warp.  The first blocks make the word boxes (where there
+// are any), which would have no use for a launch of their own.
+__global__ void __launch_bounds__(kTT) unit_list_kernel(TableArgs a, uint2* ulist,
+                                                        uint32_t box_blocks) {
     pdl_sync();
+    if (blockIdx.x < box_blocks) {
+        word_box(a, blockIdx.x * kTT + threadIdx.x);
+        return;
+    }
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ntiles = *a.ntiles;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = (blockIdx.x - box_blocks) * kTT + threadIdx.x;
     if (t - lane >= ntiles) return;  // (whole warps)
     uint32_t b = 0, e = 0, u0 = 0;
     if (t < ntiles) {
@@ -2060,11 +2064,6 @@ void launch_count(const TableArgs& a, int nblocks, cudaStream_t s) {
         launch(count_kernel<false>, nblocks, kWPB * 32, s, a);
 }
 
-void launch_word_boxes(const TableArgs& a, cudaStream_t s) {
-    const uint32_t nb = (a.n + 3u) / 4u;
-    launch(word_boxes_kernel, (nb + kTT - 1) / kTT, kTT, s, a);
-}
-
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s) {
     if (a.mixed)
         launch(table_kernel<true, true>, nblocks, kTT, s, a);
@@ -2087,7 +2086,8 @@ void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* u
 
 void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s) {
     if (!a.n) return;
-    launch(unit_list_kernel, (a.n + kTT - 1) / kTT, kTT, s, a, ulist);
+    const uint32_t boxes = a.wbox ? ((a.n + 3u) / 4u + kTT - 1) / kTT : 0u;
+    launch(unit_list_kernel, boxes + (a.n + kTT - 1) / kTT, kTT, s, a, ulist, boxes);
 }
 
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s) {
