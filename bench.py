@@ -54,7 +54,7 @@ def parse():
     p.add_argument("--no-reuse-compare", action="store_true",
                    help="skip the measurement without reuse across variants")
     p.add_argument("--no-labels-only", action="store_true",
-                   help="skip the labels-only measurement (border rows of the tables)")
+                   help="skip the labels-only measurement (only the table rows that the labelling reads)")
     p.add_argument("--serving-table", default="border", choices=["border", "all"],
                    help="table rows written by the serving workload's requests")
     p.add_argument("--entry-bytes", type=int, default=0, choices=[0, 2, 4],
@@ -62,9 +62,9 @@ def parse():
     p.add_argument("--streams", type=int, default=0,
                    help="concurrent dataset streams of the library (0: autotuned)")
     p.add_argument("--tile-cells", type=int, default=0,
-                   help="grid cells per tile group (0: autotuned per table)")
+                   help="grid cells per tile group (0: by the library's rule)")
     p.add_argument("--compare-fixed", action="store_true",
-                   help="also time the step with the untuned shapes (one-cell tiles, "
+                   help="also time the step with fixed shapes (one-cell tiles, "
                         "min(4, datasets) streams); on by default for --workload multi")
     p.add_argument("--unit-candidates", type=int, default=0, choices=[0, 1024, 2048, 4096],
                    help="candidates per work unit (0: by dataset size)")
@@ -379,7 +379,8 @@ def run_ours(args):
     # inner loop, 4.5 warp-instruction lanes per test (per 2 candidates and
     # query: 2 fma.f32x2, 2 sub.f32x2, 4 funnel shifts; 2 shared loads per
     # 4 tests), i.e. 32 / 4.5 tests per warp-instruction, 4 warp-instructions
-    # per cycle per SM
+    # per cycle per SM.  Pairs that the kernel settles by the boxes of whole
+    # words, without that loop, count as tests: the fraction can pass 1
     nsm = torch.cuda.get_device_properties(local).multi_processor_count
     sm_hz = (clk or {}).get("sm_mhz", 2070.0) * 1e6
     count_s = sum(s["ms_count"] for s in stats) / len(stats) / 1e3
@@ -405,7 +406,7 @@ def run_ours(args):
                    "precision": "mixed (FP32 filter, FP64 band re-test)",
                    "schedule": "batched (tables shared per eps; union-find chained over "
                                "minpts; larger-eps components prune cell-pair searches)",
-                   "table_entries": {"compact": "16-bit (position within a 4096-candidate work unit)",
+                   "table_entries": {"compact": "16-bit (position within a work unit of 512 to 4096 candidates)",
                                      "wide": "32-bit (cell-ordered index)"}.get(entry, "mixed"),
                    "l2": "flushed between steps (256 MB write)",
                    "parallelism": f"replicas x{world}"},
@@ -472,7 +473,7 @@ def run_ours(args):
 
     if args.compare_fixed or (args.workload == "multi" and args.tile_cells == 0
                               and args.streams == 0):
-        # the untuned shapes: one-cell tiles everywhere, min(4, datasets) streams
+        # fixed shapes: one-cell tiles everywhere, min(4, datasets) streams
         fixed = dict(tile_cells=1, streams=min(4, len(dss)))
         step(**fixed)
         ms_f = []

@@ -3,8 +3,9 @@
 // Per dataset: bounding box, the reference's visit order and multiple-point
 // boxes (shared by all variants), then per group of variants with the same
 // epsilon: the grid, the count pass, the CSR neighbour table (whole, or in
-// row chunks when it exceeds the memory budget) and, for each minpts of the
-// group, union-find and labelling from scratch.  Several datasets of one call
+// row chunks when it exceeds the memory budget) and the labelling of all
+// minpts of the group: over cells, which reads no table, or, on grids whose
+// cells are no cliques, one union-find over points for each.  Several datasets of one call
 // run concurrently on worker streams.
 #include <float.h>
 #include <math.h>

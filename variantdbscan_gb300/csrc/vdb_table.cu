@@ -3,12 +3,15 @@
 // table written from that bitmap).
 //
 // Work is split into units: a tile is up to 64 consecutive cell-ordered points
-// of one cell; its candidates are the points of the cells within reach in the
+// (32 in small inputs) of one group of cells; its candidates are the points of the cells within reach in the
 // rows cy-rho..cy+rho, i.e. 2*rho+1 contiguous ranges of the cell-ordered
 // arrays; a unit is one tile and one chunk of unit_words*32 of its
 // candidates.  Persistent warps take units from a global counter; each warp
-// holds one tile's queries (lane l: queries l and l+32) and stages its
-// candidates in its own slice of shared memory.
+// holds one tile's queries and stages its candidates in its own slice of shared
+// memory.  Tiles of more than kLaneCand queries are tested lane = query (lane l:
+// queries l and l+32), the others and all FP64 tests lane = candidate, and
+// tiles of a few queries and candidates by a thread per point.  Tiles of
+// thousands of candidates first compare the candidates' boxes, word by word.
 //
 // The neighbour predicate is the reference's (src/DBScan.cpp:665-702 with the
 // R-tree candidate rule of src/RTree.h:1613-1625):
@@ -26,8 +29,10 @@
 // per 32 consecutive candidates (bit j: candidate j is a neighbour), laid out
 // [word][query] so that a warp's 32 queries store 128 contiguous bytes.  The
 // table pass turns each word into table entries (lane = bit), in candidate
-// order, so every row comes out sorted.  An entry is 16 bits (the neighbour's
-// position within its work unit of 1024 to 4096 candidates; readers decode it
+// order: rows of 32-bit entries come out sorted, rows of 16-bit entries unit
+// after unit, within a unit first the words that were expanded, then the runs
+// of words that are neighbours as a whole.  An entry is 16 bits (the neighbour's
+// position within its work unit of 512 to 4096 candidates; readers decode it
 // through the tile's row segments and the count pass's per-unit counts) or 32 bits (the
 // cell-ordered index).  Entries accepted in one direction only are flagged
 // afterwards from the asymmetric-pair list.  When the bitmap does not fit in
@@ -1213,7 +1218,10 @@ __device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* sl
     }
 }
 
-// 16-bit tables: two queries per pass.  The round's words are transposed
+// 16-bit tables.  The count pass flags the words that are outside eps of the
+// whole tile (skipped here) and those inside it (runs of three or more are
+// copied from staged runs of ids, full_round); the others are packed into
+// rounds of 16 words.  Two queries per pass: the round's words are transposed
 // into the query slots as above (lane = query); then lanes 0-15 expand one
 // query of a pair and lanes 16-31 the other, lane j of a half taking bits j
 // and j + 16 of every word.  The work of a query that does not depend on its
@@ -1225,7 +1233,10 @@ __device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* sl
 // 16-bit entries need only the tile's candidate count), 8 blocks of 3 warps
 // (80 registers, 26.4 KB of shared memory) share an SM; the extra warps hide
 // more of the kernel's dependency latency (2M sweep: 34.7 ms of tables against
-// 40.3 with two buffers per half at 6 blocks).
+// 40.3 with two buffers per half at 6 blocks).  Bound by the issue of shared
+// stores where most words are mixed, by the table's writes where most are
+// whole: 1M sweep, eps 0.1 / 0.2 / 0.4 / 0.8: 0.26 / 0.53 / 1.10 / 2.67 ms, 1.0
+// to 4.7 TB/s of entries (eps 0.8 3.24 ms before the runs were copied).
 __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     pdl_sync();
     using E = uint16_t;
@@ -1977,8 +1988,9 @@ __global__ void plan_chunks_kernel(const uint32_t* __restrict__ tiles,
 }
 
 // Flags the table entries accepted in one direction only (the count pass
-// recorded them): b in row a when dir == 1, a in row b when dir == 2.  Rows are
-// sorted by neighbour index.
+// recorded them): b in row a when dir == 1, a in row b when dir == 2.  Rows of
+// 32-bit entries are sorted; of a unit's 16-bit entries those before its runs
+// of whole words are (a one-way pair is never in a run).
 __global__ void asym_flags_kernel(TableArgs a) {
     pdl_sync();
     uint32_t na = *a.asym_n;
