@@ -404,8 +404,8 @@ def run_ours(args):
         "data": "synthetic (seeded Gaussian blobs + uniform background)",
         "config": {"workload": desc,
                    "precision": "mixed (FP32 filter, FP64 band re-test)",
-                   "schedule": "batched (tables shared per eps; union-find chained over "
-                               "minpts; larger-eps components prune cell-pair searches)",
+                   "schedule": "batched (tables shared per eps, whose minpts are labelled "
+                               "together; larger-eps components prune cell-pair searches)",
                    "table_entries": {"compact": "16-bit (position within a work unit of 512 to 4096 candidates)",
                                      "wide": "32-bit (cell-ordered index)"}.get(entry, "mixed"),
                    "l2": "flushed between steps (256 MB write)",

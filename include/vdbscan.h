@@ -111,12 +111,12 @@ typedef struct {
                                table bytes); 4 = 32 bits (the cell-ordered index);
                                0 = 16 bits with VDB_TABLE_ALL, 32 with VDB_TABLE_BORDER */
     int32_t no_reuse;       /* nonzero: label every variant from scratch.  By default
-                               (batched schedule) a variant's union-find starts from the
-                               components of the larger minpts before it at the same
-                               epsilon, and cell pairs whose cores lie in different
+                               (batched schedule) cell pairs whose cores lie in different
                                components at a larger epsilon (and a smaller or equal
-                               minpts) are not searched: both only save work, the labels
-                               are those of a from-scratch run */
+                               minpts) are not searched, and on grids whose cells are no
+                               cliques a variant's union-find starts from the components
+                               of the larger minpts before it at the same epsilon: both
+                               only save work, the labels are those of a from-scratch run */
     int32_t tile_cells;     /* grid cells per tile group of the neighbour search (1 to 64);
                                0 = the library's choice: 2 on grids of more than two cells
                                per point, else 1 */

@@ -421,7 +421,7 @@ struct Options {
     int table_rows = VDB_TABLE_ALL;
     int table_hash = 0;
     int entry_bytes = 0;  // 0 / 2: compact entries where they fit; 4: always 32-bit
-    bool reuse = true;    // labellings start from earlier variants' components
+    bool reuse = true;    // labellings use earlier variants' components
     int tile_cells = 0;   // cells per tile group G; 0 = default_tile_cells
     int unit_words = 0;   // work-unit size in bitmap words; 0 = by dataset size
     bool graph = false;   // repeated calls replayed as one CUDA graph
@@ -1529,7 +1529,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 ca.cscan = cscan;
                 ca.cbest = cbest;
                 ca.m = (int)std::min<size_t>(slots.size() - s0, kSlots);
-                ca.chain = o.reuse ? 1 : 0;
                 ca.parent = cells_buf;
                 ca.seed = cells_buf + cells_slots * n8;
                 ca.cst = cells_buf + 2 * cells_slots * n8;
@@ -1548,12 +1547,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                     ca.comp_prev[v] = comp_source(mp);
                 }
                 for (int v = 0; v < ca.m; v++) ca.comp_out[v] = comp_dest(slots[s0 + v].second);
-                if (s0 > 0 && ca.chain) {
-                    // go on from the last slot before
-                    CK(cudaMemcpyAsync(ca.parent, ca.parent + (size_t)(kSlots - 1) * n,
-                                       (size_t)n * 4, cudaMemcpyDeviceToDevice, s));
-                    ca.continued = 1;
-                }
                 launch_cells(ca, nrows, group_asym != 0, cells_ws, s);
                 CK(cudaGetLastError());
             }

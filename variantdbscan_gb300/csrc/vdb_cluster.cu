@@ -418,8 +418,8 @@ __device__ __forceinline__ uint32_t test_pair(const CellArgs& a, const PairTest&
 // exist instead of probing every offset.
 //
 // The middle row's threads also set the slots' start state: no seeds, no
-// cluster starts, every cell its own root in the first slot; and each cell's
-// largest degree with its point (cbest, zero before).
+// cluster starts; and each cell's largest degree with its point (cbest, zero
+// before).
 __global__ void cell_setup_kernel(CellArgs a) {
     pdl_sync();
     if (blockIdx.y == (uint32_t)a.ep->rho) {
@@ -429,7 +429,6 @@ __global__ void cell_setup_kernel(CellArgs a) {
         const bool in = k < a.n;
         if (k < (uint32_t)a.m) a.st->starts_done[k] = 0u;
         if (in) {
-            if (!a.continued) a.parent[k] = k;
             for (int v = 0; v < a.m; v++) a.seed[(size_t)v * a.n + k] = kNone;
         }
         const uint32_t c = in ? a.cscan[k + 1] - 1u : kNone;
@@ -466,23 +465,32 @@ __global__ void cell_setup_kernel(CellArgs a) {
     a.crng[(size_t)r * a.n + c] = out;
 }
 
-// Hooks: a cell that has cores for the first time in slot v is a tree of its
-// own and nobody else writes its parent, so it can be hung under an earlier
-// cell without atomics: under the first cell of the run of joined cells that
-// it ends (within the warp), else under a joined cell of the row before.
-// Returns cell c's parent (whole warps; old: its parent so far).
-__device__ __forceinline__ uint32_t hook_parent(const CellArgs& a, const PairTest& t, uint32_t c,
-                                                bool in, uint32_t mp, uint32_t mp_before,
-                                                uint32_t old) {
-    const uint32_t lane = threadIdx.x & 31;
+// Hooks (y: slot): at the start every cell is a tree of its own and nobody else
+// writes its parent, so it can be hung under an earlier cell without atomics:
+// under the first cell of the run of joined cells that it ends (within the
+// warp), else under a joined cell of the row before.
+//
+// The slots do not build on one another.  A slot could start from the
+// components of the one before (its minpts is smaller), but the hooks find most
+// of them again, and the slots' kernels, each too small to fill the chip below
+// 10^5 points, run as one launch (clustering of 60k points, 4 minpts of one
+// epsilon, 138 -> 84 us; 2M points 564 -> 570).
+__global__ void cell_hook_kernel(CellArgs a) {
+    pdl_sync();
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t ncl = *a.ncl;
+    if (c - lane >= ncl) return;  // (whole warps)
+    const bool in = c < ncl;
+    const PairTest t = pair_test(a);
+    const uint32_t mp = a.mp[blockIdx.y];
     const int rho = a.ep->rho;
     const unsigned long long bA = in ? a.cbest[c] : 0ull;
     const uint32_t ku = best_point(bA);
-    const bool fresh = in && best_deg(bA) >= mp && best_deg(bA) < mp_before && ku < a.n;
+    const bool core = in && best_deg(bA) >= mp && ku < a.n;
     bool left = false;
     int cx = 0;
     float2 pu = make_float2(0.f, 0.f);
-    if (fresh) {
+    if (core) {
         cx = (int)a.ccx[c];
         pu = a.glocal[ku];
         if (c > 0) {
@@ -494,39 +502,29 @@ __device__ __forceinline__ uint32_t hook_parent(const CellArgs& a, const PairTes
         }
     }
     const uint32_t heads = ~__ballot_sync(kFull, left);
-    if (!fresh) return old;
+    uint32_t p = c;
     if (left) {
         // the run's first cell in this warp, or the cell before the warp's
         const uint32_t upto = heads & ((2u << lane) - 1u);
-        return upto ? c - lane + 31u - (uint32_t)__clz((int)upto) : c - lane - 1u;
-    }
-    if (rho >= 1) {
+        p = upto ? c - lane + 31u - (uint32_t)__clz((int)upto) : c - lane - 1u;
+    } else if (core && rho >= 1) {
         const uint2 rg = a.crng[(size_t)(rho - 1) * a.n + c];
-        for (uint32_t o = rg.x; o < rg.y; o++) {
+        for (uint32_t o = rg.x; o < rg.y && p == c; o++) {
             const int dx = (int)a.ccx[o] - cx;
             const unsigned long long bB = a.cbest[o];
             const uint32_t kv = best_point(bB);
             if (dx >= -1 && dx <= 1 && o < c && best_deg(bB) >= mp && kv < a.n &&
                 test_pair(a, t, ku, kv, pu, a.glocal[kv], dx, -1) == 3u)
-                return o;
+                p = o;
         }
     }
-    return old;
-}
-
-__global__ void cell_hook_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    const uint32_t ncl = *a.ncl;
-    if (c - lane >= ncl || a.continued) return;  // (whole warps)
-    const uint32_t p = hook_parent(a, pair_test(a), c, c < ncl, a.mp[0], kNone, c);
-    if (c < ncl) a.parent[c] = p;
+    if (in) a.parent[(size_t)blockIdx.y * a.n + c] = p;
 }
 
 constexpr uint32_t kLanePairs = 4;     // cells of at most so many point pairs: one lane
 constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes over the pairs
 
-// Unions of slot v: every pair of cells within reach whose roots differ is
+// Unions (z: slot): every pair of cells within reach whose roots differ is
 // searched for one core-core pair accepted in both directions.  A lane takes a
 // cell and one row of its half neighbourhood: it screens the roots and tests
 // the cells' points of largest degree (and all pairs of next to empty cells);
@@ -536,8 +534,9 @@ constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes
 // the cheap unions few are left.  The clustering of the 2M sweep at eps 0.2 took
 // 0.88 ms with the cheap unions and a flatten as kernels before it, 0.67 like
 // this; 1M uniform points at eps 0.05 0.50 -> 0.41 ms.
-__global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a, int v) {
+__global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a) {
     pdl_sync();
+    const int v = blockIdx.z;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t ncl = *a.ncl;
     const uint32_t mp = a.mp[v];
@@ -568,14 +567,18 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a, int
         }
     }
     // A row's cells are screened at once (their loads overlap): those with
-    // cores and another parent, as far as it is known, stay in `left`.
+    // cores that are not, as far as two steps up their tree show, in the cell's
+    // own tree stay in `left`.
     uint32_t left = 0;
     const uint32_t o0 = o;
     {
-        const uint32_t pc = c < ncl ? parent[c] : 0u;
+        const uint32_t root = o < oe ? uf_find(parent, c) : 0u;
 #pragma unroll 5
-        for (uint32_t j = 0; j < (o < oe ? min(oe - o, 32u) : 0u); j++)
-            if (best_deg(a.cbest[o + j]) >= mp && parent[o + j] != pc) left |= 1u << j;
+        for (uint32_t j = 0; j < (o < oe ? min(oe - o, 32u) : 0u); j++) {
+            if (best_deg(a.cbest[o + j]) < mp) continue;
+            const uint32_t p1 = parent[o + j];
+            if (p1 != root && parent[p1] != root) left |= 1u << j;
+        }
     }
     // Every lane takes the cells left in its row: the cells' points of largest
     // degree first, which in dense regions mostly pair, or all points of next
@@ -709,24 +712,13 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a, int
     if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
 }
 
-// Roots of slot v, which are also the next slot's start: a smaller minpts keeps
-// every core and every connection, and its new cells are hooked.
-__global__ void cell_flatten_kernel(CellArgs a, int v) {
+// The cells' roots (y: slot).
+__global__ void cell_flatten_kernel(CellArgs a) {
     pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-    const uint32_t ncl = *a.ncl;
-    if (c - lane >= ncl) return;  // (whole warps)
-    uint32_t* parent = a.parent + (size_t)v * a.n;
-    uint32_t r = 0;
-    if (c < ncl) {
-        r = uf_find_ro(parent, c);
-        parent[c] = r;
-    }
-    if (v + 1 < a.m) {
-        const uint32_t p = hook_parent(a, pair_test(a), c, c < ncl, a.mp[v + 1],
-                                       a.chain ? a.mp[v] : kNone, a.chain ? r : c);
-        if (c < ncl) parent[a.n + c] = p;
-    }
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= *a.ncl) return;
+    uint32_t* parent = a.parent + (size_t)blockIdx.y * a.n;
+    parent[c] = uf_find_ro(parent, c);
 }
 
 // seed[root] = first visit position among the component's cores (y: slot).
@@ -1070,11 +1062,10 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     if (!a.n) return;
     const dim3 per_slot(nblk(a.n), (unsigned)a.m);
     launch(cell_setup_kernel, dim3(nblk(std::max(a.n, a.nw)), (unsigned)nrows), kThreads, s, a);
-    launch(cell_hook_kernel, nblk(a.n), kThreads, s, a);
-    for (int v = 0; v < a.m; v++) {
-        launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1)), kThreads, s, a, v);
-        launch(cell_flatten_kernel, nblk(a.n), kThreads, s, a, v);
-    }
+    launch(cell_hook_kernel, per_slot, kThreads, s, a);
+    launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1), (unsigned)a.m), kThreads,
+           s, a);
+    launch(cell_flatten_kernel, per_slot, kThreads, s, a);
     launch(cell_seed_kernel, per_slot, kThreads, s, a);
     if (one_way) {
         launch(cell_resolve_kernel, a.m, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);

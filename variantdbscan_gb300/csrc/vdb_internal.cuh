@@ -598,8 +598,6 @@ struct CellArgs {
     const uint32_t* cscan;      // cell of point k: cscan[k + 1] - 1
     unsigned long long* cbest;  // per cell: largest degree and a point that has it (n entries)
     int m;                      // slots
-    int chain;                  // nonzero: a slot starts from the components of the one before
-    int continued;              // nonzero: parent of slot 0 holds such a start already
     uint32_t mp[kSlots];        // minpts (0xffffffff: no cores)
     uint32_t copies[kSlots];    // variants that get the slot's labels
     // nested-epsilon reuse: comp_prev[v][pos] = component (its cluster start)
