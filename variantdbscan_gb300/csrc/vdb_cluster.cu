@@ -712,24 +712,23 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a) {
     if (lane == 0 && skipped) atomicAdd(&a.st->reuse_skips, (unsigned long long)skipped);
 }
 
-// The cells' roots (y: slot).
-__global__ void cell_flatten_kernel(CellArgs a) {
-    pdl_sync();
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= *a.ncl) return;
-    uint32_t* parent = a.parent + (size_t)blockIdx.y * a.n;
-    parent[c] = uf_find_ro(parent, c);
-}
-
-// seed[root] = first visit position among the component's cores (y: slot).
+// Roots, and seed[root] = first visit position among the component's cores (y:
+// slot).  Each core walks up its cell's tree, in a few steps that its
+// neighbours in cell order share; the cell's first point leaves the root.
 __global__ void cell_seed_kernel(CellArgs a) {
     pdl_sync();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     const int v = blockIdx.y;
-    if (k >= a.n || a.deg[k] < a.mp[v]) return;
-    const uint32_t c = a.cscan[k + 1] - 1u;
+    if (k >= a.n) return;
+    const bool core = a.deg[k] >= a.mp[v];
+    const uint32_t before = a.cscan[k], c = a.cscan[k + 1] - 1u;
+    const bool first = before == c;  // of its cell
+    if (!core && !first) return;
     if (!VDB_GUARD(a.st, c < a.n, 16, c)) return;
-    const uint32_t r = a.parent[(size_t)v * a.n + c];
+    uint32_t* parent = a.parent + (size_t)v * a.n;
+    const uint32_t r = uf_find_ro(parent, c);
+    if (first) parent[c] = r;
+    if (!core) return;
     // neighbours in cell order mostly share a root: one atomic per root and warp
     const uint32_t same = __match_any_sync(__activemask(), r);
     const uint32_t mn = __reduce_min_sync(same, a.gpos[k]);
@@ -1065,7 +1064,6 @@ void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
     launch(cell_hook_kernel, per_slot, kThreads, s, a);
     launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1), (unsigned)a.m), kThreads,
            s, a);
-    launch(cell_flatten_kernel, per_slot, kThreads, s, a);
     launch(cell_seed_kernel, per_slot, kThreads, s, a);
     if (one_way) {
         launch(cell_resolve_kernel, a.m, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);
