@@ -107,3 +107,11 @@ def test_boxes_of_signed_coordinates(ctx, vdb, orc, n, shift):
         x[-1] = bad
         with pytest.raises(vdb.VDBError):
             ctx.run([vdb.BatchItem(x, y, eps, mp, 70)])
+
+
+@pytest.mark.parametrize("n", [262144, 262145, 786432, 786433])
+def test_sort_tiles(ctx, vdb, orc, n):
+    # the sizes at which the sorts change their tiles
+    rng = np.random.default_rng(n)
+    x, y = rng.uniform(0, 40, n), rng.uniform(0, 40, n)
+    _check(ctx, vdb, orc, x, y, np.array([0.03, 0.02]), np.array([3, 2], np.uint32))

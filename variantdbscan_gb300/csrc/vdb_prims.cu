@@ -167,8 +167,11 @@ __global__ void __launch_bounds__(kDigits) radix_pass_kernel(
 }
 
 // Keys per thread: short tiles for small sorts, so that they spread over the
-// chip (50k keys: 49 tiles of 1,024 instead of 13 of 4,096).
-int sort_items(uint32_t n) { return n <= (1u << 18) ? 2 : n <= (1u << 20) ? 8 : 16; }
+// chip (50k keys: 49 tiles of 1,024 instead of 13 of 4,096), long ones where
+// they still fill it.  Index of one epsilon (five passes), us, with 2 / 4 / 8 / 16
+// keys: 130k points 123 / 124 / 127 / 150, 262k 160 / 158 / 162 / 171, 524k 199 / 188
+// / 207 / 201, 800k 253 / 232 / 236 / 226, 1M 294 / 269 / 259 / 246.
+int sort_items(uint32_t n) { return n <= (1u << 18) ? 2 : n <= (3u << 18) ? 4 : 16; }
 
 template <int ITEMS>
 void run_pass(uint32_t nb, const uint32_t* keys_in, const uint2* in, uint2* out, uint32_t* okeys,
@@ -212,7 +215,7 @@ void radix_sort(const uint32_t* keys, uint32_t n, int bits, int drop, void* zero
         const uint32_t* kin = i == 0 ? keys : nullptr;
         const uint2* in = i == 0 ? nullptr : buf[(i - 1) & 1];
         uint2* out = last ? nullptr : buf[i & 1];
-        auto pass = items == 2 ? run_pass<2> : items == 8 ? run_pass<8> : run_pass<16>;
+        auto pass = items == 2 ? run_pass<2> : items == 4 ? run_pass<4> : run_pass<16>;
         pass(nb, kin, in, out, last ? okeys : nullptr, last ? ovals : nullptr, last ? oinv : nullptr,
              n, i * kDigitBits, last ? drop : 0, hist + (size_t)i * kDigits,
              state + (size_t)i * nb * kDigits, ticket + i, st, s);
