@@ -329,6 +329,7 @@ void finish_eps(EpsParams& p, const GridParams& g) {
     p.xb.ax = ordered(sqrt(p.tbox));
     p.wf = (float)g.w;
     p.near2 = (float)(p.eps * p.eps * (1.0 + 0x1p-8));
+    p.iw = (float)(1.0 / g.w);
 }
 
 // Distance-test parameters of eps on grid g.  Cells (i, j) relative to a query

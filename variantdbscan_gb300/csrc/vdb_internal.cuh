@@ -195,6 +195,7 @@ struct EpsParams {
     ExactBounds xb; // of eps, thr and tbox
     float wf;       // the cells' width, FP32
     float near2;    // eps^2 (1 + 2^-8), FP32
+    float iw;       // 1 / the cells' width, FP32
     float lo32;     // FP32 d2 < lo32: neighbour (no FP64 re-test)
     float hi32;     // FP32 d2 > hi32: not a neighbour
     // count pass filter on the quadratic form nS = |c|^2/2 + (|q|^2 - L32)/2 - q.c

@@ -42,6 +42,15 @@ __global__ void __launch_bounds__(kLookThreads) scan_kernel(const uint32_t* __re
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) sum += v[i];
     unsigned long long run = block_lookback(sum, tile, ls, st);
+    if (base + kScanItems < n) {
+        // (out is 16-byte aligned: whole sectors at a time)
+#pragma unroll
+        for (int i = 0; i < kScanItems; i += 2) {
+            reinterpret_cast<ulonglong2*>(out + base)[i / 2] = make_ulonglong2(run, run + v[i]);
+            run += (unsigned long long)v[i] + v[i + 1];
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         if (base + i < n) out[base + i] = run;
