@@ -72,25 +72,28 @@ __global__ void __launch_bounds__(kThreads) visit_keys_kernel(
         s_f[threadIdx.x] = (float)((double)kVisitBins / w);
     }
     counts_clear(s_h, passes);
-    auto bin = [&](double v, int axis) {
+    // (bins as integers: compared and converted as doubles they took 26 us of the
+    // FP64 pipe's time at 2M points, 7 at 1M)
+    constexpr uint32_t kNoBin = 0xffffffffu;
+    auto bin = [&](double v, int axis) -> uint32_t {
         const double a = __dadd_rn(v, s_p[2 + axis]);
         const float r = (float)a * s_f[axis];
         bool sure;
         const float f = floor_if_sure(r, 1e-3f, &sure);
-        if (sure && factor_ok(s_f[axis]) && f >= 0.0f && f <= (float)(kVisitBins - 1)) return (double)f;
-        return floor(__dmul_rn(__ddiv_rn(a, s_p[axis]), (double)kVisitBins));
+        if (sure && factor_ok(s_f[axis]) && f >= 0.0f && f <= (float)(kVisitBins - 1))
+            return (uint32_t)f;
+        const double b = floor(__dmul_rn(__ddiv_rn(a, s_p[axis]), (double)kVisitBins));
+        return b >= 0.0 && b <= (double)(kVisitBins - 1) ? (uint32_t)b : kNoBin;
     };
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        double fx = bin(x[i], 0), fy = bin(y[i], 1);
-        const bool ok = fx >= 0.0 && fx <= (double)(kVisitBins - 1) && fy >= 0.0 &&
-                        fy <= (double)(kVisitBins - 1);
-        if (!ok) {
+        uint32_t bx = bin(x[i], 0), by = bin(y[i], 1);
+        if (bx == kNoBin || by == kNoBin) {
             atomicOr(&st->flags, kStatDegenerate);
-            fx = 0.0;
-            fy = 0.0;
+            bx = 0;
+            by = 0;
         }
-        const uint32_t key = (uint32_t)fx * kVisitBins + (uint32_t)fy;
+        const uint32_t key = bx * kVisitBins + by;
         keys[i] = key;
         counts_add(s_h, passes, key);
     }
