@@ -374,8 +374,8 @@ __global__ void write_labels_kernel(ClusterArgs a) {
 // thresholds): the cores of a cell always share a component, so the
 // union-find runs over the non-empty cells, and a border point is settled by
 // its neighbour cells' cluster starts.  The neighbour table is not read.  All
-// minpts of one epsilon (slots, largest minpts first) share the kernels that
-// do not depend on one another.
+// minpts of one epsilon (slots) are labelled side by side, a launch of each
+// kernel for all.
 
 // cbest[c] = largest degree of the cell (high word) and the first point that
 // has it (complemented, low word): the cell has cores at minpts m iff the

@@ -577,7 +577,7 @@ struct ClusterArgs {
     const EpsParams* ep;        // reach pattern of the grid
 };
 // Clustering on grids whose cells are cliques: all minpts of one epsilon
-// (slots, largest minpts first), up to kSlots at a time.
+// (slots), up to kSlots at a time.
 constexpr int kSlots = 8;
 struct CellArgs {
     uint32_t n;
