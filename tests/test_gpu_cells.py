@@ -115,3 +115,26 @@ def test_sort_tiles(ctx, vdb, orc, n):
     rng = np.random.default_rng(n)
     x, y = rng.uniform(0, 40, n), rng.uniform(0, 40, n)
     _check(ctx, vdb, orc, x, y, np.array([0.03, 0.02]), np.array([3, 2], np.uint32))
+
+
+@pytest.mark.parametrize("entry_bytes", [2, 4])
+@pytest.mark.parametrize("gap", [100, 1000, 7000, 100000])
+def test_dense_regions_far_apart_in_the_same_rows(ctx, vdb, orc, gap, entry_bytes):
+    # two dense lattice regions with nothing but empty cells between them (gap: in
+    # cells of the middle epsilon), thousands of pairs at exactly eps: a run of
+    # points that begins in the one region and ends in the other has a box whose
+    # edges are far from its first point
+    rng = np.random.default_rng(gap)
+    n1, n2, step = 3500, 30000, 0.004
+    x = np.concatenate([rng.uniform(1.0, 1.06, n1), rng.uniform(0.0, 0.06, n2) + 1.0 + gap * 0.01])
+    x, y = np.rint(x / step) * step, np.rint(rng.uniform(40.0, 40.06, n1 + n2) / step) * step
+    eps = np.array([0.01, 0.02, 0.05])
+    mp = np.array([700, 9000, 20000], np.uint32)
+    want = orc.variants(x, y, eps, mp, 70)
+    item = vdb.BatchItem(x, y, eps, mp, 70)
+    out, st = ctx.run([item], table_hash=True, entry_bytes=entry_bytes)
+    np.testing.assert_array_equal(out[0], want)
+    assert st["table_hash"] == sum(orc.table_hash(x, y, e, 70) for e in eps) & M64
+    out, sb = ctx.run([item], table="border", entry_bytes=entry_bytes)
+    np.testing.assert_array_equal(out[0], want)
+    assert sb["pairs"] == st["pairs"]

@@ -193,11 +193,28 @@ constexpr uint32_t kLaneCand = 16;
 // lies in a small box where the data are dense (points of a cell are ordered
 // by subcell).  box[i] bounds the points [4i, 4i + 36), relative to the cell
 // origin of point 4i, so it covers the 32 candidates of any word that starts
-// at points 4i..4i+3; x0 > x1 when the run spans two grid rows.  Tiles of at
-// least kBoxCand candidates compare each word's box with their queries' first:
-// a box wholly inside or outside eps settles 64 x 32 pairs without a test.
+// at points 4i..4i+3; x0 > x1 when the run spans two grid rows, or more than
+// kBoxCells cells of one (an edge far from point 4i is rounded at that distance:
+// see box_pad).  Tiles of at least kBoxCand candidates compare each word's box
+// with their queries' first: a box wholly inside or outside eps settles 64 x 32
+// pairs without a test.
 constexpr uint32_t kBoxCand = 2048;
 constexpr uint32_t kBoxRun = 36;
+constexpr uint32_t kBoxCells = 16;
+// How far a box's edges are moved out along x and y in a tile of G cells with
+// reach r in its own row (the largest): more than what the roundings can have
+// moved them in.  With u = 2^-24, cells of width w and |positions| in the tile
+// at most R = (G + r + 1) w, a point's stored x is off by at most
+// u (kBoxCells + 1) w; the shift into the tile's coordinates, the pad's own
+// subtraction and the candidate's coordinate that the box has to contain add at
+// most u R each (an edge further out than R is one of a point between the run's
+// first and the word's: rounding is monotone, it is no further in than the
+// word's own).  Together u w (kBoxCells + 1 + 3 (G + r + 1)), against a pad of
+// u w 16 (G + 2 r + 4), which is larger for all G, r >= 1.
+__device__ __forceinline__ float box_pad(float wf, uint32_t G, int r) {
+    static_assert(kBoxCells + 1 + 3 * (1 + 1 + 1) <= 16 * (1 + 2 + 4), "the pad covers the roundings");
+    return 0x1p-20f * wf * (float)((int)G + 2 * r + 4);
+}
 __device__ __forceinline__ void word_box(const TableArgs& a, uint32_t i) {
     const uint32_t k0 = 4u * i;
     if (k0 >= a.n) return;
@@ -205,7 +222,8 @@ __device__ __forceinline__ void word_box(const TableArgs& a, uint32_t i) {
     const uint32_t e = min(k0 + kBoxRun, a.n);
     const float wf = a.ep->wf;
     float4 b = make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
-    if (a.gkey[e - 1] / a.g.ncx_pad == cy0) {
+    const uint32_t key1 = a.gkey[e - 1];
+    if (key1 - key0 <= kBoxCells && key1 / a.g.ncx_pad == cy0) {
         for (uint32_t k = k0; k < e; k++) {
             const float2 loc = a.glocal[k];
             const float x = __fmaf_rn((float)(a.gkey[k] - key0), wf, loc.x);
@@ -653,13 +671,13 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
             const bool boxes = a.wbox && C >= kBoxCand;
             if (boxes) settled = true;
             float bx0 = 0.f, bx1 = 0.f, by0 = 0.f, by1 = 0.f;  // the queries' box (fmin/fmax skip NaN)
-            float pad = 0.f;  // more than the roundings of a box's edges (16 of them)
+            float pad = 0.f;
             if (boxes) {
                 bx0 = warp_min(fminf(qx[0], qx[1]));
                 bx1 = warp_max(fmaxf(qx[0], qx[1]));
                 by0 = warp_min(fminf(qy[0], qy[1]));
                 by1 = warp_max(fmaxf(qy[0], qy[1]));
-                pad = 0x1p-20f * wf * (float)((int)G + 2 * ep->reach[rho] + 4);
+                pad = box_pad(wf, G, ep->reach[rho]);
             }
 
             // blocks of 32 words: lane l looks at word wb + l
@@ -675,12 +693,14 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
                         if (g1 <= rows.off[i + 1] && VDB_GUARD(a.st, k < a.n, 3, k)) {
                             const float4 b = a.wbox[k >> 2];
                             if (b.x <= b.y) {
-                                // Rounding is monotone: the largest |q - c| per
-                                // axis, rounded, is at least every rounded
-                                // |q - c|, and its FP32 d2 at least every
-                                // pair's; the smallest likewise.  So d2max <
-                                // lo32 (d2min > hi32) decides all pairs of the
-                                // two boxes as their own FP32 d2 would.
+                                // The padded box holds the FP32 coordinates of
+                                // the word's candidates.  Rounding is monotone:
+                                // the largest |q - c| per axis, rounded, is at
+                                // least every rounded |q - c|, and its FP32 d2
+                                // at least every pair's; the smallest likewise.
+                                // So d2max < lo32 (d2min > hi32) decides all
+                                // pairs of the two boxes as their own FP32 d2
+                                // would.
                                 const float dcx = (float)(int)(a.gkey[k & ~3u] - rows.base[i]);
                                 const float x0 = __fmaf_rn(dcx, wf, b.x) - pad;
                                 const float x1 = __fmaf_rn(dcx, wf, b.y) + pad;
