@@ -138,3 +138,24 @@ def test_dense_regions_far_apart_in_the_same_rows(ctx, vdb, orc, gap, entry_byte
     out, sb = ctx.run([item], table="border", entry_bytes=entry_bytes)
     np.testing.assert_array_equal(out[0], want)
     assert sb["pairs"] == st["pairs"]
+
+
+@pytest.mark.parametrize("cpe", [4, 15, 16, 17, 24, 31, 32])
+def test_many_cells_per_epsilon(ctx, vdb, orc, cpe):
+    # up to 65 rows of up to 65 cells around each cell, most of them with points;
+    # minpts near the degrees: cores and border points everywhere
+    rng = np.random.default_rng(3)
+    n = 9000
+    x, y = rng.uniform(0, 6, n), rng.uniform(0, 4, n)
+    x[:1500], y[:1500] = rng.normal(1.5, 0.4, 1500), rng.normal(3.0, 0.4, 1500)
+    eps = np.array([1.0, 1.0, 1.0, 0.4, 0.4])
+    mp = np.array([980, 1250, 2250, 160, 560], np.uint32)
+    _check(ctx, vdb, orc, x, y, eps, mp, cells_per_eps=cpe)
+    # two clusters that meet at one pair of cells, with up to 57 cells of noise
+    # before it in the row: (0, 0) has its mass below, (0.95, 0.15) to the right
+    px = np.concatenate([np.full(300, 0.2), np.zeros(5), np.full(5, 0.95), np.full(300, 1.9)])
+    py = np.concatenate([np.full(300, -0.9), np.zeros(5), np.full(305, 0.15)])
+    rx = np.arange(-0.9, 0.88, 1 / 32)
+    x, y = np.concatenate([px, rx]), np.concatenate([py, np.full(len(rx), 0.15)])
+    assert orc.variants(x, y, np.ones(1), np.array([200], np.uint32), 70).max() == 1
+    _check(ctx, vdb, orc, x, y, np.ones(2), np.array([200, 3], np.uint32), cells_per_eps=cpe)

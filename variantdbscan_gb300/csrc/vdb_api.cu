@@ -411,6 +411,11 @@ EpsParams make_eps(double eps, const GridParams& g, const HostBox& hb, bool want
     return p;
 }
 
+// Cells of a grid row within reach of a cell, at most.
+int row_cells(const EpsParams& p) {
+    return 2 * *std::max_element(p.reach, p.reach + 2 * p.rho + 1) + 1;
+}
+
 struct Options {
     int precision = VDB_PRECISION_MIXED;
     int schedule = VDB_SCHEDULE_BATCHED;
@@ -1548,7 +1553,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                     ca.comp_prev[v] = comp_source(mp);
                 }
                 for (int v = 0; v < ca.m; v++) ca.comp_out[v] = comp_dest(slots[s0 + v].second);
-                launch_cells(ca, nrows, group_asym != 0, cells_ws, s);
+                launch_cells(ca, nrows, row_cells(ep), group_asym != 0, cells_ws, s);
                 CK(cudaGetLastError());
             }
         } else if (!chunked) {
@@ -2520,7 +2525,7 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
         ca.asym_count = asym_n;
         ca.asym_cap = kNoallocAsymCap;
         ca.st = st;
-        launch_cells(ca, 2 * ep.rho + 1, true, resolve_ws, s);
+        launch_cells(ca, 2 * ep.rho + 1, row_cells(ep), true, resolve_ws, s);
     } else {
         ClusterArgs ca;
         memset(&ca, 0, sizeof ca);

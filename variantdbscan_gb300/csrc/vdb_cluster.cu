@@ -526,7 +526,8 @@ constexpr uint32_t kFlatPairs = 1024;  // of at most so many: all of them, lanes
 
 // Unions (z: slot): every pair of cells within reach whose roots differ is
 // searched for one core-core pair accepted in both directions.  A lane takes a
-// cell and one row of its half neighbourhood: it screens the roots and tests
+// cell and one row of its half neighbourhood (y; 32 cells of it at a time, a row
+// has at most 5 at the default cell size): it screens the roots and tests
 // the cells' points of largest degree (and all pairs of next to empty cells);
 // only then the pairs that are still apart are searched by the whole warp,
 // lanes over the point pairs (or, for large cells, over the first cell's points
@@ -544,7 +545,9 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a) {
     const float near2 = a.ep->near2;
     const float wf = t.wf;
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t dy = (blockIdx.y + 1u) % gridDim.y;  // (the next row's many pairs first)
+    const uint32_t hrows = (uint32_t)a.ep->rho + 1u;
+    const uint32_t dy = (blockIdx.y + 1u) % hrows;  // (the next row's many pairs first)
+    const uint32_t skip = blockIdx.y / hrows * 32u;  // cells of the row that other blocks take
     if (c - lane >= ncl) return;  // (whole warps)
     uint32_t* parent = a.parent + (size_t)v * a.n;
     const uint32_t* __restrict__ comp = a.comp_prev[v];
@@ -556,8 +559,8 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a) {
         ku = best_point(bA);
         if (best_deg(bA) >= mp && ku < a.n) {
             const uint2 rg = a.crng[(size_t)((uint32_t)a.ep->rho + dy) * a.n + c];
-            o = dy ? rg.x : c + 1;
-            oe = rg.y;
+            o = (dy ? rg.x : c + 1) + skip;
+            oe = min(rg.y, o + 32u);
             if (o < oe) {
                 cx = (int)a.ccx[c];
                 sA = a.clist[c];
@@ -574,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 6) cell_pairs_kernel(CellArgs a) {
     {
         const uint32_t root = o < oe ? uf_find(parent, c) : 0u;
 #pragma unroll 5
-        for (uint32_t j = 0; j < (o < oe ? min(oe - o, 32u) : 0u); j++) {
+        for (uint32_t j = 0; j < (o < oe ? oe - o : 0u); j++) {
             if (best_deg(a.cbest[o + j]) < mp) continue;
             const uint32_t p1 = parent[o + j];
             if (p1 != root && parent[p1] != root) left |= 1u << j;
@@ -854,7 +857,9 @@ __device__ __forceinline__ uint32_t start_label(const CellArgs& a, int v, uint32
 // start after p's own visit position cannot label it (p was visited first, as
 // noise).  The lanes of a warp search side by side while there are at most
 // kLaneCores points for each lane that searches; a few lanes' larger searches
-// are done by the warp one after the other, lanes over the cells' points.
+// are done by the warp one after the other, lanes over the cells' points (a lane
+// holds a row, so not on grids of more than 32 rows, 16 and more cells per
+// epsilon).
 constexpr uint32_t kLaneCores = 16;
 __global__ void __launch_bounds__(kThreads, 8) cell_labels_kernel(CellArgs a) {
     pdl_sync();
@@ -923,7 +928,7 @@ __global__ void __launch_bounds__(kThreads, 8) cell_labels_kernel(CellArgs a) {
             }
             bool hit = false;
             const uint32_t searching = (uint32_t)__popc(__ballot_sync(kFull, busy));
-            const bool wide = busy && npts > kLaneCores * searching;
+            const bool wide = busy && nrows <= 32 && npts > kLaneCores * searching;
             if (busy && !wide) {
                 for (int j = 0; j < nrows && !hit; j++) {
                     const int dy = (j + 1) / 2 * ((j & 1) ? 1 : -1);  // nearest rows first
@@ -1056,14 +1061,15 @@ void launch_border_and_write(const ClusterArgs& a, int nblocks, cudaStream_t s) 
     launch_label_write(a, s);
 }
 
-void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws,
+void launch_cells(const CellArgs& a, int nrows, int row_cells, bool one_way, void* resolve_ws,
                   cudaStream_t s) {
     if (!a.n) return;
+    const unsigned parts = (unsigned)(row_cells + 31) / 32u;
     const dim3 per_slot(nblk(a.n), (unsigned)a.m);
     launch(cell_setup_kernel, dim3(nblk(std::max(a.n, a.nw)), (unsigned)nrows), kThreads, s, a);
     launch(cell_hook_kernel, per_slot, kThreads, s, a);
-    launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1), (unsigned)a.m), kThreads,
-           s, a);
+    launch(cell_pairs_kernel, dim3(nblk(a.n), (unsigned)(nrows / 2 + 1) * parts, (unsigned)a.m),
+           kThreads, s, a);
     launch(cell_seed_kernel, per_slot, kThreads, s, a);
     if (one_way) {
         launch(cell_resolve_kernel, a.m, 32, s, a, (uint32_t*)resolve_ws, kResolveCap);

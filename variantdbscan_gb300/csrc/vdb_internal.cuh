@@ -622,9 +622,10 @@ struct CellArgs {
 };
 // Words of the start bits of n visit positions (whole 32-byte groups).
 inline uint32_t start_words(uint32_t n) { return ((n + 31u) / 32u + 7u) & ~7u; }
-// nrows: 2*rho+1; one_way: the table has one-way pairs; resolve_ws:
-// m * resolve_scratch_bytes()
-void launch_cells(const CellArgs& a, int nrows, bool one_way, void* resolve_ws, cudaStream_t s);
+// nrows: 2*rho+1; row_cells: cells of a row within reach of a cell, at most;
+// one_way: the table has one-way pairs; resolve_ws: m * resolve_scratch_bytes()
+void launch_cells(const CellArgs& a, int nrows, int row_cells, bool one_way, void* resolve_ws,
+                  cudaStream_t s);
 size_t resolve_scratch_bytes();
 // comp[gpos[k]] = seed of the component of core k, kNone for other points
 // (after launch_uf_finish)
