@@ -96,7 +96,9 @@ typedef struct {
     int32_t precision;      /* VDB_PRECISION_* */
     int32_t schedule;       /* VDB_SCHEDULE_* */
     int32_t location;       /* VDB_LOC_*: where x, y and labels live */
-    int32_t cells_per_eps;  /* grid cells per epsilon (1..4); 0 = the library's choice (2) */
+    int32_t cells_per_eps;  /* grid cells per epsilon (1..4 are useful, more than 32 are
+                               taken as 32); 0 = the library's choice (2).  Labels and
+                               tables do not depend on it */
     int32_t verbose;
     int64_t table_budget_bytes; /* neighbour-table budget; 0 = derived from free memory */
     int32_t streams;        /* datasets of one call run concurrently on this many CUDA

@@ -159,3 +159,12 @@ def test_many_cells_per_epsilon(ctx, vdb, orc, cpe):
     x, y = np.concatenate([px, rx]), np.concatenate([py, np.full(len(rx), 0.15)])
     assert orc.variants(x, y, np.ones(1), np.array([200], np.uint32), 70).max() == 1
     _check(ctx, vdb, orc, x, y, np.ones(2), np.array([200, 3], np.uint32), cells_per_eps=cpe)
+
+
+@pytest.mark.parametrize("cpe", [33, 50, 1000])
+def test_more_cells_per_epsilon_than_the_rows_hold(ctx, vdb, orc, cpe):
+    # the kernels hold 65 rows of cells: finer cells than 32 per epsilon are not made
+    rng = np.random.default_rng(cpe)
+    x, y = rng.uniform(0, 3, 2000), rng.uniform(0, 3, 2000)
+    eps, mp = np.array([1.0, 0.3]), np.array([600, 60], np.uint32)
+    _check(ctx, vdb, orc, x, y, eps, mp, cells_per_eps=cpe)

@@ -486,6 +486,9 @@ struct Group {
 // cell pairs the clustering searches (measured slower at every eps of the
 // variant sweep and the lattice), so the cell size is a fixed choice.
 constexpr int kCellsPerEps = 2;
+// the finest cells whose reach of an epsilon the kernels' rows hold (labels and
+// tables do not depend on the cell size)
+constexpr int kMaxCellsPerEps = (kMaxRows - 1) / 2;
 
 // Tile groups: a tile is up to 64 consecutive cell-ordered points of one group
 // of G cells of a grid row; its candidates are the cells within reach of the
@@ -1119,7 +1122,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             launch_gather(oa, s);
         } else {
             const size_t ta = tm.mark();
-            const int r = o.cells_per_eps > 0 ? o.cells_per_eps : kCellsPerEps;
+            const int r = o.cells_per_eps > 0 ? std::min(o.cells_per_eps, kMaxCellsPerEps)
+                                              : kCellsPerEps;
             if (isinf(eps)) {
                 g = make_grid(hb, 1.0, 1);
                 g.w = INFINITY;
