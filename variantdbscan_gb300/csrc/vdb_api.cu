@@ -573,6 +573,8 @@ void check_flags(const DeviceStatus& st) {
         throw VdbError{VDB_ERR_CUDA, "fill pass disagrees with count pass"};
     if (f & kStatUnionStall)
         throw VdbError{VDB_ERR_CUDA, "union-find retry limit reached"};
+    if (f & kStatTooManyUnits)
+        throw VdbError{VDB_ERR_NOMEM, "2^31 work units or more for one epsilon"};
 }
 
 constexpr uint32_t kAsymCap = 1u << 20;
@@ -1249,16 +1251,19 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 st_flags = (uint32_t)rec->take();
                 GraphCheck chk;
                 memset(&chk, 0, sizeof chk);
+                // (a failed scan's sizes are not to be compared)
                 chk.c[0] = graph_cond(d_nunits, kGcLe32, nunits);
-                chk.n = 1;
+                chk.c[1] = graph_cond(&d_st->flags, kGcMask32, kStatGuard | kStatTooManyUnits, 0);
+                chk.n = 2;
                 if (!no_rows) {
-                    chk.c[1] = graph_cond(d_nwords, kGcLe64, bm_words);
-                    chk.c[2] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
-                    chk.n = 3;
+                    chk.c[2] = graph_cond(d_nwords, kGcLe64, bm_words);
+                    chk.c[3] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
+                    chk.n = 4;
                 }
                 capture_checkpoint(*rec, s, chk);
             } else {
                 read_status(ctx, s);
+                check_flags(*ctx->h_status);  // (before the sizes are used)
                 status_before_count = *ctx->h_status;
                 if (!no_rows) bm_words = ctx->h_status->nwords;
                 nunits = ctx->h_status->nunits;

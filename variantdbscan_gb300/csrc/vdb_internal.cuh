@@ -64,6 +64,7 @@ enum : uint32_t {
     kStatUnionStall = 1u << 5,       // union-find retry limit reached
     kStatGuard = 1u << 6,            // an index guard failed (see guard_site)
     kStatBitmapTooLarge = 1u << 7,   // a tile's test bitmap exceeds 2^32 words (use the fill pass)
+    kStatTooManyUnits = 1u << 8,     // 2^31 work units or more: their offsets and number are void
 };
 
 constexpr uint32_t kResolveCap = 4096;   // directed component edges per variant

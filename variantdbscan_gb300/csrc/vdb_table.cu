@@ -1821,8 +1821,10 @@ __device__ __forceinline__ void tile_rows(const TableArgs& a, const EpsParams* _
 // of its test bitmap, ceil(C/32) per query, and its work units,
 // ceil(ceil(C/32) / unit_words); the offsets of both, and of the units that
 // warps take (those of tiles that are not small), by a single-pass scan (boff
-// may be null: no bitmap).  Blocks past the last tile only clear their part of
-// deg (and the one-way pairs' counter).
+// may be null: no bitmap).  A scan's word holds 31 bits of units: where they are
+// more (dense data of 10^7 points and more; their list alone would take 16 GB),
+// kStatTooManyUnits is set and the offsets are not to be used.  Blocks past the
+// last tile only clear their part of deg (and the one-way pairs' counter).
 __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
     uint32_t* __restrict__ loff, unsigned long long* __restrict__ nwords,
@@ -1872,6 +1874,8 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     block_lookbacks<2>(before, tile, states, a.st);
     if (t < ntiles) {
         const uint32_t u0 = (uint32_t)(before[0] & 0x7fffffffull), l0 = (uint32_t)(before[0] >> 31);
+        // (the first tile to pass the 31 bits sees it, what comes before it is right)
+        if (u0 + nu > 0x7fffffffu) atomicOr(&a.st->flags, kStatTooManyUnits);
         uoff[t] = u0;
         loff[t] = l0;
         if (boff) boff[t] = before[1];
