@@ -145,3 +145,29 @@ def test_noalloc_rejects_sizes_beyond_the_limit(lib):
     dummy = ctypes.c_void_p(16)
     rc = lib.vdb_run_noalloc(dummy, dummy, MAX_POINTS + 1, 0.5, 10, 70, dummy, None)
     assert rc == VDB_ERR_TOO_LARGE
+
+
+def test_noalloc_near_the_limit_on_pairs(lib):
+    # 115 sites, 350 points each: 13.975 million pairs of 40,000 points are just
+    # within what the array's table has room for beside the other temporaries
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(2)
+    site = np.minimum(np.arange(40_000) // 350, 114)
+    x = np.where(site == 114, 190.0, site % 20 * 10.0) + rng.uniform(0, 1e-3, 40_000)
+    y = np.where(site == 114, 130.0, site // 20 * 10.0) + rng.uniform(0, 1e-3, 40_000)
+    got = _noalloc(lib, torch, x, y, 1.0, 5, 70)
+    assert got.max() == 115
+    np.testing.assert_array_equal(got, _batched(x, y, 1.0, 5, 70))
+
+
+def test_noalloc_near_the_limit_on_pairs_of_a_coarse_grid(lib):
+    # a point far away coarsens the cells to 16 epsilons, so that every point is
+    # a candidate of all the others: many work units beside a table of 11.9
+    # million pairs
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(7)
+    u = rng.uniform(0, 1, (MAX_POINTS - 1, 2)) * 2.0804443359375
+    x, y = np.append(u[:, 0], 1000.0), np.append(u[:, 1], 1000.0)
+    got = _noalloc(lib, torch, x, y, 0.0625, 190, 70)
+    assert got.max() > 0 and (got == 0).sum() > 1
+    np.testing.assert_array_equal(got, _batched(x, y, 0.0625, 190, 70))

@@ -2463,6 +2463,9 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     uint32_t nunits = 0;
     CK(cudaMemcpyAsync(&nunits, d_nunits, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
+    // (the unit list's room is the table's, or the cells' lists', once the
+    // points are counted)
+    const size_t used = cv.used;
     uint2* ulist = cv.take<uint2>((size_t)nunits + 1);
     ta.tile_uoff = tuoff;
     ta.tile_loff = tloff;
@@ -2479,10 +2482,13 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     CK(cudaStreamSynchronize(s));
     check_flags(hs);
     const unsigned long long E = hs.entries;
+    cv.used = used;
     // the limit on the neighbour pairs: what a table of 32-bit entries has
-    // beside 160 bytes per point, the cells and the one-way pairs
-    const size_t held = (size_t)n * 160 + (g.ncells + 1) * 4 +
-                        (size_t)kNoallocAsymCap * sizeof(AsymPair) + ((size_t)1 << 18);
+    // beside 162 bytes per point, the multiple-point boxes, the cells and the
+    // one-way pairs
+    const size_t held = (size_t)n * 152 + (size_t)nmpb * sizeof(MpbBox) +
+                        std::max((size_t)n * 10, (size_t)98304) + (g.ncells + 1) * 4 +
+                        (size_t)kNoallocAsymCap * sizeof(AsymPair);
     const size_t room = held < kNoallocBytes ? (kNoallocBytes - held) / sizeof(uint32_t) : 0;
     if (E > room)
         throw VdbError{VDB_ERR_TOO_LARGE, "neighbour table exceeds the fixed scratch array"};
