@@ -27,3 +27,33 @@ def test_more_work_units_than_their_offsets_hold(vdb, orc):
         out, _ = c.run([vdb.BatchItem(x[:3000], y[:3000], [0.02], [5], 70)], table=table)
         np.testing.assert_array_equal(out[0], orc.variants(x[:3000], y[:3000], [0.02], [5], 70))
     c.close()
+
+
+@pytest.mark.parametrize("cpe", [0, 1])
+def test_labelling_when_the_table_fills_the_memory(vdb, cpe):
+    # a table that takes all the memory it is given, eight minpts to label after
+    # it: the labelling's own memory has to be there (cells_per_eps 1 labels from
+    # the table, over points)
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(12)
+    n = 1_000_000
+    x, y = rng.uniform(0, 100, n), rng.uniform(0, 100, n)
+    eps = np.full(8, 1.2)
+    mp = np.array([300, 350, 400, 430, 450, 470, 500, 550], np.uint32)
+    item = vdb.BatchItem(x, y, eps, mp, 70)
+    c = vdb.Context()
+    want, sw = c.run([item], cells_per_eps=cpe)
+    c.close()
+    assert sw["table_chunks"] == 1
+    c = vdb.Context()
+    c.run([vdb.BatchItem(x[:5000], y[:5000], eps[:2], mp[:2], 70)], cells_per_eps=cpe)
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - (960 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        out, st = c.run([item], cells_per_eps=cpe)
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+        c.close()
+    np.testing.assert_array_equal(out[0], want[0])
+    assert st["table_chunks"] > 1

@@ -907,8 +907,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* cells_ws = nullptr;
     size_t cells_slots = 0, cells_ws_slots = 0;
     const uint32_t nw = start_words(n);
-    uint2* crng = nullptr;  // neighbour cells of every cell and row
-    size_t crng_cap = 0;
+    const size_t n8 = ((size_t)n + 7) & ~(size_t)7;       // (keeps the bit words aligned)
+    const size_t slot_words = 3 * n8 + 2 * (size_t)nw;    // of cells_buf
     UfState whole;
     memset(&whole, 0, sizeof whole);
     auto new_state = [&]() {
@@ -962,8 +962,11 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint64_t cell_cap = 0;
     uint32_t* crow = nullptr;   // sparse grids: row directory
     uint64_t crow_cap = 0;
-    uint32_t *trow_s = nullptr, *trow_e = nullptr;  // tile row ranges (sparse grids, compact tables)
-    size_t trow_cap = 0;
+    // tile row ranges (sparse grids, compact tables: trow_s, trow_e), and once
+    // the table is written the neighbour cells of every cell and row in their place
+    uint2* row_ranges = nullptr;
+    size_t row_ranges_cap = 0;
+    uint32_t *trow_s = nullptr, *trow_e = nullptr;
 
     const bool want_mixed = o.precision == VDB_PRECISION_MIXED;
     // (small inputs: tiles of 32, twice as many and half as long)
@@ -1205,17 +1208,36 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // VDB_TABLE_BORDER writes the rows that the labelling reads: none
             // on grids whose cells are cliques
             no_rows = o.table_rows == VDB_TABLE_BORDER && clique;
-            if (g.sparse || (compact_ok && !no_rows)) {
+            const bool tile_ranges = g.sparse || (compact_ok && !no_rows);
+            if (tile_ranges || clique) {
                 const size_t nr = (size_t)n * (size_t)(2 * ep.rho + 1);
-                if (nr > trow_cap) {
-                    if (trow_s) ar.put(trow_s);
-                    if (trow_e) ar.put(trow_e);
-                    trow_s = ar.get<uint32_t>(nr);
-                    trow_e = ar.get<uint32_t>(nr);
-                    trow_cap = nr;
+                if (nr > row_ranges_cap) {
+                    if (row_ranges) ar.put(row_ranges);
+                    row_ranges = ar.get<uint2>(nr);
+                    row_ranges_cap = nr;
                 }
-                ta_args.trow_s = trow_s;
-                ta_args.trow_e = trow_e;
+                if (tile_ranges) {
+                    ta_args.trow_s = trow_s = (uint32_t*)row_ranges;
+                    ta_args.trow_e = trow_e = trow_s + nr;
+                }
+            }
+            // the labelling's state comes before the bitmap and the table, which
+            // are sized by the memory that is left.  All minpts side by side, or
+            // fewer at a time where they would take more than a tenth of it.
+            const size_t want_slots = std::min<size_t>(slots.size(), kSlots);
+            if (!clique) {
+                if (!whole.parent) whole = new_state();
+            } else if (want_slots > cells_slots) {
+                size_t k = want_slots;
+                if (!capturing && k * slot_words * 4 > kSmallAlloc) {
+                    const double room = 0.1 * avail_bytes(ctx);
+                    while (k > 1 && (double)(k * slot_words * 4) > room) k--;
+                }
+                if (k > cells_slots) {
+                    if (cells_buf) ar.put(cells_buf);
+                    cells_buf = ar.get<uint32_t>(k * slot_words);
+                    cells_slots = k;
+                }
             }
             ta_args.crow = crow;
             ta_args.ccx = ccx;
@@ -1504,25 +1526,13 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             // are written, chunk by chunk, and that is all)
             if (chunked)
                 for (const RowChunk& c : chunk_list) build_chunk(ta_args, c, group_asym);
-            const size_t want = std::min<size_t>(slots.size(), kSlots);
-            const size_t n8 = ((size_t)n + 7) & ~(size_t)7;  // (keeps the bit words aligned)
-            if (want > cells_slots) {
-                if (cells_buf) ar.put(cells_buf);
-                cells_buf = ar.get<uint32_t>(want * (3 * n8 + 2 * (size_t)nw));
-                cells_slots = want;
-            }
             const int nrows = 2 * ep.rho + 1;
-            if ((size_t)n * nrows > crng_cap) {
-                if (crng) ar.put(crng);
-                crng_cap = (size_t)n * nrows;
-                crng = ar.get<uint2>(crng_cap);
-            }
-            if (group_asym && want > cells_ws_slots) {
+            if (group_asym && cells_slots > cells_ws_slots) {
                 if (cells_ws) ar.put(cells_ws);
-                cells_ws = ar.get<uint32_t>(want * (resolve_scratch_bytes() / 4));
-                cells_ws_slots = want;
+                cells_ws = ar.get<uint32_t>(cells_slots * (resolve_scratch_bytes() / 4));
+                cells_ws_slots = cells_slots;
             }
-            for (size_t s0 = 0; s0 < slots.size(); s0 += kSlots) {
+            for (size_t s0 = 0; s0 < slots.size(); s0 += cells_slots) {
                 CellArgs ca;
                 memset(&ca, 0, sizeof ca);
                 ca.n = n;
@@ -1538,12 +1548,12 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 ca.cell_start = cell_start;
                 ca.crow = crow;
                 ca.ccx = ccx;
-                ca.crng = crng;
+                ca.crng = row_ranges;
                 ca.clist = clist;
                 ca.ncl = cscan + n;
                 ca.cscan = cscan;
                 ca.cbest = cbest;
-                ca.m = (int)std::min<size_t>(slots.size() - s0, kSlots);
+                ca.m = (int)std::min<size_t>(slots.size() - s0, cells_slots);
                 ca.parent = cells_buf;
                 ca.seed = cells_buf + cells_slots * n8;
                 ca.cst = cells_buf + 2 * cells_slots * n8;
