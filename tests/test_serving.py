@@ -127,3 +127,17 @@ def test_calibration_sets_the_per_point_footprint():
                                          + (1 << 20))) <= 2
     res = srv.serve(reqs, rate=float("inf"))
     assert res.footprint_ratio == pytest.approx(1.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,minpts,side", [(20000, 1, 1.0), (300000, 3, 5.0), (300000, 16, 1.0),
+                                           (1500000, 8, 10.0), (1500000, 8, 100.0)])
+def test_estimate_before_calibration_covers_the_measured_footprint(n, minpts, side):
+    rng = np.random.default_rng(n)
+    mp = np.arange(4, 4 + minpts, dtype=np.uint32)
+    eps = np.repeat([0.02, 0.01], minpts)
+    r = sv.Request(0.0, rng.uniform(0, side, n), rng.uniform(0, side, n), eps, np.tile(mp, 2))
+    run = sv.library_runner_factory()(1 << 30)
+    run(r)
+    run.ctx.close()
+    assert r.device_bytes - r.table_bytes <= sv.footprint(r, 0)

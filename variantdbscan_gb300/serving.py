@@ -17,13 +17,18 @@ from dataclasses import dataclass, field
 
 import numpy as np
 
-# device bytes of one dataset besides the neighbour table and the labels:
-# a fixed part (the one-way pair list, scratch of the sorts and scans, a dense
-# cell array of up to 4M cells) and a part per point (inputs, visit order, cell
-# order, union-find state, tiles, counts, row offsets), until Server.calibrate
-# measures both on sample requests
+# device bytes of one labels-only dataset besides the neighbour table and the
+# labels, until Server.calibrate measures both parts on sample requests: a fixed
+# part (the one-way pair list, a dense cell array of up to 4M cells, blocks
+# rounded up) and a part per point that the densest and the sparsest requests
+# stay below.  Always: inputs, visit order, cell order, tiles, counts, offsets,
+# sorts, row ranges, 216; clustering state, 12 for each of up to 8 minpts of an
+# epsilon, 98, and 4 for every minpts kept for the next epsilon.  Dense grids:
+# cells, up to 128.  Where the cells are coarser than half an epsilon (a small
+# epsilon over a wide box): union-find over points, 24, and work units, 264 each,
+# of sparse points up to one for each.
 INDEX_BASE_BYTES = 64 << 20
-INDEX_BYTES_PER_POINT = 200
+INDEX_BYTES_PER_POINT = 768
 
 
 @dataclass
