@@ -168,3 +168,18 @@ def test_more_cells_per_epsilon_than_the_rows_hold(ctx, vdb, orc, cpe):
     x, y = rng.uniform(0, 3, 2000), rng.uniform(0, 3, 2000)
     eps, mp = np.array([1.0, 0.3]), np.array([600, 60], np.uint32)
     _check(ctx, vdb, orc, x, y, eps, mp, cells_per_eps=cpe)
+
+
+@pytest.mark.parametrize("entry_bytes", [2, 4])
+def test_rows_built_twice_are_hashed_once(ctx, vdb, orc, entry_bytes):
+    # row chunks that the labelling reads (cells that are no cliques) are built
+    # for the unions and again for the border points
+    rng = np.random.default_rng(6)
+    n = 30011
+    x, y = rng.uniform(0, 40, n), rng.uniform(0, 40, n)
+    eps, mp = np.array([0.5, 0.5]), np.array([9, 14], np.uint32)
+    kw = dict(entry_bytes=entry_bytes, table_hash=True, cells_per_eps=1)
+    out, st = ctx.run([vdb.BatchItem(x, y, eps, mp, 70)], budget=200000, **kw)
+    np.testing.assert_array_equal(out[0], orc.variants(x, y, eps, mp, 70))
+    assert st["table_hash"] == orc.table_hash(x, y, 0.5, 70) & M64
+    assert st["table_chunks"] > 2

@@ -1021,7 +1021,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     bool table_counter_fresh = false;  // zero since the group's memset
     // builds the rows of chunk c into nbr (expand from the bitmap, or the
     // fill pass when there is no bitmap)
-    auto build_chunk = [&](TableArgs& t, const RowChunk& c, uint32_t nasym) {
+    auto build_chunk = [&](TableArgs& t, const RowChunk& c, uint32_t nasym, bool again = false) {
         const size_t m0 = tm.mark();
         t.off_base = c.e_lo;
         t.tile_lo = c.t_lo;
@@ -1039,8 +1039,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
         } else {
             launch_fill(t, nb_fill, s);
         }
-        // hash of the rows just built
-        if (o.table_hash) launch_table_hash(t, gorig, nb_warps, s);
+        // hash of the rows just built (again: hashed before)
+        if (o.table_hash && !again) launch_table_hash(t, gorig, nb_warps, s);
         CK(cudaGetLastError());
         table_marks.push_back({m0, tm.mark()});
         chunks++;
@@ -1612,7 +1612,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 save_comp(cas[si], slots[si].second);
             }
             for (const RowChunk& c : chunk_list) {
-                build_chunk(ta_args, c, group_asym);
+                build_chunk(ta_args, c, group_asym, true);
                 for (ClusterArgs& ca : cas) {
                     chunk_rows(ca, c);
                     launch_border_pull(ca, nb_warps, s);
