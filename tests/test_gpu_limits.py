@@ -57,3 +57,22 @@ def test_labelling_when_the_table_fills_the_memory(vdb, cpe):
         c.close()
     np.testing.assert_array_equal(out[0], want[0])
     assert st["table_chunks"] > 1
+
+
+@pytest.mark.parametrize("kw", [dict(eps=[0.4], budget=100000), dict(eps=[-1.0], budget=0)])
+def test_stats_of_a_call_that_no_graph_captures(vdb, kw):
+    # row chunks and empty neighbourhoods are not captured: the first call with
+    # graph=True records a run before it finds out
+    rng = np.random.default_rng(9)
+    x, y = rng.uniform(0, 30, 20000), rng.uniform(0, 30, 20000)
+    lab = np.zeros((1, 20000), np.uint32)
+    item = vdb.BatchItem(x, y, kw["eps"], [6], 70, lab)
+    c = vdb.Context()
+    want, sw = c.run([item], budget=kw["budget"], table_hash=True)
+    for _ in range(2):
+        out, st = c.run([item], budget=kw["budget"], table_hash=True, graph=True)
+        assert st["graph"] == 4  # unsupported: ran directly
+        for k in ("pairs", "candidates", "tables", "table_chunks", "clusters", "table_hash",
+                  "entry_bytes", "worker_streams"):
+            assert st[k] == sw[k], k
+    c.close()

@@ -2201,6 +2201,8 @@ int run_graph(vdb_context* ctx, const vdb_dataset* ds, int nds, const Options& o
     }
     while (ctx->graphs.size() >= kMaxGraphs) drop_graph(ctx, ctx->graphs.front());
     ctx->graphs.push_back(ge);
+    // (a call that cannot be captured runs once more: that run's stats count)
+    if (stats && !ge->ok) memset(stats, 0, sizeof *stats);
     if (stats) stats->graph_checks = ge->checks;
     return ge->ok ? VDB_GRAPH_CAPTURED : VDB_GRAPH_UNSUPPORTED;
 }
