@@ -183,3 +183,25 @@ def test_rows_built_twice_are_hashed_once(ctx, vdb, orc, entry_bytes):
     np.testing.assert_array_equal(out[0], orc.variants(x, y, eps, mp, 70))
     assert st["table_hash"] == orc.table_hash(x, y, 0.5, 70) & M64
     assert st["table_chunks"] > 2
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [33, 63, 64, 65, 97, 1500, 131100])
+def test_tables_without_a_bitmap(ctx, vdb, orc, n, precision):
+    # a far point makes one cell of all the others: every point a candidate of
+    # all, few of them neighbours, so that the table fits a budget which the
+    # bitmap of the tests exceeds (tiles of 32, of 64 from 2^17 points on)
+    rng = np.random.default_rng(n)
+    side = 1.0 if n < 1000 else 2.0
+    x, y = rng.uniform(0, side, n), rng.uniform(0, side, n)
+    x[0], y[0] = 1e5, 1e5
+    eps, mp = np.array([0.004 if n > 1e5 else 0.02]), np.array([3], np.uint32)
+    item = vdb.BatchItem(x, y, eps, mp, 70)
+    want = orc.variants(x, y, eps, mp, 70)
+    for entry_bytes in (2, 4):
+        kw = dict(table_hash=True, precision=precision, entry_bytes=entry_bytes)
+        _, sw = ctx.run([item], **kw)
+        out, st = ctx.run([item], budget=sw["entry_bytes"], **kw)
+        np.testing.assert_array_equal(out[0], want)
+        assert st["table_chunks"] == 1
+        assert st["table_hash"] == sw["table_hash"] == orc.table_hash(x, y, eps[0], 70) & M64
