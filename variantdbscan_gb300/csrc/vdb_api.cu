@@ -971,8 +971,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     const bool want_mixed = o.precision == VDB_PRECISION_MIXED;
     // (small inputs: tiles of 32, twice as many and half as long)
     const int tq = n < kSmallTilePoints ? table_tile_queries() / 2 : table_tile_queries();
-    const int nb_count = ctx->nsm * ctx->blocks_count[want_mixed];
-    const int nb_fill = ctx->nsm * ctx->blocks_fill[want_mixed];
     const int nb_expand16 = ctx->nsm * ctx->blocks_expand[1];
     const int nb_expand32 = ctx->nsm * ctx->blocks_expand[0];
     const int nb_warps = ctx->nsm * 8;
@@ -1037,7 +1035,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             launch_expand(t, t.compact ? nb_expand16 : nb_expand32, s);
             if (nasym) launch_asym_flags(t, s);
         } else {
-            launch_fill(t, nb_fill, s);
+            launch_fill(t, ctx->nsm * ctx->blocks_fill[t.mixed], s);
         }
         // hash of the rows just built (again: hashed before)
         if (o.table_hash && !again) launch_table_hash(t, gorig, nb_warps, s);
@@ -1362,7 +1360,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                     CK(cudaMemsetAsync(count_counter, 0, 4, s));
                     CK(cudaMemsetAsync(gz.off, 0, scan_state_bytes(n), s));
                 }
-                launch_count(ta_args, nb_count, s);
+                launch_count(ta_args, ctx->nsm * ctx->blocks_count[mixed], s);
                 CK(cudaGetLastError());
                 tc = tm.mark();
                 if (!no_rows) scan_u32_to_u64(deg, off, n, gz.off, d_st, s);
