@@ -76,3 +76,31 @@ def test_stats_of_a_call_that_no_graph_captures(vdb, kw):
                   "entry_bytes", "worker_streams"):
             assert st[k] == sw[k], k
     c.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_work_units_when_memory_is_short(vdb, graph):
+    # a far point makes one cell of all the others, but the cells look nearly
+    # empty: units of 1,024 candidates, 1.1M of them, take 330 MB where 150 are
+    # left; the largest ones take 80
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(13)
+    n = 270_000
+    x, y = rng.uniform(0, 1, n), rng.uniform(0, 1, n)
+    x[0], y[0] = 1e6, 1e6
+    item = vdb.BatchItem(x, y, [0.002], [3], 70, np.zeros((1, n), np.uint32))
+    c = vdb.Context()
+    want, _ = c.run([vdb.BatchItem(x, y, [0.002], [3], 70)])
+    c.close()
+    c = vdb.Context()
+    c.run([vdb.BatchItem(x[1:5000], y[1:5000], [0.02], [3], 70)])
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - (300 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        for _ in range(2 if graph else 1):
+            out, st = c.run([item], graph=graph)
+            np.testing.assert_array_equal(out[0], want[0])
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+        c.close()

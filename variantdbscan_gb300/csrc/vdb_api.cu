@@ -144,6 +144,9 @@ struct VdbError {
 // Buffers up to this size are taken without weighing them against the free
 // memory first (a question to the driver of 5 to 10 us).
 constexpr size_t kSmallAlloc = (size_t)64 << 20;
+// Work units are weighed from this size on (a fraction of a percent of the
+// device's memory; below it they are taken, and the largest units if that fails).
+constexpr size_t kLargeAlloc = (size_t)1 << 30;
 
 // Allocations of one call, returned to the context pool when it ends.
 // The bytes it holds (as the pool rounds them) and their peak: the call's
@@ -1254,64 +1257,107 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             ta_args.st = d_st;
             // layout of the count pass's test bitmap (one word per query and
             // 32 candidates of its tile), which the table pass expands
-            unit_words = o.unit_words > 0 ? (uint32_t)o.unit_words : default_unit_words(n, g.ncells);
-            ta_args.unit_words = unit_words;
-            launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, tloff, d_nwords, d_nunits,
-                              gz.words, s);
+            unit_words = capturing          ? (uint32_t)rec->take()
+                         : o.unit_words > 0 ? (uint32_t)o.unit_words
+                                            : default_unit_words(n, g.ncells);
+            // 16-bit entries (positions within work units)
+            compact = compact_ok;
+            ta_args.compact = compact ? 1 : 0;
+            ta_args.ptile = ptile;
             uint64_t bm_words = 0;
             uint32_t nunits = 0;
             uint32_t st_flags = 0;
             DeviceStatus status_before_count;
             memset(&status_before_count, 0, sizeof status_before_count);
-            if (capturing) {
-                // buffers sized with headroom over the record, checked
-                // against what they hold
-                bm_words = graph_room(rec->take());
-                nunits = (uint32_t)std::min<uint64_t>(graph_room(rec->take()), 0xfffffffeu);
-                st_flags = (uint32_t)rec->take();
-                GraphCheck chk;
-                memset(&chk, 0, sizeof chk);
-                // (a failed scan's sizes are not to be compared)
-                chk.c[0] = graph_cond(d_nunits, kGcLe32, nunits);
-                chk.c[1] = graph_cond(&d_st->flags, kGcMask32, kStatGuard | kStatTooManyUnits, 0);
-                chk.n = 2;
-                if (!no_rows) {
-                    chk.c[2] = graph_cond(d_nwords, kGcLe64, bm_words);
-                    chk.c[3] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
-                    chk.n = 4;
+            // work units: (tile, chunk of unit_words bitmap words)
+            const size_t flag_words = compact && !no_rows ? flag_blocks(kUnitWords) : 0;
+            const size_t unit_bytes = sizeof(uint2) + (no_rows ? 0 : 4 * (size_t)kUnitQ) +
+                                      flag_words * sizeof(uint2);
+            auto put_units = [&]() {
+                if (ulist) ar.put(ulist);
+                if (parts) ar.put(parts);
+                if (wflags) ar.put(wflags);
+                ulist = nullptr;
+                parts = nullptr;
+                wflags = nullptr;
+                unit_cap = 0;
+            };
+            auto take_units = [&]() {
+                if ((uint64_t)nunits + 1 > unit_cap) {
+                    put_units();
+                    ulist = ar.get<uint2>((size_t)nunits + 1);
+                    unit_cap = (uint64_t)nunits + 1;
                 }
-                capture_checkpoint(*rec, s, chk);
-            } else {
+                if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
+                // (sized for any unit size: a later epsilon may take larger units)
+                if (!wflags && flag_words) wflags = ar.get<uint2>(unit_cap * flag_words);
+            };
+            for (;;) {
+                ta_args.unit_words = unit_words;
+                launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, tloff, d_nwords,
+                                  d_nunits, gz.words, s);
+                if (capturing) {
+                    // buffers sized with headroom over the record, checked
+                    // against what they hold
+                    bm_words = graph_room(rec->take());
+                    nunits = (uint32_t)std::min<uint64_t>(graph_room(rec->take()), 0xfffffffeu);
+                    st_flags = (uint32_t)rec->take();
+                    GraphCheck chk;
+                    memset(&chk, 0, sizeof chk);
+                    // (a failed scan's sizes are not to be compared)
+                    chk.c[0] = graph_cond(d_nunits, kGcLe32, nunits);
+                    chk.c[1] = graph_cond(&d_st->flags, kGcMask32, kStatGuard | kStatTooManyUnits, 0);
+                    chk.n = 2;
+                    if (!no_rows) {
+                        chk.c[2] = graph_cond(d_nwords, kGcLe64, bm_words);
+                        chk.c[3] = graph_cond(&d_st->flags, kGcMask32, kStatBitmapTooLarge, st_flags);
+                        chk.n = 4;
+                    }
+                    capture_checkpoint(*rec, s, chk);
+                    take_units();
+                    break;
+                }
                 read_status(ctx, s);
-                check_flags(*ctx->h_status);  // (before the sizes are used)
+                // Where the units by the rule are too many (a far point makes the
+                // points per cell look few) the largest ones are taken: more than a
+                // tenth of the memory, more than there is, or than offsets hold.
+                uint32_t flags = ctx->h_status->flags;
+                const bool can = o.unit_words <= 0 && unit_words < kUnitWords;
+                bool larger = can && (flags & kStatTooManyUnits);
+                if (!larger) {
+                    check_flags(*ctx->h_status);  // (before the sizes are used)
+                    nunits = ctx->h_status->nunits;
+                    larger = can && nunits * unit_bytes > kLargeAlloc &&
+                             (double)(nunits * unit_bytes) > 0.1 * avail_bytes(ctx);
+                }
+                if (!larger) {
+                    try {
+                        take_units();
+                    } catch (const VdbError& e) {
+                        if (!can || e.code != VDB_ERR_NOMEM) throw;
+                        put_units();
+                        larger = true;
+                    }
+                }
+                if (!larger) break;
+                unit_words = kUnitWords;
+                flags &= ~(uint32_t)kStatTooManyUnits;
+                memcpy(ctx->h_pinned, &flags, sizeof flags);
+                CK(cudaMemcpyAsync(&d_st->flags, ctx->h_pinned, sizeof flags,
+                                   cudaMemcpyHostToDevice, s));
+                CK(cudaMemsetAsync(gz.words, 0, words_state_bytes(n), s));
+            }
+            if (!capturing) {
                 status_before_count = *ctx->h_status;
                 if (!no_rows) bm_words = ctx->h_status->nwords;
-                nunits = ctx->h_status->nunits;
                 st_flags = ctx->h_status->flags & kStatBitmapTooLarge;
                 if (recording) {
+                    rec->put(unit_words);
                     rec->put(bm_words);
                     rec->put(nunits);
                     rec->put(st_flags);
                 }
             }
-            // 16-bit entries (positions within work units)
-            compact = compact_ok;
-            ta_args.compact = compact ? 1 : 0;
-            ta_args.ptile = ptile;
-            // work units: (tile, chunk of unit_words bitmap words)
-            if ((uint64_t)nunits + 1 > unit_cap) {
-                if (ulist) ar.put(ulist);
-                if (parts) ar.put(parts);
-                if (wflags) ar.put(wflags);
-                wflags = nullptr;
-                unit_cap = (uint64_t)nunits + 1;
-                ulist = ar.get<uint2>(unit_cap);
-                parts = nullptr;
-            }
-            if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
-            // (sized for any unit size: a later epsilon may take larger units)
-            if (!wflags && compact && !no_rows)
-                wflags = ar.get<uint2>(unit_cap * flag_blocks(kUnitWords));
             ta_args.wflags = compact && !no_rows ? wflags : nullptr;
             ta_args.tile_uoff = tuoff;
             ta_args.tile_loff = tloff;
