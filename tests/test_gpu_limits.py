@@ -104,3 +104,18 @@ def test_work_units_when_memory_is_short(vdb, graph):
         del hold
         torch.cuda.empty_cache()
         c.close()
+
+
+@pytest.mark.parametrize("entry_bytes", [2, 4])
+def test_memory_of_sparse_data(vdb, entry_bytes):
+    # a few points per tile: counts per unit and query (256 bytes a unit) are kept
+    # for the tiles that warps take only, so the index, the bitmap and the
+    # labelling stay below 320 bytes a point beside the table
+    rng = np.random.default_rng(14)
+    n = 1_000_000
+    x, y = rng.uniform(0, 100, n), rng.uniform(0, 100, n)
+    c = vdb.Context()
+    out, st = c.run([vdb.BatchItem(x, y, [0.3], [6], 70)], entry_bytes=entry_bytes)
+    c.close()
+    assert out[0].max() > 0
+    assert st["device_bytes"] - st["table_bytes"] < 320 * n

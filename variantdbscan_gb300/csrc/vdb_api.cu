@@ -599,7 +599,7 @@ struct UfState {
 // Splits the table into row chunks of whole tiles holding at most cap
 // entries each (greedy, in tile order).
 std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, Arena& ar, const uint32_t* tiles,
-                                      const uint32_t* ntiles_dev, const uint32_t* tloff,
+                                      const uint32_t* ntiles_dev, const uint32_t* tuoff,
                                       const unsigned long long* off, uint32_t n, uint64_t cap,
                                       cudaStream_t s) {
     static_assert(sizeof(ChunkPlan) <= 4096, "the plan fits the pinned buffer");
@@ -607,7 +607,7 @@ std::vector<RowChunk> plan_row_chunks(vdb_context* ctx, Arena& ar, const uint32_
     ChunkPlan* d = (ChunkPlan*)ar.get<uint64_t>(sizeof(ChunkPlan) / 8);
     ChunkPlan h;
     do {
-        launch_plan_chunks(tiles, ntiles_dev, tloff, off, n, cap, out.empty() ? 0u : h.next, d, s);
+        launch_plan_chunks(tiles, ntiles_dev, tuoff, off, n, cap, out.empty() ? 0u : h.next, d, s);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(ctx->h_pinned, d, sizeof h, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -950,11 +950,10 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
     uint32_t* ccx = ar.get<uint32_t>(n);
     unsigned long long* tboff = ar.get<unsigned long long>((size_t)n + 1);
     uint32_t* tuoff = ar.get<uint32_t>((size_t)n + 1);
-    uint32_t* tloff = ar.get<uint32_t>((size_t)n + 1);
     float4* wbox = nullptr;  // boxes of runs of points
     uint32_t* bitmap = nullptr;
     uint64_t bitmap_cap = 0;
-    uint2* ulist = nullptr;
+    uint32_t* ulist = nullptr;
     uint32_t* parts = nullptr;
     uint2* wflags = nullptr;
     uint64_t unit_cap = 0;
@@ -1271,7 +1270,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             memset(&status_before_count, 0, sizeof status_before_count);
             // work units: (tile, chunk of unit_words bitmap words)
             const size_t flag_words = compact && !no_rows ? flag_blocks(kUnitWords) : 0;
-            const size_t unit_bytes = sizeof(uint2) + (no_rows ? 0 : 4 * (size_t)kUnitQ) +
+            const size_t unit_bytes = sizeof(uint32_t) + (no_rows ? 0 : 4 * (size_t)kUnitQ) +
                                       flag_words * sizeof(uint2);
             auto put_units = [&]() {
                 if (ulist) ar.put(ulist);
@@ -1285,7 +1284,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             auto take_units = [&]() {
                 if ((uint64_t)nunits + 1 > unit_cap) {
                     put_units();
-                    ulist = ar.get<uint2>((size_t)nunits + 1);
+                    ulist = ar.get<uint32_t>((size_t)nunits + 1);
                     unit_cap = (uint64_t)nunits + 1;
                 }
                 if (!parts && !no_rows) parts = ar.get<uint32_t>(unit_cap * kUnitQ);
@@ -1294,8 +1293,8 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             };
             for (;;) {
                 ta_args.unit_words = unit_words;
-                launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, tloff, d_nwords,
-                                  d_nunits, gz.words, s);
+                launch_tile_words(ta_args, no_rows ? nullptr : tboff, tuoff, d_nwords, d_nunits,
+                                  gz.words, s);
                 if (capturing) {
                     // buffers sized with headroom over the record, checked
                     // against what they hold
@@ -1360,7 +1359,6 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
             }
             ta_args.wflags = compact && !no_rows ? wflags : nullptr;
             ta_args.tile_uoff = tuoff;
-            ta_args.tile_loff = tloff;
             ta_args.nunits = d_nunits;
             ta_args.ulist = ulist;
             ta_args.parts = no_rows ? nullptr : parts;
@@ -1497,7 +1495,7 @@ void run_dataset(vdb_context* ctx, const vdb_dataset& ds, const Options& o, vdb_
                 nbr_cap_bytes = 0;
                 const int64_t budget = o.budget > 0 ? o.budget : (int64_t)(avail_bytes(ctx) * 0.9);
                 const uint64_t cap = (uint64_t)std::max<int64_t>(budget / (int64_t)esz, 1);
-                chunk_list = plan_row_chunks(ctx, ar, tiles, d_ntiles, tloff, off, n, cap, s);
+                chunk_list = plan_row_chunks(ctx, ar, tiles, d_ntiles, tuoff, off, n, cap, s);
                 uint64_t mx = 1;
                 for (const RowChunk& c : chunk_list) mx = std::max<uint64_t>(mx, c.e_hi - c.e_lo);
                 const size_t w = std::max<size_t>(words_for(mx), 1);
@@ -2514,17 +2512,15 @@ void run_noalloc(const double* x, const double* y, uint32_t n, double eps, uint3
     ta.unit_words = kUnitWordsTiny;
     // work units of the count pass (no bitmap here: the fill pass writes the table)
     uint32_t* tuoff = cv.take<uint32_t>((size_t)n + 1);
-    uint32_t* tloff = cv.take<uint32_t>((size_t)n + 1);
-    launch_tile_words(ta, nullptr, tuoff, tloff, &st->nwords, d_nunits, gz.words, s);
+    launch_tile_words(ta, nullptr, tuoff, &st->nwords, d_nunits, gz.words, s);
     uint32_t nunits = 0;
     CK(cudaMemcpyAsync(&nunits, d_nunits, 4, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     // (the unit list's room is the table's, or the cells' lists', once the
     // points are counted)
     const size_t used = cv.used;
-    uint2* ulist = cv.take<uint2>((size_t)nunits + 1);
+    uint32_t* ulist = cv.take<uint32_t>((size_t)nunits + 1);
     ta.tile_uoff = tuoff;
-    ta.tile_loff = tloff;
     ta.nunits = d_nunits;
     ta.ulist = ulist;
     ta.ptile = ptile;

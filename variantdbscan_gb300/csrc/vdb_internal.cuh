@@ -84,7 +84,7 @@ struct DeviceStatus {
     // sizes of the current epsilon, which the host reads back with the rest
     unsigned long long nwords;     // words of the test bitmap
     unsigned long long entries;    // entries of the neighbour table
-    uint32_t nunits, nlist;        // work units; those that warps take
+    uint32_t nunits;               // work units
     uint32_t ntiles;
     uint32_t asym_n;               // one-way pairs recorded
     uint32_t starts_done[8];       // blocks done per slot of cell_starts_kernel
@@ -430,20 +430,19 @@ struct TableArgs {
     uint32_t* bitmap;               // count pass: per-tile test bitmaps (nullptr: none)
     const unsigned long long* tile_boff;  // first bitmap word of each tile
     // work units of the count and table passes: (tile, chunk of unit_words
-    // bitmap words); tile t has the units tile_uoff[t]..tile_uoff[t+1].  Warps
-    // take the units of ulist (unit, tile), which leaves out those of small
-    // tiles; tile t's are tile_loff[t]..tile_loff[t+1] of it.
+    // bitmap words); tile t has the units tile_uoff[t]..tile_uoff[t+1], which
+    // warps take, and ulist holds their tile.  Small tiles have none: a thread
+    // per point takes them, and their rows are one piece.
     uint32_t unit_words;            // bitmap words per unit (default_unit_words)
-    const uint2* ulist;
+    const uint32_t* ulist;
     const uint32_t* tile_uoff;
-    const uint32_t* tile_loff;
-    const uint32_t* nunits;         // device: units, units in ulist
+    const uint32_t* nunits;         // device scalar
     uint32_t* parts;                // per unit and query slot: neighbours in that chunk
     uint2* wflags;                  // per unit and block of 32 words: words wholly inside eps of
                                     // the tile, wholly outside (16-bit tables; else null)
     unsigned long long* pair_sum;   // count pass: adds the neighbours counted (nullptr: not)
     // one row chunk of the table: the fill pass takes tiles from tile_lo on,
-    // the expand pass entries [unit_lo, unit_hi) of ulist, and the small tiles
+    // the expand pass units [unit_lo, unit_hi), and the small tiles
     // and the asymmetric flags touch rows [row_lo, row_hi) only
     uint32_t tile_lo;
     uint32_t unit_lo, unit_hi;
@@ -465,7 +464,8 @@ constexpr uint32_t kUnitQ = 64;        // query slots per unit (tiles hold <= 64
 // by unit, 32 entries at a time: fn(neighbour cell-ordered index, one-way
 // flag, valid) on every lane (the decoding shuffles need the whole warp; lanes
 // past the end get valid = false).  parts[u * kUnitQ + slot]: the row's
-// entries in unit u; unit_words: the table's unit size in bitmap words.
+// entries in unit u (not looked at where the tile has one unit, or none, as small
+// tiles: the row is one piece); unit_words: the table's unit size in bitmap words.
 template <class Fn>
 static __device__ __forceinline__ void walk_compact_row(
     const uint16_t* __restrict__ nb16, unsigned long long row0, unsigned long long row1, uint32_t k,
@@ -475,27 +475,31 @@ static __device__ __forceinline__ void walk_compact_row(
     uint32_t unit_words, int lane, Fn&& fn) {
     const uint32_t t = ptile[k];
     const uint32_t slot = k - tiles[t];
-    const uint32_t u0 = tile_uoff[t], u1 = tile_uoff[t + 1];
+    const uint32_t u0 = tile_uoff[t];
+    const uint32_t u1 = max(tile_uoff[t + 1], u0 + 1u);
     const TileSegs sg = load_tile_segs(trow_s, trow_e, t, nrows, lane);
-    unsigned long long j = row0;
+    const uint32_t len = (uint32_t)(row1 - row0);
+    uint32_t j = 0;  // entries of the row before unit ub
     for (uint32_t ub = u0; ub < u1; ub += 32) {
         const uint32_t u = ub + (uint32_t)lane;
-        const uint32_t c = (u < u1 && slot < kUnitQ) ? parts[(unsigned long long)u * kUnitQ + slot] : 0u;
+        uint32_t c = 0;
+        if (u < u1 && slot < kUnitQ)
+            c = u1 - u0 == 1u ? len : parts[(unsigned long long)u * kUnitQ + slot];
         uint32_t incl = c;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= d) incl += v;
         }
-        const unsigned long long jb = j + (incl - c);
+        const uint32_t jb = j + (incl - c);
         for (uint32_t nz = __ballot_sync(0xffffffffu, c != 0u); nz; nz &= nz - 1u) {
             const int src = __ffs(nz) - 1;
             const uint32_t cu = __shfl_sync(0xffffffffu, c, src);
-            const unsigned long long js = __shfl_sync(0xffffffffu, jb, src);
+            const uint32_t js = __shfl_sync(0xffffffffu, jb, src);
             const uint32_t gbase = (ub + (uint32_t)src - u0) * (unit_words * 32u);
             for (uint32_t e0 = 0; e0 < cu; e0 += 32) {
-                const bool valid = e0 + (uint32_t)lane < cu && js + e0 + (uint32_t)lane < row1;
-                const uint16_t ev = valid ? nb16[js + e0 + (uint32_t)lane] : (uint16_t)0;
+                const bool valid = e0 + (uint32_t)lane < cu && js + e0 + (uint32_t)lane < len;
+                const uint16_t ev = valid ? nb16[row0 + js + e0 + (uint32_t)lane] : (uint16_t)0;
                 const uint32_t id = decode_candidate(sg, nrows, gbase + (ev & kPosMask16));
                 fn(id, (ev & kAsymFlag16) != 0, valid);
             }
@@ -507,17 +511,17 @@ void launch_count(const TableArgs& a, int nblocks, cudaStream_t s);
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s);
 size_t words_state_bytes(uint32_t n);
 void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
-                       uint32_t* loff, unsigned long long* nwords, uint32_t* nunits,
-                       void* zeroed, cudaStream_t s);
-void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s);
+                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
+                       cudaStream_t s);
+void launch_unit_list(const TableArgs& a, uint32_t* ulist, cudaStream_t s);
 // adds the hash of rows [row_lo, row_hi) of the table to st->table_hash
 // (gorig: input index of every cell-ordered point)
 void launch_table_hash(const TableArgs& a, const uint32_t* gorig, int nblocks, cudaStream_t s);
 void launch_expand(const TableArgs& a, int nblocks, cudaStream_t s);
 void launch_asym_flags(const TableArgs& a, cudaStream_t s);
 
-// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi), with the
-// entries [u_lo, u_hi) of the unit list, table entries [e_lo, e_hi).  The whole
+// Rows [r_lo, r_hi) of the neighbour table = tiles [t_lo, t_hi) = work units
+// [u_lo, u_hi), table entries [e_lo, e_hi).  The whole
 // table: t_hi = u_hi = 0xffffffff (no limits).
 struct RowChunk {
     uint32_t t_lo, t_hi, u_lo, u_hi, r_lo, r_hi;
@@ -533,7 +537,7 @@ struct ChunkPlan {
 };
 // The next (up to kPlanChunks) row chunks from tile t0: whole tiles, at most cap
 // entries each, greedy in tile order.
-void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tloff,
+void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tuoff,
                         const unsigned long long* off, uint32_t n, uint64_t cap, uint32_t t0,
                         ChunkPlan* plan, cudaStream_t s);
 int table_block_threads();

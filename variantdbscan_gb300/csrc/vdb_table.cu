@@ -265,7 +265,7 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
     bool mine = false;
     if (k < a.n) {
         t = a.ptile[k];
-        mine = a.tile_loff[t + 1] == a.tile_loff[t];
+        mine = a.tile_uoff[t + 1] == a.tile_uoff[t];
     }
     if (!__any_sync(kFull, mine)) return;
     uint32_t cnt = 0, retest = 0, g = 0;
@@ -332,7 +332,6 @@ __device__ void small_count(const TableArgs& a, uint32_t k) {
         }
         if ((g & 31u) && bm) bm[(unsigned long long)(g >> 5) * Q] = word;
         a.deg[k] = cnt;
-        if (a.parts) a.parts[(unsigned long long)a.tile_uoff[t] * kUnitQ + (k - qs)] = cnt;
     }
     const uint32_t tests = __reduce_add_sync(kFull, g), again = __reduce_add_sync(kFull, retest);
     const uint32_t pairs = __reduce_add_sync(kFull, cnt);
@@ -353,7 +352,7 @@ __global__ void __launch_bounds__(kTT) small_count_kernel(TableArgs a) {
 template <typename E>
 __device__ void small_expand(const TableArgs& a, uint32_t k) {
     const uint32_t t = a.ptile[k];
-    if (a.tile_loff[t + 1] != a.tile_loff[t]) return;
+    if (a.tile_uoff[t + 1] != a.tile_uoff[t]) return;
     const uint32_t qs = a.tiles[t], Q = a.tiles[t + 1] - qs;
     const uint32_t* __restrict__ bm = a.bitmap + a.tile_boff[t] + (k - qs);
     E* dst = reinterpret_cast<E*>(a.nbr) + (a.off[k] - a.off_base);
@@ -419,7 +418,7 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
     const float wf = a.ep->wf;
-    const uint32_t nlist = a.nunits[1];
+    const uint32_t nunits = *a.nunits;
     const uint32_t ncx_pad = a.g.ncx_pad, G = a.g.G;
     const float fnan = __int_as_float(0x7fc00000);
     const double dnan = __longlong_as_double(0x7ff8000000000000ll);
@@ -437,10 +436,8 @@ __global__ void __launch_bounds__(kWPB * 32, 3) count_kernel(TableArgs a) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nlist) break;
-        const uint2 ut = a.ulist[u];
-        u = ut.x;
-        const uint32_t t = ut.y;
+        if (u >= nunits) break;
+        const uint32_t t = a.ulist[u];
         const uint32_t chunk = u - a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ)) {
@@ -981,7 +978,7 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
     const float wf = a.ep->wf;
-    const uint32_t nlist = min(a.nunits[1], a.unit_hi);  // the row chunk's part of the list
+    const uint32_t nunits = min(*a.nunits, a.unit_hi);  // up to the row chunk's last
     if (a.n <= kSmallFused)
         for (uint64_t k = a.row_lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.row_hi;
              k += (uint64_t)gridDim.x * blockDim.x)
@@ -997,10 +994,8 @@ __global__ void __launch_bounds__(kXPB * 32, 6) expand_kernel(TableArgs a) {
         uint32_t u = 0;
         if (lane == 0) u = a.unit_lo + atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nlist) break;
-        const uint2 ut = a.ulist[u];
-        u = ut.x;
-        const uint32_t t = ut.y;
+        if (u >= nunits) break;
+        const uint32_t t = a.ulist[u];
         const uint32_t u0 = a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ && u0 <= u)) {
@@ -1276,7 +1271,7 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho;
     const int nrows = 2 * rho + 1;
-    const uint32_t nlist = min(a.nunits[1], a.unit_hi);
+    const uint32_t nunits = min(*a.nunits, a.unit_hi);
     if (a.n <= kSmallFused)
         for (uint64_t k = a.row_lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.row_hi;
              k += (uint64_t)gridDim.x * blockDim.x)
@@ -1291,10 +1286,8 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
         uint32_t u = 0;
         if (lane == 0) u = a.unit_lo + atomicAdd(a.tile_counter, 1u);
         u = __shfl_sync(kFull, u, 0);
-        if (u >= nlist) break;
-        const uint2 ut = a.ulist[u];
-        u = ut.x;
-        const uint32_t t = ut.y;
+        if (u >= nunits) break;
+        const uint32_t t = a.ulist[u];
         const uint32_t u0 = a.tile_uoff[t];
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         if (!(qs < qe && qe <= a.n && qe - qs <= kUnitQ && u0 <= u)) {
@@ -1825,16 +1818,15 @@ __device__ __forceinline__ void tile_rows(const TableArgs& a, const EpsParams* _
 
 // A thread per tile: its row segments (kept in trow_s/e where set), the words
 // of its test bitmap, ceil(C/32) per query, and its work units,
-// ceil(ceil(C/32) / unit_words); the offsets of both, and of the units that
-// warps take (those of tiles that are not small), by a single-pass scan (boff
-// may be null: no bitmap).  A scan's word holds 31 bits of units: where they are
-// more (dense data of 10^7 points and more; their list alone would take 16 GB),
-// kStatTooManyUnits is set and the offsets are not to be used.  Blocks past the
-// last tile only clear their part of deg (and the one-way pairs' counter).
+// ceil(ceil(C/32) / unit_words), or none if it is small; the offsets of both by a
+// single-pass scan (boff may be null: no bitmap).  Where there are more units than
+// 31 bits hold (dense data of 10^7 points and more; their counts would take 500
+// GB), kStatTooManyUnits is set and the offsets are not to be used.  Blocks past
+// the last tile only clear their part of deg (and the one-way pairs' counter).
 __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     TableArgs a, unsigned long long* __restrict__ boff, uint32_t* __restrict__ uoff,
-    uint32_t* __restrict__ loff, unsigned long long* __restrict__ nwords,
-    uint32_t* __restrict__ nunits, LookState lu, LookState lw) {
+    unsigned long long* __restrict__ nwords, uint32_t* __restrict__ nunits, LookState lu,
+    LookState lw) {
     pdl_sync();
     const uint32_t tile = lookback_ticket(lu);
     const uint32_t t = tile * kLookThreads + threadIdx.x;
@@ -1845,7 +1837,7 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
     const EpsParams* __restrict__ ep = a.ep;
     const int rho = ep->rho, nrows = 2 * rho + 1;
     unsigned long long w = 0;
-    uint32_t nu = 0, nl = 0;
+    uint32_t nu = 0;
     if (t < ntiles) {
         const uint32_t qs = a.tiles[t], qe = a.tiles[t + 1];
         const uint32_t key0 = a.gkey[qs];
@@ -1868,37 +1860,33 @@ __global__ void __launch_bounds__(kLookThreads) tile_words_kernel(
         }
         const uint32_t tw = (c + 31u) >> 5;
         w = (unsigned long long)tw * (qe - qs);
-        nu = (tw + a.unit_words - 1) / a.unit_words;
-        nl = c <= (a.mixed ? kSmallCand : kSmallCand64) && qe - qs <= kSmallQueries ? 0u : nu;
+        if (c > (a.mixed ? kSmallCand : kSmallCand64) || qe - qs > kSmallQueries)
+            nu = (tw + a.unit_words - 1) / a.unit_words;
         if (w > 0xffffffffull) {
             atomicOr(&a.st->flags, kStatBitmapTooLarge);
             w = 0;
         }
     }
-    unsigned long long before[2] = {nu | ((unsigned long long)nl << 31), boff ? w : 0ull};
+    unsigned long long before[2] = {nu, boff ? w : 0ull};
     unsigned long long* const states[2] = {lu.tiles, lw.tiles};
     block_lookbacks<2>(before, tile, states, a.st);
     if (t < ntiles) {
-        const uint32_t u0 = (uint32_t)(before[0] & 0x7fffffffull), l0 = (uint32_t)(before[0] >> 31);
-        // (the first tile to pass the 31 bits sees it, what comes before it is right)
-        if (u0 + nu > 0x7fffffffu) atomicOr(&a.st->flags, kStatTooManyUnits);
+        const uint32_t u0 = (uint32_t)before[0];
         uoff[t] = u0;
-        loff[t] = l0;
         if (boff) boff[t] = before[1];
         if (t == ntiles - 1) {
+            if (before[0] + nu > 0x7fffffffull) atomicOr(&a.st->flags, kStatTooManyUnits);
             uoff[ntiles] = u0 + nu;
-            loff[ntiles] = l0 + nl;
-            nunits[0] = u0 + nu;
-            nunits[1] = l0 + nl;
+            *nunits = u0 + nu;
             if (boff) *nwords = before[1] + w;
         }
     }
 }
 
-// ulist: (unit, tile) of the units that warps take: a thread per tile, long
-// lists by the whole warp.  The first blocks make the word boxes (where there
-// are any), which would have no use for a launch of their own.
-__global__ void __launch_bounds__(kTT) unit_list_kernel(TableArgs a, uint2* ulist,
+// ulist: the tile of every unit, a thread per tile, long lists by the whole
+// warp.  The first blocks make the word boxes (where there are any), which would
+// have no use for a launch of their own.
+__global__ void __launch_bounds__(kTT) unit_list_kernel(TableArgs a, uint32_t* ulist,
                                                         uint32_t box_blocks) {
     pdl_sync();
     if (blockIdx.x < box_blocks) {
@@ -1909,19 +1897,17 @@ __global__ void __launch_bounds__(kTT) unit_list_kernel(TableArgs a, uint2* ulis
     const uint32_t ntiles = *a.ntiles;
     const uint32_t t = (blockIdx.x - box_blocks) * kTT + threadIdx.x;
     if (t - lane >= ntiles) return;  // (whole warps)
-    uint32_t b = 0, e = 0, u0 = 0;
+    uint32_t b = 0, e = 0;
     if (t < ntiles) {
-        b = a.tile_loff[t];
-        e = a.tile_loff[t + 1];
-        u0 = a.tile_uoff[t];
+        b = a.tile_uoff[t];
+        e = a.tile_uoff[t + 1];
     }
     if (e - b <= 8u)
-        for (uint32_t i = b; i < e; i++) ulist[i] = make_uint2(u0 + (i - b), t);
+        for (uint32_t i = b; i < e; i++) ulist[i] = t;
     for (uint32_t l = __ballot_sync(kFull, e - b > 8u); l; l &= l - 1u) {
         const int src = __ffs(l) - 1;
         const uint32_t bb = __shfl_sync(kFull, b, src), ee = __shfl_sync(kFull, e, src);
-        const uint32_t uu = __shfl_sync(kFull, u0, src), tt = t - lane + (uint32_t)src;
-        for (uint32_t i = bb + lane; i < ee; i += 32) ulist[i] = make_uint2(uu + (i - bb), tt);
+        for (uint32_t i = bb + lane; i < ee; i += 32) ulist[i] = t - lane + (uint32_t)src;
     }
 }
 
@@ -1979,7 +1965,7 @@ __global__ void table_hash_kernel(TableArgs a, const uint32_t* __restrict__ gori
 // each chunked table of 2M points by 1.4 ms.
 __global__ void plan_chunks_kernel(const uint32_t* __restrict__ tiles,
                                    const uint32_t* __restrict__ ntiles,
-                                   const uint32_t* __restrict__ tloff,
+                                   const uint32_t* __restrict__ tuoff,
                                    const unsigned long long* __restrict__ off, uint32_t n,
                                    uint64_t cap, uint32_t t0, ChunkPlan* plan) {
     pdl_sync();
@@ -2003,7 +1989,7 @@ __global__ void plan_chunks_kernel(const uint32_t* __restrict__ tiles,
             refused = 1;
         } else {
             if (lane == 0)
-                plan->list[k] = RowChunk{t,         lo, tloff[t], tloff[lo], tiles[t], tiles[lo],
+                plan->list[k] = RowChunk{t,         lo, tuoff[t], tuoff[lo], tiles[t], tiles[lo],
                                          e0, off[tiles[lo]]};
             k++;
             t = lo;
@@ -2048,17 +2034,21 @@ __global__ void asym_flags_kernel(TableArgs a) {
             }
             const uint32_t u0 = a.tile_uoff[t], nu = a.tile_uoff[t + 1] - u0;
             const uint32_t c = g / (a.unit_words * 32u), pos = g % (a.unit_words * 32u);
-            if (!VDB_GUARD(a.st, g != 0xffffffffu && c < nu && slot < kUnitQ, 5, target)) continue;
-            for (uint32_t u = u0; u < u0 + c; u++) lo += a.parts[(unsigned long long)u * kUnitQ + slot];
-            // (a one-way pair was tested: it is not in the runs that follow the
-            // unit's other entries)
-            uint32_t in_runs = 0;
-            if (a.wflags && a.tile_loff[t + 1] != a.tile_loff[t])
-                for (uint32_t b = 0; b < flag_blocks(a.unit_words); b++)
-                    in_runs += 32u * (uint32_t)__popc(full_runs(
-                                         a.wflags[(unsigned long long)(u0 + c) * flag_blocks(a.unit_words) + b].x,
-                                         c * a.unit_words + 32u * b, before));
-            hi = lo + a.parts[(unsigned long long)(u0 + c) * kUnitQ + slot] - in_runs;
+            if (!VDB_GUARD(a.st, g != 0xffffffffu && c < max(nu, 1u) && slot < kUnitQ, 5, target))
+                continue;
+            if (nu) {  // (a small tile's row is one piece)
+                for (uint32_t u = u0; u < u0 + c; u++)
+                    lo += a.parts[(unsigned long long)u * kUnitQ + slot];
+                // (a one-way pair was tested: it is not in the runs that follow the
+                // unit's other entries)
+                uint32_t in_runs = 0;
+                if (a.wflags)
+                    for (uint32_t b = 0; b < flag_blocks(a.unit_words); b++)
+                        in_runs += 32u * (uint32_t)__popc(full_runs(
+                                             a.wflags[(unsigned long long)(u0 + c) * flag_blocks(a.unit_words) + b].x,
+                                             c * a.unit_words + 32u * b, before));
+                hi = lo + a.parts[(unsigned long long)(u0 + c) * kUnitQ + slot] - in_runs;
+            }
             if (hi > end) hi = end;
             if (lo > hi) lo = hi;
             const unsigned long long seg_end = hi;
@@ -2118,15 +2108,15 @@ size_t words_state_bytes(uint32_t n) {
 }
 
 void launch_tile_words(const TableArgs& a, unsigned long long* boff, uint32_t* uoff,
-                       uint32_t* loff, unsigned long long* nwords, uint32_t* nunits, void* zeroed,
+                       unsigned long long* nwords, uint32_t* nunits, void* zeroed,
                        cudaStream_t s) {
     if (!a.n) return;
     const unsigned nb = (a.n + kLookThreads - 1) / kLookThreads;
-    launch(tile_words_kernel, nb, kLookThreads, s, a, boff, uoff, loff, nwords, nunits, look_state(zeroed),
+    launch(tile_words_kernel, nb, kLookThreads, s, a, boff, uoff, nwords, nunits, look_state(zeroed),
         look_state((char*)zeroed + words_state_bytes(a.n) / 2));
 }
 
-void launch_unit_list(const TableArgs& a, uint2* ulist, cudaStream_t s) {
+void launch_unit_list(const TableArgs& a, uint32_t* ulist, cudaStream_t s) {
     if (!a.n) return;
     const uint32_t boxes = a.wbox ? ((a.n + 3u) / 4u + kTT - 1) / kTT : 0u;
     launch(unit_list_kernel, boxes + (a.n + kTT - 1) / kTT, kTT, s, a, ulist, boxes);
@@ -2156,10 +2146,10 @@ void launch_asym_flags(const TableArgs& a, cudaStream_t s) {
     launch(asym_flags_kernel, 64, kTT, s, a);
 }
 
-void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tloff,
+void launch_plan_chunks(const uint32_t* tiles, const uint32_t* ntiles, const uint32_t* tuoff,
                         const unsigned long long* off, uint32_t n, uint64_t cap, uint32_t t0,
                         ChunkPlan* plan, cudaStream_t s) {
-    launch(plan_chunks_kernel, 1, 32, s, tiles, ntiles, tloff, off, n, cap, t0, plan);
+    launch(plan_chunks_kernel, 1, 32, s, tiles, ntiles, tuoff, off, n, cap, t0, plan);
 }
 
 int table_blocks_per_sm(bool fill, bool mixed) {
