@@ -45,9 +45,10 @@ struct Pool {
         const size_t g = (size_t)2 << 20;
         return (b + g - 1) / g * g;
     }
-    // the largest cached block that serves b bytes: up to twice their size for
-    // small ones (the datasets of a batch reuse one another's buffers whatever
-    // worker gets them), a quarter more for large ones
+    // the smallest cached block of at least b bytes serves them if it is no larger
+    // than this: 4 MB more than twice as large up to 64 MB (the datasets of a batch
+    // reuse one another's buffers whatever worker gets them), then 64 MB or a
+    // quarter larger.  A call's footprint counts the blocks, not what it asked for.
     static size_t fits(size_t b) {
         return b + std::max(b / 4, std::min(b, (size_t)64 << 20)) + ((size_t)4 << 20);
     }
@@ -582,7 +583,6 @@ void check_flags(const DeviceStatus& st) {
 
 constexpr uint32_t kAsymCap = 1u << 20;
 
-// Free device memory plus blocks this context holds in its pool.
 // Free device memory plus blocks this context holds in its pool, divided
 // among the contexts that run concurrently on the device.
 double avail_bytes(vdb_context* ctx) {

@@ -1,7 +1,6 @@
 // Device side of graph replay (vdb_options.graph): the checkpoint kernel that
 // re-checks, on each replay of a captured call, the device values the host
-// read while recording it, and the kernel that stores per-table parameters
-// (a captured call cannot copy them from host memory that changes later).
+// read while recording it.
 #include "vdb_internal.cuh"
 
 namespace vdb {
@@ -17,9 +16,6 @@ __global__ void graph_check_kernel(GraphCheck chk, uint32_t* bad,
     for (int i = 0; i < chk.n && i < kGraphConds; i++) {
         const GraphCond& c = chk.c[i];
         switch (c.kind) {
-            case kGcEq64:
-                ok = ok && *(const unsigned long long*)c.ptr == c.a;
-                break;
             case kGcLe64: {
                 const unsigned long long v = *(const unsigned long long*)c.ptr;
                 ok = ok && v <= c.a;

@@ -156,7 +156,7 @@ __device__ __forceinline__ uint32_t cell_of(double v, double v0, double w, float
 
 // Place of subcell (x, y) along the Hilbert curve over 2^sub x 2^sub subcells:
 // from the coarsest quadrant down, each level turned the way the curve enters
-// it.  Every run of the curve is connected, so a run of points has a small box
+// it (the textbook walk over quadrants, after Hilbert 1891).  Every run of the curve is connected, so a run of points has a small box
 // (along the Z order every second step is a diagonal or a jump).
 __device__ __forceinline__ uint32_t curve_index(uint32_t x, uint32_t y, uint32_t sub) {
     uint32_t d = 0;

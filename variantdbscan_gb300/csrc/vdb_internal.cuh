@@ -638,14 +638,13 @@ void launch_save_components(const ClusterArgs& a, uint32_t* comp, cudaStream_t s
 
 // Graph replay (vdb_options.graph).  A checkpoint re-checks device values
 // that the host read while recording the call: each condition compares one
-// value with what the host planned for (kGcEq64: equal 64-bit word; kGcLe64 /
-// kGcLe32: at most a, and kGcLe64 adds the value to *sum when sum is set;
-// kGcMask32: (value & a) == b; kGcGeF64 / kGcLeF64: a double at least / at
-// most the double whose bits are a).  If all hold and no earlier checkpoint
+// value with what the host planned for (kGcLe64 / kGcLe32: at most a, and
+// kGcLe64 adds the value to *sum when sum is set; kGcMask32: (value & a) == b;
+// kGcGeF64 / kGcLeF64: a double at least / at most the double whose bits are
+// a).  If all hold and no earlier checkpoint
 // failed the conditional node after it runs; otherwise *bad = index (first
 // failure) and the rest of the replay is skipped.
-enum : uint32_t { kGcEq64 = 1, kGcLe64 = 2, kGcLe32 = 3, kGcMask32 = 4, kGcGeF64 = 5,
-                  kGcLeF64 = 6 };
+enum : uint32_t { kGcLe64 = 1, kGcLe32 = 2, kGcMask32 = 3, kGcGeF64 = 4, kGcLeF64 = 5 };
 constexpr int kGraphConds = 8;
 struct GraphCond {
     const void* ptr;
@@ -661,8 +660,7 @@ struct GraphCheck {
 };
 void launch_graph_check(const GraphCheck& chk, uint32_t* bad, cudaGraphConditionalHandle next,
                         cudaStream_t s);
-// *dst = v by a kernel (a captured host-to-device copy would read the host
-// buffer at replay time).
+// ---------------------------------------------------- clustering over points
 void launch_uf_init(const ClusterArgs& a, bool fresh, cudaStream_t s);
 void launch_uf_union(const ClusterArgs& a, int nblocks, cudaStream_t s);
 void launch_uf_finish(const ClusterArgs& a, void* resolve_ws, cudaStream_t s);

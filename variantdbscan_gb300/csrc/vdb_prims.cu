@@ -75,11 +75,11 @@ void scan_u32_to_u64(const uint32_t* in, unsigned long long* out, uint32_t n, vo
 
 // ------------------------------------------------------------------ radix sort
 //
-// Digits of 9 bits (27-bit keys take three passes, the 17 bits of the visit
-// order two).  The kernel that makes the keys also counts all their digits
-// (SortPlan::hist), so a pass is one kernel: a block ranks its tile's keys per
-// digit, looks back over the tiles before it, a thread per digit, and writes
-// every pair to its place.  Pairs travel as 8 bytes between passes; the last
+// A one-sweep sort (Adinets and Merrill 2022) with digits of 9 bits (27-bit keys
+// take three passes, the 17 bits of the visit order two).  The kernel that makes
+// the keys also counts all their digits, so a pass is one kernel: a block ranks
+// its tile's keys per digit, looks back over the tiles before it, a thread per
+// digit, and writes every pair to its place.  Pairs travel as 8 bytes between passes; the last
 // pass writes the two arrays.  Measured on 1M keys of 25 bits: 3 launches and
 // 85 us against 20 launches and 140 us with separate histogram and scan
 // kernels per 8-bit digit.

@@ -36,7 +36,7 @@
 // through the tile's row segments and the count pass's per-unit counts) or 32 bits (the
 // cell-ordered index).  Entries accepted in one direction only are flagged
 // afterwards from the asymmetric-pair list.  When the bitmap does not fit in
-// device memory, the fill kernel (blocks of kTT threads, kQPT queries each)
+// device memory, the fill kernel (blocks of kTT threads, kQPT queries a thread)
 // re-tests the candidates and writes the table directly.
 #include "vdb_lookback.cuh"
 
@@ -1178,7 +1178,8 @@ __device__ __forceinline__ uint32_t full_runs(uint32_t inside, uint32_t w0, uint
 // with the id that falls on the boundary.  Four runs at a time fit the slots'
 // memory.  cur: the row's place of id0, nc entries are carried before it; the
 // row is written up to its last 32-byte boundary (last: up to its end) and the
-// entries after that are carried.
+// entries after that are carried.  A run is 3 words or more, but cut into pieces
+// of 16: len is at least 32.
 __device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* slots,
                                         uint16_t* carry, bool wrow, uint32_t id0, uint32_t len, bool last,
                                         unsigned long long cur, uint32_t nc, int lane) {
@@ -1186,7 +1187,7 @@ __device__ __noinline__ void full_round(uint16_t* __restrict__ nbr, uint32_t* sl
     static_assert(4u * kRun * sizeof(uint16_t) <= 32u * kXS * sizeof(uint32_t), "four runs fit");
     const unsigned long long wcur = cur - nc, end = cur + len;
     const unsigned long long A = (cur + 7ull) & ~7ull;
-    const unsigned long long wto = last ? end : end & ~15ull;  // (at least A: len >= 64)
+    const unsigned long long wto = last ? end : end & ~15ull;  // (past A: len >= 32)
     const unsigned long long B = wto & ~7ull;
     const uint32_t first = (uint32_t)(A - cur);  // entries of the run before A
     if (wrow) {
@@ -1493,8 +1494,11 @@ __global__ void __launch_bounds__(kXPB * 32, 8) expand16_kernel(TableArgs a) {
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-template <bool MIXED, bool FILL>
-__global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
+// Table pass without a bitmap: a block per tile re-tests its candidates and
+// writes each query's row (off, off_base).  The tests are the count pass's, the
+// FP32 ones on the plain squared distance.
+template <bool MIXED>
+__global__ void __launch_bounds__(kTT) fill_kernel(TableArgs a) {
     pdl_sync();
     __shared__ float2 s_rel[kChunk];
     __shared__ double2 s_xy[kChunk];
@@ -1508,7 +1512,7 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t lt = (1u << lane) - 1u;
     const EpsParams* __restrict__ ep = a.ep;
-    const double eps = ep->eps, thr = ep->thr, tbox = ep->tbox;
+    const double thr = ep->thr, tbox = ep->tbox;
     const ExactBounds xb = ep->xb;
     const float lo = ep->lo32, hi = ep->hi32;
     const int rho = ep->rho;
@@ -1529,13 +1533,10 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
             __syncthreads();
             continue;
         }
-        const uint32_t Q = qe - qs;
         const uint32_t key0 = a.gkey[qs];
         const uint32_t cy = key0 / ncx_pad;
         const uint32_t cx0 = (key0 - cy * ncx_pad) / G * G;
         const uint32_t tile_base = cy * ncx_pad + cx0;
-        // bitmap of this tile (count pass only)
-        const unsigned long long bm0 = (!FILL && a.bitmap) ? a.tile_boff[t] : 0ull;
 
         if (tid < nrows) {
             uint32_t st, len, base;
@@ -1553,7 +1554,6 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
                 acc += s_seg_off[i + 1];
                 s_seg_off[i + 1] = acc;
             }
-            if (!FILL) atomicAdd(&a.st->candidates, (unsigned long long)acc * Q);
         }
         __syncthreads();
         const uint32_t C = s_seg_off[nrows];
@@ -1568,13 +1568,12 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
         const bool two = qs + (uint32_t)(tid & ~31) * kQPT + 32u < qe;
         float qx[kQPT], qy[kQPT];
         double2 qd[kQPT];
-        uint32_t qk[kQPT], cnt[kQPT];
+        uint32_t qk[kQPT];
         unsigned long long cur[kQPT], rend[kQPT];
 #pragma unroll
         for (int q = 0; q < kQPT; q++) {
             const uint32_t k = q0 + 32u * q;
             qk[q] = k;
-            cnt[q] = 0;
             cur[q] = rend[q] = 0;
             if (k < qe) {
                 const float2 loc = a.glocal[k];
@@ -1582,10 +1581,8 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
                 qx[q] = __fmaf_rn((float)dcx, wf, loc.x);
                 qy[q] = loc.y;
                 qd[q] = a.gxy[k];
-                if (FILL) {
-                    cur[q] = a.off[k] - a.off_base;
-                    rend[q] = a.off[k + 1] - a.off_base;
-                }
+                cur[q] = a.off[k] - a.off_base;
+                rend[q] = a.off[k + 1] - a.off_base;
             } else {
                 qx[q] = qy[q] = __int_as_float(0x7fc00000);
                 qd[q] = make_double2(__longlong_as_double(0x7ff8000000000000ll),
@@ -1674,66 +1671,39 @@ __global__ void __launch_bounds__(kTT) table_kernel(TableArgs a) {
                                 m[q] |= 1u << jj;
                                 if (!(r & 2u)) asy[q] |= 1u << jj;
                             }
-                            if (!FILL && (r == 1u || r == 2u) && qk[q] < kq) {
-                                const uint32_t slot = atomicAdd(a.asym_n, 1u);
-                                if (slot < a.asym_cap) {
-                                    AsymPair ap;
-                                    ap.a = qk[q];
-                                    ap.b = kq;
-                                    ap.dir = r;
-                                    ap.pad = 0u;
-                                    a.asym[slot] = ap;
-                                } else {
-                                    atomicOr(&a.st->flags, kStatAsymOverflow);
-                                }
-                            }
                         }
                     }
                 }
-                if (FILL) {
 #pragma unroll
-                    for (int q = 0; q < kQPT; q++) {
-                        uint32_t act = __ballot_sync(kFull, m[q] != 0u);
-                        while (act) {
-                            const int src = __ffs(act) - 1;
-                            act &= act - 1u;
-                            const uint32_t mm = __shfl_sync(kFull, m[q], src);
-                            const uint32_t am = __shfl_sync(kFull, asy[q], src);
-                            const unsigned long long c0 = __shfl_sync(kFull, cur[q], src);
-                            const unsigned long long ce = __shfl_sync(kFull, rend[q], src);
-                            if ((mm >> lane) & 1u) {
-                                const unsigned long long dst = c0 + __popc(mm & lt);
-                                if (dst < ce) {
-                                    const bool one_way = (am >> lane) & 1u;
-                                    if (a.compact)  // position in its work unit's candidates
-                                        reinterpret_cast<uint16_t*>(a.nbr)[dst] =
-                                            (uint16_t)(((cb + j0 + (uint32_t)lane) &
-                                                        (a.unit_words * 32u - 1u)) |
-                                                       (one_way ? kAsymFlag16 : 0u));
-                                    else
-                                        a.nbr[dst] = s_id[j0 + lane] | (one_way ? kAsymFlag : 0u);
-                                } else {
-                                    atomicOr(&a.st->flags, kStatRowOverflow);
-                                }
+                for (int q = 0; q < kQPT; q++) {
+                    uint32_t act = __ballot_sync(kFull, m[q] != 0u);
+                    while (act) {
+                        const int src = __ffs(act) - 1;
+                        act &= act - 1u;
+                        const uint32_t mm = __shfl_sync(kFull, m[q], src);
+                        const uint32_t am = __shfl_sync(kFull, asy[q], src);
+                        const unsigned long long c0 = __shfl_sync(kFull, cur[q], src);
+                        const unsigned long long ce = __shfl_sync(kFull, rend[q], src);
+                        if ((mm >> lane) & 1u) {
+                            const unsigned long long dst = c0 + __popc(mm & lt);
+                            if (dst < ce) {
+                                const bool one_way = (am >> lane) & 1u;
+                                if (a.compact)  // position in its work unit's candidates
+                                    reinterpret_cast<uint16_t*>(a.nbr)[dst] =
+                                        (uint16_t)(((cb + j0 + (uint32_t)lane) &
+                                                    (a.unit_words * 32u - 1u)) |
+                                                   (one_way ? kAsymFlag16 : 0u));
+                                else
+                                    a.nbr[dst] = s_id[j0 + lane] | (one_way ? kAsymFlag : 0u);
+                            } else {
+                                atomicOr(&a.st->flags, kStatRowOverflow);
                             }
-                            if (lane == src) cur[q] += __popc(mm);
                         }
-                    }
-                } else {
-                    const unsigned long long wrow = bm0 + (unsigned long long)((cb + j0) >> 5) * Q;
-#pragma unroll
-                    for (int q = 0; q < kQPT; q++) {
-                        cnt[q] += __popc(m[q]);
-                        if (a.bitmap && qk[q] < qe) a.bitmap[wrow + (qk[q] - qs)] = m[q];
+                        if (lane == src) cur[q] += __popc(mm);
                     }
                 }
             }
             __syncthreads();
-        }
-        if (!FILL) {
-#pragma unroll
-            for (int q = 0; q < kQPT; q++)
-                if (qk[q] < qe) a.deg[qk[q]] = cnt[q];
         }
         __syncthreads();
     }
@@ -2098,9 +2068,9 @@ void launch_count(const TableArgs& a, int nblocks, cudaStream_t s) {
 
 void launch_fill(const TableArgs& a, int nblocks, cudaStream_t s) {
     if (a.mixed)
-        launch(table_kernel<true, true>, nblocks, kTT, s, a);
+        launch(fill_kernel<true>, nblocks, kTT, s, a);
     else
-        launch(table_kernel<false, true>, nblocks, kTT, s, a);
+        launch(fill_kernel<false>, nblocks, kTT, s, a);
 }
 
 size_t words_state_bytes(uint32_t n) {
@@ -2156,9 +2126,9 @@ int table_blocks_per_sm(bool fill, bool mixed) {
     int nb = 0;
     if (fill) {
         if (mixed)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, table_kernel<true, true>, kTT, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fill_kernel<true>, kTT, 0);
         else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, table_kernel<false, true>, kTT, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fill_kernel<false>, kTT, 0);
     } else {
         if (mixed)
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, count_kernel<true>, kWPB * 32, 0);
