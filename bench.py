@@ -67,7 +67,7 @@ def parse():
                    help="also time the step with fixed shapes (one-cell tiles, "
                         "min(4, datasets) streams); on by default for --workload multi")
     p.add_argument("--unit-candidates", type=int, default=0, choices=[0, 1024, 2048, 4096],
-                   help="candidates per work unit (0: by dataset size)")
+                   help="candidates per work unit (0: by the library's rule)")
     p.add_argument("--graph", action="store_true",
                    help="time the main steps as graph replays (vdb_options.graph)")
     p.add_argument("--graph-compare", action="store_true",
